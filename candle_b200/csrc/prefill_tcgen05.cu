@@ -139,72 +139,6 @@ __global__ void __launch_bounds__(256) quantize_q8k_tiles_kernel(const T *__rest
                              TileBlob::tile_rows(tokens, tt), tl, lane);
 }
 
-// ---- grouped (expert-indexed) mode ------------------------------------------------------------------------
-// Jobs m = 0..M-1 are (token, expert) pairs sorted by expert (candle-nn/src/moe.rs:286-337): pair = sorted_token_ids[m],
-// expert = expert_ids[m]; input row = pair when routing weights are given, else pair / topk; output row = pair, scaled
-// by topk_weights[pair] when given.  The jobs of one expert are cut into tiles of 128; a table of (expert, first job,
-// valid rows) per tile is built on the device (the host never sees the routing), over-sized to ceil(M / 128) + experts
-// tiles; tiles past the last one have zero valid rows and their CTAs leave at once.
-struct GroupInfo {
-    const int *tiles;                  // [max_tiles][4]: expert, first job, valid rows, 0; null: dense mode
-    const int32_t *sorted_token_ids;
-    const float *topk_weights;
-    long long expert_stride;           // bytes between experts
-    int topk;
-};
-
-// One CTA.  expert_ids ascending (ids outside [0, num_experts) - another rank's experts - may sit at either end).
-__global__ void __launch_bounds__(1024) moe_tiles_kernel(const int32_t *__restrict__ expert_ids, int m, int num_experts,
-                                                         int max_tiles, int *__restrict__ tiles) {
-    __shared__ int start[1025], first_tile[1025];
-    const int tid = threadIdx.x;
-    for (int e = tid; e <= num_experts; e += 1024) {       // start[e] = first job whose expert is >= e
-        int lo = 0, hi = m;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (expert_ids[mid] < e) lo = mid + 1; else hi = mid;
-        }
-        start[e] = lo;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int t = 0;
-        for (int e = 0; e < num_experts; ++e) { first_tile[e] = t; t += (start[e + 1] - start[e] + kTokTile - 1) / kTokTile; }
-        first_tile[num_experts] = t;
-    }
-    __syncthreads();
-    for (int e = tid; e < num_experts; e += 1024) {
-        const int cnt = start[e + 1] - start[e];
-        for (int j = 0; j * kTokTile < cnt; ++j) {
-            int *t = tiles + 4 * (first_tile[e] + j);
-            t[0] = e; t[1] = start[e] + j * kTokTile; t[2] = min(kTokTile, cnt - j * kTokTile); t[3] = 0;
-        }
-    }
-    for (int t = first_tile[num_experts] + tid; t < max_tiles; t += 1024) { tiles[4 * t] = 0; tiles[4 * t + 1] = 0; tiles[4 * t + 2] = 0; tiles[4 * t + 3] = 0; }
-}
-
-// One warp per (tile row, super-block): the input row of that job, or zeros for the padding rows of a tile.
-template <typename T>
-__global__ void __launch_bounds__(256) quantize_q8k_tiles_grouped_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k,
-                                                                         int max_tiles, GroupInfo gi) {
-    const int lane = threadIdx.x & 31;
-    const int nsb = k / 256;
-    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (item >= (int64_t)max_tiles * kTokTile * nsb) return;
-    const int sb = (int)(item % nsb);
-    const int64_t slot = item / nsb;
-    const int tt = (int)(slot / kTokTile), tl = (int)(slot % kTokTile);
-    const int *ti = gi.tiles + 4 * tt;
-    if (ti[2] == 0) return;                                 // unused tile: nobody reads its blob
-    const T *xr = nullptr;
-    if (tl < ti[2]) {
-        const int pair = gi.sorted_token_ids[ti[1] + tl];
-        const int64_t in_row = gi.topk_weights ? pair : pair / gi.topk;
-        xr = x + in_row * k + sb * 256 + lane * 8;
-    }
-    quantize_q8k_row_part<T>(xr, y + TileBlob::offset(max_tiles * kTokTile, nsb, tt, sb), kTokTile, tl, lane);
-}
-
 // ---- weight planes -----------------------------------------------------------------------------------------
 // RawBlock<T>: the GGUF bytes one producer thread needs for (weight row r, super-block sb, half h, part jh) and their
 // expansion into two int8 planes of 16-byte K slabs:  plane j of row r, slab s  ->  stB + s*kSlabB + (64*j + r)*16,
@@ -342,31 +276,13 @@ template <> struct RawBlock<CQ_Q6_K> {
 //   E(i) after M(i) [bar_acc] and after the relay arrive on bar_vis, which carries the visibility of the scale rings.
 // The scale rings are 8 deep: an entry is rewritten for i+8 only after M(i+5), which itself waited for E(i+3).
 // Warps: 0-7 epilogue (TMEM lane quadrant = warp % 4, weight rows 32 * (warp / 4) ..), 8-15 producers, 16 MMA, 17 loader.
-struct TileCtx {
-    const uint8_t *w;       // weight matrix of this tile (grouped mode: of its expert)
-    int row0, tt, valid, job0;
-};
-// false: nothing to do for tile t (grouped mode, unused tile).  Every role evaluates this for the same t, so all skip alike.
-__device__ __forceinline__ bool tile_ctx(int t, int ntt, const uint8_t *w, const GroupInfo &gi, TileCtx &c) {
-    c.row0 = (t / ntt) * kRowTile;
-    c.tt = t % ntt;
-    c.valid = kTokTile;
-    c.job0 = 0;
-    c.w = w;
-    if (gi.tiles) {
-        const int *ti = gi.tiles + 4 * c.tt;
-        c.valid = ti[2];
-        if (c.valid == 0) return false;
-        c.w = w + (long long)ti[0] * gi.expert_stride;
-        c.job0 = ti[1];
-    }
-    return true;
-}
+struct TileCtx { int row0, tt; };
+__device__ __forceinline__ TileCtx tile_ctx(int t, int ntt) { return TileCtx{(t / ntt) * kRowTile, t % ntt}; }
 
 template <int WTYPE>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, void *__restrict__ out_v, int out_kind, int k,
-                   int nrows, int tokens, int stride_out, int dbg, int ntt, int ntiles, const GroupInfo gi) {
+                   int nrows, int tokens, int stride_out, int dbg, int ntt, int ntiles) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bar_fullA = reinterpret_cast<uint64_t *>(smem);         // [3] activations landed (TMA bytes)
     uint64_t *bar_fullB = bar_fullA + 3;                               // [3] weight planes written (all producer threads)
@@ -423,27 +339,21 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
             uint8_t *z = stB0 + st * kStageB + (16 + which) * kSlabB + ((which ? 0 : kRowTile) + row) * 16;
             *reinterpret_cast<uint4 *>(z) = make_uint4(0u, 0u, 0u, 0u);
         }
-        auto row_of = [&](const TileCtx &c) -> const uint8_t * {
-            int grow = c.row0 + r;
+        auto row_of = [&](int t) -> const uint8_t * {
+            int grow = tile_ctx(t, ntt).row0 + r;
             if (grow >= nrows) grow = nrows - 1;        // ragged last tile: duplicate a valid row, never stored
-            return c.w + (size_t)grow * row_bytes;
-        };
-        auto next_tile = [&](int t, TileCtx &c) -> int {      // first tile >= t of this CTA that has work, or ntiles
-            while (t < ntiles && !tile_ctx(t, ntt, w, gi, c)) t += gridDim.x;
-            return t;
+            return w + (size_t)grow * row_bytes;
         };
         // the GGUF bytes of the next super-block (of this or of the next tile) are fetched one iteration ahead of their use
-        TileCtx cx;
-        int t = next_tile(blockIdx.x, cx);
-        const uint8_t *wrow = t < ntiles ? row_of(cx) : nullptr;
+        int t = blockIdx.x;
+        const uint8_t *wrow = t < ntiles ? row_of(t) : nullptr;
         RawBlock<WTYPE> nxt_raw;
         if (t < ntiles) nxt_raw.load(wrow, 0, h, jh);
         int it = 0;
         bool alive = true;
         while (t < ntiles && alive) {
-            TileCtx nx;
-            const int tn = next_tile(t + gridDim.x, nx);
-            const uint8_t *wnext = tn < ntiles ? row_of(nx) : nullptr;
+            const int tn = t + gridDim.x;
+            const uint8_t *wnext = tn < ntiles ? row_of(tn) : nullptr;
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int s = it % kStagesB;
                 uint8_t *stB = stB0 + s * kStageB;
@@ -465,8 +375,7 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
             int it = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-                TileCtx cx;
-                if (!tile_ctx(t, ntt, w, gi, cx)) continue;
+                const TileCtx cx = tile_ctx(t, ntt);
                 const int tile_rows = (int)TileBlob::tile_rows(tokens, cx.tt);
                 for (int sb = 0; sb < nsb; ++sb, ++it) {
                     const int a = it % kStagesA;
@@ -490,8 +399,6 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
         int it = 0;
         bool alive = true;
         for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-            TileCtx cx;
-            if (!tile_ctx(t, ntt, w, gi, cx)) continue;
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int a = it % kStagesA, s = it % kStagesB, c = it & 1;
                 if (!wait_or_abort(&bar_fullA[a], (it / kStagesA) & 1, abort_flag) ||
@@ -525,8 +432,7 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
         int it = 0;
         bool alive = true;
         for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-            TileCtx cx;
-            if (!tile_ctx(t, ntt, w, gi, cx)) continue;
+            const TileCtx cx = tile_ctx(t, ntt);
             const int tok = cx.tt * kTokTile + tok_local;
             float acc[kMyRows];
 #pragma unroll
@@ -584,20 +490,8 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
                 mbar_arrive(&bar_free[c]);
             }
             if (!alive) break;
-            bool store = tok < tokens;
-            int64_t orow = tok;
-            if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight
-                store = tok_local < cx.valid;
-                if (store) {
-                    const int pair = gi.sorted_token_ids[cx.job0 + tok_local];
-                    orow = pair;
-                    if (gi.topk_weights) {
-                        const float sc = gi.topk_weights[pair];
-#pragma unroll
-                        for (int i = 0; i < kMyRows; ++i) acc[i] = __fmul_rn(acc[i], sc);
-                    }
-                }
-            }
+            const bool store = tok < tokens;
+            const int64_t orow = tok;
             const int c0 = cx.row0 + rh * kMyRows;
             // The branches below are chosen by warp-uniform values only (`store` differs between the lanes of a ragged token
             // tile and must not decide whether a lane reaches the shuffles of the f32 branch).
@@ -613,7 +507,7 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
                         if (c0 + i < nrows) cq_store_out(out_v, out_kind, orow * stride_out + c0 + i, acc[i]);
                 }
               }
-            } else if (!gi.tiles && c0 + kMyRows <= nrows && (stride_out & 3) == 0 && (c0 & 3) == 0 && (((uintptr_t)out_v) & 15) == 0) {
+            } else if (c0 + kMyRows <= nrows && (stride_out & 3) == 0 && (c0 & 3) == 0 && (((uintptr_t)out_v) & 15) == 0) {
                 // f32, whole 32-row slice (warp-uniform test): three exchange steps turn "a lane holds 32 rows of its token" into
                 // "a lane holds 4 rows of 8 tokens", so that eight lanes write one token's 128 contiguous bytes per store
                 // instruction (four full lines per instruction instead of 32 quarter lines).
@@ -732,77 +626,11 @@ extern "C" void cq_prefill_gemm(int wtype, const void *vx, const void *scratch, 
     const unsigned grid = prefill_grid(ntiles);
     if (ti == 0)
         prefill_kernel<CQ_Q4_K><<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
-            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles, GroupInfo{});
+            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles);
     else
         prefill_kernel<CQ_Q6_K><<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
-            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles, GroupInfo{});
+            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles);
     cq_check_launch("prefill gemm");
-}
-
-// ---- grouped entry points (quantized mixture-of-experts, many tokens) ----
-namespace {
-int moe_max_tiles(int size_m, int num_experts) { return (size_m + kTokTile - 1) / kTokTile + num_experts; }
-size_t moe_table_bytes(int max_tiles) { return ((size_t)max_tiles * 16 + 255) / 256 * 256; }
-}  // namespace
-
-extern "C" size_t cq_moe_prefill_scratch_bytes(int size_m, int num_experts, int k) {
-    if (size_m <= 0 || num_experts <= 0 || num_experts > 1024 || k <= 0 || k % 256 != 0) return 0;
-    const int mt = moe_max_tiles(size_m, num_experts);
-    return moe_table_bytes(mt) + (size_t)mt * kTokTile * kTokBytes * (k / 256) + 256;
-}
-
-// out[pair, :] = W[expert of the pair] . x[input row of the pair] (times topk_weights[pair]) for all size_m sorted pairs, on
-// the tensor cores.  Same job rules as moe_gemm_gguf; arithmetic of the dense prefill kernel (Q8_K activations).
-// `scratch`: cq_moe_prefill_scratch_bytes(size_m, num_experts, size_k) bytes.  Rows of pairs whose expert id is outside
-// [0, num_experts) are not written.
-extern "C" void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *weights, const int32_t *sorted_token_ids,
-                                    const int32_t *expert_ids, const float *topk_weights, float *out, void *scratch, int num_experts,
-                                    int topk, int size_m, int size_n, int size_k, void *stream) {
-    if (!input || !weights || !sorted_token_ids || !expert_ids || !out || !scratch || num_experts <= 0 || num_experts > 1024 ||
-        topk <= 0 || size_m <= 0 || size_n <= 0 || size_k <= 0 || size_k % 256 != 0) {
-        cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: null pointer, empty shape, more than 1024 experts or K not a multiple of 256");
-        return;
-    }
-    if (wtype != CQ_Q4_K && wtype != CQ_Q6_K) {
-        cq_set_status(CQ_ERR_UNSUPPORTED, "moe prefill: the tensor-core kernel covers Q4_K and Q6_K");
-        return;
-    }
-    const long long expert_stride = (long long)size_n * (size_k / 256) * cq_type_size(wtype);
-    if ((uintptr_t)weights % 16 != 0 || (uintptr_t)scratch % 256 != 0 || (wtype == CQ_Q4_K ? expert_stride % 16 : expert_stride % 4) != 0) {
-        cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: misaligned weights or scratch");
-        return;
-    }
-    cudaStream_t st = (cudaStream_t)stream;
-    const int mt = moe_max_tiles(size_m, num_experts);
-    int *tiles = (int *)scratch;
-    uint8_t *blobs = (uint8_t *)scratch + moe_table_bytes(mt);
-    moe_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
-    const GroupInfo gi{tiles, sorted_token_ids, topk_weights, expert_stride, topk};
-    const int64_t items = (int64_t)mt * kTokTile * (size_k / 256);
-    const unsigned qgrid = (unsigned)((items + 7) / 8);
-    if (in_elem == CQ_F32) quantize_q8k_tiles_grouped_kernel<float><<<qgrid, 256, 0, st>>>((const float *)input, blobs, size_k, mt, gi);
-    else if (in_elem == CQ_F16) quantize_q8k_tiles_grouped_kernel<__half><<<qgrid, 256, 0, st>>>((const __half *)input, blobs, size_k, mt, gi);
-    else if (in_elem == CQ_BF16)
-        quantize_q8k_tiles_grouped_kernel<__nv_bfloat16><<<qgrid, 256, 0, st>>>((const __nv_bfloat16 *)input, blobs, size_k, mt, gi);
-    else { cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: unknown input element type"); return; }
-    static bool attr_done[2][64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int ti = wtype == CQ_Q4_K ? 0 : 1;
-    if (dev >= 0 && dev < 64 && !attr_done[ti][dev]) {
-        if (ti == 0) cudaFuncSetAttribute(prefill_kernel<CQ_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        else cudaFuncSetAttribute(prefill_kernel<CQ_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        attr_done[ti][dev] = true;
-    }
-    const int ntiles = ((size_n + kRowTile - 1) / kRowTile) * mt;
-    const unsigned grid = prefill_grid(ntiles);
-    if (ti == 0)
-        prefill_kernel<CQ_Q4_K><<<grid, kThreads, kSmemBytes, st>>>((const uint8_t *)weights, blobs, out, CQ_F32, size_k, size_n,
-                                                                     mt * kTokTile, size_n, g_prefill_dbg, mt, ntiles, gi);
-    else
-        prefill_kernel<CQ_Q6_K><<<grid, kThreads, kSmemBytes, st>>>((const uint8_t *)weights, blobs, out, CQ_F32, size_k, size_n,
-                                                                     mt * kTokTile, size_n, g_prefill_dbg, mt, ntiles, gi);
-    cq_check_launch("moe prefill gemm");
 }
 
 #ifdef CQ_EXPERIMENT

@@ -1,0 +1,218 @@
+// Shared parts of the f16 prompt kernels (prompt_kq.cu: Q4_K / Q6_K with one activation scale per 256 elements;
+// prompt_b32.cu: formats with an activation scale per 32 elements).
+//
+// Both run the quantized product on `tcgen05.mma kind::f16` with INTEGERS in f16: int8 activations, and weight codes times
+// their integer sub-scales, are whole numbers of at most 11 significant bits, so every product is exact and the f32
+// accumulator holds the exact integer sum as long as it stays below 2^24.  Against int8 operands that saves the second
+// weight plane and the int -> float conversions of the epilogue.
+//
+// Operand A (M = 128 weight rows) lives in TENSOR MEMORY: a producer thread owns one row = one TMEM lane, expands its GGUF
+// bytes in registers and stores them with `tcgen05.st`.  Through shared memory the same operand would cost a write and, per
+// MMA, a read of 4 KiB: at N = 128 the two operands' reads alone would fill the 128 B/clk shared-memory pipe.  Operand B
+// (N = up to 128 tokens, any multiple of 16, so a ragged tile pays only for the tokens it has) comes pre-tiled from the
+// quantize kernel with bulk copies.  The accumulator lane is then the weight row, so 32 lanes store 32 consecutive outputs.
+// Measured rate of this form (one CTA per SM): 16.4 / 32.3 / 64.4 clocks per MMA at N = 32 / 64 / 128, the nominal rate; with
+// A in shared memory 40 / 48 / 64, so small token tiles need the tensor-memory form.
+#pragma once
+#include "common.cuh"
+#include "tcgen05.cuh"
+#include "tensor_map.cuh"
+
+namespace cq_prompt {
+using namespace cq_tc;
+
+constexpr int kRows = 128;         // weight rows per CTA tile (MMA M = TMEM lanes)
+constexpr int kTokMax = 128;       // tokens per CTA tile (MMA N), at most
+
+// The issuing thread is the only one of its warp that runs, every instruction waits for the one before it, and one MMA of N =
+// 128 lasts 64 clocks: some 15 dependent instructions.  So a shared-memory descriptor is kept as its low word - address / 16
+// and, in the upper half, the distance / 16 between the two 16-byte halves of a K step, which for a tile of n tokens is n - and
+// the next K step is one addition of 2 n.
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"((128u >> 4) | (1u << 14)));      // 8-row groups 128 bytes apart; sm_100 descriptor
+    return r;
+}
+__device__ __forceinline__ uint32_t desc_lo(const void *smem, uint32_t n) { return (cq_smem_u32(smem) >> 4) | (n << 16); }
+// D[128 rows][n tokens] (+)= A[tmem: 128 x 16 f16] * B[smem: n x 16 f16]
+template <bool ACC> __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_b, uint32_t idesc) {
+    if constexpr (ACC)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(desc_of(desc_b)), "r"(idesc) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(tmem_a), "l"(desc_of(desc_b)), "r"(idesc) : "memory");
+}
+// the same with A in shared memory, into a fresh accumulator
+__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(desc_of(desc_a)), "l"(desc_of(desc_b)), "r"(idesc) : "memory");
+}
+// kind::f16 instruction descriptor: D = f32, A = B = f16, both K-major, M = 128, N = n.
+__device__ __forceinline__ uint32_t idesc_f16(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24); }
+
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+          "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+          "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// A warp that goes on to a warp-wide tcgen05 instruction must decide as one whether its wait gave up.
+__device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag));
+}
+// One arrival per warp: barriers count warps, not threads.
+__device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// two f32 operations per instruction; each half rounds like the scalar operation
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t pack2f(float lo, float hi) { return pack2(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t b) { return *reinterpret_cast<__half2 *>(&b); }
+__device__ __forceinline__ uint32_t hfma2_bits(uint32_t a, __half2 b, __half2 c) { return h2_bits(__hfma2(bits_h2(a), b, c)); }
+
+// K runs in groups of four with the middle two swapped (elements 0, 2, 1, 3): masking a word of four codes gives the
+// pairs (byte 0, byte 2) and (byte 1, byte 3), which is what lies in one 32-bit TMEM cell.  Both operands use this order.
+
+// Eight consecutive activations of one lane; `vec`: the row is 16-byte aligned.
+__device__ __forceinline__ void load8(const float *p, bool vec, float (&e)[8]) {
+    if (vec) {
+        const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+        e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w; e[4] = b.x; e[5] = b.y; e[6] = b.z; e[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = p[i];
+    }
+}
+template <typename T> __device__ __forceinline__ void load8(const T *p, bool vec, float (&e)[8]) {      // 16-bit types
+    if (vec) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(p);
+        const T *h = reinterpret_cast<const T *>(&a);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = cq_elem_to_float(h, i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = cq_elem_to_float(p, i);
+    }
+}
+// eight small integers as f16 in the operands' K order
+__device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
+    auto pr = [](int a, int b) { return h2_bits(__halves2half2(__short2half_rn((short)a), __short2half_rn((short)b))); };
+    return make_uint4(pr(q[0], q[2]), pr(q[1], q[3]), pr(q[4], q[6]), pr(q[5], q[7]));
+}
+
+// ---- tiles --------------------------------------------------------------------------------------------------
+// The jobs of a grouped (expert-indexed) launch; null `tiles` = dense.
+struct GroupInfo {
+    const int *tiles;                  // [max_tiles][4]: expert, first job, valid rows, first blob row; then the number of tiles in use
+    const int32_t *sorted_token_ids;
+    const float *topk_weights;
+    long long expert_rows;             // weight rows per expert
+    int topk, row_per_pair;            // input row of a pair: the pair itself, or pair / topk
+};
+
+// Tokens are cut into `ntt` tiles of `tt` (a multiple of 16, at most 128).  The activation blobs of (tile, 256-element chunk)
+// follow each other, their rows padded to a multiple of 16.
+struct Tiling {
+    int tokens, tt, ntt;
+    __host__ __device__ int rows(int t) const {
+        const int left = tokens - t * tt;
+        return ((left < tt ? left : tt) + 15) / 16 * 16;
+    }
+};
+
+struct TileCtx {
+    int row0;           // first weight row inside the matrix (of the expert)
+    long long wrow0;    // the same counted from the start of the weights
+    long long blob_row; // rows of activation blobs before this tile
+    int t, valid, n, job0;
+};
+// Tile number -> row tile and token tile; `ntt` token tiles are in use.
+__device__ __forceinline__ void tile_ctx(int tile, int ntt, const Tiling &tl, const GroupInfo &gi, TileCtx &c) {
+    c.t = tile % ntt;
+    c.row0 = (tile / ntt) * kRows;
+    c.wrow0 = c.row0;
+    c.job0 = 0;
+    if (gi.tiles) {
+        const int4 ti = *reinterpret_cast<const int4 *>(gi.tiles + 4 * c.t);
+        c.valid = ti.z;
+        c.wrow0 += ti.x * gi.expert_rows;
+        c.job0 = ti.y;
+        c.blob_row = ti.w;
+    } else {
+        c.blob_row = (long long)c.t * tl.tt;
+        const int left = tl.tokens - c.t * tl.tt;
+        c.valid = left < tl.tt ? left : tl.tt;
+    }
+    c.n = (c.valid + 15) / 16 * 16;
+}
+
+// Number of token tiles for `nrt` row tiles.  Results do not depend on it.  A tile's cost per chunk is the larger of its
+// MMA time (proportional to its tokens) and what expanding 128 weight rows takes (`floor_tok`: as many tokens' worth of MMA);
+// the launch takes as many rounds of `sms` tiles as it needs.
+inline Tiling plan_tiling(int tokens, int nrt, int sms, int floor_tok, int tok_max = kTokMax) {
+    Tiling best{tokens, 16, 0};
+    long long best_cost = -1;
+    for (int ntt = (tokens + tok_max - 1) / tok_max; ntt <= (tokens + 15) / 16; ++ntt) {
+        const int tt = ((tokens + ntt - 1) / ntt + 15) / 16 * 16;
+        if ((tokens + tt - 1) / tt != ntt) continue;
+        const long long rounds = ((long long)nrt * ntt + sms - 1) / sms;
+        const long long cost = rounds * ((tt > floor_tok ? tt : floor_tok) + 8);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best.tt = tt; best.ntt = ntt; }
+        if (rounds > 64) break;          // many rounds: smaller tiles only repeat the expansion
+    }
+    return best;
+}
+
+inline int sm_count() {
+    static int sms[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return 148;
+    if (!sms[dev]) {
+        int n = 0;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        sms[dev] = n > 0 ? n : 148;
+    }
+    return sms[dev];
+}
+
+// ---- raw weight bytes: (128 rows, one 256-element chunk) -> shared memory ---------------------------------------
+// One tiled TMA copy when rows are whole multiples of 16 bytes apart; else one bulk copy per row from the 16-byte boundary
+// below the chunk (Q6_K rows of K % 2048 != 0 and the like).  In shared memory row r starts at r * kPitch, the chunk a few bytes
+// behind it when it does not start on such a boundary.  CB: bytes of a chunk.
+template <int CB> struct Raw {
+    static constexpr bool kAligned = CB % 16 == 0;
+    static constexpr int kNeed = kAligned ? CB : (CB + 14 + 15) / 16 * 16;       // 16-byte window that covers the chunk
+    // pitch: an odd number of 16-byte units, so that eight lanes' 16-byte reads of one column fall into different banks
+    static constexpr int kPitch = (kNeed / 16) % 2 ? kNeed : kNeed + 16;
+    static constexpr int kBytes = kRows * kPitch;
+};
+
+}  // namespace cq_prompt

@@ -1,0 +1,703 @@
+// Prompt-phase quantized GEMM, out[t, r] = sum_k x[t, k] * W[r, k] for many tokens, Q4_K and Q6_K weights, dense and grouped
+// by expert, on tcgen05.mma kind::f16 (see prompt_f16.cuh for the operand scheme).
+//
+// Replaces candle's MMQ path for these formats (host: candle-core/src/quantized/fast_mmq.rs:253-400; kernels:
+// candle-kernels/src/mmq_gguf/mmq_gguf.cuh:3442-3777, mmq_quantize.cu:11-107) and its expert GEMM
+// (candle-kernels/src/moe/moe_wmma_gguf.cu:124-300).
+//
+// Arithmetic: candle's CPU path.  Activations are BlockQ8K (one f32 scale per 256 values, k_quants.rs:2320-2358, bit-identical
+// int8); a super-block contributes  d_a * (d_w * P - dmin_w * L)  (k_quants.rs:1460-1540, 2035-2092) with the integers
+//      Q4_K:  P = sum (sc_g q) . q8,   |sc_g q| <= 945: one f16 plane;   L = sum_j m_j bsum_j,  |bsum_j| <= 2032, one K = 16 step
+//      Q6_K:  P = sum (sc_j (q - 32)) . q8:  q - 32 = e + b with e even, b the lowest bit of q:  |sc_j e| <= 4096 and even,
+//             |sc_j b| <= 128, both exact in f16; the two planes add into the same accumulator
+// P is exact below 2^24; above (only reachable when most of the 256 products are near their largest value with one sign) each
+// accumulation step rounds to 24 bits, as the int -> float conversion of an integer accumulator would.  L is always exact.
+//
+// Mapping.  One CTA per SM walks tiles of 128 weight rows x up to 128 tokens.  Warps 0-7 epilogue, 8-11 producers (one
+// weight row per thread), 12 MMA issuer, 13 loader.  Tensor memory, all 512 columns: P in two buffers of 128 (the epilogue
+// of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a super-block, by which time
+// the epilogue has read the previous one), operand A in a ring of four 32-column chunks (64 k-elements of one plane).
+//
+// Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
+// for, TMEM is released and a device flag is set for the host.
+#include "../../include/candle_q_b200.h"
+#include "prompt_f16.cuh"
+
+#include <type_traits>
+
+namespace {
+using namespace cq_prompt;
+
+constexpr int kEpiWarps = 8, kProdWarps = 4;
+constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
+constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
+constexpr int kSlabs = 34;                       // 32 slabs of 8 f16 activations, 2 of f16 run sums (16 bytes per token each)
+constexpr int kTokBytes = kSlabs * 16 + 4;       // + the f32 scale
+constexpr int kStageT = 16 * kTokMax * 16;       // token stage: half a super-block, 32 KiB
+constexpr int kStagesT = 4, kAuxRing = 4;
+constexpr int kAux = 2 * kTokMax * 16 + kTokMax * 4;      // run sums, then scales of one super-block
+constexpr int kStagesW = 4;                      // operand A ring in tensor memory, 32 columns each
+constexpr int kColL = 256, kColA = 384;
+
+__device__ int g_prompt_kq_timeout_flag = 0;
+
+template <int WTYPE> struct Fmt;
+template <> struct Fmt<CQ_Q4_K> { static constexpr int kChunks = 4, kRawStages = 3; static constexpr bool kMins = true; };
+template <> struct Fmt<CQ_Q6_K> { static constexpr int kChunks = 8, kRawStages = 2; static constexpr bool kMins = false; };
+
+template <int WTYPE> constexpr int smem_bytes() {
+    return 1024 + kStagesT * kStageT + kAuxRing * kAux + 4 * kRows * 8 + 2 * kRows * 32 + Fmt<WTYPE>::kRawStages * Raw<cq_type_size(WTYPE)>::kBytes + 16;
+}
+
+// ---- activations -> f16 operand tiles -------------------------------------------------------------------------
+template <typename T> struct LoadRows {            // rows of k elements
+    const T *x;
+    int64_t k;
+    __device__ __forceinline__ void operator()(int64_t row, int col, float (&e)[8]) const { load8(x + row * k + col, ((uintptr_t)x & 15) == 0, e); }
+};
+
+// One warp per (token, super-block): BlockQ8K values (the rules of quantize_act.cu).  A block of 8 warps takes 8 consecutive
+// tokens of one super-block and goes through shared memory, so that every slab receives 128 contiguous bytes (stored straight
+// from the warps it would be 16-byte pieces, half a sector each).
+template <typename L>
+__global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__restrict__ y, int nsb, Tiling tl, GroupInfo gi) {
+    constexpr int kPitch = 8 * 16 + 16;
+    __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
+    __shared__ float sd[8];
+    cq_pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sb = blockIdx.x % nsb, g = blockIdx.x / nsb, per_tile = tl.tt / 8;
+    const int t = g / per_tile, row0 = (g % per_tile) * 8, row = row0 + warp;
+    int64_t src = -1, blob_row = (int64_t)t * tl.tt;      // input row; none: a padding row of zeros
+    int rows;
+    if (gi.tiles) {
+        if (t >= gi.tiles[4 * tl.ntt]) return;
+        const int4 ti = *reinterpret_cast<const int4 *>(gi.tiles + 4 * t);
+        rows = (ti.z + 15) / 16 * 16;
+        blob_row = ti.w;
+        if (row < ti.z) {
+            const int pair = gi.sorted_token_ids[ti.y + row];
+            src = gi.row_per_pair ? pair : pair / gi.topk;
+        }
+    } else {
+        rows = tl.rows(t);
+        const int64_t tok = (int64_t)t * tl.tt + row;
+        if (row < rows && tok < tl.tokens) src = tok;
+    }
+    if (row0 >= rows) return;           // block-uniform
+    float e[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) e[c] = 0.0f;
+    if (src >= 0) load(src, sb * 256 + lane * 8, e);
+    float amax = 0.0f, vmax = 0.0f;
+    int imax = 0x7fffffff;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        if (amax < fabsf(e[c])) { amax = fabsf(e[c]); vmax = e[c]; imax = lane * 8 + c; }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        const float oa = __shfl_xor_sync(0xffffffffu, amax, m);
+        const float ov = __shfl_xor_sync(0xffffffffu, vmax, m);
+        const int oi = __shfl_xor_sync(0xffffffffu, imax, m);
+        if (oa > amax || (oa == amax && oi < imax)) { amax = oa; vmax = ov; imax = oi; }
+    }
+    int q[8];
+    float d = 0.0f;
+    if (amax == 0.0f) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) q[c] = 0;
+    } else {
+        const float iscale = __fdiv_rn(-127.0f, vmax);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            float r = roundf(__fmul_rn(iscale, e[c]));
+            r = fminf(fmaxf(r, -128.0f), 127.0f);
+            q[c] = (int)r;
+        }
+        d = __fdiv_rn(1.0f, iscale);
+    }
+    *reinterpret_cast<uint4 *>(sm + lane * kPitch + warp * 16) = pack_q8(q);
+    int bs = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+    bs += __shfl_xor_sync(0xffffffffu, bs, 1);
+    if ((lane & 1) == 0) {              // sum of run j = lane / 2: slab 32 + j / 8, f16 j % 8
+        const int j = lane >> 1;
+        *reinterpret_cast<__half *>(sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7)) = __short2half_rn((short)bs);
+    }
+    if (lane == 0) sd[warp] = d;
+    __syncthreads();
+    uint8_t *blob = y + ((size_t)blob_row * nsb + (size_t)sb * rows) * kTokBytes;
+    for (int i = threadIdx.x; i < kSlabs * 8; i += 256)
+        *reinterpret_cast<uint4 *>(blob + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 16) = *reinterpret_cast<const uint4 *>(sm + (i >> 3) * kPitch + (i & 7) * 16);
+    if (threadIdx.x < 8) *reinterpret_cast<float *>(blob + (size_t)rows * (kSlabs * 16) + (row0 + threadIdx.x) * 4) = sd[threadIdx.x];
+}
+
+// One CTA: the tile table of a grouped launch.  expert_ids ascending (ids outside [0, num_experts) may sit at either end);
+// the jobs of one expert are cut into tiles of kTokMax.
+__global__ void __launch_bounds__(1024) group_tiles_kernel(const int32_t *__restrict__ expert_ids, int m, int num_experts, int max_tiles,
+                                                           int *__restrict__ tiles) {
+    __shared__ int start[1025], first_tile[1025], first_row[1024];
+    const int tid = threadIdx.x;
+    for (int e = tid; e <= num_experts; e += 1024) {       // start[e] = first job whose expert is >= e
+        int lo = 0, hi = m;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (expert_ids[mid] < e) lo = mid + 1; else hi = mid;
+        }
+        start[e] = lo;
+    }
+    __syncthreads();
+    if (tid < 32) {         // tiles and blob rows (a multiple of 16 per expert) before each expert: a warp scan, 32 experts at a time
+        int tiles_before = 0, rows_before = 0;
+        for (int e0 = 0; e0 < num_experts; e0 += 32) {
+            const int e = e0 + tid;
+            const int cnt = e < num_experts ? start[e + 1] - start[e] : 0;
+            const int my_tiles = (cnt + kTokMax - 1) / kTokMax, my_rows = (cnt + 15) / 16 * 16;
+            int v = my_tiles, r = my_rows;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int uv = __shfl_up_sync(0xffffffffu, v, o), ur = __shfl_up_sync(0xffffffffu, r, o);
+                if (tid >= o) { v += uv; r += ur; }
+            }
+            if (e < num_experts) { first_tile[e] = tiles_before + v - my_tiles; first_row[e] = rows_before + r - my_rows; }
+            tiles_before += __shfl_sync(0xffffffffu, v, 31);
+            rows_before += __shfl_sync(0xffffffffu, r, 31);
+        }
+        if (tid == 0) first_tile[num_experts] = tiles_before;
+    }
+    __syncthreads();
+    for (int e = tid; e < num_experts; e += 1024) {
+        const int cnt = start[e + 1] - start[e];
+        for (int j = 0; j * kTokMax < cnt; ++j)
+            *reinterpret_cast<int4 *>(tiles + 4 * (first_tile[e] + j)) =
+                make_int4(e, start[e] + j * kTokMax, min(kTokMax, cnt - j * kTokMax), first_row[e] + j * kTokMax);
+    }
+    if (tid == 0) tiles[4 * max_tiles] = first_tile[num_experts];
+}
+
+// ---- producers: the GGUF bytes of one row -> chunks of 32 TMEM cells ------------------------------------------------
+template <int WTYPE> struct Expand;
+
+// Q4_K chunk ch: elements 64 ch ..: low nibbles of bytes 32 ch .. +31 (sub-block 2 ch), then the high ones (2 ch + 1).
+// A nibble in the low mantissa bits of 1024.0 (or 16 times it, for high nibbles left in place) becomes sc * q in one fma.
+template <> struct Expand<CQ_Q4_K> {
+    const uint8_t *p;
+    uint32_t sc[2], mn[2], dm;
+    __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
+        p = rr + shift;
+        const uint4 h = *reinterpret_cast<const uint4 *>(p);
+        dm = h.x;           // get_scale_min_k4, candle-core/src/quantized/utils.rs:50-60, four sub-blocks per word
+        sc[0] = h.y & 0x3F3F3F3Fu; mn[0] = h.z & 0x3F3F3F3Fu;
+        sc[1] = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
+        mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
+    }
+    static __device__ __forceinline__ __half2 byte_h2(uint32_t w, int i) {      // byte i (< 1024) as f16, twice
+        return __hsub2(bits_h2(((w >> (8 * i)) & 0xFFu) * 0x00010001u | 0x64006400u), bits_h2(0x64006400u));
+    }
+    __device__ __forceinline__ float2 scales() const {
+        const __half2 h = bits_h2(dm);
+        return make_float2(__low2float(h), __high2float(h));
+    }
+    __device__ __forceinline__ void mins(uint8_t *slab0) const {       // f16 minimum of every 16-element run, two slabs
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+            *reinterpret_cast<uint4 *>(slab0 + s * kRows * 16) =
+                make_uint4(h2_bits(byte_h2(mn[s], 0)), h2_bits(byte_h2(mn[s], 1)), h2_bits(byte_h2(mn[s], 2)), h2_bits(byte_h2(mn[s], 3)));
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(p + 16 + 32 * CH), b = *reinterpret_cast<const uint4 *>(p + 32 + 32 * CH);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const __half2 s0 = byte_h2(sc[CH >> 1], 2 * (CH & 1)), s1 = byte_h2(sc[CH >> 1], 2 * (CH & 1) + 1);
+        const __half2 c0 = __hmul2(s0, __float2half2_rn(-1024.0f));
+        const __half2 m1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-64.0f));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t u = w[i], v = w[i] >> 8;
+            o[2 * i] = hfma2_bits((u & 0x000F000Fu) | 0x64006400u, s0, c0);
+            o[2 * i + 1] = hfma2_bits((v & 0x000F000Fu) | 0x64006400u, s0, c0);
+            o[16 + 2 * i] = hfma2_bits((u & 0x00F000F0u) | 0x64006400u, m1, c1);
+            o[16 + 2 * i + 1] = hfma2_bits((v & 0x00F000F0u) | 0x64006400u, m1, c1);
+        }
+    }
+};
+
+// Q6_K chunk ch = 4 h + 2 p + nib: elements 128 h + 32 pos + [0, 32), pos = p + 2 nib: nibble `nib` of ql[64 h + 32 p ..], bit pair
+// pos of qh[32 h ..]; cells 0-15 the even part times the scale, 16-31 the lowest bit times the scale.  The even part sits in the
+// mantissa of 64.0 (unit 1/16), so one fma with -96 sc gives sc (e - 32) exactly.
+template <> struct Expand<CQ_Q6_K> {
+    const uint8_t *p;
+    uint32_t qh[8], ql[8], sc[4];
+    __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
+        p = rr + shift;
+        cq_lds_words<4>(p + 192, sc);
+    }
+    __device__ __forceinline__ float2 scales() const { return make_float2(__half2float(*reinterpret_cast<const __half *>(p + 208)), 0.0f); }
+    __device__ __forceinline__ void mins(uint8_t *) const {}
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) {
+        constexpr int h = CH >> 2, pp = (CH >> 1) & 1, nib = CH & 1, pos = pp + 2 * nib;
+        if constexpr ((CH & 3) == 0) cq_lds_words<8>(p + 128 + 32 * h, qh);
+        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 64 * h + 32 * pp, ql);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            constexpr int j0 = 8 * h + 2 * pos;
+            const int scv = (int)(int8_t)(sc[(j0 + hf) >> 2] >> (8 * ((j0 + hf) & 3)));
+            const __half s = __short2half_rn((short)scv);
+            const __half2 s2 = __half2half2(s), c2 = __hmul2(s2, __float2half2_rn(-96.0f));
+            const uint32_t sbits = (uint32_t)__half_as_ushort(s);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i];
+#pragma unroll
+                for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
+                    const uint32_t lv = od ? l >> 8 : l;
+                    const uint32_t lo = (nib ? lv : lv << 4) & 0x00E000E0u;
+                    const int up = 8 - 2 * pos - 8 * od;        // bit pair pos of byte od -> bits 8, 9
+                    const uint32_t hi = (up >= 0 ? b << (up >= 0 ? up : 0) : b >> (up < 0 ? -up : 0)) & 0x03000300u;
+                    o[8 * hf + 2 * i + od] = hfma2_bits(lo | hi | 0x54005400u, s2, c2);
+                    o[16 + 8 * hf + 2 * i + od] = ((nib ? lv >> 4 : lv) & 0x00010001u) * sbits;
+                }
+            }
+        }
+    }
+};
+// token slab (8 k-elements) at which a chunk starts, inside its half super-block
+template <int WTYPE> __device__ __forceinline__ constexpr int chunk_slab(int ch) {
+    return WTYPE == CQ_Q4_K ? 8 * (ch & 1) : 4 * (((ch >> 1) & 1) + 2 * (ch & 1));
+}
+
+struct Args {
+    const uint8_t *w, *w2, *act;        // w2: null, or a second matrix of the same shape for the same activations
+    void *out, *out2;
+    long long total_rows;               // weight rows in memory (all experts)
+    int out_kind, nrows, nsb, stride_out, use_map, nrt;
+};
+
+template <int WTYPE>
+__global__ void __launch_bounds__(kThreads, 1)
+prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2, const Args a, const Tiling tl, const GroupInfo gi) {
+    using F = Fmt<WTYPE>;
+    using R = Raw<cq_type_size(WTYPE)>;
+    constexpr int kCB = cq_type_size(WTYPE);
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [3] raw weight bytes landed
+    uint64_t *bar_rawfree = bar_raw + 3;                            // [3] read by all producers
+    uint64_t *bar_fullT = bar_raw + 6;                              // [4] token stage (first half: + run sums and scales) landed
+    uint64_t *bar_doneT = bar_raw + 10;                             // [4] its MMAs are complete
+    uint64_t *bar_fullW = bar_raw + 14;                             // [4] operand A chunk stored (all producers)
+    uint64_t *bar_doneW = bar_raw + 18;                             // [4] its MMAs are complete
+    uint64_t *bar_acc = bar_raw + 22;                               // [2] MMAs of a super-block complete
+    uint64_t *bar_free = bar_raw + 24;                              // [2] accumulators drained (all epilogue warps)
+    uint64_t *bar_vis = bar_raw + 26;                               // [2] relay: the scale rings of this super-block are visible
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 256);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 264);
+    uint8_t *stT0 = smem + 1024;
+    uint8_t *aux0 = stT0 + kStagesT * kStageT;
+    uint8_t *ringW = aux0 + kAuxRing * kAux;            // (d, dmin) of the rows: [4][128] float2
+    uint8_t *mins0 = ringW + 4 * kRows * 8;             // operand A of the sums step: [2][2 slabs][128][16]
+    uint8_t *raw0 = mins0 + 2 * kRows * 32;             // 128-byte aligned
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nsb = a.nsb;
+    const uint32_t row_bytes = (uint32_t)nsb * kCB;
+
+    if (tid == 0) {
+        for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], 1); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < 4; ++i) {
+            cq_mbar_init(&bar_fullT[i], 1);
+            cq_mbar_init(&bar_doneT[i], 1);
+            cq_mbar_init(&bar_fullW[i], kProdWarps);
+            cq_mbar_init(&bar_doneW[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            cq_mbar_init(&bar_acc[i], 1);
+            cq_mbar_init(&bar_free[i], kEpiWarps);
+            cq_mbar_init(&bar_vis[i], 1);
+        }
+        *abort_flag = 0;
+        cq_fence_mbar_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    cq_pdl_wait();              // activations and the tile table come from the preceding launches
+    // grouped: the table says how many of its tiles are in use.  With a second matrix its tiles follow those of the first.
+    const int ntt = gi.tiles ? gi.tiles[4 * tl.ntt] : tl.ntt;
+    const int per_matrix = a.nrt * ntt, ntiles = a.w2 ? 2 * per_matrix : per_matrix;
+
+    if (warp >= kEpiWarps && warp < kMmaWarp) {
+        // ===== producers: thread = weight row = TMEM lane =====
+        const int r = tid - kEpiWarps * 32;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
+        int it = 0, wi = 0, rs = 0, rs_phase = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            long long wr = cx.wrow0 + r;
+            if (wr >= a.total_rows) wr = a.total_rows - 1;
+            // without the tensor map every row has its own distance to the 16-byte boundary below it
+            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes) & 15);
+            for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
+                if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
+                Expand<WTYPE> ex;
+                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
+                const float2 ws = ex.scales();
+                auto step = [&](auto chc) {
+                    constexpr int CH = decltype(chc)::value;
+                    if (!alive) return;
+                    uint32_t o[32];
+                    ex.template chunk<CH>(o);
+                    if constexpr (CH == F::kChunks - 1) arrive_warp(&bar_rawfree[rs], lane);
+                    const int buf = wi & 3;
+                    if (wi >= kStagesW && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
+                    tc_fence_after();
+                    if constexpr (CH == 0) {
+                        // a chunk of super-block it - 1 is done, so its MMAs had started and the epilogue has finished
+                        // it - 3: ring entry it - 4 is free; the sums step of it - 2 is complete too
+                        *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
+                        if constexpr (F::kMins) {
+                            ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
+                            fence_proxy_async_smem();
+                        }
+                    }
+                    tmem_st32(ta + buf * 32, o);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    arrive_warp(&bar_fullW[buf], lane);
+                    ++wi;
+                };
+                step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 1>{});
+                step(std::integral_constant<int, 2>{}); step(std::integral_constant<int, 3>{});
+                if constexpr (F::kChunks == 8) {
+                    step(std::integral_constant<int, 4>{}); step(std::integral_constant<int, 5>{});
+                    step(std::integral_constant<int, 6>{}); step(std::integral_constant<int, 7>{});
+                }
+                if (++rs == F::kRawStages) { rs = 0; rs_phase ^= 1; }
+            }
+        }
+    } else if (warp == kLoadWarp) {
+        // ===== loader: raw weights and activations of up to three / two super-blocks ahead =====
+        int it = 0, ti = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            const int n = cx.n;
+            const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nsb * kTokBytes;
+            for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
+                const int rs = it % F::kRawStages;
+                if (it >= F::kRawStages && !wait_or_abort(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
+                uint8_t *dst = raw0 + rs * R::kBytes;
+                if (a.use_map) {
+                    if (lane == 0) {
+                        cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
+                        cq_tmap::load_2d(dst, second ? &wmap2 : &wmap, (int)(((uint32_t)sb * kCB & ~15u) / 2), (int)cx.wrow0, &bar_raw[rs]);
+                    }
+                } else {
+                    if (lane == 0) cq_mbar_expect_tx(&bar_raw[rs], kRows * R::kNeed);
+                    __syncwarp();
+                    for (int r = lane; r < kRows; r += 32) {
+                        long long wr = cx.wrow0 + r;
+                        if (wr >= a.total_rows) wr = a.total_rows - 1;
+                        const uintptr_t src = (uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes + (uint32_t)sb * kCB) & ~(uintptr_t)15;
+                        cq_bulk_g2s(dst + r * R::kPitch, (const void *)src, R::kNeed, &bar_raw[rs]);
+                    }
+                }
+                const uint8_t *blob = blob0 + (size_t)sb * n * kTokBytes;
+                for (int half = 0; half < 2; ++half, ++ti) {
+                    const int s = ti & 3;
+                    if (ti >= kStagesT && !wait_or_abort(&bar_doneT[s], ((ti >> 2) - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (lane == 0) {
+                        const unsigned bytes = (unsigned)n * 256;
+                        if (half == 0) {
+                            // done with the stage of (it - 2, first half): its MMAs started after the epilogue of it - 4
+                            uint8_t *ax = aux0 + (it & 3) * kAux;
+                            const unsigned aux_bytes = (unsigned)n * (F::kMins ? 36 : 4);
+                            cq_mbar_expect_tx(&bar_fullT[s], bytes + aux_bytes);
+                            cq_bulk_g2s(ax + (F::kMins ? 0 : n * 32), blob + (size_t)n * (F::kMins ? 512 : 544), aux_bytes, &bar_fullT[s]);
+                        } else {
+                            cq_mbar_expect_tx(&bar_fullT[s], bytes);
+                        }
+                        cq_bulk_g2s(stT0 + s * kStageT, blob + (size_t)half * bytes, bytes, &bar_fullT[s]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
+        if (lane == 0 && (!alive || *abort_flag)) {
+            for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; j <= it; ++j)
+                (void)cq_mbar_wait_bounded(&bar_raw[j % F::kRawStages], (j / F::kRawStages) & 1);
+            for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j & 3], (j >> 2) & 1);
+        }
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        // ===== MMA issuer: one thread =====
+        if (lane == 0) {
+            constexpr int kHalf = F::kChunks / 2;
+            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)kColA;
+            int it = 0, wi = 0;
+            bool alive = true;
+            for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+                TileCtx cx;
+                const bool second = tile >= per_matrix;
+                tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+                const uint32_t n = (uint32_t)cx.n, idesc = idesc_f16(cx.n), bT = stT | (n << 16);
+                for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
+                    const int c = it & 1;
+                    const uint32_t tp = tmem_base + (uint32_t)(c * kTokMax);
+                    if (it >= 2 && !wait_or_abort(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        const int s = (2 * it + half) & 3;
+                        if (!wait_or_abort(&bar_fullT[s], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                        const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4);
+#pragma unroll
+                        for (int ch = 0; ch < kHalf; ++ch, ++wi) {
+                            const int buf = wi & 3;
+                            if (!wait_or_abort(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
+                            tc_fence_after();
+                            if (half == 0 && ch == 0) mbar_arrive(&bar_vis[c]);     // relay: what this thread has acquired is visible to the epilogue
+                            const uint32_t b1 = b0 + (uint32_t)chunk_slab<WTYPE>(ch) * n, a0 = ta + buf * 32;
+                            if (half == 0 && ch == 0) mma_f16_ts<false>(tp, a0, b1, idesc);
+                            else mma_f16_ts<true>(tp, a0, b1, idesc);
+                            mma_f16_ts<true>(tp, a0 + 8, b1 + 2 * n, idesc);
+                            // Q6_K: both planes of a chunk meet the same 32 activations
+                            mma_f16_ts<true>(tp, a0 + 16, F::kMins ? b1 + 4 * n : b1, idesc);
+                            mma_f16_ts<true>(tp, a0 + 24, F::kMins ? b1 + 6 * n : b1 + 2 * n, idesc);
+                            tc_commit(&bar_doneW[buf]);
+                        }
+                        if (!alive) break;
+                        if constexpr (F::kMins) {
+                            if (half == 1) {
+                                // L has one buffer: the epilogue of the previous super-block must have read it
+                                if (it >= 1 && !wait_or_abort(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
+                                tc_fence_after();
+                                mma_f16_ss(tmem_base + (uint32_t)kColL, desc_lo(mins0 + c * kRows * 32, kRows), desc_lo(aux0 + (it & 3) * kAux, n), idesc);
+                            }
+                        }
+                        tc_commit(&bar_doneT[s]);
+                    }
+                    if (alive) tc_commit(&bar_acc[c]);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
+        const int quad = warp & 3, ch0 = warp >> 2;
+        const int r = quad * 32 + lane;
+        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        int it = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            uint64_t acc[4][8];
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[g][i] = 0ull;
+            for (int sb = 0; sb < nsb; ++sb, ++it) {
+                const int c = it & 1;
+                if (!wait_warp(&bar_vis[c], (it >> 1) & 1, abort_flag) ||
+                    !wait_warp(&bar_acc[c], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                tc_fence_after();
+                const float2 ws = *reinterpret_cast<const float2 *>(ringW + (it & 3) * kRows * 8 + r * 8);
+                const uint64_t dw = pack2f(ws.x, ws.x), ndm = pack2f(-ws.y, -ws.y);
+                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * kAux + cx.n * 32);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const int col = (2 * g + ch0) * 16;
+                    if (col < cx.n) {           // warp-uniform
+                        uint32_t p[16], l[16];
+                        tmem_ld16(tlane + (uint32_t)(c * kTokMax + col), p);
+                        if constexpr (F::kMins) tmem_ld16(tlane + (uint32_t)(kColL + col), l);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 8; i += 2) {
+                            const float4 d4 = *reinterpret_cast<const float4 *>(da + col + 2 * i);
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
+                                const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
+                                uint64_t tv;
+                                if constexpr (F::kMins) tv = fma2(dw, pv, mul2(ndm, pack2(l[2 * (i + e)], l[2 * (i + e) + 1])));
+                                else tv = mul2(dw, pv);
+                                acc[g][i + e] = fma2(dd, tv, acc[g][i + e]);
+                            }
+                        }
+                    }
+                }
+                tc_fence_before();
+                arrive_warp(&bar_free[c], lane);
+            }
+            if (!alive) break;
+            if (cx.row0 + r < a.nrows) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const int col = (2 * g + ch0) * 16;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        if (col + i < cx.valid) {
+                            float v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
+                            int64_t orow = (int64_t)cx.t * tl.tt + col + i;
+                            if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight
+                                orow = gi.sorted_token_ids[cx.job0 + col + i];
+                                if (gi.topk_weights) v = __fmul_rn(v, gi.topk_weights[orow]);
+                            }
+                            cq_store_out(second ? a.out2 : a.out, a.out_kind, orow * a.stride_out + cx.row0 + r, v);
+                        }
+                    }
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && *abort_flag) atomicExch(&g_prompt_kq_timeout_flag, 1);
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
+}
+
+// tokens' worth of MMA time that expanding one super-block of 128 rows takes
+template <int WTYPE> constexpr int floor_tokens() { return WTYPE == CQ_Q4_K ? 56 : 72; }
+
+template <int WTYPE>
+bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k, int n, long long total_rows, int stride_out, const Tiling &tl,
+                 const GroupInfo &gi, cudaStream_t st, const void *w2 = nullptr, void *out2 = nullptr) {
+    using R = Raw<cq_type_size(WTYPE)>;
+    static_assert(smem_bytes<WTYPE>() <= 232448, "shared memory of one CTA");
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+        cudaFuncSetAttribute(prompt_kernel<WTYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WTYPE>());
+        attr_done[dev] = true;
+    }
+    const long long row_bytes = (long long)(k / 256) * cq_type_size(WTYPE);
+    CUtensorMap map{}, map2{};
+    const uintptr_t both = (uintptr_t)w | (uintptr_t)w2;
+    const bool use_map = both % 16 == 0 && row_bytes % 16 == 0 && row_bytes <= INT32_MAX && total_rows <= INT32_MAX &&
+                         cq_tmap::weight_map(w, (int)row_bytes, (int)total_rows, R::kPitch / 2, kRows, 2, map) &&
+                         (!w2 || cq_tmap::weight_map(w2, (int)row_bytes, (int)total_rows, R::kPitch / 2, kRows, 2, map2));
+    if (!use_map && R::kAligned && both % 16 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt gemm: Q4_K weights must be 16-byte aligned");
+        return false;
+    }
+    const Args a{(const uint8_t *)w, (const uint8_t *)w2, (const uint8_t *)act, out, out2, total_rows, out_elem, n, k / 256, stride_out,
+                 use_map ? 1 : 0, (n + kRows - 1) / kRows};
+    const long long ntiles = (long long)a.nrt * tl.ntt * (w2 ? 2 : 1);
+    const int grid = ntiles < sm_count() ? (int)ntiles : sm_count();
+    cq_launch_k(prompt_kernel<WTYPE>, dim3(grid), dim3(kThreads), smem_bytes<WTYPE>(), st, map, map2, a, tl, gi);
+    return true;
+}
+
+template <typename L> bool launch_quantize(const L &load, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
+    const long long blocks = (long long)tl.ntt * (tl.tt / 8) * (k / 256);
+    if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt quantize: too many tokens for one launch"); return false; }
+    cq_launch_k(quantize_kernel<L>, dim3((unsigned)blocks), dim3(256), 0, st, load, (uint8_t *)scratch, k / 256, tl, gi);
+    return true;
+}
+bool launch_quantize_rows(const void *x, int x_elem, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
+    if (x_elem == CQ_F32) return launch_quantize(LoadRows<float>{(const float *)x, k}, scratch, k, tl, gi, st);
+    if (x_elem == CQ_F16) return launch_quantize(LoadRows<__half>{(const __half *)x, k}, scratch, k, tl, gi, st);
+    if (x_elem == CQ_BF16) return launch_quantize(LoadRows<__nv_bfloat16>{(const __nv_bfloat16 *)x, k}, scratch, k, tl, gi, st);
+    cq_set_status(CQ_ERR_BAD_ARG, "prompt quantize: unknown element type");
+    return false;
+}
+
+Tiling dense_tiling(int wtype, int tokens, int n) {
+    return plan_tiling(tokens, (n + kRows - 1) / kRows, sm_count(), wtype == CQ_Q4_K ? floor_tokens<CQ_Q4_K>() : floor_tokens<CQ_Q6_K>());
+}
+int group_max_tiles(int size_m, int num_experts) { return (size_m + kTokMax - 1) / kTokMax + num_experts; }
+size_t table_bytes(int max_tiles) { return ((size_t)(max_tiles + 1) * 16 + 255) / 256 * 256; }
+// every expert pads its rows to a multiple of 16
+size_t group_blob_bytes(int size_m, int num_experts, int k) { return ((size_t)size_m + 15 * (size_t)num_experts) * kTokBytes * (k / 256); }
+
+}  // namespace
+
+extern "C" size_t cq_prompt_scratch_bytes(int tokens, int k) {
+    if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
+    // whatever the tile size, only the last tile is padded, to a multiple of 16 rows
+    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * kTokBytes + 256;
+}
+
+extern "C" void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,
+                                 int tokens, int stride_dst, void *stream) {
+    if (!vx || !x || !scratch || !dst || ncols_x <= 0 || nrows_x <= 0 || tokens <= 0 || ncols_x % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt matmul: null pointer, empty shape or K not a multiple of 256");
+        return;
+    }
+    if (wtype != CQ_Q4_K && wtype != CQ_Q6_K) {
+        cq_set_status(CQ_ERR_UNSUPPORTED, "prompt matmul: covers Q4_K and Q6_K");
+        return;
+    }
+    if ((uintptr_t)vx % (wtype == CQ_Q4_K ? 16 : 4) != 0 || (uintptr_t)scratch % 16 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt matmul: misaligned weights (16 bytes for Q4_K, 4 for Q6_K) or scratch (16)");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const Tiling tl = dense_tiling(wtype, tokens, nrows_x);
+    if (!launch_quantize_rows(x, elem, scratch, ncols_x, tl, GroupInfo{}, st)) return;
+    const bool ok = wtype == CQ_Q4_K
+                        ? launch_gemm<CQ_Q4_K>(vx, scratch, dst, elem, ncols_x, nrows_x, nrows_x, stride_dst, tl, GroupInfo{}, st)
+                        : launch_gemm<CQ_Q6_K>(vx, scratch, dst, elem, ncols_x, nrows_x, nrows_x, stride_dst, tl, GroupInfo{}, st);
+    if (ok) cq_check_launch("prompt matmul");
+}
+
+// ---- grouped entry point (quantized mixture-of-experts, many tokens) ----
+extern "C" size_t cq_moe_prefill_scratch_bytes(int size_m, int num_experts, int k) {
+    if (size_m <= 0 || num_experts <= 0 || num_experts > 1024 || k <= 0 || k % 256 != 0) return 0;
+    return table_bytes(group_max_tiles(size_m, num_experts)) + group_blob_bytes(size_m, num_experts, k) + 256;
+}
+
+// out[pair, :] = W[expert of the pair] . x[input row of the pair] (times topk_weights[pair]) for all size_m sorted pairs
+// (candle-nn/src/moe.rs:286-337): jobs sorted by expert; job m: pair = sorted_token_ids[m], expert = expert_ids[m]; input row =
+// pair when routing weights are given, else pair / topk.  The host never sees the routing: a table of tiles is built on the
+// device, over-sized to ceil(M / 128) + experts entries.  Rows of pairs whose expert id is outside [0, num_experts) are not
+// written.
+extern "C" void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *weights, const int32_t *sorted_token_ids,
+                                    const int32_t *expert_ids, const float *topk_weights, float *out, void *scratch, int num_experts,
+                                    int topk, int size_m, int size_n, int size_k, void *stream) {
+    if (!input || !weights || !sorted_token_ids || !expert_ids || !out || !scratch || num_experts <= 0 || num_experts > 1024 ||
+        topk <= 0 || size_m <= 0 || size_n <= 0 || size_k <= 0 || size_k % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: null pointer, empty shape, more than 1024 experts or K not a multiple of 256");
+        return;
+    }
+    if (wtype != CQ_Q4_K && wtype != CQ_Q6_K) {
+        cq_set_status(CQ_ERR_UNSUPPORTED, "moe prefill: the tensor-core kernel covers Q4_K and Q6_K");
+        return;
+    }
+    const long long expert_stride = (long long)size_n * (size_k / 256) * cq_type_size(wtype);
+    if ((uintptr_t)weights % 16 != 0 || (uintptr_t)scratch % 256 != 0 || (wtype == CQ_Q4_K ? expert_stride % 16 : expert_stride % 4) != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: misaligned weights or scratch");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const int mt = group_max_tiles(size_m, num_experts);
+    int *tiles = (int *)scratch;
+    uint8_t *blobs = (uint8_t *)scratch + table_bytes(mt);
+    group_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
+    const GroupInfo gi{tiles, sorted_token_ids, topk_weights, size_n, topk, topk_weights ? 1 : 0};
+    const Tiling tl{mt * kTokMax, kTokMax, mt};
+    if (!launch_quantize_rows(input, in_elem, blobs, size_k, tl, gi, st)) return;
+    const long long total = (long long)size_n * num_experts;
+    const bool ok = wtype == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st)
+                                     : launch_gemm<CQ_Q6_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st);
+    if (ok) cq_check_launch("moe prefill gemm");
+}
+
+extern "C" int cq_prompt_timeout_flag(void) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_prompt_kq_timeout_flag, sizeof v) != cudaSuccess) { (void)cudaGetLastError(); return -1; }
+    if (v) cq_set_status(CQ_ERR_TIMEOUT, "prompt matmul: a bounded wait gave up");
+    return v;
+}

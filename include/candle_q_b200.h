@@ -227,6 +227,15 @@ void cq_prefill_quantize(const void *x, int x_elem, void *scratch, int k, int to
 void cq_prefill_gemm(int wtype, const void *vx, const void *scratch, void *dst, int out_elem, int ncols_x, int nrows_x,
                      int tokens, int stride_dst, void *stream);
 int cq_prefill_timeout_flag(void);
+
+/* The prompt product as QMatMul::forward runs it, Q4_K and Q6_K, the arithmetic of the pair above: x [tokens, k] of `elem`
+ * -> dst[t * stride_dst + row] of the same type, quantization and product in one call.  k % 256 == 0; scratch:
+ * cq_prompt_scratch_bytes, 16-byte aligned; weights 16-byte (Q4_K) or 4-byte (Q6_K) aligned.
+ *   cq_prompt_timeout_flag : 1 if a launch (dense or grouped) on the current device gave up a bounded wait (synchronises). */
+size_t cq_prompt_scratch_bytes(int tokens, int k);
+void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
+                      int stride_dst, void *stream);
+int cq_prompt_timeout_flag(void);
 /* The same for the 32-element block formats Q4_0 (wtype 2) and Q8_0 (8): candle-kernels/src/mmq_gguf/mmq_gguf.cuh:305-364,
  * 927-1062, 1169-1296 behind ffi.rs:471-630.  Activations are quantized like candle's CPU path (BlockQ8_0, k_quants.rs:
  * 658-687); every 32-element block is one tcgen05 MMA step into a fresh TMEM accumulator that the epilogue scales by

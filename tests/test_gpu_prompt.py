@@ -1,0 +1,67 @@
+"""The prompt products QMatMul.forward runs: f16 operands holding integers, weights expanded into tensor memory.
+
+Q4_K / Q6_K (cq_prompt_matmul) against the CPU path's matmul (the tolerance of the other prompt tests: only the order of f32
+additions differs), and bit for bit against the int8 kernel behind cq_prefill_gemm: the same integers, the same f32 operations
+in the same order.
+"""
+import numpy as np
+import pytest
+import torch
+
+from candle_b200 import capi
+from helpers import make_case, rel_err
+
+pytestmark = pytest.mark.gpu
+ELEM = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
+
+
+def _run(scratch_bytes, matmul, flag, wtype, w_dev, x_dev, k, n):
+    tokens, st = x_dev.shape[0], torch.cuda.current_stream().cuda_stream
+    scratch = torch.full((scratch_bytes + 64,), 0xFF, dtype=torch.uint8, device=x_dev.device)     # 0xFFFF: f16 NaN
+    out = torch.full((tokens * n + 32,), float("nan"), dtype=x_dev.dtype, device=x_dev.device)
+    matmul(wtype, w_dev.data_ptr(), x_dev.data_ptr(), ELEM[x_dev.dtype], out.data_ptr(), scratch.data_ptr(), k, n, tokens, n, st)
+    capi.check("prompt")
+    torch.cuda.synchronize()
+    assert flag() == 0
+    assert bool((scratch[-64:] == 0xFF).all()), "scratch written past its end"
+    assert bool(torch.isnan(out[tokens * n:].float()).all()) and not bool(torch.isnan(out[:tokens * n].float()).any())
+    return out[:tokens * n].view(tokens, n)
+
+
+def _prompt(lib, wtype, w_dev, x_dev, k, n):
+    return _run(lib.cq_prompt_scratch_bytes(x_dev.shape[0], k), lib.cq_prompt_matmul, lib.cq_prompt_timeout_flag, wtype, w_dev, x_dev, k, n)
+
+
+def _int8(lib, wtype, w_dev, x_dev, k, n):
+    tokens, st = x_dev.shape[0], torch.cuda.current_stream().cuda_stream
+    scratch = torch.zeros(lib.cq_prefill_scratch_bytes(tokens, k), dtype=torch.uint8, device=x_dev.device)
+    out = torch.empty((tokens, n), dtype=x_dev.dtype, device=x_dev.device)
+    lib.cq_prefill_quantize(x_dev.data_ptr(), ELEM[x_dev.dtype], scratch.data_ptr(), k, tokens, st)
+    lib.cq_prefill_gemm(wtype, w_dev.data_ptr(), scratch.data_ptr(), out.data_ptr(), ELEM[x_dev.dtype], k, n, tokens, n, st)
+    capi.check("prefill")
+    return out
+
+
+# one super-block, one ragged row tile; a full tile and one row more; tokens around the multiples of 16 and of 128; more tiles
+# than SMs (several per CTA); K whose Q6_K rows start off a 16-byte boundary (256, 768, 1280) and on one (2048)
+@pytest.mark.parametrize("tokens,k,n", [(1, 256, 1), (17, 512, 65), (16, 256, 128), (128, 768, 129), (129, 1280, 200), (333, 2048, 512),
+                                        (300, 4096, 96), (2000, 512, 2050)])
+@pytest.mark.parametrize("wtype,dtype", [(12, torch.float32), (14, torch.float32), (12, torch.bfloat16), (14, torch.float16)])
+def test_prompt_matmul(lib, oracle, cuda_dev, tokens, k, n, wtype, dtype):
+    _, x, wq = make_case(oracle, wtype, k, n, tokens, seed=tokens + k + n)
+    if wtype == 14:     # negative, zero and extreme sub-block scales
+        wq.reshape(-1, 210)[0, 192:208] = np.array([-128, 127, 0, -1, 1, -64, 64, 5, -5, 100, -100, 33, -33, 2, -2, 0], dtype=np.int8).view(np.uint8)
+    x_dev = torch.from_numpy(x).to(cuda_dev).to(dtype)
+    w_dev = torch.from_numpy(wq).to(cuda_dev)
+    out = _prompt(lib, wtype, w_dev, x_dev, k, n)
+    if dtype == torch.float32 and tokens <= 333:
+        assert rel_err(out.cpu().numpy(), oracle.matmul(wtype, x, wq, n)) <= 1e-5
+    assert torch.equal(out, _int8(lib, wtype, w_dev, x_dev, k, n))
+
+
+def test_prompt_matmul_unaligned_activations(lib, oracle, cuda_dev):
+    _, x, wq = make_case(oracle, 12, 512, 70, 40, seed=3)
+    w_dev = torch.from_numpy(wq).to(cuda_dev)
+    buf = torch.zeros(40 * 512 + 1, device=cuda_dev)
+    buf[1:] = torch.from_numpy(x).to(cuda_dev).view(-1)
+    assert torch.equal(_prompt(lib, 12, w_dev, buf[1:].view(40, 512), 512, 70), _prompt(lib, 12, w_dev, buf[1:].clone().view(40, 512), 512, 70))
