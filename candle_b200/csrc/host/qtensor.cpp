@@ -195,14 +195,17 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
         lib_check("qmatmul prefill");
         return;
     }
-    // The 32-element block formats Q4_0 / Q8_0 have their own tensor-core prompt kernel (Q8_0 activations, the CPU path's
-    // arithmetic, in every mode); K must be a whole number of 256-element stages.
-    if (rows > kPrefillMinRows && (dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0) && k % 256 == 0) {
-        const size_t need = cq_prefill32_scratch_bytes((int)rows, (int)k);
-        uint8_t *scratch = (uint8_t *)workspace_ensure(device_, need);
-        cq_prefill32_quantize(x, (int)x_dtype, scratch, (int)k, (int)rows, stream);
-        cq_prefill32_gemm((int)dtype_, ptr_, scratch, out, (int)x_dtype, (int)k, (int)n, (int)rows, (int)n, stream);
-        lib_check("qmatmul prefill (block formats)");
+    // Formats with an activation scale per 32 elements: Q4_0 / Q8_0 (Q8_0 activations, the CPU path's arithmetic, in every mode)
+    // and the six others (Q8_1, the decode kernels' arithmetic, hence already from the first row that no longer fits one
+    // decode launch, and not in the CPU-exact mode).  K must be a whole number of 256-element stages.
+    const bool plain32 = dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0;
+    const bool q8_1_only = !plain32 && dtype_ != GgmlDType::Q4K && dtype_ != GgmlDType::Q6K;
+    const bool any_address = dtype_ == GgmlDType::Q2K || dtype_ == GgmlDType::Q3K;
+    if (k % 256 == 0 && ((plain32 && rows > kPrefillMinRows) ||
+                         (q8_1_only && rows > MMVQ_MAX_BATCH && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0)))) {
+        uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt32_scratch_bytes((int)dtype_, (int)rows, (int)k));
+        cq_prompt32_matmul((int)dtype_, ptr_, x, (int)x_dtype, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
+        lib_check("qmatmul prefill (scales per 32)");
         return;
     }
     // Decode path: up to 8 rows per launch.  Other formats with more rows are walked in slices of 8 rows.

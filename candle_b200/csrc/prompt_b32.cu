@@ -1,0 +1,701 @@
+// Prompt-phase quantized GEMM for activations with one scale per 32 elements, on tcgen05.mma kind::f16 (prompt_f16.cuh):
+//   Q8_0, Q4_0                            BlockQ8_0 activations, candle's CPU arithmetic (k_quants.rs:294-311, 720-738)
+//   Q4_1, Q5_0, Q5_1, Q2_K, Q3_K, Q5_K     Q8_1 activations, the arithmetic of the decode kernels (mmvq_gguf.cu:208-334, 357-381,
+//                                          492-531; gemv_chunks.cuh), which these formats use at every row count
+//
+// Both sides of a product carry a scale per 32 elements, so nothing beyond the integer sub-scales of a K-quant can be folded
+// into the operands: every 32-element block is two K = 16 steps into a FRESH accumulator slot, exact (sums below 2^24: at most
+// 31 * 63 * 127 * 32), and the epilogue adds  d_a * (d_w * I) [+ m_w * s_a]  to f32 running sums, two at a time.
+// Against int8 operands the epilogue needs no int -> float conversion, which was two of its five operations per value.
+//
+// Summation: Q8_0 / Q4_0 add block after block, as the kernel behind cq_prefill32_gemm does (the same f32 operations, the same
+// bits).  The Q8_1 formats were summed by the decode kernels' balanced tree until now; a plain chain of K / 32 additions would
+// lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
+//
+// Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 128 (Q8_0 / Q4_0) or 64 tokens (the compensated sums take three
+// registers per value), warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader; tensor memory: 384 columns of
+// accumulator slots, 128 of operand A.  Every wait is bounded as there.
+#include "../../include/candle_q_b200.h"
+#include "prompt_f16.cuh"
+
+#include <type_traits>
+
+namespace {
+using namespace cq_prompt;
+
+constexpr int kEpiWarps = 8, kProdWarps = 4;
+constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
+constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
+constexpr int kColA = 384;
+
+__device__ int g_prompt_b32_timeout_flag = 0;
+
+// kMins: terms m_w * s_a per block;  kSum: what s_a is
+enum { kNoSum, kFloatSum, kIntSum };
+template <int WTYPE> struct Fmt {       // Q8_0, Q4_0
+    static constexpr bool kQ81 = false;
+    static constexpr int kMins = 0, kSum = kNoSum, kTok = 128, kStagesT = 3;
+};
+template <int MINS, int SUM> struct FmtQ81 {
+    static constexpr bool kQ81 = true;
+    static constexpr int kMins = MINS, kSum = SUM, kTok = 64, kStagesT = 4;
+};
+template <> struct Fmt<CQ_Q4_1> : FmtQ81<1, kFloatSum> {};
+template <> struct Fmt<CQ_Q5_0> : FmtQ81<1, kFloatSum> {};
+template <> struct Fmt<CQ_Q5_1> : FmtQ81<1, kFloatSum> {};
+template <> struct Fmt<CQ_Q5_K> : FmtQ81<1, kIntSum> {};
+template <> struct Fmt<CQ_Q2_K> : FmtQ81<2, kIntSum> {};     // one per 16 elements
+template <> struct Fmt<CQ_Q3_K> : FmtQ81<0, kNoSum> {};
+
+template <int WTYPE> constexpr int chunk_bytes() { return 256 / cq_block_elems(WTYPE) * cq_type_size(WTYPE); }
+template <int MINS> constexpr int tok_bytes() { return 512 + 32 + 32 * MINS; }        // f16 values, scales, sums of one chunk
+template <int MINS> constexpr int wscale_bytes() { return MINS == 0 ? 4 : MINS == 1 ? 8 : 16; }
+template <int WTYPE> struct Smem {
+    using F = Fmt<WTYPE>;
+    static constexpr int kStageT = 16 * F::kTok * 16, kAux = F::kTok * (32 + 32 * F::kMins), kRingW = 8 * kRows * wscale_bytes<F::kMins>();
+    static constexpr int kBytes = 1024 + F::kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
+};
+
+// ---- activations ---------------------------------------------------------------------------------------------------
+// One warp per (token, chunk of 256), 8 tokens of one chunk per block, through shared memory (see prompt_kq.cu).
+template <typename T, bool Q81, int MINS, int SUM>
+__global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k, Tiling tl) {
+    constexpr int kPitch = 8 * 16 + 16, kVals = 8 * (1 + MINS);
+    __shared__ __align__(16) uint8_t sm[32 * kPitch];
+    __shared__ float sv[kVals][8];      // [value][token]: block scales, then sums
+    cq_pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nch = k / 256;
+    const int c = blockIdx.x % nch, g = blockIdx.x / nch, per_tile = tl.tt / 8;
+    const int t = g / per_tile, row0 = (g % per_tile) * 8, row = row0 + warp;
+    const int rows = tl.rows(t);
+    if (row0 >= rows) return;           // block-uniform
+    const int64_t tok = (int64_t)t * tl.tt + row;
+    float e[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) e[i] = 0.0f;
+    if (row < rows && tok < tl.tokens) load8(x + tok * k + c * 256 + lane * 8, ((uintptr_t)x & 15) == 0, e);
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(e[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float d = __fdiv_rn(amax, 127.0f);
+    int q[8];
+    if constexpr (Q81) {                // mmvq_gguf.cu:811-911
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q[i] = (amax == 0.0f) ? 0 : (int)(int8_t)roundf(__fdiv_rn(e[i], d));
+    } else {                            // k_quants.rs:658-687
+        const float id = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float r = roundf(__fmul_rn(e[i], id));
+            r = fminf(fmaxf(r, -128.0f), 127.0f);
+            q[i] = (int)r;
+        }
+    }
+    const float dh = __half2float(__float2half_rn(d));
+    *reinterpret_cast<uint4 *>(sm + lane * kPitch + warp * 16) = pack_q8(q);
+    const int b = lane >> 2;
+    if ((lane & 3) == 0) sv[b][warp] = dh;
+    if constexpr (SUM == kFloatSum) {
+        // the f16-rounded sum of the inputs, added in the order of a 32-lane xor butterfly over the block (16, 8, 4, 2, 1)
+        float s[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(e[i], __shfl_xor_sync(0xffffffffu, e[i], 2));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], 1));
+        const float t0 = __fadd_rn(__fadd_rn(s[0], s[4]), __fadd_rn(s[2], s[6])), t1 = __fadd_rn(__fadd_rn(s[1], s[5]), __fadd_rn(s[3], s[7]));
+        if ((lane & 3) == 0) sv[8 + b][warp] = __half2float(__float2half_rn(__fadd_rn(t0, t1)));
+    } else if constexpr (SUM == kIntSum) {      // scale times the sum of the int8 values, per block or per 16
+        int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if constexpr (MINS == 1) s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if constexpr (MINS == 1) { if ((lane & 3) == 0) sv[8 + b][warp] = __fmul_rn(dh, (float)s); }
+        else { if ((lane & 1) == 0) sv[8 + 8 * ((lane >> 1) & 1) + b][warp] = __fmul_rn(dh, (float)s); }
+    }
+    __syncthreads();
+    uint8_t *blob = y + ((size_t)t * tl.tt * nch + (size_t)c * rows) * tok_bytes<MINS>();
+    for (int i = threadIdx.x; i < 32 * 8; i += 256)
+        *reinterpret_cast<uint4 *>(blob + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 16) = *reinterpret_cast<const uint4 *>(sm + (i >> 3) * kPitch + (i & 7) * 16);
+    for (int i = threadIdx.x; i < kVals * 8; i += 256)
+        *reinterpret_cast<float *>(blob + (size_t)rows * 512 + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 4) = sv[i >> 3][i & 7];
+}
+
+// ---- producers: chunk CH = 0..3 covers blocks 2 CH (cells 0-15) and 2 CH + 1 (cells 16-31) -----------------------------
+struct WScale { float d, m0, m1; };
+
+// 32-bit word at byte offset OFF (even) of a row chunk held as 16-byte vectors from vector V0 on
+template <int OFF, int V0, int NV> __device__ __forceinline__ uint32_t word_at(const uint4 (&v)[NV]) {
+    constexpr int w = OFF / 4 - 4 * V0;
+    auto get = [&](int i) -> uint32_t { const uint4 &q = v[i >> 2]; return (i & 3) == 0 ? q.x : (i & 3) == 1 ? q.y : (i & 3) == 2 ? q.z : q.w; };
+    if constexpr (OFF % 4 == 0) return get(w);
+    else return __funnelshift_r(get(w), get(w + 1), 16);
+}
+__device__ __forceinline__ float h16(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xFFFFu))); }
+// pairs (byte 0, byte 2) and (byte 1, byte 3) of a word of small unsigned codes, minus `off`, as f16
+__device__ __forceinline__ void codes4(uint32_t w, float off, uint32_t &a, uint32_t &b) {
+    const __half2 o = __float2half2_rn(1024.0f + off);
+    a = h2_bits(__hsub2(bits_h2((w & 0x00FF00FFu) | 0x64006400u), o));
+    b = h2_bits(__hsub2(bits_h2(((w >> 8) & 0x00FF00FFu) | 0x64006400u), o));
+}
+
+template <int WTYPE> struct Expand;
+
+// the 32-element block formats: their chunk is a whole number of 16-byte vectors
+template <int WTYPE> struct ExpandBlock {
+    static constexpr int kBlk = cq_type_size(WTYPE);
+    static constexpr bool kHasM = WTYPE == CQ_Q4_1 || WTYPE == CQ_Q5_1, kFive = WTYPE == CQ_Q5_0 || WTYPE == CQ_Q5_1;
+    const uint8_t *p;
+    __device__ __forceinline__ void header(const uint8_t *rr, int) { p = rr; }
+    template <int B, int V0, int NV> __device__ __forceinline__ WScale block(const uint4 (&v)[NV], uint32_t *o) const {
+        constexpr int off = B * kBlk, qs = off + 2 + (kHasM ? 2 : 0) + (kFive ? 4 : 0);
+        WScale s;
+        s.d = h16(word_at<off, V0>(v));
+        s.m1 = 0.0f;
+        s.m0 = kHasM ? h16(word_at<off + 2, V0>(v)) : __fmul_rn(-16.0f, s.d);      // Q5_0: the codes stay unsigned, -16 d s
+        if constexpr (WTYPE == CQ_Q8_0) {
+            auto four = [&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const uint32_t w = word_at<qs + 4 * i, V0>(v);
+                const __half2 c = __float2half2_rn(1152.0f);        // int8 + 128 in the mantissa of 1024
+                o[2 * i] = h2_bits(__hsub2(bits_h2((w & 0x00FF00FFu) ^ 0x64806480u), c));
+                o[2 * i + 1] = h2_bits(__hsub2(bits_h2(((w >> 8) & 0x00FF00FFu) ^ 0x64806480u), c));
+            };
+            four(std::integral_constant<int, 0>{}); four(std::integral_constant<int, 1>{}); four(std::integral_constant<int, 2>{});
+            four(std::integral_constant<int, 3>{}); four(std::integral_constant<int, 4>{}); four(std::integral_constant<int, 5>{});
+            four(std::integral_constant<int, 6>{}); four(std::integral_constant<int, 7>{});
+        } else {
+            uint32_t qh = 0;
+            if constexpr (kFive) qh = word_at<qs - 4, V0>(v);
+            auto four = [&](auto ic) {          // elements 4 i .. and 16 + 4 i ..
+                constexpr int i = decltype(ic)::value;
+                const uint32_t w = word_at<qs + 4 * i, V0>(v);
+                uint32_t lo = w & 0x0F0F0F0Fu, hi = (w >> 4) & 0x0F0F0F0Fu;
+                if constexpr (kFive) {          // bit e of qh -> bit 4 of element e
+                    lo |= ((((qh >> (4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
+                    hi |= ((((qh >> (16 + 4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
+                }
+                constexpr float minus = WTYPE == CQ_Q4_0 ? 8.0f : 0.0f;
+                codes4(lo, minus, o[2 * i], o[2 * i + 1]);
+                codes4(hi, minus, o[8 + 2 * i], o[8 + 2 * i + 1]);
+            };
+            four(std::integral_constant<int, 0>{}); four(std::integral_constant<int, 1>{});
+            four(std::integral_constant<int, 2>{}); four(std::integral_constant<int, 3>{});
+        }
+        return s;
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
+        constexpr int v0 = 2 * CH * kBlk / 16, nv = (2 * (CH + 1) * kBlk + 15) / 16 - v0;
+        uint4 v[nv + 1];
+#pragma unroll
+        for (int i = 0; i < nv; ++i) v[i] = *reinterpret_cast<const uint4 *>(p + 16 * (v0 + i));
+        v[nv] = make_uint4(0u, 0u, 0u, 0u);       // word_at may name (not use) the word after the last
+        s[0] = block<2 * CH, v0>(v, o);
+        s[1] = block<2 * CH + 1, v0>(v, o + 16);
+    }
+};
+template <> struct Expand<CQ_Q8_0> : ExpandBlock<CQ_Q8_0> {};
+template <> struct Expand<CQ_Q4_0> : ExpandBlock<CQ_Q4_0> {};
+template <> struct Expand<CQ_Q4_1> : ExpandBlock<CQ_Q4_1> {};
+template <> struct Expand<CQ_Q5_0> : ExpandBlock<CQ_Q5_0> {};
+template <> struct Expand<CQ_Q5_1> : ExpandBlock<CQ_Q5_1> {};
+
+// Q5_K: Q4_K with the fifth bits of sub-block g in bit g of 32 bytes; codes times the 6-bit scale, at most 31 * 63 = 1953.
+template <> struct Expand<CQ_Q5_K> {
+    const uint8_t *p;
+    uint32_t sc[2], mn[2], dm;
+    __device__ __forceinline__ void header(const uint8_t *rr, int) {
+        p = rr;
+        const uint4 h = *reinterpret_cast<const uint4 *>(p);
+        dm = h.x;
+        sc[0] = h.y & 0x3F3F3F3Fu; mn[0] = h.z & 0x3F3F3F3Fu;
+        sc[1] = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
+        mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
+        const uint4 a = *reinterpret_cast<const uint4 *>(p + 48 + 32 * CH), b = *reinterpret_cast<const uint4 *>(p + 64 + 32 * CH);
+        const uint4 ha = *reinterpret_cast<const uint4 *>(p + 16), hb = *reinterpret_cast<const uint4 *>(p + 32);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+        auto byte_of = [](const uint32_t (&t)[2], int j) { return (t[j >> 2] >> (8 * (j & 3))) & 0xFFu; };
+        auto twice = [](uint32_t v) { return __hsub2(bits_h2(v * 0x00010001u | 0x64006400u), bits_h2(0x64006400u)); };
+        const __half2 dmh = bits_h2(dm);
+        const float d = __low2float(dmh), dmin = __high2float(dmh);
+        s[0] = WScale{d, -__fmul_rn(dmin, (float)byte_of(mn, 2 * CH)), 0.0f};
+        s[1] = WScale{d, -__fmul_rn(dmin, (float)byte_of(mn, 2 * CH + 1)), 0.0f};
+        const __half2 s0 = twice(byte_of(sc, 2 * CH)), s1 = twice(byte_of(sc, 2 * CH + 1));
+        const __half2 c0 = __hmul2(s0, __float2half2_rn(-1024.0f));
+        const __half2 m1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-64.0f));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+#pragma unroll
+            for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
+                const uint32_t u = od ? w[i] >> 8 : w[i], v = od ? h[i] >> 8 : h[i];
+                const uint32_t lo = (u & 0x000F000Fu) | ((2 * CH >= 4 ? v >> (2 * CH - 4) : v << (4 - 2 * CH)) & 0x00100010u);
+                // high nibbles stay in place, so their codes are 16-fold: the fifth bit goes to bit 8
+                const uint32_t hi = (u & 0x00F000F0u) | ((v << (7 - 2 * CH)) & 0x01000100u);
+                o[2 * i + od] = hfma2_bits(lo | 0x64006400u, s0, c0);
+                o[16 + 2 * i + od] = hfma2_bits(hi | 0x64006400u, m1, c1);
+            }
+        }
+    }
+};
+
+// Q2_K / Q3_K: block b = 4 n + pos: bit pair pos of bytes 32 n .. of the codes; a scale per 16 elements, number 2 b + half.
+template <> struct Expand<CQ_Q2_K> {
+    const uint8_t *p;
+    uint32_t q[8], sc[4];
+    float d, dmin;
+    __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
+        p = rr + shift;         // a multiple of 4 when the base is, else of 2
+        cq_lds_words<4>(p, sc);
+        uint32_t dm[1];
+        cq_lds_words<1>(p + 80, dm);
+        d = h16(dm[0]); dmin = h16(dm[0] >> 16);
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
+        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 16 + 16 * CH, q);
+#pragma unroll
+        for (int bb = 0; bb < 2; ++bb) {
+            const int b = 2 * CH + bb, pos = b & 3;
+            float m[2];
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const uint32_t by = (sc[(2 * b + hf) >> 2] >> (8 * ((2 * b + hf) & 3))) & 0xFFu;
+                m[hf] = -__fmul_rn(dmin, (float)(by >> 4));
+                const __half2 sv = __hsub2(bits_h2((by & 0xFu) * 0x00010001u | 0x64006400u), bits_h2(0x64006400u));
+                const __half2 cv = __hmul2(sv, __float2half2_rn(-1024.0f));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t u = q[4 * hf + i] >> (2 * pos);
+                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits((u & 0x00030003u) | 0x64006400u, sv, cv);
+                    o[16 * bb + 8 * hf + 2 * i + 1] = hfma2_bits(((u >> 8) & 0x00030003u) | 0x64006400u, sv, cv);
+                }
+            }
+            s[bb] = WScale{d, m[0], m[1]};
+        }
+    }
+};
+template <> struct Expand<CQ_Q3_K> {
+    const uint8_t *p;
+    uint32_t q[8], hm[8], sc[3];
+    float d;
+    __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
+        p = rr + shift;         // even
+        cq_lds_words<3>(p + 96, sc);
+        cq_lds_words<8>(p, hm);
+        d = __half2float(*reinterpret_cast<const __half *>(p + 108));
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
+        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 32 + 16 * CH, q);
+#pragma unroll
+        for (int bb = 0; bb < 2; ++bb) {
+            const int b = 2 * CH + bb, pos = b & 3;
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int j = 2 * b + hf;       // scale number: 4 low bits from bytes 0-7, 2 high bits from bytes 8-11
+                const uint32_t lo4 = (sc[(j & 7) >> 2] >> (8 * (j & 3) + (j < 8 ? 0 : 4))) & 0xFu, hi2 = (sc[2] >> (8 * (j & 3) + 2 * (j >> 2))) & 3u;
+                const __half2 sv = __hsub2(bits_h2((lo4 | hi2 << 4) * 0x00010001u | 0x64006400u), __float2half2_rn(1056.0f));
+                const __half2 four = __float2half2_rn(1028.0f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    // two bits, plus 4 when the mask bit is set, minus 4
+                    const uint32_t u = ((q[4 * hf + i] >> (2 * pos)) & 0x03030303u) | (((hm[4 * hf + i] >> b) & 0x01010101u) << 2);
+                    o[16 * bb + 8 * hf + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2((u & 0x00FF00FFu) | 0x64006400u), four), sv));
+                    o[16 * bb + 8 * hf + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(((u >> 8) & 0x00FF00FFu) | 0x64006400u), four), sv));
+                }
+            }
+            s[bb] = WScale{d, 0.0f, 0.0f};
+        }
+    }
+};
+
+struct Args {
+    const uint8_t *w, *act;
+    void *out;
+    int out_kind, nrows, nch, stride_out, use_map, ntiles;
+};
+
+template <int WTYPE>
+__global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
+    using F = Fmt<WTYPE>;
+    using S = Smem<WTYPE>;
+    constexpr int kCB = chunk_bytes<WTYPE>(), kMins = F::kMins, kTok = F::kTok, kStagesT = F::kStagesT, kSlots = 384 / kTok;
+    using R = Raw<kCB>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [2] raw weight bytes landed
+    uint64_t *bar_rawfree = bar_raw + 2;                            // [2] read by all producers
+    uint64_t *bar_fullT = bar_raw + 4;                              // [4] token stage (first half: + scales) landed
+    uint64_t *bar_doneT = bar_raw + 8;                              // [4] its MMAs are complete
+    uint64_t *bar_fullW = bar_raw + 12;                             // [4] operand A chunk stored (all producers)
+    uint64_t *bar_doneW = bar_raw + 16;                             // [4] its MMAs are complete
+    uint64_t *bar_vis = bar_raw + 20;                               // [4] relay: the scales of this operand chunk are visible
+    uint64_t *bar_acc = bar_raw + 24;                               // [6] the MMAs of a block are complete
+    uint64_t *bar_free = bar_raw + 30;                              // [6] accumulator slot read (all epilogue warps)
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 520);
+    uint8_t *stT0 = smem + 1024;
+    uint8_t *aux0 = stT0 + kStagesT * S::kStageT;       // [4] scales [8][n], then sums [kMins][8][n]
+    uint8_t *ringW = aux0 + 4 * S::kAux;                // [4][8 blocks][128 rows] weight scales (and minima)
+    uint8_t *raw0 = ringW + 4 * S::kRingW;              // 128-byte aligned
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nch = a.nch;
+    const uint32_t row_bytes = (uint32_t)nch * kCB;
+    const GroupInfo gi{};
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_raw[i], 1); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < 4; ++i) {
+            cq_mbar_init(&bar_fullT[i], 1);
+            cq_mbar_init(&bar_doneT[i], 1);
+            cq_mbar_init(&bar_fullW[i], kProdWarps);
+            cq_mbar_init(&bar_doneW[i], 1);
+            cq_mbar_init(&bar_vis[i], 1);
+        }
+        for (int i = 0; i < 6; ++i) { cq_mbar_init(&bar_acc[i], 1); cq_mbar_init(&bar_free[i], kEpiWarps); }
+        *abort_flag = 0;
+        cq_fence_mbar_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    cq_pdl_wait();
+
+    if (warp >= kEpiWarps && warp < kMmaWarp) {
+        // ===== producers: thread = weight row = TMEM lane =====
+        const int r = tid - kEpiWarps * 32;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
+        int it = 0, wi = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            long long wr = cx.wrow0 + r;
+            if (wr >= a.nrows) wr = a.nrows - 1;
+            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
+            for (int c = 0; c < nch && alive; ++c, ++it) {
+                const int rs = it & 1;
+                if (!wait_warp(&bar_raw[rs], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                Expand<WTYPE> ex;
+                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
+                uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
+                auto step = [&](auto chc) {
+                    constexpr int CH = decltype(chc)::value;
+                    if (!alive) return;
+                    uint32_t o[32];
+                    WScale s[2];
+                    ex.template chunk<CH>(o, s);
+                    if constexpr (CH == 3) arrive_warp(&bar_rawfree[rs], lane);
+                    const int buf = wi & 3;
+                    if (wi >= 4 && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
+                    tc_fence_after();
+                    // the first operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most kSlots <= 6
+                    // blocks behind them, has finished it - 3: entry it - 4 of the ring is free
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        uint8_t *dst = rw + (2 * CH + b) * kRows * wscale_bytes<kMins>();
+                        if constexpr (kMins == 0) *reinterpret_cast<float *>(dst) = s[b].d;
+                        else if constexpr (kMins == 1) *reinterpret_cast<float2 *>(dst) = make_float2(s[b].d, s[b].m0);
+                        else *reinterpret_cast<float4 *>(dst) = make_float4(s[b].d, s[b].m0, s[b].m1, 0.0f);
+                    }
+                    tmem_st32(ta + buf * 32, o);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    arrive_warp(&bar_fullW[buf], lane);
+                    ++wi;
+                };
+                step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 1>{});
+                step(std::integral_constant<int, 2>{}); step(std::integral_constant<int, 3>{});
+            }
+        }
+    } else if (warp == kLoadWarp) {
+        // ===== loader =====
+        int it = 0, ti = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            const int n = cx.n;
+            const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes<kMins>();
+            for (int c = 0; c < nch && alive; ++c, ++it) {
+                const int rs = it & 1;
+                if (it >= 2 && !wait_or_abort(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                uint8_t *dst = raw0 + rs * R::kBytes;
+                if (a.use_map) {
+                    if (lane == 0) {
+                        cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
+                        cq_tmap::load_2d(dst, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
+                    }
+                } else {
+                    if (lane == 0) cq_mbar_expect_tx(&bar_raw[rs], kRows * R::kNeed);
+                    __syncwarp();
+                    for (int r = lane; r < kRows; r += 32) {
+                        long long wr = cx.wrow0 + r;
+                        if (wr >= a.nrows) wr = a.nrows - 1;
+                        const uintptr_t src = (uintptr_t)(a.w + wr * row_bytes + (uint32_t)c * kCB) & ~(uintptr_t)15;
+                        cq_bulk_g2s(dst + r * R::kPitch, (const void *)src, R::kNeed, &bar_raw[rs]);
+                    }
+                }
+                const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes<kMins>();
+                for (int half = 0; half < 2; ++half, ++ti) {
+                    const int s = ti % kStagesT;
+                    if (ti >= kStagesT && !wait_or_abort(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (lane == 0) {
+                        const unsigned bytes = (unsigned)n * 256;
+                        if (half == 0) {
+                            // a stage of chunk it - 2 (or later) is done: its MMAs had started, so the epilogue has finished it - 4
+                            const unsigned aux_bytes = (unsigned)n * (32 + 32 * kMins);
+                            cq_mbar_expect_tx(&bar_fullT[s], bytes + aux_bytes);
+                            cq_bulk_g2s(aux0 + (it & 3) * S::kAux, blob + (size_t)n * 512, aux_bytes, &bar_fullT[s]);
+                        } else {
+                            cq_mbar_expect_tx(&bar_fullT[s], bytes);
+                        }
+                        cq_bulk_g2s(stT0 + s * S::kStageT, blob + (size_t)half * bytes, bytes, &bar_fullT[s]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
+        if (lane == 0 && (!alive || *abort_flag)) {
+            for (int j = it >= 2 ? it - 1 : 0; j <= it; ++j) (void)cq_mbar_wait_bounded(&bar_raw[j & 1], (j >> 1) & 1);
+            for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j % kStagesT], (j / kStagesT) & 1);
+        }
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        // ===== MMA issuer, one thread: a block = two K = 16 steps into a fresh slot =====
+        if (lane == 0) {
+            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)kColA;
+            int it = 0, wi = 0, s = 0, s_phase = 0, slot = 0, round = 0;      // token stage; accumulator slot and how often all have been used
+            bool alive = true;
+            for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+                TileCtx cx;
+                tile_ctx(tile, tl.ntt, tl, gi, cx);
+                const uint32_t n = (uint32_t)cx.n, idesc = idesc_f16(cx.n), bT = stT | (n << 16);
+                for (int c = 0; c < nch && alive; ++c, ++it) {
+#pragma unroll
+                    for (int ch = 0; ch < 4; ++ch, ++wi) {
+                        const int buf = wi & 3;
+                        if (((ch & 1) == 0 && !wait_or_abort(&bar_fullT[s], s_phase, abort_flag)) ||
+                            !wait_or_abort(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
+                        const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = ta + buf * 32;
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            if (round > 0 && !wait_or_abort(&bar_free[slot], (round - 1) & 1, abort_flag)) { alive = false; break; }
+                            tc_fence_after();
+                            if (b == 0) mbar_arrive(&bar_vis[buf]);     // what this thread has acquired is visible to the epilogue
+                            const uint32_t td = tmem_base + (uint32_t)(slot * kTok);
+                            mma_f16_ts<false>(td, a0 + b * 16, b0 + 4 * b * n, idesc);
+                            mma_f16_ts<true>(td, a0 + b * 16 + 8, b0 + (4 * b + 2) * n, idesc);
+                            tc_commit(&bar_acc[slot]);
+                            if (++slot == kSlots) { slot = 0; ++round; }
+                        }
+                        if (!alive) break;
+                        tc_commit(&bar_doneW[buf]);
+                        if (ch & 1) {
+                            tc_commit(&bar_doneT[s]);
+                            if (++s == kStagesT) { s = 0; s_phase ^= 1; }
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
+        constexpr int kG = kTok / 32;
+        constexpr bool kComp = F::kQ81;
+        const int quad = warp & 3, ch0 = warp >> 2;
+        const int r = quad * 32 + lane;
+        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        const uint64_t minus1 = pack2f(-1.0f, -1.0f), one = pack2f(1.0f, 1.0f);
+        int it = 0, slot = 0, round = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            uint64_t acc[kG][8];                                              // running sums (or those of this chunk)
+            uint64_t sum[kComp ? kG : 1][8], low[kComp ? kG : 1][8];          // compensated sum of the chunks
+#pragma unroll
+            for (int g = 0; g < kG; ++g)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    acc[g][i] = 0ull;
+                    if constexpr (kComp) { sum[g][i] = 0ull; low[g][i] = 0ull; }
+                }
+            for (int c = 0; c < nch && alive; ++c, ++it) {
+                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux);
+                const uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
+                for (int b = 0; b < 8; ++b) {
+                    if (((b & 1) == 0 && !wait_warp(&bar_vis[b >> 1], it & 1, abort_flag)) ||
+                        !wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
+                    tc_fence_after();
+                    const uint8_t *wp = rw + b * kRows * wscale_bytes<kMins>();
+                    float wd, m0 = 0.0f, m1 = 0.0f;
+                    if constexpr (kMins == 0) wd = *reinterpret_cast<const float *>(wp);
+                    else if constexpr (kMins == 1) { const float2 v = *reinterpret_cast<const float2 *>(wp); wd = v.x; m0 = v.y; }
+                    else { const float4 v = *reinterpret_cast<const float4 *>(wp); wd = v.x; m0 = v.y; m1 = v.z; }
+                    const uint64_t dw = pack2f(wd, wd), mm0 = pack2f(m0, m0), mm1 = pack2f(m1, m1);
+#pragma unroll
+                    for (int g = 0; g < kG; ++g) {
+                        const int col = (2 * g + ch0) * 16;
+                        if (col < cx.n) {           // warp-uniform
+                            uint32_t p[16];
+                            tmem_ld16(tlane + (uint32_t)(slot * kTok + col), p);
+                            tmem_ld_wait();
+                            const float *dp = da + b * cx.n + col;
+#pragma unroll
+                            for (int i = 0; i < 8; i += 2) {
+                                const float4 d4 = *reinterpret_cast<const float4 *>(dp + 2 * i);
+                                float4 s4, t4;
+                                if constexpr (kMins >= 1) s4 = *reinterpret_cast<const float4 *>(dp + 8 * cx.n + 2 * i);
+                                if constexpr (kMins >= 2) t4 = *reinterpret_cast<const float4 *>(dp + 16 * cx.n + 2 * i);
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) {
+                                    const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
+                                    const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
+                                    // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel; else d_a (d_w I)
+                                    uint64_t v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
+                                    if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
+                                    if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
+                                    acc[g][i + e] = v;
+                                }
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    arrive_warp(&bar_free[slot], lane);
+                    if (++slot == kSlots) { slot = 0; ++round; }
+                }
+                if constexpr (kComp) {      // sum += acc with the rounding error kept in `low` (two-sum)
+#pragma unroll
+                    for (int g = 0; g < kG; ++g)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const uint64_t x = acc[g][i], s0 = sum[g][i], s1 = fma2(one, x, s0), bb = fma2(minus1, s0, s1);
+                            const uint64_t e0 = fma2(minus1, fma2(minus1, bb, s1), s0), e1 = fma2(minus1, bb, x);
+                            low[g][i] = fma2(one, fma2(one, e0, e1), low[g][i]);
+                            sum[g][i] = s1;
+                            acc[g][i] = 0ull;
+                        }
+                }
+            }
+            if (!alive) break;
+            if (cx.row0 + r < a.nrows) {
+#pragma unroll
+                for (int g = 0; g < kG; ++g) {
+                    const int col = (2 * g + ch0) * 16;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        if (col + i < cx.valid) {
+                            float v;
+                            if constexpr (kComp) {
+                                const float s = (i & 1) ? hi2(sum[g][i >> 1]) : lo2(sum[g][i >> 1]);
+                                const float l = (i & 1) ? hi2(low[g][i >> 1]) : lo2(low[g][i >> 1]);
+                                v = fabsf(s) <= 3.0e38f ? __fadd_rn(s, l) : s;      // an infinite (or NaN) sum has no error term
+                            } else {
+                                v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
+                            }
+                            cq_store_out(a.out, a.out_kind, ((int64_t)cx.t * tl.tt + col + i) * a.stride_out + cx.row0 + r, v);
+                        }
+                    }
+                }
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && *abort_flag) atomicExch(&g_prompt_b32_timeout_flag, 1);
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
+}
+
+template <int WTYPE, typename T>
+void launch_quantize(const void *x, void *scratch, int k, const Tiling &tl, unsigned blocks, cudaStream_t st) {
+    using F = Fmt<WTYPE>;
+    cq_launch_k(quantize_kernel<T, F::kQ81, F::kMins, F::kSum>, dim3(blocks), dim3(256), 0, st, (const T *)x, (uint8_t *)scratch, k, tl);
+}
+
+template <int WTYPE>
+bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, int k, int n, int tokens, int stride_dst, cudaStream_t st) {
+    using F = Fmt<WTYPE>;
+    using R = Raw<chunk_bytes<WTYPE>()>;
+    static_assert(Smem<WTYPE>::kBytes <= 232448, "shared memory of one CTA");
+    static bool attr_done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_done[dev]) {
+        cudaFuncSetAttribute(prompt32_kernel<WTYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<WTYPE>::kBytes);
+        attr_done[dev] = true;
+    }
+    const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
+    // expanding a chunk costs about what the epilogue needs for 40 tokens (8 warps, ~1.25 - 2 instructions per value and block)
+    const Tiling tl = plan_tiling(tokens, nrt, sm_count(), 40, F::kTok);
+    const long long blocks = (long long)tl.ntt * (tl.tt / 8) * nch;
+    if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32: too many tokens for one launch"); return false; }
+    const long long row_bytes = (long long)nch * chunk_bytes<WTYPE>();
+    CUtensorMap map{};
+    const bool use_map = (uintptr_t)w % 16 == 0 && row_bytes % 16 == 0 && row_bytes <= INT32_MAX &&
+                         cq_tmap::weight_map(w, (int)row_bytes, n, R::kPitch / 2, kRows, 2, map);
+    if (!use_map && R::kAligned && (uintptr_t)w % 16 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt32: weights of this format must be 16-byte aligned");
+        return false;
+    }
+    if (elem == CQ_F32) launch_quantize<WTYPE, float>(x, scratch, k, tl, (unsigned)blocks, st);
+    else if (elem == CQ_F16) launch_quantize<WTYPE, __half>(x, scratch, k, tl, (unsigned)blocks, st);
+    else launch_quantize<WTYPE, __nv_bfloat16>(x, scratch, k, tl, (unsigned)blocks, st);
+    const Args a{(const uint8_t *)w, (const uint8_t *)scratch, dst, elem, n, nch, stride_dst, use_map ? 1 : 0, nrt * tl.ntt};
+    const int grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
+    cq_launch_k(prompt32_kernel<WTYPE>, dim3(grid), dim3(kThreads), Smem<WTYPE>::kBytes, st, map, a, tl);
+    return true;
+}
+
+int mins_of(int wtype) {
+    return (wtype == CQ_Q4_1 || wtype == CQ_Q5_0 || wtype == CQ_Q5_1 || wtype == CQ_Q5_K) ? 1 : wtype == CQ_Q2_K ? 2 : 0;
+}
+
+}  // namespace
+
+extern "C" size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k) {
+    if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
+    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)(512 + 32 + 32 * mins_of(wtype)) + 256;
+}
+
+extern "C" void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,
+                                   int tokens, int stride_dst, void *stream) {
+    if (!vx || !x || !scratch || !dst || ncols_x <= 0 || nrows_x <= 0 || tokens <= 0 || ncols_x % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: null pointer, empty shape or K not a multiple of 256");
+        return;
+    }
+    if ((uintptr_t)scratch % 16 != 0 || (uintptr_t)vx % 2 != 0 || elem < CQ_F32 || elem > CQ_BF16) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: misaligned scratch or weights, or unknown element type");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    bool ok = false;
+    switch (wtype) {
+    case CQ_Q4_0: ok = launch<CQ_Q4_0>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q8_0: ok = launch<CQ_Q8_0>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q4_1: ok = launch<CQ_Q4_1>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_0: ok = launch<CQ_Q5_0>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_1: ok = launch<CQ_Q5_1>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q2_K: ok = launch<CQ_Q2_K>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q3_K: ok = launch<CQ_Q3_K>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_K: ok = launch<CQ_Q5_K>(vx, x, elem, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    default: cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32 matmul: Q4_K and Q6_K have their own kernel"); return;
+    }
+    if (ok) cq_check_launch("prompt32 matmul");
+}
+
+extern "C" int cq_prompt32_timeout_flag(void) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_prompt_b32_timeout_flag, sizeof v) != cudaSuccess) { (void)cudaGetLastError(); return -1; }
+    if (v) cq_set_status(CQ_ERR_TIMEOUT, "prompt32 matmul: a bounded wait gave up");
+    return v;
+}

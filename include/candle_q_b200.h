@@ -246,6 +246,14 @@ void cq_prefill32_gemm(int wtype, const void *vx, const void *scratch, void *dst
                        int tokens, int stride_dst, void *stream);
 int cq_prefill32_timeout_flag(void);
 
+/* The prompt product of the formats with an activation scale per 32 elements, as QMatMul::forward runs it: Q8_0 / Q4_0 in the
+ * arithmetic of the pair above, Q4_1 / Q5_0 / Q5_1 / Q2_K / Q3_K / Q5_K in the Q8_1 arithmetic of the decode kernels.  Arguments as
+ * cq_prompt_matmul; weights 16-byte aligned (Q2_K / Q3_K: 2). */
+size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k);
+void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
+                        int stride_dst, void *stream);
+int cq_prompt32_timeout_flag(void);
+
 /* Glue kernels of the decoder harness (f32, fixed order of additions, one launch each).  They stand where candle's
  * quantized models run chains of tensor ops (candle-transformers/src/models/quantized_llama.rs:56-62, 178-262).
  *   cq_attention_f32     : causal attention over an f32 KV cache, one CTA per (sequence, head, query), so that a head

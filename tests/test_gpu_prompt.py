@@ -9,6 +9,7 @@ import pytest
 import torch
 
 from candle_b200 import capi
+from candle_b200.quantized import GgmlDType, QMatMul, QTensor
 from helpers import make_case, rel_err
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,52 @@ def test_prompt_matmul_unaligned_activations(lib, oracle, cuda_dev):
     buf = torch.zeros(40 * 512 + 1, device=cuda_dev)
     buf[1:] = torch.from_numpy(x).to(cuda_dev).view(-1)
     assert torch.equal(_prompt(lib, 12, w_dev, buf[1:].view(40, 512), 512, 70), _prompt(lib, 12, w_dev, buf[1:].clone().view(40, 512), 512, 70))
+
+
+# ---- activation scales per 32 elements ------------------------------------------------------------------------------
+NAMES = {2: "Q4_0", 3: "Q4_1", 6: "Q5_0", 7: "Q5_1", 8: "Q8_0", 10: "Q2K", 11: "Q3K", 13: "Q5K"}
+
+
+def _prompt32(lib, wtype, w_dev, x_dev, k, n):
+    return _run(lib.cq_prompt32_scratch_bytes(wtype, x_dev.shape[0], k), lib.cq_prompt32_matmul, lib.cq_prompt32_timeout_flag, wtype, w_dev,
+                x_dev, k, n)
+
+
+@pytest.mark.parametrize("tokens,k,n", [(1, 256, 1), (9, 512, 65), (64, 256, 128), (65, 768, 129), (128, 1280, 200), (200, 2048, 300),
+                                        (2000, 512, 2050)])
+@pytest.mark.parametrize("wtype", sorted(NAMES))
+def test_prompt32_matmul(lib, oracle, cuda_dev, tokens, k, n, wtype):
+    _, x, wq = make_case(oracle, wtype, k, n, tokens, seed=tokens + k + n)
+    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
+    out = _prompt32(lib, wtype, w_dev, x_dev, k, n)
+    if wtype in (2, 8):     # the int8 kernel's integers and f32 operations in its order: the same bits
+        scratch = torch.zeros(lib.cq_prefill32_scratch_bytes(tokens, k), dtype=torch.uint8, device=cuda_dev)
+        ref, st = torch.empty_like(out), torch.cuda.current_stream().cuda_stream
+        lib.cq_prefill32_quantize(x_dev.data_ptr(), capi.F32, scratch.data_ptr(), k, tokens, st)
+        lib.cq_prefill32_gemm(wtype, w_dev.data_ptr(), scratch.data_ptr(), ref.data_ptr(), capi.F32, k, n, tokens, n, st)
+        capi.check("prefill32")
+        assert torch.equal(out, ref)
+    else:                   # f32 sums in another order
+        pick = np.unique(np.linspace(0, tokens - 1, 64).astype(int))
+        ref = oracle.cuda_mmvq(wtype, wq, oracle.cuda_quantize_q8_1(x[pick]), k, n)
+        assert rel_err(out.cpu().numpy()[pick], ref) <= 2e-6
+
+
+@pytest.mark.parametrize("wtype", [7, 8, 10, 11, 13])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_prompt32_half_types(lib, oracle, cuda_dev, wtype, dtype):
+    """16-bit activations give the f32 result of the same values, rounded once."""
+    _, x, wq = make_case(oracle, wtype, 1024, 130, 77, seed=5)
+    w_dev, xt = torch.from_numpy(wq).to(cuda_dev), torch.from_numpy(x).to(cuda_dev).to(dtype)
+    assert torch.equal(_prompt32(lib, wtype, w_dev, xt, 1024, 130), _prompt32(lib, wtype, w_dev, xt.float(), 1024, 130).to(dtype))
+
+
+@pytest.mark.parametrize("wtype", [3, 10, 13])
+def test_qmatmul_routes_rows_past_one_decode_launch(oracle, cuda_dev, wtype):
+    """Rows 9 and up of the Q8_1 formats go to the prompt kernel: the values of the decode kernel, f32 sums in another order."""
+    _, x, wq = make_case(oracle, wtype, 512, 96, 21, seed=8)
+    mm = QMatMul.from_qtensor(QTensor.from_data(wq, GgmlDType[NAMES[wtype]], (96, 512), cuda_dev))
+    xd = torch.from_numpy(x).to(cuda_dev)
+    y = mm.forward(xd.view(3, 7, 512)).view(21, 96)
+    ref = torch.cat([mm.forward(xd[i:i + 7]) for i in (0, 7, 14)])
+    assert rel_err(y.cpu().numpy(), ref.cpu().numpy()) <= 2e-6
