@@ -27,7 +27,9 @@ constexpr int kTokMax = 128;       // tokens per CTA tile (MMA N), at most
 // The issuing thread is the only one of its warp that runs, every instruction waits for the one before it, and one MMA of N =
 // 128 lasts 64 clocks: some 15 dependent instructions.  So a shared-memory descriptor is kept as its low word - address / 16
 // and, in the upper half, the distance / 16 between the two 16-byte halves of a K step, which for a tile of n tokens is n - and
-// the next K step is one addition of 2 n.
+// the next K step is one addition of 2 n.  What the roles hand each other is kept coarse for the same reason: a wait that has to
+// be woken costs 110 - 190 clocks, a commit 45 to issue and 180 until it is seen (measured), and with a hand-off every four MMAs
+// these alone took 2500 clocks per 256 k-elements, twice what the MMAs of 128 tokens take.
 __device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"((128u >> 4) | (1u << 14)));      // 8-row groups 128 bytes apart; sm_100 descriptor
@@ -72,6 +74,13 @@ __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
 }
+
+// Register budgets per warpgroup (kernels of 640 threads = 96 registers each at launch, 61,440 in all): the two epilogue
+// warpgroups go up to 128, the two producer warpgroups down to 88, the one of the issuing and loading warps to 48:
+// 256 * 128 + 256 * 88 + 128 * 48 = 61,440.
+constexpr int kRegsEpi = 128, kRegsProd = 88, kRegsMisc = 48;
+template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // two f32 operations per instruction; each half rounds like the scalar operation
 __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {

@@ -8,15 +8,17 @@
 // Arithmetic: candle's CPU path.  Activations are BlockQ8K (one f32 scale per 256 values, k_quants.rs:2320-2358, bit-identical
 // int8); a super-block contributes  d_a * (d_w * P - dmin_w * L)  (k_quants.rs:1460-1540, 2035-2092) with the integers
 //      Q4_K:  P = sum (sc_g q) . q8,   |sc_g q| <= 945: one f16 plane;   L = sum_j m_j bsum_j,  |bsum_j| <= 2032, one K = 16 step
-//      Q6_K:  P = sum (sc_j (q - 32)) . q8:  q - 32 = e + b with e even, b the lowest bit of q:  |sc_j e| <= 4096 and even,
-//             |sc_j b| <= 128, both exact in f16; the two planes add into the same accumulator
+//      Q6_K:  P = sum (sc_j (q - 32)) . q8:  q - 32 = n + 16 (b - 2) with the nibble n and the bit pair b:  |sc_j n| <= 1920 and
+//             |sc_j 16 (b - 2)| <= 4096, a multiple of 16, are exact in f16; the two planes add into the same accumulator
 // P is exact below 2^24; above (only reachable when most of the 256 products are near their largest value with one sign) each
 // accumulation step rounds to 24 bits, as the int -> float conversion of an integer accumulator would.  L is always exact.
 //
-// Mapping.  One CTA per SM walks tiles of 128 weight rows x up to 128 tokens.  Warps 0-7 epilogue, 8-11 producers (one
-// weight row per thread), 12 MMA issuer, 13 loader.  Tensor memory, all 512 columns: P in two buffers of 128 (the epilogue
-// of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a super-block, by which time
-// the epilogue has read the previous one), operand A in a ring of four 32-column chunks (64 k-elements of one plane).
+// Mapping.  One CTA per SM walks tiles of 128 weight rows x up to 128 tokens.  Warps 0-7 epilogue, 8-15 producers (two sets of
+// four, a weight row per thread), 16 MMA issuer, 17 loader.  K advances in stages of 64 TMEM columns of operand A = eight MMAs: 128
+// elements of Q4_K, 64 of Q6_K (two planes); the sets take turns.  One barrier says that a stage's operands are there (its
+// producer set and the copied activations), one commit that its MMAs are complete.  Tensor memory, all 512 columns: P in two
+// buffers of 128 (the epilogue of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a
+// super-block, by which time the epilogue has read the previous one), operand A in two (Q4_K) or four stages.
 //
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
@@ -28,25 +30,25 @@
 namespace {
 using namespace cq_prompt;
 
-constexpr int kEpiWarps = 8, kProdWarps = 4;
+constexpr int kEpiWarps = 8, kProdWarps = 8;     // producers: two sets of four
 constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
-constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
+constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two warps only fill their warpgroup
 constexpr int kSlabs = 34;                       // 32 slabs of 8 f16 activations, 2 of f16 run sums (16 bytes per token each)
 constexpr int kTokBytes = kSlabs * 16 + 4;       // + the f32 scale
-constexpr int kStageT = 16 * kTokMax * 16;       // token stage: half a super-block, 32 KiB
-constexpr int kStagesT = 4, kAuxRing = 4;
+constexpr int kRingT = 2 * 32 * kTokMax * 16;    // token stages: two super-blocks, 128 KiB
+constexpr int kAuxRing = 4;
 constexpr int kAux = 2 * kTokMax * 16 + kTokMax * 4;      // run sums, then scales of one super-block
-constexpr int kStagesW = 4;                      // operand A ring in tensor memory, 32 columns each
-constexpr int kColL = 256, kColA = 384;
+constexpr int kColL = 256;
 
 __device__ int g_prompt_kq_timeout_flag = 0;
 
+// kSps: stages per super-block; kNA: stages of operand A; kNT: token stages
 template <int WTYPE> struct Fmt;
-template <> struct Fmt<CQ_Q4_K> { static constexpr int kChunks = 4, kRawStages = 3; static constexpr bool kMins = true; };
-template <> struct Fmt<CQ_Q6_K> { static constexpr int kChunks = 8, kRawStages = 2; static constexpr bool kMins = false; };
+template <> struct Fmt<CQ_Q4_K> { static constexpr int kSps = 2, kNA = 2, kNT = 4, kRawStages = 3, kColA = 384; static constexpr bool kMins = true; };
+template <> struct Fmt<CQ_Q6_K> { static constexpr int kSps = 4, kNA = 4, kNT = 8, kRawStages = 2, kColA = 256; static constexpr bool kMins = false; };
 
 template <int WTYPE> constexpr int smem_bytes() {
-    return 1024 + kStagesT * kStageT + kAuxRing * kAux + 4 * kRows * 8 + 2 * kRows * 32 + Fmt<WTYPE>::kRawStages * Raw<cq_type_size(WTYPE)>::kBytes + 16;
+    return 1024 + kRingT + kAuxRing * kAux + 4 * kRows * 8 + 2 * kRows * 32 + Fmt<WTYPE>::kRawStages * Raw<cq_type_size(WTYPE)>::kBytes + 16;
 }
 
 // ---- activations -> f16 operand tiles -------------------------------------------------------------------------
@@ -60,7 +62,7 @@ template <typename T> struct LoadRows {            // rows of k elements
 // tokens of one super-block and goes through shared memory, so that every slab receives 128 contiguous bytes (stored straight
 // from the warps it would be 16-byte pieces, half a sector each).
 template <typename L>
-__global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__restrict__ y, int nsb, Tiling tl, GroupInfo gi) {
+__global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__restrict__ y, int nsb, int q6k, Tiling tl, GroupInfo gi) {
     constexpr int kPitch = 8 * 16 + 16;
     __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
     __shared__ float sd[8];
@@ -116,7 +118,10 @@ __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__
         }
         d = __fdiv_rn(1.0f, iscale);
     }
-    *reinterpret_cast<uint4 *>(sm + lane * kPitch + warp * 16) = pack_q8(q);
+    // Slab of this lane's 8 elements.  A Q6_K stage holds the two 32-element groups that share their ql bytes: with lane =
+    // 16 h + 4 (p + 2 nib) + j the order is h, p, nib, j.
+    const int slab = q6k ? (lane & 0x13) | ((lane & 4) << 1) | ((lane & 8) >> 1) : lane;
+    *reinterpret_cast<uint4 *>(sm + slab * kPitch + warp * 16) = pack_q8(q);
     int bs = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
     bs += __shfl_xor_sync(0xffffffffu, bs, 1);
     if ((lane & 1) == 0) {              // sum of run j = lane / 2: slab 32 + j / 8, f16 j % 8
@@ -174,10 +179,10 @@ __global__ void __launch_bounds__(1024) group_tiles_kernel(const int32_t *__rest
     if (tid == 0) tiles[4 * max_tiles] = first_tile[num_experts];
 }
 
-// ---- producers: the GGUF bytes of one row -> chunks of 32 TMEM cells ------------------------------------------------
+// ---- producers: the GGUF bytes of one row -> stages of 64 TMEM cells ------------------------------------------------
 template <int WTYPE> struct Expand;
 
-// Q4_K chunk ch: elements 64 ch ..: low nibbles of bytes 32 ch .. +31 (sub-block 2 ch), then the high ones (2 ch + 1).
+// Q4_K, a stage is two chunks; chunk ch: elements 64 ch ..: low nibbles of bytes 32 ch .. +31 (sub-block 2 ch), then the high ones (2 ch + 1).
 // A nibble in the low mantissa bits of 1024.0 (or 16 times it, for high nibbles left in place) becomes sc * q in one fma.
 template <> struct Expand<CQ_Q4_K> {
     const uint8_t *p;
@@ -203,7 +208,11 @@ template <> struct Expand<CQ_Q4_K> {
             *reinterpret_cast<uint4 *>(slab0 + s * kRows * 16) =
                 make_uint4(h2_bits(byte_h2(mn[s], 0)), h2_bits(byte_h2(mn[s], 1)), h2_bits(byte_h2(mn[s], 2)), h2_bits(byte_h2(mn[s], 3)));
     }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) {
+    template <int ST> __device__ __forceinline__ void stage(uint32_t (&o)[2][32]) const {
+        chunk<2 * ST>(o[0]);
+        chunk<2 * ST + 1>(o[1]);
+    }
+    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) const {
         const uint4 a = *reinterpret_cast<const uint4 *>(p + 16 + 32 * CH), b = *reinterpret_cast<const uint4 *>(p + 32 + 32 * CH);
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         const __half2 s0 = byte_h2(sc[CH >> 1], 2 * (CH & 1)), s1 = byte_h2(sc[CH >> 1], 2 * (CH & 1) + 1);
@@ -220,49 +229,47 @@ template <> struct Expand<CQ_Q4_K> {
     }
 };
 
-// Q6_K chunk ch = 4 h + 2 p + nib: elements 128 h + 32 pos + [0, 32), pos = p + 2 nib: nibble `nib` of ql[64 h + 32 p ..], bit pair
-// pos of qh[32 h ..]; cells 0-15 the even part times the scale, 16-31 the lowest bit times the scale.  The even part sits in the
-// mantissa of 64.0 (unit 1/16), so one fma with -96 sc gives sc (e - 32) exactly.
+// Q6_K stage 2 h + p: the two 32-element groups pos = p (low nibbles) and p + 2 (high ones) of ql[64 h + 32 p ..], bit pairs pos of
+// qh[32 h ..]; 16 cells of sc * nibble, then 16 of sc * 16 (bits - 2), per group.  Codes sit in the mantissa of 64.0 (unit 1/16),
+// nibble at bits 4-7, bit pair at 8-9, so one fma with -64 sc or -96 sc gives each part exactly.
 template <> struct Expand<CQ_Q6_K> {
     const uint8_t *p;
-    uint32_t qh[8], ql[8], sc[4];
+    uint32_t sc[4];
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;
         cq_lds_words<4>(p + 192, sc);
     }
     __device__ __forceinline__ float2 scales() const { return make_float2(__half2float(*reinterpret_cast<const __half *>(p + 208)), 0.0f); }
     __device__ __forceinline__ void mins(uint8_t *) const {}
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) {
-        constexpr int h = CH >> 2, pp = (CH >> 1) & 1, nib = CH & 1, pos = pp + 2 * nib;
-        if constexpr ((CH & 3) == 0) cq_lds_words<8>(p + 128 + 32 * h, qh);
-        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 64 * h + 32 * pp, ql);
+    template <int ST> __device__ __forceinline__ void stage(uint32_t (&o)[2][32]) {
+        constexpr int h = ST >> 1, pp = ST & 1;
+        uint32_t ql[8], qh[8];
+        cq_lds_words<8>(p + 64 * h + 32 * pp, ql);
+        cq_lds_words<8>(p + 128 + 32 * h, qh);
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-            constexpr int j0 = 8 * h + 2 * pos;
-            const int scv = (int)(int8_t)(sc[(j0 + hf) >> 2] >> (8 * ((j0 + hf) & 3)));
-            const __half s = __short2half_rn((short)scv);
-            const __half2 s2 = __half2half2(s), c2 = __hmul2(s2, __float2half2_rn(-96.0f));
-            const uint32_t sbits = (uint32_t)__half_as_ushort(s);
+        for (int nib = 0; nib < 2; ++nib) {
+            const int pos = pp + 2 * nib;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i];
+            for (int hf = 0; hf < 2; ++hf) {
+                const int j = 8 * h + 2 * pos + hf;
+                const __half2 s2 = __half2half2(__short2half_rn((short)(int8_t)(sc[j >> 2] >> (8 * (j & 3)))));
+                const __half2 cl = __hmul2(s2, __float2half2_rn(-64.0f)), ch = __hmul2(s2, __float2half2_rn(-96.0f));
 #pragma unroll
-                for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
-                    const uint32_t lv = od ? l >> 8 : l;
-                    const uint32_t lo = (nib ? lv : lv << 4) & 0x00E000E0u;
-                    const int up = 8 - 2 * pos - 8 * od;        // bit pair pos of byte od -> bits 8, 9
-                    const uint32_t hi = (up >= 0 ? b << (up >= 0 ? up : 0) : b >> (up < 0 ? -up : 0)) & 0x03000300u;
-                    o[8 * hf + 2 * i + od] = hfma2_bits(lo | hi | 0x54005400u, s2, c2);
-                    o[16 + 8 * hf + 2 * i + od] = ((nib ? lv >> 4 : lv) & 0x00010001u) * sbits;
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i];
+#pragma unroll
+                    for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
+                        const int dn = 8 * od + (nib ? 0 : -4), up = 8 - 2 * pos - 8 * od;
+                        const uint32_t lv = dn >= 0 ? l >> (dn >= 0 ? dn : 0) : l << (dn < 0 ? -dn : 0);
+                        const uint32_t hv = up >= 0 ? b << (up >= 0 ? up : 0) : b >> (up < 0 ? -up : 0);
+                        o[nib][8 * hf + 2 * i + od] = hfma2_bits((lv & 0x00F000F0u) | 0x54005400u, s2, cl);
+                        o[nib][16 + 8 * hf + 2 * i + od] = hfma2_bits((hv & 0x03000300u) | 0x54005400u, s2, ch);
+                    }
                 }
             }
         }
     }
 };
-// token slab (8 k-elements) at which a chunk starts, inside its half super-block
-template <int WTYPE> __device__ __forceinline__ constexpr int chunk_slab(int ch) {
-    return WTYPE == CQ_Q4_K ? 8 * (ch & 1) : 4 * (((ch >> 1) & 1) + 2 * (ch & 1));
-}
 
 struct Args {
     const uint8_t *w, *w2, *act;        // w2: null, or a second matrix of the same shape for the same activations
@@ -276,21 +283,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2, const Args a, const Tiling tl, const GroupInfo gi) {
     using F = Fmt<WTYPE>;
     using R = Raw<cq_type_size(WTYPE)>;
-    constexpr int kCB = cq_type_size(WTYPE);
+    constexpr int kCB = cq_type_size(WTYPE), kStageT = kRingT / F::kNT;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [3] raw weight bytes landed
-    uint64_t *bar_rawfree = bar_raw + 3;                            // [3] read by all producers
-    uint64_t *bar_fullT = bar_raw + 6;                              // [4] token stage (first half: + run sums and scales) landed
-    uint64_t *bar_doneT = bar_raw + 10;                             // [4] its MMAs are complete
-    uint64_t *bar_fullW = bar_raw + 14;                             // [4] operand A chunk stored (all producers)
-    uint64_t *bar_doneW = bar_raw + 18;                             // [4] its MMAs are complete
-    uint64_t *bar_acc = bar_raw + 22;                               // [2] MMAs of a super-block complete
-    uint64_t *bar_free = bar_raw + 24;                              // [2] accumulators drained (all epilogue warps)
-    uint64_t *bar_vis = bar_raw + 26;                               // [2] relay: the scale rings of this super-block are visible
+    uint64_t *bar_rawfree = bar_raw + 3;                            // [3] read by both producer sets
+    uint64_t *bar_full = bar_raw + 6;                               // [kNT] stage: operand A stored (four warps), activations landed
+    uint64_t *bar_done = bar_raw + 14;                              // [kNT] its MMAs are complete
+    uint64_t *bar_free = bar_raw + 22;                              // [2] accumulators drained (all epilogue warps)
+    uint64_t *bar_vis = bar_raw + 24;                               // [2] relay: the scale rings of this super-block are visible
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 256);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 264);
     uint8_t *stT0 = smem + 1024;
-    uint8_t *aux0 = stT0 + kStagesT * kStageT;
+    uint8_t *aux0 = stT0 + kRingT;
     uint8_t *ringW = aux0 + kAuxRing * kAux;            // (d, dmin) of the rows: [4][128] float2
     uint8_t *mins0 = ringW + 4 * kRows * 8;             // operand A of the sums step: [2][2 slabs][128][16]
     uint8_t *raw0 = mins0 + 2 * kRows * 32;             // 128-byte aligned
@@ -301,17 +305,8 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 
     if (tid == 0) {
         for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], 1); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
-        for (int i = 0; i < 4; ++i) {
-            cq_mbar_init(&bar_fullT[i], 1);
-            cq_mbar_init(&bar_doneT[i], 1);
-            cq_mbar_init(&bar_fullW[i], kProdWarps);
-            cq_mbar_init(&bar_doneW[i], 1);
-        }
-        for (int i = 0; i < 2; ++i) {
-            cq_mbar_init(&bar_acc[i], 1);
-            cq_mbar_init(&bar_free[i], kEpiWarps);
-            cq_mbar_init(&bar_vis[i], 1);
-        }
+        for (int i = 0; i < F::kNT; ++i) { cq_mbar_init(&bar_full[i], 4 + 1); cq_mbar_init(&bar_done[i], 1); }
+        for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_free[i], kEpiWarps); cq_mbar_init(&bar_vis[i], 1); }
         *abort_flag = 0;
         cq_fence_mbar_init();
     }
@@ -328,61 +323,11 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const int ntt = gi.tiles ? gi.tiles[4 * tl.ntt] : tl.ntt;
     const int per_matrix = a.nrt * ntt, ntiles = a.w2 ? 2 * per_matrix : per_matrix;
 
-    if (warp >= kEpiWarps && warp < kMmaWarp) {
-        // ===== producers: thread = weight row = TMEM lane =====
-        const int r = tid - kEpiWarps * 32;
-        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
-        int it = 0, wi = 0, rs = 0, rs_phase = 0;
-        bool alive = true;
-        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
-            TileCtx cx;
-            const bool second = tile >= per_matrix;
-            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
-            long long wr = cx.wrow0 + r;
-            if (wr >= a.total_rows) wr = a.total_rows - 1;
-            // without the tensor map every row has its own distance to the 16-byte boundary below it
-            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes) & 15);
-            for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
-                if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
-                Expand<WTYPE> ex;
-                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
-                const float2 ws = ex.scales();
-                auto step = [&](auto chc) {
-                    constexpr int CH = decltype(chc)::value;
-                    if (!alive) return;
-                    uint32_t o[32];
-                    ex.template chunk<CH>(o);
-                    if constexpr (CH == F::kChunks - 1) arrive_warp(&bar_rawfree[rs], lane);
-                    const int buf = wi & 3;
-                    if (wi >= kStagesW && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
-                    tc_fence_after();
-                    if constexpr (CH == 0) {
-                        // a chunk of super-block it - 1 is done, so its MMAs had started and the epilogue has finished
-                        // it - 3: ring entry it - 4 is free; the sums step of it - 2 is complete too
-                        *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
-                        if constexpr (F::kMins) {
-                            ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
-                            fence_proxy_async_smem();
-                        }
-                    }
-                    tmem_st32(ta + buf * 32, o);
-                    tmem_st_wait();
-                    tc_fence_before();
-                    arrive_warp(&bar_fullW[buf], lane);
-                    ++wi;
-                };
-                step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 1>{});
-                step(std::integral_constant<int, 2>{}); step(std::integral_constant<int, 3>{});
-                if constexpr (F::kChunks == 8) {
-                    step(std::integral_constant<int, 4>{}); step(std::integral_constant<int, 5>{});
-                    step(std::integral_constant<int, 6>{}); step(std::integral_constant<int, 7>{});
-                }
-                if (++rs == F::kRawStages) { rs = 0; rs_phase ^= 1; }
-            }
-        }
-    } else if (warp == kLoadWarp) {
+    if (warp >= kMmaWarp) {
+    regs_down<kRegsMisc>();
+    if (warp == kLoadWarp) {
         // ===== loader: raw weights and activations of up to three / two super-blocks ahead =====
-        int it = 0, ti = 0;
+        int it = 0, h = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
             TileCtx cx;
@@ -410,39 +355,42 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                     }
                 }
                 const uint8_t *blob = blob0 + (size_t)sb * n * kTokBytes;
-                for (int half = 0; half < 2; ++half, ++ti) {
-                    const int s = ti & 3;
-                    if (ti >= kStagesT && !wait_or_abort(&bar_doneT[s], ((ti >> 2) - 1) & 1, abort_flag)) { alive = false; break; }
+                for (int st = 0; st < F::kSps; ++st, ++h) {
+                    const int s = h % F::kNT;
+                    if (h >= F::kNT && !wait_warp(&bar_done[s], (h / F::kNT - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
-                        const unsigned bytes = (unsigned)n * 256;
-                        if (half == 0) {
-                            // done with the stage of (it - 2, first half): its MMAs started after the epilogue of it - 4
+                        const unsigned bytes = (unsigned)n * (512 / F::kSps);
+                        if (st == 0) {
+                            // done with the first stage of it - 2: its MMAs started after the epilogue of it - 4
                             uint8_t *ax = aux0 + (it & 3) * kAux;
                             const unsigned aux_bytes = (unsigned)n * (F::kMins ? 36 : 4);
-                            cq_mbar_expect_tx(&bar_fullT[s], bytes + aux_bytes);
-                            cq_bulk_g2s(ax + (F::kMins ? 0 : n * 32), blob + (size_t)n * (F::kMins ? 512 : 544), aux_bytes, &bar_fullT[s]);
+                            cq_mbar_expect_tx(&bar_full[s], bytes + aux_bytes);
+                            cq_bulk_g2s(ax + (F::kMins ? 0 : n * 32), blob + (size_t)n * (F::kMins ? 512 : 544), aux_bytes, &bar_full[s]);
                         } else {
-                            cq_mbar_expect_tx(&bar_fullT[s], bytes);
+                            cq_mbar_expect_tx(&bar_full[s], bytes);
                         }
-                        cq_bulk_g2s(stT0 + s * kStageT, blob + (size_t)half * bytes, bytes, &bar_fullT[s]);
+                        cq_bulk_g2s(stT0 + s * kStageT, blob + (size_t)st * bytes, bytes, &bar_full[s]);
                     }
                     __syncwarp();
                 }
             }
         }
-        // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
+        // after a give-up the copies of raw bytes must land (or give up themselves) before the shared memory goes away, and those
+        // of activations have a second to (their barrier also waits for producers that may have left)
         if (lane == 0 && (!alive || *abort_flag)) {
             for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; j <= it; ++j)
                 (void)cq_mbar_wait_bounded(&bar_raw[j % F::kRawStages], (j / F::kRawStages) & 1);
-            for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j & 3], (j >> 2) & 1);
+            for (int j = h > F::kNT ? h - F::kNT : 0; j < h; ++j) {
+                if (cq_mbar_wait_bounded(&bar_full[j % F::kNT], (j / F::kNT) & 1)) continue;
+                break;
+            }
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
         // ===== MMA issuer: one thread =====
         if (lane == 0) {
-            constexpr int kHalf = F::kChunks / 2;
-            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)kColA;
-            int it = 0, wi = 0;
+            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)F::kColA;
+            int it = 0;
             bool alive = true;
             for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
                 TileCtx cx;
@@ -452,44 +400,90 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                     const int c = it & 1;
                     const uint32_t tp = tmem_base + (uint32_t)(c * kTokMax);
-                    if (it >= 2 && !wait_or_abort(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                    // the epilogue has read P of it - 2 (Q4_K: known from the wait for L below)
+                    if (!F::kMins && it >= 2 && !wait_or_abort(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int s = (2 * it + half) & 3;
-                        if (!wait_or_abort(&bar_fullT[s], (it >> 1) & 1, abort_flag)) { alive = false; break; }
-                        const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4);
+                    for (int st = 0; st < F::kSps; ++st) {
+                        const int h = it * F::kSps + st, s = h % F::kNT;
+                        if (!wait_or_abort(&bar_full[s], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
+                        tc_fence_after();
+                        if (st == 0) mbar_arrive(&bar_vis[c]);      // relay: what this thread has acquired is visible to the epilogue
+                        const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = ta + (uint32_t)((h % F::kNA) * 64);
 #pragma unroll
-                        for (int ch = 0; ch < kHalf; ++ch, ++wi) {
-                            const int buf = wi & 3;
-                            if (!wait_or_abort(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
+                        for (int j = 0; j < 8; ++j) {
+                            // Q6_K: a group's two planes (two steps each) meet the same 32 activations
+                            const uint32_t b1 = b0 + (uint32_t)(F::kMins ? 2 * j : 4 * (j >> 2) + 2 * (j & 1)) * n;
+                            if (st == 0 && j == 0) mma_f16_ts<false>(tp, a0, b1, idesc);
+                            else mma_f16_ts<true>(tp, a0 + 8 * j, b1, idesc);
+                        }
+                        if (F::kMins && st == F::kSps - 1) {
+                            // L has one buffer: the epilogue of the previous super-block must have read it
+                            if (it >= 1 && !wait_or_abort(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
                             tc_fence_after();
-                            if (half == 0 && ch == 0) mbar_arrive(&bar_vis[c]);     // relay: what this thread has acquired is visible to the epilogue
-                            const uint32_t b1 = b0 + (uint32_t)chunk_slab<WTYPE>(ch) * n, a0 = ta + buf * 32;
-                            if (half == 0 && ch == 0) mma_f16_ts<false>(tp, a0, b1, idesc);
-                            else mma_f16_ts<true>(tp, a0, b1, idesc);
-                            mma_f16_ts<true>(tp, a0 + 8, b1 + 2 * n, idesc);
-                            // Q6_K: both planes of a chunk meet the same 32 activations
-                            mma_f16_ts<true>(tp, a0 + 16, F::kMins ? b1 + 4 * n : b1, idesc);
-                            mma_f16_ts<true>(tp, a0 + 24, F::kMins ? b1 + 6 * n : b1 + 2 * n, idesc);
-                            tc_commit(&bar_doneW[buf]);
+                            mma_f16_ss(tmem_base + (uint32_t)kColL, desc_lo(mins0 + c * kRows * 32, kRows), desc_lo(aux0 + (it & 3) * kAux, n), idesc);
                         }
-                        if (!alive) break;
-                        if constexpr (F::kMins) {
-                            if (half == 1) {
-                                // L has one buffer: the epilogue of the previous super-block must have read it
-                                if (it >= 1 && !wait_or_abort(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
-                                tc_fence_after();
-                                mma_f16_ss(tmem_base + (uint32_t)kColL, desc_lo(mins0 + c * kRows * 32, kRows), desc_lo(aux0 + (it & 3) * kAux, n), idesc);
-                            }
-                        }
-                        tc_commit(&bar_doneT[s]);
+                        tc_commit(&bar_done[s]);
                     }
-                    if (alive) tc_commit(&bar_acc[c]);
                 }
             }
         }
         __syncwarp();
+    }
+    } else if (warp >= kEpiWarps) {
+        regs_down<kRegsProd>();
+        // ===== producers: thread = weight row = TMEM lane; set 0 takes the even stages, set 1 the odd ones =====
+        const int set = (warp - kEpiWarps) >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)F::kColA;
+        int it = 0, rs = 0, rs_phase = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            long long wr = cx.wrow0 + r;
+            if (wr >= a.total_rows) wr = a.total_rows - 1;
+            // without the tensor map every row has its own distance to the 16-byte boundary below it
+            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes) & 15);
+            for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
+                if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
+                Expand<WTYPE> ex;
+                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
+                const float2 ws = ex.scales();
+                auto step = [&](auto stc) {
+                    constexpr int ST = decltype(stc)::value;
+                    if (!alive) return;
+                    uint32_t o[2][32];
+                    ex.template stage<ST>(o);
+                    if constexpr (ST >= F::kSps - 2) arrive_warp(&bar_rawfree[rs], lane);
+                    const int h = it * F::kSps + ST, before = h - F::kNA;       // the stage whose columns are taken over
+                    if (before >= 0 && !wait_warp(&bar_done[before % F::kNT], (before / F::kNT) & 1, abort_flag)) { alive = false; return; }
+                    tc_fence_after();
+                    // a stage of super-block it - 1 is done, so its MMAs had started and the epilogue has finished it - 3: ring entry
+                    // it - 4 is free; the sums step of it - 2 is complete too
+                    if constexpr (ST == 0) *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
+                    if constexpr (F::kMins && ST == 1) {
+                        ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
+                        fence_proxy_async_smem();
+                    }
+                    const uint32_t dst = ta + (uint32_t)((h % F::kNA) * 64);
+                    tmem_st32(dst, o[0]);
+                    tmem_st32(dst + 32, o[1]);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    arrive_warp(&bar_full[h % F::kNT], lane);
+                };
+                if (set == 0) {
+                    step(std::integral_constant<int, 0>{});
+                    if constexpr (F::kSps == 4) step(std::integral_constant<int, 2>{});
+                } else {
+                    step(std::integral_constant<int, 1>{});
+                    if constexpr (F::kSps == 4) step(std::integral_constant<int, 3>{});
+                }
+                if (++rs == F::kRawStages) { rs = 0; rs_phase ^= 1; }
+            }
+        }
     } else {
+        regs_up<kRegsEpi>();
         // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
         const int quad = warp & 3, ch0 = warp >> 2;
         const int r = quad * 32 + lane;
@@ -507,8 +501,10 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 for (int i = 0; i < 8; ++i) acc[g][i] = 0ull;
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int c = it & 1;
+                // the last stage of the super-block is done; its barrier cannot come round again before this epilogue is through
+                const int h = it * F::kSps + F::kSps - 1;
                 if (!wait_warp(&bar_vis[c], (it >> 1) & 1, abort_flag) ||
-                    !wait_warp(&bar_acc[c], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                    !wait_warp(&bar_done[h % F::kNT], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
                 tc_fence_after();
                 const float2 ws = *reinterpret_cast<const float2 *>(ringW + (it & 3) * kRows * 8 + r * 8);
                 const uint64_t dw = pack2f(ws.x, ws.x), ndm = pack2f(-ws.y, -ws.y);
@@ -600,16 +596,16 @@ bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k,
     return true;
 }
 
-template <typename L> bool launch_quantize(const L &load, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
+template <typename L> bool launch_quantize(int wtype, const L &load, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
     const long long blocks = (long long)tl.ntt * (tl.tt / 8) * (k / 256);
     if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt quantize: too many tokens for one launch"); return false; }
-    cq_launch_k(quantize_kernel<L>, dim3((unsigned)blocks), dim3(256), 0, st, load, (uint8_t *)scratch, k / 256, tl, gi);
+    cq_launch_k(quantize_kernel<L>, dim3((unsigned)blocks), dim3(256), 0, st, load, (uint8_t *)scratch, k / 256, wtype == CQ_Q6_K ? 1 : 0, tl, gi);
     return true;
 }
-bool launch_quantize_rows(const void *x, int x_elem, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
-    if (x_elem == CQ_F32) return launch_quantize(LoadRows<float>{(const float *)x, k}, scratch, k, tl, gi, st);
-    if (x_elem == CQ_F16) return launch_quantize(LoadRows<__half>{(const __half *)x, k}, scratch, k, tl, gi, st);
-    if (x_elem == CQ_BF16) return launch_quantize(LoadRows<__nv_bfloat16>{(const __nv_bfloat16 *)x, k}, scratch, k, tl, gi, st);
+bool launch_quantize_rows(int wtype, const void *x, int x_elem, void *scratch, int k, const Tiling &tl, const GroupInfo &gi, cudaStream_t st) {
+    if (x_elem == CQ_F32) return launch_quantize(wtype, LoadRows<float>{(const float *)x, k}, scratch, k, tl, gi, st);
+    if (x_elem == CQ_F16) return launch_quantize(wtype, LoadRows<__half>{(const __half *)x, k}, scratch, k, tl, gi, st);
+    if (x_elem == CQ_BF16) return launch_quantize(wtype, LoadRows<__nv_bfloat16>{(const __nv_bfloat16 *)x, k}, scratch, k, tl, gi, st);
     cq_set_status(CQ_ERR_BAD_ARG, "prompt quantize: unknown element type");
     return false;
 }
@@ -646,7 +642,7 @@ extern "C" void cq_prompt_matmul(int wtype, const void *vx, const void *x, int e
     }
     cudaStream_t st = (cudaStream_t)stream;
     const Tiling tl = dense_tiling(wtype, tokens, nrows_x);
-    if (!launch_quantize_rows(x, elem, scratch, ncols_x, tl, GroupInfo{}, st)) return;
+    if (!launch_quantize_rows(wtype, x, elem, scratch, ncols_x, tl, GroupInfo{}, st)) return;
     const bool ok = wtype == CQ_Q4_K
                         ? launch_gemm<CQ_Q4_K>(vx, scratch, dst, elem, ncols_x, nrows_x, nrows_x, stride_dst, tl, GroupInfo{}, st)
                         : launch_gemm<CQ_Q6_K>(vx, scratch, dst, elem, ncols_x, nrows_x, nrows_x, stride_dst, tl, GroupInfo{}, st);
@@ -688,7 +684,7 @@ extern "C" void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, c
     group_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
     const GroupInfo gi{tiles, sorted_token_ids, topk_weights, size_n, topk, topk_weights ? 1 : 0};
     const Tiling tl{mt * kTokMax, kTokMax, mt};
-    if (!launch_quantize_rows(input, in_elem, blobs, size_k, tl, gi, st)) return;
+    if (!launch_quantize_rows(wtype, input, in_elem, blobs, size_k, tl, gi, st)) return;
     const long long total = (long long)size_n * num_experts;
     const bool ok = wtype == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st)
                                      : launch_gemm<CQ_Q6_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st);
