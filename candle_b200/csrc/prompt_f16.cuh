@@ -24,12 +24,19 @@ using namespace cq_tc;
 constexpr int kRows = 128;         // weight rows per CTA tile (MMA M = TMEM lanes)
 constexpr int kTokMax = 128;       // tokens per CTA tile (MMA N), at most
 
-// The issuing thread is the only one of its warp that runs, every instruction waits for the one before it, and one MMA of N =
-// 128 lasts 64 clocks: some 15 dependent instructions.  So a shared-memory descriptor is kept as its low word - address / 16
-// and, in the upper half, the distance / 16 between the two 16-byte halves of a K step, which for a tile of n tokens is n - and
-// the next K step is one addition of 2 n.  What the roles hand each other is kept coarse for the same reason: a wait that has to
-// be woken costs 110 - 190 clocks, a commit 45 to issue and 180 until it is seen (measured), and with a hand-off every four MMAs
-// these alone took 2500 clocks per 256 k-elements, twice what the MMAs of 128 tokens take.
+// Issuing.  An MMA takes its descriptors and addresses from uniform registers.  Computed by one diverged thread they sit in vector
+// registers and are moved over one by one, ~115 clocks per MMA (measured: 2300 clocks of issue per 256 k-elements, where the
+// MMAs of 128 tokens last 1090).  So the whole warp runs the issuing loop on values the compiler can keep uniform - loop
+// counters, kernel arguments, constants, and a tile's token count passed through a warp reduction - and one elected lane
+// executes the instruction.  A shared-memory descriptor is kept as its low word: address / 16 and, in the upper half, the
+// distance / 16 between the two 16-byte halves of a K step, which for a tile of n tokens is n; the next K step is 2 n further.
+// Hand-offs are kept coarse: a wait that has to be woken costs 110 - 190 clocks, a commit 45 to issue and 180 until it is seen.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }      // the same in every lane
 __device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"((128u >> 4) | (1u << 14)));      // 8-row groups 128 bytes apart; sm_100 descriptor
@@ -134,6 +141,18 @@ template <typename T> __device__ __forceinline__ void load8(const T *p, bool vec
 __device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
     auto pr = [](int a, int b) { return h2_bits(__halves2half2(__short2half_rn((short)a), __short2half_rn((short)b))); };
     return make_uint4(pr(q[0], q[2]), pr(q[1], q[3]), pr(q[4], q[6]), pr(q[5], q[7]));
+}
+
+// 16 consecutive tokens' values of one weight row; `row(i)` gives the output row, values past `valid` are not stored
+template <typename F> __device__ __forceinline__ void store16(const uint64_t (&v)[8], void *out, int kind, int64_t stride, int col, int valid, F &&row) {
+    auto each = [&](auto put) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (i < valid) put(row(i) * stride + col, (i & 1) ? hi2(v[i >> 1]) : lo2(v[i >> 1]));
+    };
+    if (kind == CQ_F32) each([&](int64_t o, float x) { ((float *)out)[o] = x; });
+    else if (kind == CQ_F16) each([&](int64_t o, float x) { ((__half *)out)[o] = __float2half(x); });
+    else each([&](int64_t o, float x) { ((__nv_bfloat16 *)out)[o] = __float2bfloat16(x); });
 }
 
 // ---- tiles --------------------------------------------------------------------------------------------------

@@ -208,23 +208,26 @@ template <> struct Expand<CQ_Q4_K> {
             *reinterpret_cast<uint4 *>(slab0 + s * kRows * 16) =
                 make_uint4(h2_bits(byte_h2(mn[s], 0)), h2_bits(byte_h2(mn[s], 1)), h2_bits(byte_h2(mn[s], 2)), h2_bits(byte_h2(mn[s], 3)));
     }
-    template <int ST> __device__ __forceinline__ void stage(uint32_t (&o)[2][32]) const {
-        chunk<2 * ST>(o[0]);
-        chunk<2 * ST + 1>(o[1]);
-    }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32]) const {
-        const uint4 a = *reinterpret_cast<const uint4 *>(p + 16 + 32 * CH), b = *reinterpret_cast<const uint4 *>(p + 32 + 32 * CH);
-        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const __half2 s0 = byte_h2(sc[CH >> 1], 2 * (CH & 1)), s1 = byte_h2(sc[CH >> 1], 2 * (CH & 1) + 1);
-        const __half2 c0 = __hmul2(s0, __float2half2_rn(-1024.0f));
-        const __half2 m1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-64.0f));
+    // One copy of the code for both stages (and both producer sets): straight-line code of every stage did not fit the
+    // instruction caches and ran at five clocks per instruction.
+    __device__ __forceinline__ void stage(int st, uint32_t (&o)[2][32]) const {
+        const uint32_t scw = st ? sc[1] : sc[0];
+        const uint8_t *q = p + 16 + 64 * st;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t u = w[i], v = w[i] >> 8;
-            o[2 * i] = hfma2_bits((u & 0x000F000Fu) | 0x64006400u, s0, c0);
-            o[2 * i + 1] = hfma2_bits((v & 0x000F000Fu) | 0x64006400u, s0, c0);
-            o[16 + 2 * i] = hfma2_bits((u & 0x00F000F0u) | 0x64006400u, m1, c1);
-            o[16 + 2 * i + 1] = hfma2_bits((v & 0x00F000F0u) | 0x64006400u, m1, c1);
+        for (int c = 0; c < 2; ++c) {
+            const uint4 a = *reinterpret_cast<const uint4 *>(q + 32 * c), b = *reinterpret_cast<const uint4 *>(q + 16 + 32 * c);
+            const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            const __half2 s0 = byte_h2(scw, 2 * c), s1 = byte_h2(scw, 2 * c + 1);
+            const __half2 c0 = __hmul2(s0, __float2half2_rn(-1024.0f));
+            const __half2 m1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-64.0f));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t u = w[i], v = w[i] >> 8;
+                o[c][2 * i] = hfma2_bits((u & 0x000F000Fu) | 0x64006400u, s0, c0);
+                o[c][2 * i + 1] = hfma2_bits((v & 0x000F000Fu) | 0x64006400u, s0, c0);
+                o[c][16 + 2 * i] = hfma2_bits((u & 0x00F000F0u) | 0x64006400u, m1, c1);
+                o[c][16 + 2 * i + 1] = hfma2_bits((v & 0x00F000F0u) | 0x64006400u, m1, c1);
+            }
         }
     }
 };
@@ -241,25 +244,24 @@ template <> struct Expand<CQ_Q6_K> {
     }
     __device__ __forceinline__ float2 scales() const { return make_float2(__half2float(*reinterpret_cast<const __half *>(p + 208)), 0.0f); }
     __device__ __forceinline__ void mins(uint8_t *) const {}
-    template <int ST> __device__ __forceinline__ void stage(uint32_t (&o)[2][32]) {
-        constexpr int h = ST >> 1, pp = ST & 1;
+    __device__ __forceinline__ void stage(int st, uint32_t (&o)[2][32]) const {
+        const int h = st >> 1, pp = st & 1;
         uint32_t ql[8], qh[8];
         cq_lds_words<8>(p + 64 * h + 32 * pp, ql);
         cq_lds_words<8>(p + 128 + 32 * h, qh);
 #pragma unroll
-        for (int nib = 0; nib < 2; ++nib) {
-            const int pos = pp + 2 * nib;
+        for (int nib = 0; nib < 2; ++nib) {         // pos = pp + 2 nib, scales 8 h + 2 pos + {0, 1}
+            const uint32_t scw = (h ? sc[2 + nib] : sc[nib]) >> (16 * pp);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                const int j = 8 * h + 2 * pos + hf;
-                const __half2 s2 = __half2half2(__short2half_rn((short)(int8_t)(sc[j >> 2] >> (8 * (j & 3)))));
+                const __half2 s2 = __half2half2(__short2half_rn((short)(int8_t)(scw >> (8 * hf))));
                 const __half2 cl = __hmul2(s2, __float2half2_rn(-64.0f)), ch = __hmul2(s2, __float2half2_rn(-96.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i];
+                    const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i] >> (2 * pp);
 #pragma unroll
                     for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
-                        const int dn = 8 * od + (nib ? 0 : -4), up = 8 - 2 * pos - 8 * od;
+                        const int dn = 8 * od + (nib ? 0 : -4), up = 8 - 4 * nib - 8 * od;
                         const uint32_t lv = dn >= 0 ? l >> (dn >= 0 ? dn : 0) : l << (dn < 0 ? -dn : 0);
                         const uint32_t hv = up >= 0 ? b << (up >= 0 ? up : 0) : b >> (up < 0 ? -up : 0);
                         o[nib][8 * hf + 2 * i + od] = hfma2_bits((lv & 0x00F000F0u) | 0x54005400u, s2, cl);
@@ -387,28 +389,30 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
-        // ===== MMA issuer: one thread =====
-        if (lane == 0) {
-            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)F::kColA;
-            int it = 0;
-            bool alive = true;
-            for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
-                TileCtx cx;
-                const bool second = tile >= per_matrix;
-                tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
-                const uint32_t n = (uint32_t)cx.n, idesc = idesc_f16(cx.n), bT = stT | (n << 16);
-                for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
-                    const int c = it & 1;
-                    const uint32_t tp = tmem_base + (uint32_t)(c * kTokMax);
-                    // the epilogue has read P of it - 2 (Q4_K: known from the wait for L below)
-                    if (!F::kMins && it >= 2 && !wait_or_abort(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+        // ===== MMA issuer: the warp runs the loop, one elected lane issues =====
+        const uint32_t stT = uniform(cq_smem_u32(stT0) >> 4), mins = uniform(cq_smem_u32(mins0) >> 4), aux = uniform(cq_smem_u32(aux0) >> 4);
+        const uint32_t tm = uniform(tmem_base);
+        int it = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            const uint32_t n = uniform((uint32_t)cx.n), idesc = idesc_f16((int)n), bT = stT | (n << 16);
+#pragma unroll 1
+            for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
+                const int c = it & 1;
+                const uint32_t tp = tm + (uint32_t)(c * kTokMax);
+                // the epilogue has read P of it - 2 (Q4_K: known from the wait for L below)
+                if (!F::kMins && it >= 2 && !wait_warp(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
 #pragma unroll
-                    for (int st = 0; st < F::kSps; ++st) {
-                        const int h = it * F::kSps + st, s = h % F::kNT;
-                        if (!wait_or_abort(&bar_full[s], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
-                        tc_fence_after();
-                        if (st == 0) mbar_arrive(&bar_vis[c]);      // relay: what this thread has acquired is visible to the epilogue
-                        const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = ta + (uint32_t)((h % F::kNA) * 64);
+                for (int st = 0; st < F::kSps; ++st) {
+                    const int h = it * F::kSps + st, s = h % F::kNT;
+                    if (!wait_warp(&bar_full[s], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
+                    tc_fence_after();
+                    const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = tm + (uint32_t)(F::kColA + (h % F::kNA) * 64);
+                    if (elect_one()) {
+                        if (st == 0) mbar_arrive(&bar_vis[c]);      // relay: what this warp has acquired is visible to the epilogue
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
                             // Q6_K: a group's two planes (two steps each) meet the same 32 activations
@@ -416,18 +420,20 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                             if (st == 0 && j == 0) mma_f16_ts<false>(tp, a0, b1, idesc);
                             else mma_f16_ts<true>(tp, a0 + 8 * j, b1, idesc);
                         }
-                        if (F::kMins && st == F::kSps - 1) {
-                            // L has one buffer: the epilogue of the previous super-block must have read it
-                            if (it >= 1 && !wait_or_abort(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
-                            tc_fence_after();
-                            mma_f16_ss(tmem_base + (uint32_t)kColL, desc_lo(mins0 + c * kRows * 32, kRows), desc_lo(aux0 + (it & 3) * kAux, n), idesc);
-                        }
-                        tc_commit(&bar_done[s]);
                     }
+                    if (F::kMins && st == F::kSps - 1) {
+                        // L has one buffer: the epilogue of the previous super-block must have read it
+                        if (it >= 1 && !wait_warp(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
+                        tc_fence_after();
+                        if (elect_one())
+                            mma_f16_ss(tm + (uint32_t)kColL, (mins + (uint32_t)c * (kRows * 32 >> 4)) | ((uint32_t)kRows << 16),
+                                       (aux + (uint32_t)(it & 3) * (kAux >> 4)) | (n << 16), idesc);
+                    }
+                    __syncwarp();
+                    if (elect_one()) tc_commit(&bar_done[s]);
                 }
             }
         }
-        __syncwarp();
     }
     } else if (warp >= kEpiWarps) {
         regs_down<kRegsProd>();
@@ -449,19 +455,18 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 Expand<WTYPE> ex;
                 ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
                 const float2 ws = ex.scales();
-                auto step = [&](auto stc) {
-                    constexpr int ST = decltype(stc)::value;
-                    if (!alive) return;
+#pragma unroll 1
+                for (int st = set; st < F::kSps; st += 2) {
                     uint32_t o[2][32];
-                    ex.template stage<ST>(o);
-                    if constexpr (ST >= F::kSps - 2) arrive_warp(&bar_rawfree[rs], lane);
-                    const int h = it * F::kSps + ST, before = h - F::kNA;       // the stage whose columns are taken over
-                    if (before >= 0 && !wait_warp(&bar_done[before % F::kNT], (before / F::kNT) & 1, abort_flag)) { alive = false; return; }
+                    ex.stage(st, o);
+                    if (st >= F::kSps - 2) arrive_warp(&bar_rawfree[rs], lane);
+                    const int h = it * F::kSps + st, before = h - F::kNA;       // the stage whose columns are taken over
+                    if (before >= 0 && !wait_warp(&bar_done[before % F::kNT], (before / F::kNT) & 1, abort_flag)) { alive = false; break; }
                     tc_fence_after();
                     // a stage of super-block it - 1 is done, so its MMAs had started and the epilogue has finished it - 3: ring entry
                     // it - 4 is free; the sums step of it - 2 is complete too
-                    if constexpr (ST == 0) *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
-                    if constexpr (F::kMins && ST == 1) {
+                    if (st == 0) *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
+                    if (F::kMins && st == 1) {
                         ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
                         fence_proxy_async_smem();
                     }
@@ -471,13 +476,6 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                     tmem_st_wait();
                     tc_fence_before();
                     arrive_warp(&bar_full[h % F::kNT], lane);
-                };
-                if (set == 0) {
-                    step(std::integral_constant<int, 0>{});
-                    if constexpr (F::kSps == 4) step(std::integral_constant<int, 2>{});
-                } else {
-                    step(std::integral_constant<int, 1>{});
-                    if constexpr (F::kSps == 4) step(std::integral_constant<int, 3>{});
                 }
                 if (++rs == F::kRawStages) { rs = 0; rs_phase ^= 1; }
             }
@@ -537,20 +535,25 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             }
             if (!alive) break;
             if (cx.row0 + r < a.nrows) {
+                void *out = second ? a.out2 : a.out;
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
-                    const int col = (2 * g + ch0) * 16;
+                    const int col = (2 * g + ch0) * 16, left = cx.valid - col;
+                    if (left <= 0) continue;
+                    if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight (f32)
+                        const int32_t *pairs = gi.sorted_token_ids + cx.job0 + col;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (col + i < cx.valid) {
-                            float v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
-                            int64_t orow = (int64_t)cx.t * tl.tt + col + i;
-                            if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight
-                                orow = gi.sorted_token_ids[cx.job0 + col + i];
-                                if (gi.topk_weights) v = __fmul_rn(v, gi.topk_weights[orow]);
+                        for (int i = 0; i < 16; ++i) {
+                            if (i < left) {
+                                const int pair = pairs[i];
+                                float v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
+                                if (gi.topk_weights) v = __fmul_rn(v, gi.topk_weights[pair]);
+                                ((float *)out)[(int64_t)pair * a.stride_out + cx.row0 + r] = v;
                             }
-                            cq_store_out(second ? a.out2 : a.out, a.out_kind, orow * a.stride_out + cx.row0 + r, v);
                         }
+                    } else {
+                        const int64_t tok = (int64_t)cx.t * tl.tt + col;
+                        store16(acc[g], out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
                     }
                 }
             }
