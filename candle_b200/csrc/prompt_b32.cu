@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes<kMins>();
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 const int rs = it & 1;
-                if (it >= 2 && !wait_or_abort(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                if (it >= 2 && !wait_bar(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
                 uint8_t *dst = raw0 + rs * R::kBytes;
                 if (a.use_map) {
                     if (lane == 0) {
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes<kMins>();
                 for (int half = 0; half < 2; ++half, ++ti) {
                     const int s = ti % kStagesT;
-                    if (ti >= kStagesT && !wait_or_abort(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (ti >= kStagesT && !wait_bar(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         const unsigned bytes = (unsigned)n * 256;
                         if (half == 0) {
@@ -482,12 +482,12 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch, ++wi) {
                         const int buf = wi & 3;
-                        if (((ch & 1) == 0 && !wait_or_abort(&bar_fullT[s], s_phase, abort_flag)) ||
-                            !wait_or_abort(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
+                        if (((ch & 1) == 0 && !wait_bar(&bar_fullT[s], s_phase, abort_flag)) ||
+                            !wait_bar(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
                         const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = ta + buf * 32;
 #pragma unroll
                         for (int b = 0; b < 2; ++b) {
-                            if (round > 0 && !wait_or_abort(&bar_free[slot], (round - 1) & 1, abort_flag)) { alive = false; break; }
+                            if (round > 0 && !wait_bar(&bar_free[slot], (round - 1) & 1, abort_flag)) { alive = false; break; }
                             tc_fence_after();
                             if (b == 0) mbar_arrive(&bar_vis[buf]);     // what this thread has acquired is visible to the epilogue
                             const uint32_t td = tmem_base + (uint32_t)(slot * kTok);

@@ -72,9 +72,29 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// Bounded wait like wait_or_abort, with a hint that lets the hardware suspend the thread until the phase completes (at most about
+// 0.1 ms at a time): fourteen waiting warps that poll took more than half of all issue slots, from the producers above all.
+__device__ __forceinline__ bool try_wait_suspended(uint64_t *bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(cq_smem_u32(bar)), "r"(parity), "r"(100000u) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool wait_slow(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
+    const long long t0 = clock64();
+    while (!try_wait_suspended(bar, parity)) {
+        if (*abort_flag) return false;
+        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1; return false; }
+    }
+    return true;
+}
+__device__ __forceinline__ bool wait_bar(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
+    return try_wait_suspended(bar, parity) || wait_slow(bar, parity, abort_flag);
+}
+
 // A warp that goes on to a warp-wide tcgen05 instruction must decide as one whether its wait gave up.
 __device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag));
 }
 // One arrival per warp: barriers count warps, not threads.
 __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {

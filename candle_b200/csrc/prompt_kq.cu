@@ -339,7 +339,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nsb * kTokBytes;
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                 const int rs = it % F::kRawStages;
-                if (it >= F::kRawStages && !wait_or_abort(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
+                if (it >= F::kRawStages && !wait_bar(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                 uint8_t *dst = raw0 + rs * R::kBytes;
                 if (a.use_map) {
                     if (lane == 0) {
@@ -454,7 +454,13 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
                 Expand<WTYPE> ex;
                 ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
-                const float2 ws = ex.scales();
+                // This set's wait in super-block it - 1 was for a stage of it - 2: its MMAs had started, so the epilogue had finished it - 4
+                // (the ring entry written here), and set 1's was for the last one, with the sums step that read this copy of the minima.
+                if (set == 0) *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ex.scales();
+                else if (F::kMins) {
+                    ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
+                    fence_proxy_async_smem();
+                }
 #pragma unroll 1
                 for (int st = set; st < F::kSps; st += 2) {
                     uint32_t o[2][32];
@@ -463,13 +469,6 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                     const int h = it * F::kSps + st, before = h - F::kNA;       // the stage whose columns are taken over
                     if (before >= 0 && !wait_warp(&bar_done[before % F::kNT], (before / F::kNT) & 1, abort_flag)) { alive = false; break; }
                     tc_fence_after();
-                    // a stage of super-block it - 1 is done, so its MMAs had started and the epilogue has finished it - 3: ring entry
-                    // it - 4 is free; the sums step of it - 2 is complete too
-                    if (st == 0) *reinterpret_cast<float2 *>(ringW + (it & 3) * kRows * 8 + r * 8) = ws;
-                    if (F::kMins && st == 1) {
-                        ex.mins(mins0 + (it & 1) * kRows * 32 + r * 16);
-                        fence_proxy_async_smem();
-                    }
                     const uint32_t dst = ta + (uint32_t)((h % F::kNA) * 64);
                     tmem_st32(dst, o[0]);
                     tmem_st32(dst + 32, o[1]);
