@@ -12,9 +12,9 @@
 // bits).  The Q8_1 formats were summed by the decode kernels' balanced tree until now; a plain chain of K / 32 additions would
 // lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
 //
-// Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 128 (Q8_0 / Q4_0) or 64 tokens (the compensated sums take three
-// registers per value), warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader; tensor memory: 384 columns of
-// accumulator slots, 128 of operand A.  Every wait is bounded as there.
+// Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
+// warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader; tensor memory: three accumulator slots of two blocks (128
+// columns), 128 columns of operand A.  The roles hand over two blocks at a time.  Every wait is bounded as there.
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
 
@@ -34,7 +34,7 @@ __device__ int g_prompt_b32_timeout_flag = 0;
 enum { kNoSum, kFloatSum, kIntSum };
 template <int WTYPE> struct Fmt {       // Q8_0, Q4_0
     static constexpr bool kQ81 = false;
-    static constexpr int kMins = 0, kSum = kNoSum, kTok = 128, kStagesT = 3;
+    static constexpr int kMins = 0, kSum = kNoSum, kTok = 64, kStagesT = 4;
 };
 template <int MINS, int SUM> struct FmtQ81 {
     static constexpr bool kQ81 = true;
@@ -320,7 +320,7 @@ template <int WTYPE>
 __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
     using F = Fmt<WTYPE>;
     using S = Smem<WTYPE>;
-    constexpr int kCB = chunk_bytes<WTYPE>(), kMins = F::kMins, kTok = F::kTok, kStagesT = F::kStagesT, kSlots = 384 / kTok;
+    constexpr int kCB = chunk_bytes<WTYPE>(), kMins = F::kMins, kTok = F::kTok, kStagesT = F::kStagesT, kSlots = 3;
     using R = Raw<kCB>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [2] raw weight bytes landed
@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     uint64_t *bar_fullW = bar_raw + 12;                             // [4] operand A chunk stored (all producers)
     uint64_t *bar_doneW = bar_raw + 16;                             // [4] its MMAs are complete
     uint64_t *bar_vis = bar_raw + 20;                               // [4] relay: the scales of this operand chunk are visible
-    uint64_t *bar_acc = bar_raw + 24;                               // [6] the MMAs of a block are complete
-    uint64_t *bar_free = bar_raw + 30;                              // [6] accumulator slot read (all epilogue warps)
+    uint64_t *bar_acc = bar_raw + 24;                               // [3] the MMAs of two blocks are complete
+    uint64_t *bar_free = bar_raw + 30;                              // [3] accumulator slot read (all epilogue warps)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 520);
     uint8_t *stT0 = smem + 1024;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             cq_mbar_init(&bar_doneW[i], 1);
             cq_mbar_init(&bar_vis[i], 1);
         }
-        for (int i = 0; i < 6; ++i) { cq_mbar_init(&bar_acc[i], 1); cq_mbar_init(&bar_free[i], kEpiWarps); }
+        for (int i = 0; i < kSlots; ++i) { cq_mbar_init(&bar_acc[i], 1); cq_mbar_init(&bar_free[i], kEpiWarps); }
         *abort_flag = 0;
         cq_fence_mbar_init();
     }
@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     const int buf = wi & 3;
                     if (wi >= 4 && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
                     tc_fence_after();
-                    // the first operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most kSlots <= 6
-                    // blocks behind them, has finished it - 3: entry it - 4 of the ring is free
+                    // the first operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most three
+                    // operand chunks behind them, has finished it - 3: entry it - 4 of the ring is free
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         uint8_t *dst = rw + (2 * CH + b) * kRows * wscale_bytes<kMins>();
@@ -469,44 +469,41 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
-        // ===== MMA issuer, one thread: a block = two K = 16 steps into a fresh slot =====
-        if (lane == 0) {
-            const uint32_t stT = cq_smem_u32(stT0) >> 4, ta = tmem_base + (uint32_t)kColA;
-            int it = 0, wi = 0, s = 0, s_phase = 0, slot = 0, round = 0;      // token stage; accumulator slot and how often all have been used
-            bool alive = true;
-            for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
-                TileCtx cx;
-                tile_ctx(tile, tl.ntt, tl, gi, cx);
-                const uint32_t n = (uint32_t)cx.n, idesc = idesc_f16(cx.n), bT = stT | (n << 16);
-                for (int c = 0; c < nch && alive; ++c, ++it) {
+        // ===== MMA issuer (the warp runs the loop, one elected lane issues): a block = two K = 16 steps into fresh columns =====
+        const uint32_t stT = uniform(cq_smem_u32(stT0) >> 4), tm = uniform(tmem_base);
+        int it = 0, wi = 0, s = 0, s_phase = 0, slot = 0, round = 0;      // token stage; accumulator slot and how often all have been used
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            const uint32_t n = uniform((uint32_t)cx.n), idesc = idesc_f16((int)n), bT = stT | (n << 16);
+#pragma unroll 1
+            for (int c = 0; c < nch && alive; ++c, ++it) {
 #pragma unroll
-                    for (int ch = 0; ch < 4; ++ch, ++wi) {
-                        const int buf = wi & 3;
-                        if (((ch & 1) == 0 && !wait_bar(&bar_fullT[s], s_phase, abort_flag)) ||
-                            !wait_bar(&bar_fullW[buf], (wi >> 2) & 1, abort_flag)) { alive = false; break; }
-                        const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = ta + buf * 32;
-#pragma unroll
-                        for (int b = 0; b < 2; ++b) {
-                            if (round > 0 && !wait_bar(&bar_free[slot], (round - 1) & 1, abort_flag)) { alive = false; break; }
-                            tc_fence_after();
-                            if (b == 0) mbar_arrive(&bar_vis[buf]);     // what this thread has acquired is visible to the epilogue
-                            const uint32_t td = tmem_base + (uint32_t)(slot * kTok);
-                            mma_f16_ts<false>(td, a0 + b * 16, b0 + 4 * b * n, idesc);
-                            mma_f16_ts<true>(td, a0 + b * 16 + 8, b0 + (4 * b + 2) * n, idesc);
-                            tc_commit(&bar_acc[slot]);
-                            if (++slot == kSlots) { slot = 0; ++round; }
-                        }
-                        if (!alive) break;
+                for (int ch = 0; ch < 4; ++ch, ++wi) {
+                    const int buf = wi & 3;
+                    if (((ch & 1) == 0 && !wait_warp(&bar_fullT[s], s_phase, abort_flag)) ||
+                        !wait_warp(&bar_fullW[buf], (wi >> 2) & 1, abort_flag) ||
+                        (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag))) { alive = false; break; }
+                    tc_fence_after();
+                    const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = tm + (uint32_t)(kColA + buf * 32);
+                    const uint32_t td = tm + (uint32_t)(slot * 2 * kTok);
+                    if (elect_one()) {
+                        mbar_arrive(&bar_vis[buf]);     // what this warp has acquired is visible to the epilogue
+                        mma_f16_ts<false>(td, a0, b0, idesc);
+                        mma_f16_ts<true>(td, a0 + 8, b0 + 2 * n, idesc);
+                        mma_f16_ts<false>(td + kTok, a0 + 16, b0 + 4 * n, idesc);
+                        mma_f16_ts<true>(td + kTok, a0 + 24, b0 + 6 * n, idesc);
+                        tc_commit(&bar_acc[slot]);
+                        if (ch & 1) tc_commit(&bar_doneT[s]);
                         tc_commit(&bar_doneW[buf]);
-                        if (ch & 1) {
-                            tc_commit(&bar_doneT[s]);
-                            if (++s == kStagesT) { s = 0; s_phase ^= 1; }
-                        }
                     }
+                    __syncwarp();
+                    if (++slot == kSlots) { slot = 0; ++round; }
+                    if ((ch & 1) && ++s == kStagesT) { s = 0; s_phase ^= 1; }
                 }
             }
         }
-        __syncwarp();
     } else {
         // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
         constexpr int kG = kTok / 32;
@@ -532,39 +529,43 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux);
                 const uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
-                for (int b = 0; b < 8; ++b) {
-                    if (((b & 1) == 0 && !wait_warp(&bar_vis[b >> 1], it & 1, abort_flag)) ||
-                        !wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
+#pragma unroll 1
+                for (int ch = 0; ch < 4; ++ch) {
+                    if (!wait_warp(&bar_vis[ch], it & 1, abort_flag) || !wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
                     tc_fence_after();
-                    const uint8_t *wp = rw + b * kRows * wscale_bytes<kMins>();
-                    float wd, m0 = 0.0f, m1 = 0.0f;
-                    if constexpr (kMins == 0) wd = *reinterpret_cast<const float *>(wp);
-                    else if constexpr (kMins == 1) { const float2 v = *reinterpret_cast<const float2 *>(wp); wd = v.x; m0 = v.y; }
-                    else { const float4 v = *reinterpret_cast<const float4 *>(wp); wd = v.x; m0 = v.y; m1 = v.z; }
-                    const uint64_t dw = pack2f(wd, wd), mm0 = pack2f(m0, m0), mm1 = pack2f(m1, m1);
 #pragma unroll
-                    for (int g = 0; g < kG; ++g) {
-                        const int col = (2 * g + ch0) * 16;
-                        if (col < cx.n) {           // warp-uniform
-                            uint32_t p[16];
-                            tmem_ld16(tlane + (uint32_t)(slot * kTok + col), p);
-                            tmem_ld_wait();
-                            const float *dp = da + b * cx.n + col;
+                    for (int bb = 0; bb < 2; ++bb) {
+                        const int b = 2 * ch + bb;
+                        const uint8_t *wp = rw + b * kRows * wscale_bytes<kMins>();
+                        float wd, m0 = 0.0f, m1 = 0.0f;
+                        if constexpr (kMins == 0) wd = *reinterpret_cast<const float *>(wp);
+                        else if constexpr (kMins == 1) { const float2 v = *reinterpret_cast<const float2 *>(wp); wd = v.x; m0 = v.y; }
+                        else { const float4 v = *reinterpret_cast<const float4 *>(wp); wd = v.x; m0 = v.y; m1 = v.z; }
+                        const uint64_t dw = pack2f(wd, wd), mm0 = pack2f(m0, m0), mm1 = pack2f(m1, m1);
 #pragma unroll
-                            for (int i = 0; i < 8; i += 2) {
-                                const float4 d4 = *reinterpret_cast<const float4 *>(dp + 2 * i);
-                                float4 s4, t4;
-                                if constexpr (kMins >= 1) s4 = *reinterpret_cast<const float4 *>(dp + 8 * cx.n + 2 * i);
-                                if constexpr (kMins >= 2) t4 = *reinterpret_cast<const float4 *>(dp + 16 * cx.n + 2 * i);
+                        for (int g = 0; g < kG; ++g) {
+                            const int col = (2 * g + ch0) * 16;
+                            if (col < cx.n) {           // warp-uniform
+                                uint32_t p[16];
+                                tmem_ld16(tlane + (uint32_t)((2 * slot + bb) * kTok + col), p);
+                                tmem_ld_wait();
+                                const float *dp = da + b * cx.n + col;
 #pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
-                                    const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
-                                    // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel; else d_a (d_w I)
-                                    uint64_t v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
-                                    if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
-                                    if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
-                                    acc[g][i + e] = v;
+                                for (int i = 0; i < 8; i += 2) {
+                                    const float4 d4 = *reinterpret_cast<const float4 *>(dp + 2 * i);
+                                    float4 s4, t4;
+                                    if constexpr (kMins >= 1) s4 = *reinterpret_cast<const float4 *>(dp + 8 * cx.n + 2 * i);
+                                    if constexpr (kMins >= 2) t4 = *reinterpret_cast<const float4 *>(dp + 16 * cx.n + 2 * i);
+#pragma unroll
+                                    for (int e = 0; e < 2; ++e) {
+                                        const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
+                                        const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
+                                        // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel; else d_a (d_w I)
+                                        uint64_t v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
+                                        if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
+                                        if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
+                                        acc[g][i + e] = v;
+                                    }
                                 }
                             }
                         }
@@ -590,21 +591,18 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             if (cx.row0 + r < a.nrows) {
 #pragma unroll
                 for (int g = 0; g < kG; ++g) {
-                    const int col = (2 * g + ch0) * 16;
+                    const int col = (2 * g + ch0) * 16, left = cx.valid - col;
+                    if (left <= 0) continue;
+                    if constexpr (kComp) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (col + i < cx.valid) {
-                            float v;
-                            if constexpr (kComp) {
-                                const float s = (i & 1) ? hi2(sum[g][i >> 1]) : lo2(sum[g][i >> 1]);
-                                const float l = (i & 1) ? hi2(low[g][i >> 1]) : lo2(low[g][i >> 1]);
-                                v = fabsf(s) <= 3.0e38f ? __fadd_rn(s, l) : s;      // an infinite (or NaN) sum has no error term
-                            } else {
-                                v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
-                            }
-                            cq_store_out(a.out, a.out_kind, ((int64_t)cx.t * tl.tt + col + i) * a.stride_out + cx.row0 + r, v);
+                        for (int i = 0; i < 8; ++i) {       // an infinite (or NaN) sum has no error term
+                            const float s0 = lo2(sum[g][i]), s1 = hi2(sum[g][i]);
+                            acc[g][i] = pack2f(fabsf(s0) <= 3.0e38f ? __fadd_rn(s0, lo2(low[g][i])) : s0,
+                                               fabsf(s1) <= 3.0e38f ? __fadd_rn(s1, hi2(low[g][i])) : s1);
                         }
                     }
+                    const int64_t tok = (int64_t)cx.t * tl.tt + col;
+                    store16(acc[g], a.out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
                 }
             }
         }
