@@ -428,9 +428,20 @@ bool attention_args_ok(const void *q, const void *k_cache, const void *v_cache, 
 }
 }  // namespace
 
+// From this many queries per sequence on, cq_attention_f32 runs the kernel that reads the context once per 32 queries
+// (attn_prompt.cu, the same bits); with fewer, its CTAs would be mostly empty.
+constexpr int kPromptMinQueries = 17;
+bool cq_attention_prompt_launch(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch, int tq,
+                                int hq, int hkv, int tmax, float scale, int q_stride, cudaStream_t st);
+
 extern "C" void cq_attention_f32(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos,
                                  int batch, int tq, int hq, int hkv, int head_dim, int tmax, float scale, int q_stride, void *stream) {
     if (!attention_args_ok(q, k_cache, v_cache, out, pos, batch, tq, hq, hkv, head_dim, tmax)) return;
+    if (tq >= kPromptMinQueries &&
+        cq_attention_prompt_launch(q, k_cache, v_cache, out, pos, batch, tq, hq, hkv, tmax, scale, q_stride, (cudaStream_t)stream)) {
+        cq_check_launch("attention");
+        return;
+    }
     cq_launch_k(attention_f32_kernel<false>, dim3(hq, tq, batch), dim3(kThreads), (size_t)tmax * sizeof(float), (cudaStream_t)stream, q,
                 k_cache, v_cache, out, pos, tq, hq, hkv, tmax, scale, q_stride, 0);
     cq_check_launch("attention");

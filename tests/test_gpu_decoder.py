@@ -398,3 +398,26 @@ def test_peer_gather_gives_up_when_a_rank_never_arrives(lib, cuda_dev):
         lib.cq_peer_gather_set_limit_clocks(2_000_000_000)
         lib.cq_peer_gather_clear_timeout()
         lib.cq_clear_status()
+
+
+@pytest.mark.parametrize("Tq,pos0,Tmax", [(17, 0, 32), (32, 5, 64), (33, 100, 133), (64, 63, 128), (130, 200, 331), (200, 0, 190), (70, 1060, 1152)])
+def test_prompt_attention_gives_the_bits_of_one_query_at_a_time(lib, cuda_dev, Tq, pos0, Tmax):
+    """Many queries per sequence (32 of them per CTA) against one call per query of the per-query kernel: tiles of 32 queries,
+    128 keys and 32-key blocks at their edges, more than 1024 keys, a cache shorter than the prompt."""
+    torch.manual_seed(Tq)
+    B, Hq, Hkv, D = 2, 6, 2, 128
+    wide = torch.randn(B, Tq, Hq * D + 64, device=cuda_dev)
+    kc, vc = torch.randn(B, Hkv, Tmax, D, device=cuda_dev), torch.randn(B, Hkv, Tmax, D, device=cuda_dev)
+    st, scale = torch.cuda.current_stream().cuda_stream, 1.0 / math.sqrt(D)
+
+    def run(q, pos, out):
+        p = torch.tensor([pos], dtype=torch.int32, device=cuda_dev)
+        lib.cq_attention_f32(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), p.data_ptr(), B, q.shape[1], Hq, Hkv, D, Tmax, scale,
+                             Hq * D + 64, st)
+        capi.check("attention")
+        return out
+
+    out = run(wide, pos0, torch.full((B, Tq, Hq, D), float("nan"), device=cuda_dev))
+    for t in range(0, Tq, 1 if Tq < 80 else 7):
+        one = run(wide[:, t:t + 1].contiguous(), pos0 + t, torch.empty((B, 1, Hq, D), device=cuda_dev))
+        assert torch.equal(out[:, t], one[:, 0]), t
