@@ -102,6 +102,13 @@ def lib() -> C.CDLL:
         L.cq_attention_q8_1.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, C.c_float, i32, i32, vp]
         L.cq_set_pdl.argtypes = [i32]
         L.cq_glue_position_overflow_flag.restype = i32
+        L.cq_moe_sort_pairs.argtypes = [vp, i32, i32, vp, vp, vp]
+        L.cq_moe_block_prompt_scratch_bytes.argtypes = [i32, i32, i32, i32]
+        L.cq_moe_block_prompt_scratch_bytes.restype = C.c_size_t
+        L.cq_moe_block_prompt.argtypes = [i32, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
+        L.cq_moe_block_decode_scratch_bytes.argtypes = [i32, i32, i32, i32]
+        L.cq_moe_block_decode_scratch_bytes.restype = C.c_size_t
+        L.cq_moe_block_decode.argtypes = [i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
         L.cq_moe_route_f32.argtypes = [vp, vp, vp, i32, i32, i32, i32, vp]
         L.cq_moe_router_f32.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
         L.cq_moe_router_f32.restype = None

@@ -30,6 +30,8 @@ struct MoeArgs {
     long long expert_stride;       // bytes between experts
     int stride_col_y, nrows, nchunks, row_bytes, stage_stride;
     int num_experts, topk, indexed, input_dim1;
+    const uint8_t *w2;             // null, or a second set of experts of the same shape for the same jobs (blockIdx.z = 1)
+    float *out2;
 };
 
 struct MoeMap {     // one activation row, one output row
@@ -63,7 +65,8 @@ __global__ void moe_gemv_kernel(const MoeArgs a) {
     }
     if (expert < 0 || expert >= a.num_experts) return;      // whole CTA leaves together: this pair takes no part
     const MoeMap map{a.y + (int64_t)in_row * a.stride_col_y * CQ_Q8_BYTES, (int64_t)out_row * a.nrows, scale};
-    gemv_body<TYPE, ACT, 1, RB>(a.w + (int64_t)expert * a.expert_stride, map, a.out, CQ_F32, a.nchunks, a.nrows, a.row_bytes,
+    const bool second = blockIdx.z != 0;
+    gemv_body<TYPE, ACT, 1, RB>((second ? a.w2 : a.w) + (int64_t)expert * a.expert_stride, map, second ? a.out2 : a.out, CQ_F32, a.nchunks, a.nrows, a.row_bytes,
                                 a.stage_stride, (int)blockIdx.y, (int)gridDim.y, &g_moe_timeout_flag);
 }
 
@@ -92,7 +95,7 @@ template <int TYPE, int ACT> bool launch_moe(MoeArgs a, int K, int N, int jobs, 
     a.expert_stride = (long long)N * row_bytes;
     int gy = p.grid > 65535 ? 65535 : p.grid;
     if (gy < 1) gy = 1;
-    ((MoeKernel)p.k->fn)<<<dim3((unsigned)jobs, (unsigned)gy), p.T, p.smem, st>>>(a);
+    ((MoeKernel)p.k->fn)<<<dim3((unsigned)jobs, (unsigned)gy, a.w2 ? 2u : 1u), p.T, p.smem, st>>>(a);
     return cq_check_launch("moe gemv");
 }
 
@@ -225,6 +228,109 @@ extern "C" void moe_gemm_gguf_prefill(const void *input, const uint8_t *weights,
     }
     moe_ffi(input, input_dtype == 0 ? CQ_F16 : CQ_BF16, weights, sorted_token_ids, expert_ids, topk_weights, output, num_experts,
             topk, size_m, size_n, size_k, gguf_dtype, (cudaStream_t)(uintptr_t)stream);
+}
+
+// ---- a whole expert block for few tokens (candle-transformers/src/fused_moe.rs:233-301) ----
+namespace {
+// Q8_1 containers of up * silu(gate); grid (ceil(f / 1024), rows), 256 threads, four values each (f a multiple of 32)
+__global__ void __launch_bounds__(256) gate_up_q8_1_kernel(const float *__restrict__ gate, const float *__restrict__ up, uint8_t *__restrict__ out,
+                                                           int f, int stride_blocks) {
+    const int i = blockIdx.x * 256 + threadIdx.x;       // four values
+    const bool in = 4 * i < f;
+    float e[4] = {0.f, 0.f, 0.f, 0.f};
+    if (in) {
+        const float4 g = reinterpret_cast<const float4 *>(gate + (size_t)blockIdx.y * f)[i], u = reinterpret_cast<const float4 *>(up + (size_t)blockIdx.y * f)[i];
+        e[0] = __fmul_rn(u.x, __fdiv_rn(g.x, __fadd_rn(1.0f, expf(-g.x))));
+        e[1] = __fmul_rn(u.y, __fdiv_rn(g.y, __fadd_rn(1.0f, expf(-g.y))));
+        e[2] = __fmul_rn(u.z, __fdiv_rn(g.z, __fadd_rn(1.0f, expf(-g.z))));
+        e[3] = __fmul_rn(u.w, __fdiv_rn(g.w, __fadd_rn(1.0f, expf(-g.w))));
+    }
+    cq_q8_1_store_block(e, out + ((size_t)blockIdx.y * stride_blocks + (i >> 3)) * CQ_Q8_BYTES, in);
+}
+
+// Pairs grouped by expert, ascending inside a group (a stable sort by expert).  One CTA per expert: it counts the pairs of lower
+// experts, then collects its own in order - every CTA reads all ids (32 KB for 1024 tokens x 8) instead of a sort's passes.
+__global__ void __launch_bounds__(1024) sort_pairs_kernel(const int32_t *__restrict__ ids, int pairs, int32_t *__restrict__ expert_ids,
+                                                          int32_t *__restrict__ sorted) {
+    __shared__ int warp_cnt[32];
+    const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int below = 0;
+    for (int i = tid; i < pairs; i += 1024) below += ids[i] < e;
+    below = __reduce_add_sync(0xffffffffu, below);
+    if (lane == 0) warp_cnt[warp] = below;
+    __syncthreads();
+    int base = __reduce_add_sync(0xffffffffu, warp_cnt[lane]);
+    for (int i0 = 0; i0 < pairs; i0 += 1024) {
+        const int i = i0 + tid;
+        const bool mine = i < pairs && ids[i] == e;
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+        __syncthreads();                // warp_cnt of the last step has been read
+        if (lane == 0) warp_cnt[warp] = __popc(m);
+        __syncthreads();
+        const int c = warp_cnt[lane];
+        const int before = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0), all = __reduce_add_sync(0xffffffffu, c);
+        if (mine) {
+            const int o = base + before + __popc(m & ((1u << lane) - 1));
+            expert_ids[o] = e;
+            sorted[o] = i;
+        }
+        base += all;
+    }
+}
+}  // namespace
+
+// ids: i32 [pairs], each in [0, num_experts) -> expert_ids ascending and the pair numbers in that order.
+extern "C" void cq_moe_sort_pairs(const int32_t *ids, int pairs, int num_experts, int32_t *expert_ids, int32_t *sorted_token_ids, void *stream) {
+    if (!ids || !expert_ids || !sorted_token_ids || pairs <= 0 || num_experts <= 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe sort: null pointer or empty shape");
+        return;
+    }
+    sort_pairs_kernel<<<num_experts, 1024, 0, (cudaStream_t)stream>>>(ids, pairs, expert_ids, sorted_token_ids);
+    cq_check_launch("moe sort");
+}
+
+// The expert products of a block for few tokens: x f32 [tokens, hidden] is quantized once, gate and up run as one launch (the
+// tasks of cq_indexed_moe_forward), up * silu(gate) is stored as Q8_1 containers, down, then the weighted sum over a token's
+// experts: five launches.  The arithmetic of moe_gemm_gguf; wtype / wtype_down: formats of gate and up / of down.
+extern "C" size_t cq_moe_block_decode_scratch_bytes(int tokens, int topk, int hidden, int ffn) {
+    if (tokens <= 0 || topk <= 0 || hidden <= 0 || ffn <= 0) return 0;
+    const size_t pairs = (size_t)tokens * topk, kh = (hidden + 511) / 512 * 16 * CQ_Q8_BYTES, kf = (ffn + 511) / 512 * 16 * CQ_Q8_BYTES;
+    return (tokens * kh + pairs * kf + 255) / 256 * 256 + pairs * ((size_t)ffn * 8 + (size_t)hidden * 4);
+}
+
+extern "C" void cq_moe_block_decode(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down,
+                                    const int32_t *ids, const float *topk_weights, float *out, void *scratch, int num_experts, int topk,
+                                    int tokens, int hidden, int ffn, void *stream) {
+    if (!x || !gate || !up || !down || !ids || !topk_weights || !out || !scratch || tokens <= 0 || topk <= 0 || num_experts <= 0 ||
+        (int64_t)tokens * topk > 65535 || (uintptr_t)scratch % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe block: null pointer, empty shape, more than 65535 pairs or misaligned scratch");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const int pairs = tokens * topk, kh = (hidden + 511) / 512 * 512, kf = (ffn + 511) / 512 * 512;
+    const size_t q_bytes = ((size_t)tokens * (kh / 32) + (size_t)pairs * (kf / 32)) * CQ_Q8_BYTES;
+    uint8_t *qx = (uint8_t *)scratch, *qa = qx + (size_t)tokens * (kh / 32) * CQ_Q8_BYTES;
+    float *g = (float *)(qx + (q_bytes + 255) / 256 * 256);
+    float *u = g + (size_t)pairs * ffn, *y = u + (size_t)pairs * ffn;
+    if (!check_common(gate, qx, g, wtype, ffn, hidden, pairs, "block") || !check_common(up, qx, u, wtype, ffn, hidden, pairs, "block") ||
+        !check_common(down, qa, y, wtype_down, hidden, ffn, pairs, "block"))
+        return;
+    cq_quantize_act(x, CQ_ELEM_F32, qx, hidden, kh, tokens, CQ_ACT_Q8_1_ENC, st);
+    MoeArgs a{};
+    a.w = (const uint8_t *)gate; a.w2 = (const uint8_t *)up; a.y = qx; a.out = g; a.out2 = u; a.expert_ids = ids;
+    a.stride_col_y = kh / 32; a.num_experts = num_experts; a.topk = topk; a.indexed = 1; a.input_dim1 = 1;
+    bool ok = dispatch(wtype, CQ_ACT_Q8_1, a, hidden, ffn, pairs, st);
+    if (ok) {
+        gate_up_q8_1_kernel<<<dim3((ffn + 1023) / 1024, pairs), 256, 0, st>>>(g, u, qa, ffn, kf / 32);
+        a.w = (const uint8_t *)down; a.w2 = nullptr; a.y = qa; a.out = y; a.out2 = nullptr;
+        a.stride_col_y = kf / 32; a.input_dim1 = topk;
+        ok = dispatch(wtype_down, CQ_ACT_Q8_1, a, ffn, hidden, pairs, st);
+    }
+    if (!ok) {
+        if (cq_last_status() == CQ_OK) cq_set_status(CQ_ERR_UNSUPPORTED, "moe block: shape outside what the kernel covers");
+        return;
+    }
+    cq_moe_weighted_sum_f32(y, topk_weights, out, tokens, topk, hidden, st);
 }
 
 extern "C" int cq_moe_timeout_flag(void) {

@@ -58,6 +58,34 @@ template <typename T> struct LoadRows {            // rows of k elements
     __device__ __forceinline__ void operator()(int64_t row, int col, float (&e)[8]) const { load8(x + row * k + col, ((uintptr_t)x & 15) == 0, e); }
 };
 
+__device__ __forceinline__ float round16(float v, int kind) {
+    return kind == CQ_F16 ? __half2float(__float2half_rn(v)) : __bfloat162float(__float2bfloat16_rn(v));
+}
+// f32 rows rounded to the 16-bit type `kind`
+struct LoadRounded {
+    const float *x;
+    int64_t k;
+    int kind;
+    __device__ __forceinline__ void operator()(int64_t row, int col, float (&e)[8]) const {
+        load8(x + row * k + col, ((uintptr_t)x & 15) == 0, e);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = round16(e[i], kind);
+    }
+};
+// up * silu(gate) of two f32 matrices, rounded to the 16-bit type `kind`: the input of an expert block's down projection
+struct LoadGateUp {
+    const float *gate, *up;
+    int64_t k;
+    int kind;
+    __device__ __forceinline__ void operator()(int64_t row, int col, float (&e)[8]) const {
+        float g[8];
+        load8(gate + row * k + col, true, g);
+        load8(up + row * k + col, true, e);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) e[i] = round16(__fmul_rn(e[i], __fdiv_rn(g[i], __fadd_rn(1.0f, expf(-g[i])))), kind);
+    }
+};
+
 // One warp per (token, super-block): BlockQ8K values (the rules of quantize_act.cu).  A block of 8 warps takes 8 consecutive
 // tokens of one super-block and goes through shared memory, so that every slab receives 128 contiguous bytes (stored straight
 // from the warps it would be 16-byte pieces, half a sector each).
@@ -691,6 +719,52 @@ extern "C" void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, c
     const bool ok = wtype == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st)
                                      : launch_gemm<CQ_Q6_K>(weights, blobs, out, CQ_F32, size_k, size_n, total, size_n, tl, gi, st);
     if (ok) cq_check_launch("moe prefill gemm");
+}
+
+// ---- the expert matmuls of a mixture-of-experts block, many tokens (candle-transformers/src/fused_moe.rs:262-295) ----
+// The three products with what lies between them: x is rounded to `kind` (the reference casts before its prompt kernel) and
+// quantized ONCE for gate and up, which run as one launch; up * silu(gate), rounded to `kind`, is computed while the down
+// projection's operand is quantized.  As three calls of cq_moe_prefill_gemm the same block built the tile table three times and
+// quantized x twice, and moved gate, up and their product through memory four times more.
+extern "C" size_t cq_moe_block_prompt_scratch_bytes(int size_m, int num_experts, int hidden, int ffn) {
+    if (size_m <= 0 || num_experts <= 0 || num_experts > 1024 || hidden <= 0 || ffn <= 0 || hidden % 256 != 0 || ffn % 256 != 0) return 0;
+    return table_bytes(group_max_tiles(size_m, num_experts)) + group_blob_bytes(size_m, num_experts, hidden > ffn ? hidden : ffn) + 256 +
+           (size_t)size_m * ffn * 8;
+}
+
+extern "C" void cq_moe_block_prompt(int wtype, int wtype_down, const float *x, int kind, const void *gate, const void *up, const void *down,
+                                    const int32_t *sorted_token_ids, const int32_t *expert_ids, const float *topk_weights, float *out,
+                                    void *scratch, int num_experts, int topk, int size_m, int hidden, int ffn, void *stream) {
+    if (!x || !gate || !up || !down || !sorted_token_ids || !expert_ids || !topk_weights || !out || !scratch || topk <= 0 ||
+        cq_moe_block_prompt_scratch_bytes(size_m, num_experts, hidden, ffn) == 0 || (kind != CQ_F16 && kind != CQ_BF16)) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe block: null pointer, empty or odd shape, more than 1024 experts, or a rounding type that is not 16-bit");
+        return;
+    }
+    if ((wtype != CQ_Q4_K && wtype != CQ_Q6_K) || (wtype_down != CQ_Q4_K && wtype_down != CQ_Q6_K)) {
+        cq_set_status(CQ_ERR_UNSUPPORTED, "moe block: the tensor-core kernel covers Q4_K and Q6_K");
+        return;
+    }
+    if ((((uintptr_t)gate | (uintptr_t)up | (uintptr_t)down) % 16) != 0 || (uintptr_t)scratch % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe block: misaligned weights or scratch");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const int mt = group_max_tiles(size_m, num_experts);
+    int *tiles = (int *)scratch;
+    uint8_t *blobs = (uint8_t *)scratch + table_bytes(mt);
+    float *g = (float *)(blobs + (group_blob_bytes(size_m, num_experts, hidden > ffn ? hidden : ffn) + 255) / 256 * 256), *u = g + (size_t)size_m * ffn;
+    const Tiling tl{mt * kTokMax, kTokMax, mt};
+    group_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
+    const GroupInfo gu{tiles, sorted_token_ids, nullptr, ffn, topk, 0};
+    if (!launch_quantize(wtype, LoadRounded{x, hidden, kind}, blobs, hidden, tl, gu, st)) return;
+    const long long rows_gu = (long long)ffn * num_experts, rows_d = (long long)hidden * num_experts;
+    bool ok = wtype == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(gate, blobs, g, CQ_F32, hidden, ffn, rows_gu, ffn, tl, gu, st, up, u)
+                               : launch_gemm<CQ_Q6_K>(gate, blobs, g, CQ_F32, hidden, ffn, rows_gu, ffn, tl, gu, st, up, u);
+    const GroupInfo gd{tiles, sorted_token_ids, topk_weights, hidden, topk, 1};
+    if (!ok || !launch_quantize(wtype_down, LoadGateUp{g, u, ffn, kind}, blobs, ffn, tl, gd, st)) return;
+    ok = wtype_down == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(down, blobs, out, CQ_F32, ffn, hidden, rows_d, hidden, tl, gd, st)
+                               : launch_gemm<CQ_Q6_K>(down, blobs, out, CQ_F32, ffn, hidden, rows_d, hidden, tl, gd, st);
+    if (ok) cq_check_launch("moe block");
 }
 
 extern "C" int cq_prompt_timeout_flag(void) {

@@ -15,9 +15,10 @@ from __future__ import annotations
 import torch
 import torch.distributed as dist
 
+from . import capi
 from .capi import CandleQError
-from .moe import moe_gemm_gguf
-from .quantized import QTensor
+from .moe import _CODE, moe_gemm_gguf
+from .quantized import GgmlDType, QTensor
 
 
 def route(router_logits: torch.Tensor, num_experts_per_tok: int, norm_topk_prob: bool):
@@ -55,11 +56,55 @@ class FusedMoeGGUF:
         self.num_experts_per_tok, self.norm_topk_prob, self.prefill_dtype = num_experts_per_tok, norm_topk_prob, prefill_dtype
         self.expert_offset, self.group, self.world = expert_offset, group, world
 
+    def _block(self, x: torch.Tensor, is_prefill: bool) -> torch.Tensor | None:
+        """The block as a few launches of libcandle_q_b200 (all experts local); None: the general path has to run.  The
+        expert products are those of `moe_gemm_gguf` - same kernels, same rule for which of them a prompt takes."""
+        e, ffn, hidden = self.gate_experts.shape
+        tokens, k = x.shape[0], self.num_experts_per_tok
+        gu, down = self.gate_experts.dtype, self.down_experts.dtype
+        if self.world > 1 or self.expert_offset != 0 or e != self.gate.shape[0] or e > 1024 or not 0 < k <= min(32, e) or tokens == 0 or \
+                not x.is_cuda or self.up_experts.dtype != gu or gu not in _CODE or down not in _CODE or x.shape[1] != hidden or \
+                any(w.device != x.device for w in (self.gate_experts, self.up_experts, self.down_experts)):
+            return None
+        pairs, dev, lib = tokens * k, x.device, capi.lib()
+        kind = {torch.float16: capi.F16, torch.bfloat16: capi.BF16}.get(self.prefill_dtype)
+        if is_prefill:
+            need = lib.cq_moe_block_prompt_scratch_bytes(pairs, e, hidden, ffn)
+            if kind is None or need == 0 or pairs < max(64, 4 * e) or {gu, down} - {GgmlDType.Q4K, GgmlDType.Q6K}:
+                return None
+        else:
+            need = lib.cq_moe_block_decode_scratch_bytes(tokens, k, hidden, ffn)
+            if pairs > 65535:
+                return None
+        with torch.cuda.device(dev):
+            st = torch.cuda.current_stream(dev).cuda_stream
+            logits = torch.nn.functional.linear(x, self.gate)
+            ids = torch.empty((3, pairs), dtype=torch.int32, device=dev)        # by token; then experts and pairs, sorted
+            weights = torch.empty((tokens, k), dtype=torch.float32, device=dev)
+            scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+            lib.cq_moe_route_f32(logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, e, k, 1 if self.norm_topk_prob else 0, st)
+            g, u, d = (w.device_ptr() for w in (self.gate_experts, self.up_experts, self.down_experts))
+            if is_prefill:
+                out = torch.empty((pairs, hidden), dtype=torch.float32, device=dev)
+                lib.cq_moe_sort_pairs(ids.data_ptr(), pairs, e, ids[1].data_ptr(), ids[2].data_ptr(), st)
+                lib.cq_moe_block_prompt(int(gu), int(down), x.data_ptr(), kind, g, u, d, ids[2].data_ptr(), ids[1].data_ptr(),
+                                        weights.data_ptr(), out.data_ptr(), scratch.data_ptr(), e, k, pairs, hidden, ffn, st)
+                out = out.view(tokens, k, hidden).sum(dim=1)
+            else:
+                out = torch.empty((tokens, hidden), dtype=torch.float32, device=dev)
+                lib.cq_moe_block_decode(int(gu), int(down), x.data_ptr(), g, u, d, ids.data_ptr(), weights.data_ptr(), out.data_ptr(),
+                                        scratch.data_ptr(), e, k, tokens, hidden, ffn, st)
+        capi.check("moe block")
+        return out
+
     def forward(self, xs: torch.Tensor, is_prefill: bool) -> torch.Tensor:
         batch, seq_len, hidden = xs.shape
         original_dtype = xs.dtype
         x = xs.reshape(-1, hidden).to(torch.float32).contiguous()
         num_tokens, k = x.shape[0], self.num_experts_per_tok
+        out = self._block(x, is_prefill)
+        if out is not None:
+            return out.to(original_dtype).reshape(batch, seq_len, hidden)
         topk_weights, topk_ids = route(torch.nn.functional.linear(x, self.gate), k, self.norm_topk_prob)
         expert_ids, sorted_token_ids = sort_pairs(topk_ids)
         local_ids = expert_ids - self.expert_offset          # ids outside [0, local experts) are skipped by the kernels
