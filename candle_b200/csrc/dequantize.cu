@@ -4,8 +4,10 @@
 // host candle-core/src/quantized/cuda.rs:105-316, `QTensor::dequantize` / `dequantize_f16` / `embedding`,
 // candle-core/src/quantized/mod.rs:689-748) for Q4_0, Q8_0, Q4_K and Q6_K.  Values are those of the CPU `to_float`
 // (k_quants.rs:219-239, 640-656, 1667-1694, 2247-2278) bit for bit: the same f32 operations in the same order, none
-// fused.  The kernel is bound by its output (4 bytes per element against 0.56 - 1.06 read): a warp writes the 256
-// elements of a super-block (or of eight 32-element blocks) as one contiguous kilobyte, 8 consecutive elements per lane.
+// fused.  The kernel is bound by its output (2 or 4 bytes per element against 0.33 - 1.06 read): a warp writes the 256 elements
+// of a super-block (or of eight 32-element blocks) as one contiguous run, 8 consecutive elements per lane, in 16-byte stores.
+// A lane's 8 code bytes come in two or three aligned words (with a load per byte and a store per element, Q4_K 14336 x 4096 to
+// f16 took 100 us, a quarter of the HBM rate).
 #include "../../include/candle_q_b200.h"
 #include "common.cuh"
 
@@ -14,23 +16,37 @@ namespace {
 __device__ __forceinline__ uint8_t ldb(const uint8_t *p) { return *p; }
 __device__ __forceinline__ float ldh(const uint8_t *p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short *>(p))); }
 
+// Eight bytes from a 2-byte aligned address: aligned words, the third only when the run starts in the middle of one (then it
+// ends in the third's first half, so nothing outside the run's own words is touched).
+struct Bytes8 {
+    uint32_t w[2];
+    __device__ __forceinline__ explicit Bytes8(const uint8_t *p) {
+        const uint32_t *a = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
+        w[0] = a[0]; w[1] = a[1];
+        if ((uintptr_t)p & 2) {
+            const uint32_t t = a[2];
+            w[0] = __funnelshift_r(w[0], w[1], 16);
+            w[1] = __funnelshift_r(w[1], t, 16);
+        }
+    }
+    __device__ __forceinline__ int operator[](int i) const { return (int)((w[i >> 2] >> (8 * (i & 3))) & 0xFFu); }
+};
+
 // The 8 values e0..e0+7 (e0 a multiple of 8) of the 256-element unit `u` of a row that starts at `row`.
 template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *row, int64_t u, int e0, float (&v)[8]) {
     if constexpr (TYPE == CQ_Q8_0) {
         const uint8_t *b = row + (u * 8 + e0 / 32) * 34;
         const float d = ldh(b);
+        const Bytes8 q(b + 2 + e0 % 32);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = __fmul_rn((float)(int8_t)ldb(b + 2 + (e0 % 32) + i), d);
+        for (int i = 0; i < 8; ++i) v[i] = __fmul_rn((float)(int8_t)q[i], d);
     } else if constexpr (TYPE == CQ_Q4_0) {
         const uint8_t *b = row + (u * 8 + e0 / 32) * 18;
         const float d = ldh(b);
         const int j0 = e0 % 32;                 // elements j < 16: low nibbles of qs[j]; j >= 16: high nibbles of qs[j - 16]
+        const Bytes8 by(b + 2 + j0 % 16);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int j = j0 + i;
-            const int q = j < 16 ? (ldb(b + 2 + j) & 0xF) : (ldb(b + 2 + j - 16) >> 4);
-            v[i] = __fmul_rn((float)(q - 8), d);
-        }
+        for (int i = 0; i < 8; ++i) v[i] = __fmul_rn((float)((j0 < 16 ? by[i] & 0xF : by[i] >> 4) - 8), d);
     } else if constexpr (TYPE == CQ_Q4_1 || TYPE == CQ_Q5_0 || TYPE == CQ_Q5_1) {
         // k_quants.rs:392-412 (q * d + m), :496-518 ((q - 16) * d), :604-629 (q * d + m); bit e of qh belongs to element e
         constexpr bool FIVE = TYPE != CQ_Q4_1, HAS_M = TYPE != CQ_Q5_0;
@@ -40,10 +56,11 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         uint32_t qh = 0;
         if constexpr (FIVE) qh = (uint32_t)ph[0] | ((uint32_t)ph[1] << 8) | ((uint32_t)ph[2] << 16) | ((uint32_t)ph[3] << 24);
         const int j0 = e0 % 32;
+        const Bytes8 by(pq + j0 % 16);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int j = j0 + i;
-            int q = j < 16 ? (ldb(pq + j) & 0xF) : (ldb(pq + j - 16) >> 4);
+            int q = j0 < 16 ? by[i] & 0xF : by[i] >> 4;
             if constexpr (FIVE) q |= (int)((qh >> j) & 1u) << 4;
             if constexpr (TYPE == CQ_Q5_0) v[i] = __fmul_rn((float)(q - 16), d);
             else v[i] = __fadd_rn(__fmul_rn((float)q, d), m);
@@ -57,7 +74,7 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         if (sub < 4) { sc = s[sub] & 63; mn = s[sub + 4] & 63; }
         else { sc = (s[sub + 4] & 0xF) | ((s[sub - 4] >> 6) << 4); mn = (s[sub + 4] >> 4) | ((s[sub] >> 6) << 4); }
         const float d1 = __fmul_rn(d, (float)sc), m1 = __fmul_rn(dmin, (float)mn);
-        const uint8_t *q = b + 16 + 32 * j + (l0 % 32);
+        const Bytes8 q(b + 16 + 32 * j + (l0 % 32));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int nib = l0 >= 32 ? (q[i] >> 4) : (q[i] & 0xF);
@@ -72,7 +89,7 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         if (sub < 4) { sc = s[sub] & 63; mn = s[sub + 4] & 63; }
         else { sc = (s[sub + 4] & 0xF) | ((s[sub - 4] >> 6) << 4); mn = (s[sub + 4] >> 4) | ((s[sub] >> 6) << 4); }
         const float d1 = __fmul_rn(d, (float)sc), m1 = __fmul_rn(dmin, (float)mn);
-        const uint8_t *q = b + 48 + 32 * (sub / 2) + l0, *qh = b + 16 + l0;
+        const Bytes8 q(b + 48 + 32 * (sub / 2) + l0), qh(b + 16 + l0);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int nib = (sub & 1) ? (q[i] >> 4) : (q[i] & 0xF);
@@ -85,7 +102,7 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         const int n = e0 / 128, pos = (e0 % 128) / 32, l0 = e0 % 32;
         const int sc = ldb(b + 8 * n + 2 * pos + l0 / 16);
         const float dl = __fmul_rn(d, (float)(sc & 0xF)), ml = __fmul_rn(dmin, (float)(sc >> 4));
-        const uint8_t *q = b + 16 + 32 * n + l0;
+        const Bytes8 q(b + 16 + 32 * n + l0);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = __fsub_rn(__fmul_rn(dl, (float)((q[i] >> (2 * pos)) & 3)), ml);
     } else if constexpr (TYPE == CQ_Q3_K) {         // k_quants.rs:1372-1421: d * (scale - 32) * (q - (mask bit ? 0 : 4))
@@ -96,7 +113,7 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         const int lo = j < 8 ? (ldb(b + 96 + j) & 0xF) : (ldb(b + 96 + j - 8) >> 4);
         const int sc = (lo | (((ldb(b + 104 + (j & 3)) >> (2 * (j >> 2))) & 3) << 4)) - 32;
         const float dl = __fmul_rn(d, (float)sc);
-        const uint8_t *q = b + 32 + 32 * n + l0, *hm = b + l0;
+        const Bytes8 q(b + 32 + 32 * n + l0), hm(b + l0);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int val = ((q[i] >> (2 * pos)) & 3) - (((hm[i] >> (4 * n + pos)) & 1) ? 0 : 4);
@@ -106,7 +123,7 @@ template <int TYPE> __device__ __forceinline__ void unit_values(const uint8_t *r
         const uint8_t *b = row + u * 210;
         const float d = ldh(b + 208);
         const int n = e0 / 128, pos = (e0 % 128) / 32, l0 = e0 % 32;       // 128-half, 32-apart position, first l
-        const uint8_t *ql = b + 64 * n + 32 * (pos & 1) + l0, *qh = b + 128 + 32 * n + l0;
+        const Bytes8 ql(b + 64 * n + 32 * (pos & 1) + l0), qh(b + 128 + 32 * n + l0);
         const int8_t sc = (int8_t)ldb(b + 192 + 8 * n + 2 * pos + l0 / 16);
         const float ds = __fmul_rn(d, (float)sc);
 #pragma unroll
@@ -123,6 +140,8 @@ __device__ __forceinline__ void store8(void *out, int kind, int64_t i, const flo
         float4 *o = reinterpret_cast<float4 *>((float *)out + i);
         o[0] = make_float4(v[0], v[1], v[2], v[3]);
         o[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else if (kind != CQ_F32 && n_valid == 8 && ((uintptr_t)out & 15) == 0) {      // i is a multiple of 8
+        cq_store_out8_16bit((uint16_t *)out + i, kind, v);
     } else {
         for (int j = 0; j < n_valid; ++j) cq_store_out(out, kind, i + j, v[j]);
     }

@@ -157,7 +157,12 @@ template <typename T> __device__ __forceinline__ void load8(const T *p, bool vec
         for (int i = 0; i < 8; ++i) e[i] = cq_elem_to_float(p, i);
     }
 }
-// eight small integers as f16 in the operands' K order
+// eight integral floats of at most 2048 as f16 in the operands' K order
+__device__ __forceinline__ uint4 pack_q8(const float (&q)[8]) {
+    return make_uint4(h2_bits(__floats2half2_rn(q[0], q[2])), h2_bits(__floats2half2_rn(q[1], q[3])), h2_bits(__floats2half2_rn(q[4], q[6])),
+                      h2_bits(__floats2half2_rn(q[5], q[7])));
+}
+// eight small integers, the same
 __device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
     auto pr = [](int a, int b) { return h2_bits(__halves2half2(__short2half_rn((short)a), __short2half_rn((short)b))); };
     return make_uint4(pr(q[0], q[2]), pr(q[1], q[3]), pr(q[4], q[6]), pr(q[5], q[7]));

@@ -119,30 +119,28 @@ __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__
 #pragma unroll
     for (int c = 0; c < 8; ++c) e[c] = 0.0f;
     if (src >= 0) load(src, sb * 256 + lane * 8, e);
-    float amax = 0.0f, vmax = 0.0f;
-    int imax = 0x7fffffff;
+    // The largest magnitude by one warp reduction over its bits (fmaxf leaves NaN out, as the comparisons of quantize_act.cu do),
+    // then the first element that has it: the first lane, the first of its eight.  The values stay in f32, where they and their
+    // sums are exact integers: conversions to int and back took a third of this kernel.
+    float m = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-        if (amax < fabsf(e[c])) { amax = fabsf(e[c]); vmax = e[c]; imax = lane * 8 + c; }
+    for (int c = 0; c < 8; ++c) m = fmaxf(m, fabsf(e[c]));
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    float v = 0.0f;
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-        const float oa = __shfl_xor_sync(0xffffffffu, amax, m);
-        const float ov = __shfl_xor_sync(0xffffffffu, vmax, m);
-        const int oi = __shfl_xor_sync(0xffffffffu, imax, m);
-        if (oa > amax || (oa == amax && oi < imax)) { amax = oa; vmax = ov; imax = oi; }
-    }
-    int q[8];
+    for (int c = 7; c >= 0; --c) v = __float_as_uint(fabsf(e[c])) == top ? e[c] : v;
+    const float vmax = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, __float_as_uint(m) == top)) - 1);
+    float q[8];
     float d = 0.0f;
-    if (amax == 0.0f) {
+    if (top == 0u) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) q[c] = 0;
+        for (int c = 0; c < 8; ++c) q[c] = 0.0f;
     } else {
         const float iscale = __fdiv_rn(-127.0f, vmax);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            float r = roundf(__fmul_rn(iscale, e[c]));
-            r = fminf(fmaxf(r, -128.0f), 127.0f);
-            q[c] = (int)r;
+            const float r = roundf(__fmul_rn(iscale, e[c]));
+            q[c] = __fadd_rn(fminf(fmaxf(r, -128.0f), 127.0f), 0.0f);      // + 0: no negative zero
         }
         d = __fdiv_rn(1.0f, iscale);
     }
@@ -150,11 +148,11 @@ __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__
     // 16 h + 4 (p + 2 nib) + j the order is h, p, nib, j.
     const int slab = q6k ? (lane & 0x13) | ((lane & 4) << 1) | ((lane & 8) >> 1) : lane;
     *reinterpret_cast<uint4 *>(sm + slab * kPitch + warp * 16) = pack_q8(q);
-    int bs = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+    float bs = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
     bs += __shfl_xor_sync(0xffffffffu, bs, 1);
     if ((lane & 1) == 0) {              // sum of run j = lane / 2: slab 32 + j / 8, f16 j % 8
         const int j = lane >> 1;
-        *reinterpret_cast<__half *>(sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7)) = __short2half_rn((short)bs);
+        *reinterpret_cast<__half *>(sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7)) = __float2half_rn(bs);
     }
     if (lane == 0) sd[warp] = d;
     __syncthreads();
