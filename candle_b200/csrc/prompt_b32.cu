@@ -13,7 +13,7 @@
 // lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
 //
 // Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
-// warps 0-7 epilogue, 8-15 producers (two sets in turns), 16 MMA issuer, 17 loader; tensor memory: three accumulator slots of two blocks (128
+// warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader; tensor memory: three accumulator slots of two blocks (128
 // columns), 128 columns of operand A.  The roles hand over two blocks at a time.  Every wait is bounded as there.
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
@@ -23,11 +23,9 @@
 namespace {
 using namespace cq_prompt;
 
-constexpr int kEpiWarps = 8, kProdWarps = 8;     // producers: two sets of four
-// register budgets as in prompt_f16.cuh, for a larger epilogue: 256 * 136 + 256 * 80 + 128 * 48 = 61,440
-constexpr int kRegsEpi32 = 136, kRegsProd32 = 80;
+constexpr int kEpiWarps = 8, kProdWarps = 4;
 constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
-constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two warps only fill their warpgroup
+constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
 constexpr int kColA = 384;
 
 __device__ int g_prompt_b32_timeout_flag = 0;
@@ -256,7 +254,7 @@ template <> struct Expand<CQ_Q2_K> {
         d = h16(dm[0]); dmin = h16(dm[0] >> 16);
     }
     template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
-        cq_lds_words<8>(p + 16 + 32 * (CH >> 1), q);
+        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 16 + 16 * CH, q);
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
             const int b = 2 * CH + bb, pos = b & 3;
@@ -289,7 +287,7 @@ template <> struct Expand<CQ_Q3_K> {
         d = __half2float(*reinterpret_cast<const __half *>(p + 108));
     }
     template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
-        cq_lds_words<8>(p + 32 + 32 * (CH >> 1), q);
+        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 32 + 16 * CH, q);
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
             const int b = 2 * CH + bb, pos = b & 3;
@@ -351,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         for (int i = 0; i < 4; ++i) {
             cq_mbar_init(&bar_fullT[i], 1);
             cq_mbar_init(&bar_doneT[i], 1);
-            cq_mbar_init(&bar_fullW[i], 4);
+            cq_mbar_init(&bar_fullW[i], kProdWarps);
             cq_mbar_init(&bar_doneW[i], 1);
             cq_mbar_init(&bar_vis[i], 1);
         }
@@ -369,9 +367,54 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     cq_pdl_wait();
 
-    if (warp >= kMmaWarp) {
-    regs_down<kRegsMisc>();
-    if (warp == kLoadWarp) {
+    if (warp >= kEpiWarps && warp < kMmaWarp) {
+        // ===== producers: thread = weight row = TMEM lane =====
+        const int r = tid - kEpiWarps * 32;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
+        int it = 0, wi = 0;
+        bool alive = true;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            long long wr = cx.wrow0 + r;
+            if (wr >= a.nrows) wr = a.nrows - 1;
+            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
+            for (int c = 0; c < nch && alive; ++c, ++it) {
+                const int rs = it & 1;
+                if (!wait_warp(&bar_raw[rs], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                Expand<WTYPE> ex;
+                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
+                uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
+                auto step = [&](auto chc) {
+                    constexpr int CH = decltype(chc)::value;
+                    if (!alive) return;
+                    uint32_t o[32];
+                    WScale s[2];
+                    ex.template chunk<CH>(o, s);
+                    if constexpr (CH == 3) arrive_warp(&bar_rawfree[rs], lane);
+                    const int buf = wi & 3;
+                    if (wi >= 4 && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
+                    tc_fence_after();
+                    // the first operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most three
+                    // operand chunks behind them, has finished it - 3: entry it - 4 of the ring is free
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        uint8_t *dst = rw + (2 * CH + b) * kRows * wscale_bytes<kMins>();
+                        if constexpr (kMins == 0) *reinterpret_cast<float *>(dst) = s[b].d;
+                        else if constexpr (kMins == 1) *reinterpret_cast<float2 *>(dst) = make_float2(s[b].d, s[b].m0);
+                        else *reinterpret_cast<float4 *>(dst) = make_float4(s[b].d, s[b].m0, s[b].m1, 0.0f);
+                    }
+                    tmem_st32(ta + buf * 32, o);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    arrive_warp(&bar_fullW[buf], lane);
+                    ++wi;
+                };
+                step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 1>{});
+                step(std::integral_constant<int, 2>{}); step(std::integral_constant<int, 3>{});
+            }
+        }
+    } else if (warp == kLoadWarp) {
         // ===== loader =====
         int it = 0, ti = 0;
         bool alive = true;
@@ -461,56 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 }
             }
         }
-    }
-    } else if (warp >= kEpiWarps) {
-        regs_down<kRegsProd32>();
-        // ===== producers: thread = weight row = TMEM lane =====
-        const int set = (warp - kEpiWarps) >> 2, r = (warp & 3) * 32 + lane;      // set 0: operand chunks 0 and 2, set 1: 1 and 3
-        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
-        int it = 0;
-        bool alive = true;
-        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
-            TileCtx cx;
-            tile_ctx(tile, tl.ntt, tl, gi, cx);
-            long long wr = cx.wrow0 + r;
-            if (wr >= a.nrows) wr = a.nrows - 1;
-            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
-            for (int c = 0; c < nch && alive; ++c, ++it) {
-                const int rs = it & 1;
-                if (!wait_warp(&bar_raw[rs], (it >> 1) & 1, abort_flag)) { alive = false; break; }
-                Expand<WTYPE> ex;
-                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
-                uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
-                auto step = [&](auto chc) {
-                    constexpr int CH = decltype(chc)::value;
-                    if (!alive) return;
-                    uint32_t o[32];
-                    WScale s[2];
-                    ex.template chunk<CH>(o, s);
-                    if constexpr (CH >= 2) arrive_warp(&bar_rawfree[rs], lane);
-                    constexpr int buf = CH;
-                    if (it >= 1 && !wait_warp(&bar_doneW[buf], (it - 1) & 1, abort_flag)) { alive = false; return; }
-                    tc_fence_after();
-                    // this operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most three
-                    // operand chunks behind them, has finished it - 3: entry it - 4 of the ring is free
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        uint8_t *dst = rw + (2 * CH + b) * kRows * wscale_bytes<kMins>();
-                        if constexpr (kMins == 0) *reinterpret_cast<float *>(dst) = s[b].d;
-                        else if constexpr (kMins == 1) *reinterpret_cast<float2 *>(dst) = make_float2(s[b].d, s[b].m0);
-                        else *reinterpret_cast<float4 *>(dst) = make_float4(s[b].d, s[b].m0, s[b].m1, 0.0f);
-                    }
-                    tmem_st32(ta + buf * 32, o);
-                    tmem_st_wait();
-                    tc_fence_before();
-                    arrive_warp(&bar_fullW[buf], lane);
-                };
-                if (set == 0) { step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 2>{}); }
-                else { step(std::integral_constant<int, 1>{}); step(std::integral_constant<int, 3>{}); }
-            }
-        }
     } else {
-        regs_up<kRegsEpi32>();
         // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
         constexpr int kG = kTok / 32;
         constexpr bool kComp = F::kQ81;
@@ -595,7 +589,6 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             }
             if (!alive) break;
             if (cx.row0 + r < a.nrows) {
-                const bool pairs = can_pair(a.out, a.stride_out, cx.row0 + quad * 32, a.nrows);
 #pragma unroll
                 for (int g = 0; g < kG; ++g) {
                     const int col = (2 * g + ch0) * 16, left = cx.valid - col;
@@ -609,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         }
                     }
                     const int64_t tok = (int64_t)cx.t * tl.tt + col;
-                    store16(acc[g], a.out, a.out_kind, a.stride_out, cx.row0 + r, left, pairs, [&](int i) { return tok + i; });
+                    store16(acc[g], a.out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
                 }
             }
         }

@@ -168,35 +168,16 @@ __device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
     return make_uint4(pr(q[0], q[2]), pr(q[1], q[3]), pr(q[4], q[6]), pr(q[5], q[7]));
 }
 
-// 16 consecutive tokens' values of one weight row; `row(i)` gives the output row, values past `valid` are not stored.  `pairs`
-// (16-bit outputs; uniform in the warp, which then calls as a whole): stores of two rows at once, half as many.
-template <typename F>
-__device__ __forceinline__ void store16(const uint64_t (&v)[8], void *out, int kind, int64_t stride, int col, int valid, bool pairs, F &&row) {
+// 16 consecutive tokens' values of one weight row; `row(i)` gives the output row, values past `valid` are not stored
+template <typename F> __device__ __forceinline__ void store16(const uint64_t (&v)[8], void *out, int kind, int64_t stride, int col, int valid, F &&row) {
     auto each = [&](auto put) {
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             if (i < valid) put(row(i) * stride + col, (i & 1) ? hi2(v[i >> 1]) : lo2(v[i >> 1]));
     };
     if (kind == CQ_F32) each([&](int64_t o, float x) { ((float *)out)[o] = x; });
-    else if (pairs) {       // neighbouring lanes exchange, so that one holds both rows' value of token i, the other of token i + 1
-        const int odd = threadIdx.x & 1;
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-            uint32_t mine;
-            if (kind == CQ_F16) mine = h2_bits(__floats2half2_rn(lo2(v[i >> 1]), hi2(v[i >> 1])));
-            else { const __nv_bfloat162 h = __floats2bfloat162_rn(lo2(v[i >> 1]), hi2(v[i >> 1])); mine = *reinterpret_cast<const uint32_t *>(&h); }
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, mine, 1);
-            const uint32_t w = odd ? __byte_perm(got, mine, 0x7632) : __byte_perm(mine, got, 0x5410);
-            if (i + odd < valid) *reinterpret_cast<uint32_t *>((uint16_t *)out + row(i + odd) * stride + (col - odd)) = w;
-        }
-    }
     else if (kind == CQ_F16) each([&](int64_t o, float x) { ((__half *)out)[o] = __float2half(x); });
     else each([&](int64_t o, float x) { ((__nv_bfloat16 *)out)[o] = __float2bfloat16(x); });
-}
-
-// whether the warp's 32 rows from `row0` can be stored in pairs
-__device__ __forceinline__ bool can_pair(const void *out, int stride, int row0, int nrows) {
-    return row0 + 32 <= nrows && (stride & 1) == 0 && ((uintptr_t)out & 3) == 0;
 }
 
 // ---- tiles --------------------------------------------------------------------------------------------------

@@ -561,7 +561,6 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             if (!alive) break;
             if (cx.row0 + r < a.nrows) {
                 void *out = second ? a.out2 : a.out;
-                const bool pairs = can_pair(out, a.stride_out, cx.row0 + quad * 32, a.nrows);
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     const int col = (2 * g + ch0) * 16, left = cx.valid - col;
@@ -579,7 +578,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                         }
                     } else {
                         const int64_t tok = (int64_t)cx.t * tl.tt + col;
-                        store16(acc[g], out, a.out_kind, a.stride_out, cx.row0 + r, left, pairs, [&](int i) { return tok + i; });
+                        store16(acc[g], out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
                     }
                 }
             }
