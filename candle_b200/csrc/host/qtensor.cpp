@@ -1,6 +1,8 @@
 // Host side of the quantized matmul (see qtensor.h) and its flat C interface (cqh_*).
 #include "qtensor.h"
 
+#include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <cstring>
 #include <map>
@@ -190,6 +192,17 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     // Prompt path: many rows of a Q4_K / Q6_K matrix go to the tensor-core kernel.  It quantizes activations like
     // candle's CPU path (Q8_K) in every mode: that is the arithmetic its integer operands are exact for.
     if (rows > kPrefillMinRows && (dtype_ == GgmlDType::Q4K || dtype_ == GgmlDType::Q6K)) {
+        // Q6_K: expanding 128 rows takes 2.0 us per super-block, the int8 kernel 1.4 us for its tiles of 64 rows x 128 tokens (the same
+        // bits).  So a launch that leaves SMs idle either way (few tiles) is faster with the smaller tiles: 4096 rows of
+        // K = 14336 and 100 tokens, 64 tiles for 148 SMs.
+        const size_t tiles128 = (n + 127) / 128 * ((rows + 127) / 128), tiles64 = (n + 63) / 64 * ((rows + 127) / 128);
+        if (dtype_ == GgmlDType::Q6K && (uintptr_t)ptr_ % 4 == 0 && (double)((tiles64 + 147) / 148) * 1.4 < (double)((tiles128 + 147) / 148) * 2.0) {
+            uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prefill_scratch_bytes((int)rows, (int)k));
+            cq_prefill_quantize(x, (int)x_dtype, scratch, (int)k, (int)rows, stream);
+            cq_prefill_gemm((int)dtype_, ptr_, scratch, out, (int)x_dtype, (int)k, (int)n, (int)rows, (int)n, stream);
+            lib_check("qmatmul prefill");
+            return;
+        }
         uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt_scratch_bytes((int)rows, (int)k));
         cq_prompt_matmul((int)dtype_, ptr_, x, (int)x_dtype, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
         lib_check("qmatmul prefill");
@@ -201,8 +214,15 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     const bool plain32 = dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0;
     const bool q8_1_only = !plain32 && dtype_ != GgmlDType::Q4K && dtype_ != GgmlDType::Q6K;
     const bool any_address = dtype_ == GgmlDType::Q2K || dtype_ == GgmlDType::Q3K;
+    // For the six the GEMV slices give the same values, so the faster is taken: a slice of eight rows streams the matrix at
+    // about 1.15 TB/s and costs 7 us at least; the prompt kernel takes a round of 148 tiles (128 weight rows x 64 tokens) per
+    // launch or more, about 1.3 us per 256 elements of K each, and 8 us.  A narrow matrix with a long K leaves most SMs without
+    // a tile: 512 rows of K = 14336 take 80 us however few the tokens, two slices 14 us.
+    const double slices = (double)((rows + MMVQ_MAX_BATCH - 1) / MMVQ_MAX_BATCH), slice_us = std::max(7.0, (double)len_ / 1.15e6);
+    const double rounds = std::ceil((double)((n + 127) / 128) * (double)((rows + 63) / 64) / 148.0);
+    const bool prompt_pays = 8.0 + rounds * (double)(k / 256) * 1.3 < slices * slice_us;
     if (k % 256 == 0 && ((plain32 && rows > kPrefillMinRows) ||
-                         (q8_1_only && rows > MMVQ_MAX_BATCH && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0)))) {
+                         (q8_1_only && rows > MMVQ_MAX_BATCH && prompt_pays && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0)))) {
         uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt32_scratch_bytes((int)dtype_, (int)rows, (int)k));
         cq_prompt32_matmul((int)dtype_, ptr_, x, (int)x_dtype, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
         lib_check("qmatmul prefill (scales per 32)");

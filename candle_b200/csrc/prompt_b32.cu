@@ -13,7 +13,7 @@
 // lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
 //
 // Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
-// warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader; tensor memory: three accumulator slots of two blocks (128
+// warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader, 14-15 raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128
 // columns), 128 columns of operand A.  The roles hand over two blocks at a time.  Every wait is bounded as there.
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
@@ -24,8 +24,8 @@ namespace {
 using namespace cq_prompt;
 
 constexpr int kEpiWarps = 8, kProdWarps = 4;
-constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
-constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
+constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
+constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two: raw bytes without a tensor map
 constexpr int kColA = 384;
 
 __device__ int g_prompt_b32_timeout_flag = 0;
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     const GroupInfo gi{};
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_raw[i], 1); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
         for (int i = 0; i < 4; ++i) {
             cq_mbar_init(&bar_fullT[i], 1);
             cq_mbar_init(&bar_doneT[i], 1);
@@ -425,21 +425,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes<kMins>();
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 const int rs = it & 1;
-                if (it >= 2 && !wait_bar(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
-                uint8_t *dst = raw0 + rs * R::kBytes;
                 if (a.use_map) {
+                    if (it >= 2 && !wait_bar(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
-                        cq_tmap::load_2d(dst, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
-                    }
-                } else {
-                    if (lane == 0) cq_mbar_expect_tx(&bar_raw[rs], kRows * R::kNeed);
-                    __syncwarp();
-                    for (int r = lane; r < kRows; r += 32) {
-                        long long wr = cx.wrow0 + r;
-                        if (wr >= a.nrows) wr = a.nrows - 1;
-                        const uintptr_t src = (uintptr_t)(a.w + wr * row_bytes + (uint32_t)c * kCB) & ~(uintptr_t)15;
-                        cq_bulk_g2s(dst + r * R::kPitch, (const void *)src, R::kNeed, &bar_raw[rs]);
+                        cq_tmap::load_2d(raw0 + rs * R::kBytes, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
                     }
                 }
                 const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes<kMins>();
@@ -464,10 +454,27 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         }
         // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
         if (lane == 0 && (!alive || *abort_flag)) {
-            for (int j = it >= 2 ? it - 1 : 0; j <= it; ++j) (void)cq_mbar_wait_bounded(&bar_raw[j & 1], (j >> 1) & 1);
+            for (int j = it >= 2 ? it - 1 : 0; a.use_map && j <= it; ++j) (void)cq_mbar_wait_bounded(&bar_raw[j & 1], (j >> 1) & 1);
             for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j % kStagesT], (j / kStagesT) & 1);
         }
         __syncwarp();
+    } else if (warp >= kRawWarp) {
+        // ===== raw bytes of rows that are not a multiple of 16 bytes apart =====
+        if (!a.use_map) {
+            int it = 0;
+            bool alive = true;
+            for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+                TileCtx cx;
+                tile_ctx(tile, tl.ntt, tl, gi, cx);
+                const uint8_t *w0 = a.w + cx.wrow0 * row_bytes;
+                for (int c = 0; c < nch; ++c, ++it) {
+                    const int rs = it & 1;
+                    if (it >= 2 && !wait_warp(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                    R::load_rows(raw0 + rs * R::kBytes, w0 + (uint32_t)c * kCB, min(a.nrows - cx.row0, kRows), row_bytes, tid - kRawWarp * 32, &bar_raw[rs]);
+                }
+            }
+            cq_cp_async_wait<0>();
+        }
     } else if (warp == kMmaWarp) {
         // ===== MMA issuer (the warp runs the loop, one elected lane issues): a block = two K = 16 steps into fresh columns =====
         const uint32_t stT = uniform(cq_smem_u32(stT0) >> 4), tm = uniform(tmem_base);
@@ -633,7 +640,6 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
         attr_done[dev] = true;
     }
     const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
-    // expanding a chunk costs about what the epilogue needs for 40 tokens (8 warps, ~1.25 - 2 instructions per value and block)
     const Tiling tl = plan_tiling(tokens, nrt, sm_count(), 40, F::kTok);
     const long long blocks = (long long)tl.ntt * (tl.tt / 8) * nch;
     if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32: too many tokens for one launch"); return false; }

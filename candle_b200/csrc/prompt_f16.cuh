@@ -226,17 +226,17 @@ __device__ __forceinline__ void tile_ctx(int tile, int ntt, const Tiling &tl, co
     c.n = (c.valid + 15) / 16 * 16;
 }
 
-// Number of token tiles for `nrt` row tiles.  Results do not depend on it.  A tile's cost per chunk is the larger of its
-// MMA time (proportional to its tokens) and what expanding 128 weight rows takes (`floor_tok`: as many tokens' worth of MMA);
-// the launch takes as many rounds of `sms` tiles as it needs.
-inline Tiling plan_tiling(int tokens, int nrt, int sms, int floor_tok, int tok_max = kTokMax) {
+// Number of token tiles for `nrt` row tiles.  Results do not depend on it.  A tile's time per chunk is affine in its tokens, `fixed`
+// tokens' worth of it whatever they are (expanding 128 weight rows and the hand-offs); the launch takes as many rounds of `sms`
+// tiles as it needs.  Q4_K on B200: 0.68 us + 4.5 ns per token, hence 150.
+inline Tiling plan_tiling(int tokens, int nrt, int sms, int fixed, int tok_max = kTokMax) {
     Tiling best{tokens, 16, 0};
     long long best_cost = -1;
     for (int ntt = (tokens + tok_max - 1) / tok_max; ntt <= (tokens + 15) / 16; ++ntt) {
         const int tt = ((tokens + ntt - 1) / ntt + 15) / 16 * 16;
         if ((tokens + tt - 1) / tt != ntt) continue;
         const long long rounds = ((long long)nrt * ntt + sms - 1) / sms;
-        const long long cost = rounds * ((tt > floor_tok ? tt : floor_tok) + 8);
+        const long long cost = rounds * (tt + fixed);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best.tt = tt; best.ntt = ntt; }
         if (rounds > 64) break;          // many rounds: smaller tiles only repeat the expansion
     }
@@ -257,15 +257,30 @@ inline int sm_count() {
 }
 
 // ---- raw weight bytes: (128 rows, one 256-element chunk) -> shared memory ---------------------------------------
-// One tiled TMA copy when rows are whole multiples of 16 bytes apart; else one bulk copy per row from the 16-byte boundary
-// below the chunk (Q6_K rows of K % 2048 != 0 and the like).  In shared memory row r starts at r * kPitch, the chunk a few bytes
+// One tiled TMA copy when rows are whole multiples of 16 bytes apart; else (Q6_K rows of K % 2048 != 0 and the like) two warps copy
+// 16-byte pieces with cp.async, consecutive lanes along a row, from the 16-byte boundary below each row's chunk - a bulk copy per
+// row was three times slower than the whole int8 kernel.  In shared memory row r starts at r * kPitch, the chunk a few bytes
 // behind it when it does not start on such a boundary.  CB: bytes of a chunk.
+constexpr int kRawThreads = 64;
 template <int CB> struct Raw {
     static constexpr bool kAligned = CB % 16 == 0;
     static constexpr int kNeed = kAligned ? CB : (CB + 14 + 15) / 16 * 16;       // 16-byte window that covers the chunk
     // pitch: an odd number of 16-byte units, so that eight lanes' 16-byte reads of one column fall into different banks
     static constexpr int kPitch = (kNeed / 16) % 2 ? kNeed : kNeed + 16;
     static constexpr int kBytes = kRows * kPitch;
+    // Pieces reach at most the last 16-byte unit that holds a byte of the chunk, rows past the matrix repeat its last one.
+    // `bar` counts kRawThreads; `w` points at the chunk of the tile's first row, `rows_left` rows are in memory from there.
+    static __device__ __forceinline__ void load_rows(uint8_t *dst, const uint8_t *w, int rows_left, uint32_t row_bytes, int thread, uint64_t *bar) {
+        constexpr int kUnits = kNeed / 16;
+#pragma unroll 1
+        for (int idx = thread; idx < kRows * kUnits; idx += kRawThreads) {
+            const int row = idx / kUnits, u = idx - row * kUnits;
+            const uint8_t *p = w + (size_t)(uint32_t)min(row, rows_left - 1) * row_bytes;
+            const uintptr_t src = ((uintptr_t)p & ~(uintptr_t)15) + 16 * u;
+            if (src < (uintptr_t)p + CB) cq_cp_async16(dst + row * kPitch + 16 * u, (const void *)src);
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(cq_smem_u32(bar)) : "memory");
+    }
 };
 
 }  // namespace cq_prompt

@@ -14,7 +14,7 @@
 // accumulation step rounds to 24 bits, as the int -> float conversion of an integer accumulator would.  L is always exact.
 //
 // Mapping.  One CTA per SM walks tiles of 128 weight rows x up to 128 tokens.  Warps 0-7 epilogue, 8-15 producers (two sets of
-// four, a weight row per thread), 16 MMA issuer, 17 loader.  K advances in stages of 64 TMEM columns of operand A = eight MMAs: 128
+// four, a weight row per thread), 16 MMA issuer, 17 loader, 18-19 raw bytes where there is no tensor map.  K advances in stages of 64 TMEM columns of operand A = eight MMAs: 128
 // elements of Q4_K, 64 of Q6_K (two planes); the sets take turns.  One barrier says that a stage's operands are there (its
 // producer set and the copied activations), one commit that its MMAs are complete.  Tensor memory, all 512 columns: P in two
 // buffers of 128 (the epilogue of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a
@@ -31,8 +31,8 @@ namespace {
 using namespace cq_prompt;
 
 constexpr int kEpiWarps = 8, kProdWarps = 8;     // producers: two sets of four
-constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1;
-constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two warps only fill their warpgroup
+constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
+constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two: raw bytes without a tensor map
 constexpr int kSlabs = 34;                       // 32 slabs of 8 f16 activations, 2 of f16 run sums (16 bytes per token each)
 constexpr int kTokBytes = kSlabs * 16 + 4;       // + the f32 scale
 constexpr int kRingT = 2 * 32 * kTokMax * 16;    // token stages: two super-blocks, 128 KiB
@@ -332,7 +332,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const uint32_t row_bytes = (uint32_t)nsb * kCB;
 
     if (tid == 0) {
-        for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], 1); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
         for (int i = 0; i < F::kNT; ++i) { cq_mbar_init(&bar_full[i], 4 + 1); cq_mbar_init(&bar_done[i], 1); }
         for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_free[i], kEpiWarps); cq_mbar_init(&bar_vis[i], 1); }
         *abort_flag = 0;
@@ -365,21 +365,11 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nsb * kTokBytes;
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                 const int rs = it % F::kRawStages;
-                if (it >= F::kRawStages && !wait_bar(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
-                uint8_t *dst = raw0 + rs * R::kBytes;
                 if (a.use_map) {
+                    if (it >= F::kRawStages && !wait_bar(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
-                        cq_tmap::load_2d(dst, second ? &wmap2 : &wmap, (int)(((uint32_t)sb * kCB & ~15u) / 2), (int)cx.wrow0, &bar_raw[rs]);
-                    }
-                } else {
-                    if (lane == 0) cq_mbar_expect_tx(&bar_raw[rs], kRows * R::kNeed);
-                    __syncwarp();
-                    for (int r = lane; r < kRows; r += 32) {
-                        long long wr = cx.wrow0 + r;
-                        if (wr >= a.total_rows) wr = a.total_rows - 1;
-                        const uintptr_t src = (uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes + (uint32_t)sb * kCB) & ~(uintptr_t)15;
-                        cq_bulk_g2s(dst + r * R::kPitch, (const void *)src, R::kNeed, &bar_raw[rs]);
+                        cq_tmap::load_2d(raw0 + rs * R::kBytes, second ? &wmap2 : &wmap, (int)(((uint32_t)sb * kCB & ~15u) / 2), (int)cx.wrow0, &bar_raw[rs]);
                     }
                 }
                 const uint8_t *blob = blob0 + (size_t)sb * n * kTokBytes;
@@ -406,7 +396,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         // after a give-up the copies of raw bytes must land (or give up themselves) before the shared memory goes away, and those
         // of activations have a second to (their barrier also waits for producers that may have left)
         if (lane == 0 && (!alive || *abort_flag)) {
-            for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; j <= it; ++j)
+            for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; a.use_map && j <= it; ++j)
                 (void)cq_mbar_wait_bounded(&bar_raw[j % F::kRawStages], (j / F::kRawStages) & 1);
             for (int j = h > F::kNT ? h - F::kNT : 0; j < h; ++j) {
                 if (cq_mbar_wait_bounded(&bar_full[j % F::kNT], (j / F::kNT) & 1)) continue;
@@ -414,6 +404,25 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             }
         }
         __syncwarp();
+    } else if (warp >= kRawWarp) {
+        // ===== raw bytes of rows that are not a multiple of 16 bytes apart =====
+        if (!a.use_map) {
+            int it = 0;
+            bool alive = true;
+            for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+                TileCtx cx;
+                const bool second = tile >= per_matrix;
+                tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+                const uint8_t *w0 = (second ? a.w2 : a.w) + cx.wrow0 * row_bytes;
+                const int rows_left = (int)min(a.total_rows - cx.wrow0, (long long)kRows);
+                for (int sb = 0; sb < nsb; ++sb, ++it) {
+                    const int rs = it % F::kRawStages;
+                    if (it >= F::kRawStages && !wait_warp(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
+                    R::load_rows(raw0 + rs * R::kBytes, w0 + (uint32_t)sb * kCB, rows_left, row_bytes, tid - kRawWarp * 32, &bar_raw[rs]);
+                }
+            }
+            cq_cp_async_wait<0>();
+        }
     } else if (warp == kMmaWarp) {
         // ===== MMA issuer: the warp runs the loop, one elected lane issues =====
         const uint32_t stT = uniform(cq_smem_u32(stT0) >> 4), mins = uniform(cq_smem_u32(mins0) >> 4), aux = uniform(cq_smem_u32(aux0) >> 4);
@@ -591,8 +600,8 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
-// tokens' worth of MMA time that expanding one super-block of 128 rows takes
-template <int WTYPE> constexpr int floor_tokens() { return WTYPE == CQ_Q4_K ? 56 : 72; }
+// the fixed part of a tile's time per super-block in tokens (plan_tiling); Q6_K is bound by its producers, 2 us at any token count
+template <int WTYPE> constexpr int fixed_tokens() { return WTYPE == CQ_Q4_K ? 150 : 400; }
 
 template <int WTYPE>
 bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k, int n, long long total_rows, int stride_out, const Tiling &tl,
@@ -639,7 +648,7 @@ bool launch_quantize_rows(int wtype, const void *x, int x_elem, void *scratch, i
 }
 
 Tiling dense_tiling(int wtype, int tokens, int n) {
-    return plan_tiling(tokens, (n + kRows - 1) / kRows, sm_count(), wtype == CQ_Q4_K ? floor_tokens<CQ_Q4_K>() : floor_tokens<CQ_Q6_K>());
+    return plan_tiling(tokens, (n + kRows - 1) / kRows, sm_count(), wtype == CQ_Q4_K ? fixed_tokens<CQ_Q4_K>() : fixed_tokens<CQ_Q6_K>());
 }
 int group_max_tiles(int size_m, int num_experts) { return (size_m + kTokMax - 1) / kTokMax + num_experts; }
 size_t table_bytes(int max_tiles) { return ((size_t)(max_tiles + 1) * 16 + 255) / 256 * 256; }
