@@ -200,7 +200,7 @@ extern "C" void moe_gemm_gguf(const float *input, const void *weights, const int
 
 // candle-kernels/src/ffi.rs:41-56: f16 (input_dtype 0) or bf16 (1) activations, f32 output.  The reference
 // de-quantizes the expert weights to half precision and multiplies with wmma (candle-kernels/src/moe/
-// moe_wmma_gguf.cu:124-300).  Here Q4_K / Q6_K experts go to the grouped tensor-core kernel (cq_moe_prefill_gemm: int8
+// moe_wmma_gguf.cu:124-300).  Here Q4_K / Q6_K experts go to the grouped tensor-core kernel (cq_moe_prefill_gemm:
 // tcgen05 MMAs over Q8_K activations, the CPU path's arithmetic) when there are at least 64 pairs and at least four per
 // expert on average - a tile unpacks its expert's weights once, which costs about as much as five GEMV jobs; fewer
 // pairs, and Q8_0 experts, take the integer GEMV of the decode entry point.

@@ -20,6 +20,10 @@
 // buffers of 128 (the epilogue of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a
 // super-block, by which time the epilogue has read the previous one), operand A in two (Q4_K) or four stages.
 //
+// Measured (4096 -> 14336, f32, quantizer included): Q4_K 2048 tokens 476 us (int8 kernel) -> 357, 128 tokens 28; Q6_K 14336 -> 4096, 512
+// tokens 171 -> 144.  Bound by the hand-offs between the roles: a super-block of 128 tokens takes about 2400 clocks, its MMAs 1090; the
+// producers' two stages (700 - 1000 clocks each, side by side) and the issuing warp (~900) are the longest.
+//
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
 #include "../../include/candle_q_b200.h"
