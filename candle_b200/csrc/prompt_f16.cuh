@@ -42,7 +42,6 @@ __device__ __forceinline__ uint64_t desc_of(uint32_t lo) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"((128u >> 4) | (1u << 14)));      // 8-row groups 128 bytes apart; sm_100 descriptor
     return r;
 }
-__device__ __forceinline__ uint32_t desc_lo(const void *smem, uint32_t n) { return (cq_smem_u32(smem) >> 4) | (n << 16); }
 // D[128 rows][n tokens] (+)= A[tmem: 128 x 16 f16] * B[smem: n x 16 f16]
 template <bool ACC> __device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t desc_b, uint32_t idesc) {
     if constexpr (ACC)
