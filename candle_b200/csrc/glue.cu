@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const float *__restrict__
 
 // Router of a mixture-of-experts block (candle-transformers/src/fused_moe.rs:233-247): softmax over the experts, the k
 // largest probabilities in descending order (lowest index first among equals), optionally divided by their sum.
+// A row with a NaN or +inf logit (or nothing but -inf) has no finite softmax: experts 0 .. k-1 with NaN weights, as a stable
+// descending sort of NaNs gives, so that ids stay in range and the NaN stays with its own token.
 // One warp per token; experts <= 1024.  The softmax sum is added lane-strided, then by an xor butterfly.
 // One warp routes one token.  VOLATILE: the logits were written by other CTAs of the running kernel (read around L1).
 template <bool VOLATILE>
@@ -166,6 +168,13 @@ __device__ __forceinline__ void moe_route_row(const float *row, int32_t *__restr
     }
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    if (sum != sum) {           // the same in every lane
+        if (lane < k) {
+            ids[(size_t)tok * k + lane] = lane;
+            weights[(size_t)tok * k + lane] = sum;
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < PER; ++i) p[i] = lane + 32 * i < experts ? __fdiv_rn(p[i], sum) : -1.0f;      // taken ones become -1 too
     float chosen = 0.0f, total = 0.0f;         // lane s keeps the probability of slot s (k <= 32)

@@ -352,7 +352,8 @@ void cq_peer_gather_set_limit_clocks(long long clocks); /* how long a poll may l
  *   cq_moe_route_f32           : softmax over `experts` (<= 1024) logits per token, the k (<= 32) largest probabilities in
  *                                descending order (lowest expert index among equals) as ids / weights [tokens, k]; with
  *                                norm_topk_prob the weights are divided by their sum
- *                                (candle-transformers/src/fused_moe.rs:233-247).
+ *                                (candle-transformers/src/fused_moe.rs:233-247).  No finite softmax (a NaN or +inf logit, or
+ *                                nothing but -inf): ids 0 .. k-1 with NaN weights.
  *   cq_qknorm_rope_store_kv_f32: optional per-head RMSNorm of q and k (weights of 128 values, null to skip), rotary
  *                                embedding (neox != 0: pairs (i, i + 64); else (2i, 2i + 1)), k and v stored into the
  *                                caches - candle-transformers/src/models/quantized_qwen3.rs:136-183.  head_dim 128. */

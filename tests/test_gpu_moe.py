@@ -231,6 +231,50 @@ def test_route_kernel_matches_the_tensor_formula(cuda_dev):
         assert torch.allclose(w, ref_w, rtol=1e-5, atol=1e-7)
 
 
+def test_route_without_a_finite_softmax(cuda_dev):
+    """NaN, +inf or nothing but -inf: ids in range, NaN weights, as the tensor formula gives; the other tokens keep their bits."""
+    from candle_b200.fused_moe import route
+    L, st = capi.lib(), torch.cuda.current_stream().cuda_stream
+    for experts, k, norm in ((60, 6, True), (128, 8, False), (4, 4, True)):
+        logits = torch.randn(6, experts, device=cuda_dev)
+        bad = logits.clone()
+        bad[1, 2], bad[3, 0] = float("nan"), float("inf")
+        bad[4] = -float("inf")
+        bad[5, 1] = -float("inf")           # finite all the same
+        out = []
+        for lg in (logits, bad):
+            ids = torch.full((6, k), -7, dtype=torch.int32, device=cuda_dev)
+            w = torch.zeros((6, k), device=cuda_dev)
+            L.cq_moe_route_f32(lg.data_ptr(), ids.data_ptr(), w.data_ptr(), 6, experts, k, 1 if norm else 0, st)
+            capi.check("route")
+            out.append((ids, w))
+        (ids0, w0), (ids, w) = out
+        ref_w, ref_ids = route(bad, k, norm)
+        assert torch.equal(ids.long(), ref_ids)
+        assert torch.equal(w[[1, 3, 4]].isnan(), torch.ones(3, k, dtype=torch.bool, device=cuda_dev))
+        assert torch.allclose(w, ref_w, rtol=1e-5, atol=1e-7, equal_nan=True)
+        assert torch.equal(ids[[0, 2]], ids0[[0, 2]]) and torch.equal(w[[0, 2]], w0[[0, 2]])
+
+
+@pytest.mark.parametrize("tokens,is_prefill", [(8, False), (64, True)])
+def test_fused_moe_keeps_a_non_finite_token_to_itself(cuda_dev, tokens, is_prefill):
+    from candle_b200.fused_moe import FusedMoeGGUF
+    from candle_b200.synth import random_blocks
+    e, topk, hidden, ffn, wt = 6, 4, 512, 768, 12
+    mk = lambda n, k, s: QTensor.from_device_blocks(random_blocks(GgmlDType(wt), e * n, k, seed=s, device=cuda_dev).reshape(-1), GgmlDType(wt), (e, n, k))
+    g = torch.Generator(device=cuda_dev).manual_seed(4)
+    moe = FusedMoeGGUF(torch.randn(e, hidden, device=cuda_dev, generator=g) * 0.1, mk(ffn, hidden, 1), mk(ffn, hidden, 2), mk(hidden, ffn, 3), topk)
+    x = torch.randn(1, tokens, hidden, device=cuda_dev, generator=g)
+    assert moe._block(x.view(-1, hidden), is_prefill) is not None
+    good = moe.forward(x, is_prefill)
+    bad = x.clone()
+    bad[0, 1, 5], bad[0, 4, 0] = float("nan"), float("inf")
+    out = moe.forward(bad, is_prefill)
+    rest = [t for t in range(tokens) if t not in (1, 4)]
+    assert torch.equal(out[0, rest], good[0, rest])
+    assert bool(out[0, [1, 4]].isnan().all())
+
+
 def test_one_launch_router_and_slot_sum(cuda_dev):
     """cq_moe_router_f32: its logits against the f32 matrix product (summation order differs), its ids and weights bit for
     bit against cq_moe_route_f32 run on those logits, the arrival counters back at zero, twice in a row.
