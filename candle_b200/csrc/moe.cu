@@ -249,20 +249,22 @@ __global__ void __launch_bounds__(256) gate_up_q8_1_kernel(const float *__restri
 }
 
 // Pairs grouped by expert, ascending inside a group (a stable sort by expert).  One CTA per expert: it counts the pairs of lower
-// experts, then collects its own in order - every CTA reads all ids (32 KB for 1024 tokens x 8) instead of a sort's passes.
+// experts, then collects its own in order - every CTA reads all ids (32 KB for 1024 tokens x 8) instead of a sort's passes.  The
+// last CTA, number `experts`, collects the ids outside [0, experts), so that every slot of both arrays is written.
 __global__ void __launch_bounds__(1024) sort_pairs_kernel(const int32_t *__restrict__ ids, int pairs, int32_t *__restrict__ expert_ids,
                                                           int32_t *__restrict__ sorted) {
     __shared__ int warp_cnt[32];
-    const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int e = blockIdx.x, experts = (int)gridDim.x - 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto key = [&](int i) { return (int)min((unsigned)ids[i], (unsigned)experts); };
     int below = 0;
-    for (int i = tid; i < pairs; i += 1024) below += ids[i] < e;
+    for (int i = tid; i < pairs; i += 1024) below += key(i) < e;
     below = __reduce_add_sync(0xffffffffu, below);
     if (lane == 0) warp_cnt[warp] = below;
     __syncthreads();
     int base = __reduce_add_sync(0xffffffffu, warp_cnt[lane]);
     for (int i0 = 0; i0 < pairs; i0 += 1024) {
         const int i = i0 + tid;
-        const bool mine = i < pairs && ids[i] == e;
+        const bool mine = i < pairs && key(i) == e;
         const unsigned m = __ballot_sync(0xffffffffu, mine);
         __syncthreads();                // warp_cnt of the last step has been read
         if (lane == 0) warp_cnt[warp] = __popc(m);
@@ -279,13 +281,13 @@ __global__ void __launch_bounds__(1024) sort_pairs_kernel(const int32_t *__restr
 }
 }  // namespace
 
-// ids: i32 [pairs], each in [0, num_experts) -> expert_ids ascending and the pair numbers in that order.
+// ids: i32 [pairs] -> expert_ids ascending and the pair numbers in that order; ids outside [0, num_experts) come last, as num_experts.
 extern "C" void cq_moe_sort_pairs(const int32_t *ids, int pairs, int num_experts, int32_t *expert_ids, int32_t *sorted_token_ids, void *stream) {
     if (!ids || !expert_ids || !sorted_token_ids || pairs <= 0 || num_experts <= 0) {
         cq_set_status(CQ_ERR_BAD_ARG, "moe sort: null pointer or empty shape");
         return;
     }
-    sort_pairs_kernel<<<num_experts, 1024, 0, (cudaStream_t)stream>>>(ids, pairs, expert_ids, sorted_token_ids);
+    sort_pairs_kernel<<<num_experts + 1, 1024, 0, (cudaStream_t)stream>>>(ids, pairs, expert_ids, sorted_token_ids);
     cq_check_launch("moe sort");
 }
 

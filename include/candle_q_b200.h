@@ -215,7 +215,8 @@ void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *
                          int topk, int size_m, int size_n, int size_k, void *stream);
 
 /* The expert part of a mixture-of-experts block (gate, up, up * silu(gate), down) with all experts in place.
- *   cq_moe_sort_pairs   : i32 ids [pairs] in [0, num_experts) -> expert_ids ascending, and the pair numbers in that order (stable).
+ *   cq_moe_sort_pairs   : i32 ids [pairs] -> expert_ids ascending, and the pair numbers in that order (stable); ids outside
+ *                         [0, num_experts) come last, as num_experts: the expert products skip those pairs.
  *   cq_moe_block_prompt : many tokens, Q4_K / Q6_K: x f32 [size_m / topk, hidden] rounded to `kind` (CQ_ELEM_F16 / BF16) -> out f32
  *                         [size_m, hidden], every pair scaled by its routing weight (the caller adds a token's pairs); the
  *                         arithmetic of three cq_moe_prefill_gemm calls on inputs of that type.  hidden, ffn multiples of 256.

@@ -452,6 +452,17 @@ def test_sort_pairs_is_the_stable_sort(cuda_dev, pairs, experts):
     assert torch.equal(out[0].long(), ref) and torch.equal(out[1].long(), order)
 
 
+def test_sort_pairs_puts_ids_out_of_range_last(cuda_dev):
+    experts, pairs = 5, 1500
+    ids = torch.randint(0, experts, (pairs,), dtype=torch.int32, device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(1))
+    ids[::7], ids[3::100], ids[5::333] = -1, 0x7fffffff, experts
+    out = torch.full((2, pairs), -9, dtype=torch.int32, device=cuda_dev)
+    capi.lib().cq_moe_sort_pairs(ids.data_ptr(), pairs, experts, out[0].data_ptr(), out[1].data_ptr(), torch.cuda.current_stream().cuda_stream)
+    capi.check("sort")
+    ref, order = torch.sort(torch.where((ids < 0) | (ids > experts), experts, ids).long(), stable=True)
+    assert torch.equal(out[0].long(), ref) and torch.equal(out[1].long(), order)
+
+
 @pytest.mark.parametrize("wt_gu,wt_down", [(12, 12), (12, 14), (14, 14)])
 @pytest.mark.parametrize("tokens,is_prefill", [(5, False), (33, True), (300, True)])
 def test_fused_moe_few_launches_against_the_general_path(cuda_dev, wt_gu, wt_down, tokens, is_prefill):
