@@ -78,7 +78,7 @@ class FusedMoeGGUF:
                 return None
         with torch.cuda.device(dev):
             st = torch.cuda.current_stream(dev).cuda_stream
-            logits = torch.nn.functional.linear(x, self.gate)
+            logits = torch.nn.functional.linear(x, self.gate).to(torch.float32).contiguous()      # autocast gives 16 bits
             ids = torch.empty((3, pairs), dtype=torch.int32, device=dev)        # by token; then experts and pairs, sorted
             weights = torch.empty((tokens, k), dtype=torch.float32, device=dev)
             scratch = torch.empty(need, dtype=torch.uint8, device=dev)

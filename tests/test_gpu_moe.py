@@ -275,6 +275,25 @@ def test_fused_moe_keeps_a_non_finite_token_to_itself(cuda_dev, tokens, is_prefi
     assert bool(out[0, [1, 4]].isnan().all())
 
 
+@pytest.mark.parametrize("tokens,is_prefill", [(8, False), (64, True)])
+def test_fused_moe_under_autocast(cuda_dev, tokens, is_prefill):
+    """Autocast makes the router's logits 16 bits wide: the routing of those values, as the general path takes them (tolerance:
+    test_fused_moe_few_launches_against_the_general_path)."""
+    from candle_b200.fused_moe import FusedMoeGGUF
+    from candle_b200.synth import random_blocks
+    e, topk, hidden, ffn, wt = 6, 4, 512, 768, 12
+    mk = lambda n, k, s: QTensor.from_device_blocks(random_blocks(GgmlDType(wt), e * n, k, seed=s, device=cuda_dev).reshape(-1), GgmlDType(wt), (e, n, k))
+    g = torch.Generator(device=cuda_dev).manual_seed(6)
+    moe = FusedMoeGGUF(torch.randn(e, hidden, device=cuda_dev, generator=g) * 0.1, mk(ffn, hidden, 1), mk(ffn, hidden, 2), mk(hidden, ffn, 3), topk)
+    x = torch.randn(1, tokens, hidden, device=cuda_dev, generator=g)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ys = moe.forward(x, is_prefill)
+        moe._block = lambda *a: None
+        ref = moe.forward(x, is_prefill)
+    assert ys.dtype == x.dtype
+    assert float((ys - ref).norm() / ref.norm()) <= (2e-3 if is_prefill else 1e-4)
+
+
 def test_one_launch_router_and_slot_sum(cuda_dev):
     """cq_moe_router_f32: its logits against the f32 matrix product (summation order differs), its ids and weights bit for
     bit against cq_moe_route_f32 run on those logits, the arrival counters back at zero, twice in a row.
