@@ -83,6 +83,7 @@ def lib() -> C.CDLL:
             getattr(L, f"launch_mmq_quantize_q8_1_{lay}").argtypes = [vp, vp, vp, i32, i64, i64, i64, i64, i64, i64, i64, i64, vp]
         for t in TYPE_NAME.values():
             getattr(L, f"launch_mmq_gguf_{t}").argtypes = [vp, vp, vp, vp, i64, i64, i64, i64, i64, i32, i32, i64, i32, vp]
+        L.cq_attention_reads_by_32.argtypes, L.cq_attention_reads_by_32.restype = [i32] * 4, i32
         L.cq_attention_f32.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, C.c_float, i32, vp]
         L.cq_rms_norm_f32.argtypes = [vp, vp, vp, i32, i32, C.c_float, vp]
         L.cq_add_rms_norm_f32.argtypes = [vp, vp, vp, vp, i32, i32, C.c_float, vp]

@@ -428,17 +428,15 @@ bool attention_args_ok(const void *q, const void *k_cache, const void *v_cache, 
 }
 }  // namespace
 
-// From this many queries per sequence on, cq_attention_f32 runs the kernel that reads the context once per 32 queries
-// (attn_prompt.cu, the same bits); with fewer, its CTAs would be mostly empty.
-constexpr int kPromptMinQueries = 17;
-bool cq_attention_prompt_launch(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch, int tq,
+// attn_prompt.cu
+void cq_attention_prompt_launch(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch, int tq,
                                 int hq, int hkv, int tmax, float scale, int q_stride, cudaStream_t st);
 
 extern "C" void cq_attention_f32(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos,
                                  int batch, int tq, int hq, int hkv, int head_dim, int tmax, float scale, int q_stride, void *stream) {
     if (!attention_args_ok(q, k_cache, v_cache, out, pos, batch, tq, hq, hkv, head_dim, tmax)) return;
-    if (tq >= kPromptMinQueries &&
-        cq_attention_prompt_launch(q, k_cache, v_cache, out, pos, batch, tq, hq, hkv, tmax, scale, q_stride, (cudaStream_t)stream)) {
+    if (cq_attention_reads_by_32(batch, tq, hq, tmax)) {
+        cq_attention_prompt_launch(q, k_cache, v_cache, out, pos, batch, tq, hq, hkv, tmax, scale, q_stride, (cudaStream_t)stream);
         cq_check_launch("attention");
         return;
     }

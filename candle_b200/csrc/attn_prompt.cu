@@ -9,7 +9,7 @@
 //            apart first), blocks in ascending order;
 //   output : keys w, w + 32, ... in ascending order for each w, the 32 partial sums in ascending order, then the division.
 // That needs all scores of a query at once, so they stay in shared memory: 128 bytes per key of the cache, which limits the
-// kernel to caches of kMaxKeys positions (longer ones keep the other kernel).
+// kernel to caches of kMaxKeys positions (longer ones keep the other kernel, and so do grids that would leave SMs idle).
 #include "../../include/candle_q_b200.h"
 #include "common.cuh"
 
@@ -209,10 +209,28 @@ attention_prompt_kernel(const float *__restrict__ q, const float *__restrict__ k
 
 }  // namespace
 
-// Called by cq_attention_f32, arguments checked there; false: the cache is too long for this kernel.
-bool cq_attention_prompt_launch(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch, int tq,
+// Which kernel cq_attention_f32 runs: 1 the one that reads the context once per 32 queries (attn_prompt.cu, the same bits), 0 a CTA
+// per query.  The first has 32 times fewer CTAs, one per SM, and each walks its whole context alone, so it needs enough of them:
+// 21 queries of 4 heads behind 954 keys take 13 us per query and 129 us by 32, 512 queries of 32 heads and 2 sequences 1180 and 343.
+// Fitted to 260 shapes (1 - 64 heads, 1 - 8 sequences, 17 - 1020 queries, caches to 1152; within 12 % on average): a CTA of the
+// first takes 17 us + 0.12 per key, a round of two CTAs per SM of the other 7 us + 0.016 per key.  The position is on the device,
+// so the first is taken only if it is the faster both at position 0 and at the end of the cache.
+extern "C" int cq_attention_reads_by_32(int batch, int tq, int hq, int tmax) {
+    if (tq < 17 || tmax > kMaxKeys || hq > 65535) return 0;
+    const double sms = cq_sm_count(), heads = (double)batch * hq;
+    const double rounds32 = heads * ((tq + 31) / 32) / sms, rounds1 = heads * tq / (2 * sms);
+    for (int last : {tq < tmax ? tq : tmax, tmax}) {            // keys of the last query
+        const double mean = last - 0.5 * (tq < last ? tq : last);
+        const double by32 = rounds32 > 1 ? rounds32 * (17 + 0.12 * mean) : 17 + 0.12 * last;
+        const double by1 = rounds1 > 1 ? rounds1 * (7 + 0.016 * mean) : 7 + 0.016 * last;
+        if (by32 >= by1) return 0;
+    }
+    return 1;
+}
+
+// Called by cq_attention_f32 for the shapes above, arguments checked there.
+void cq_attention_prompt_launch(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch, int tq,
                                 int hq, int hkv, int tmax, float scale, int q_stride, cudaStream_t st) {
-    if (tmax > kMaxKeys || hq > 65535) return false;
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -222,5 +240,4 @@ bool cq_attention_prompt_launch(const float *q, const float *k_cache, const floa
     }
     cq_launch_k(attention_prompt_kernel, dim3((tq + kQ - 1) / kQ, hq, batch), dim3(kThreads), (size_t)kFixedBytes + (size_t)tmax * kQ * 4, st, q,
                 k_cache, v_cache, out, pos, tq, hq, hkv, tmax, scale, q_stride);
-    return true;
 }

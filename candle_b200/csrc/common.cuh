@@ -116,6 +116,19 @@ static inline cudaError_t cq_launch_cluster_k(void (*kernel)(P...), dim3 grid, d
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
 }
 
+// SMs of the current device (148 when it cannot be asked).
+static inline int cq_sm_count() {
+    static int sms[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return 148; }
+    if (!sms[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) (void)cudaGetLastError();
+        sms[dev] = n > 0 ? n : 148;
+    }
+    return sms[dev];
+}
+
 // ---- device helpers ----
 __device__ __forceinline__ int cq_dp4a(int a, int b, int c) { return __dp4a(a, b, c); }
 __device__ __forceinline__ int cq_dp4a_u(unsigned a, int b, int c) {   // unsigned bytes x signed bytes

@@ -242,18 +242,7 @@ inline Tiling plan_tiling(int tokens, int nrt, int sms, int fixed, int tok_max =
     return best;
 }
 
-inline int sm_count() {
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return 148;
-    if (!sms[dev]) {
-        int n = 0;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        sms[dev] = n > 0 ? n : 148;
-    }
-    return sms[dev];
-}
+inline int sm_count() { return cq_sm_count(); }
 
 // ---- raw weight bytes: (128 rows, one 256-element chunk) -> shared memory ---------------------------------------
 // One tiled TMA copy when rows are whole multiples of 16 bytes apart; else (Q6_K rows of K % 2048 != 0 and the like) two warps copy

@@ -278,7 +278,8 @@ int cq_prompt32_timeout_flag(void);
  *   cq_attention_f32     : causal attention over an f32 KV cache, one CTA per (sequence, head, query), so that a head
  *                          gives the same bits on any GPU count.  q: batch*tq rows of q_stride floats (heads side by
  *                          side); out: [batch, tq, hq, 128]; caches: [batch, hkv, tmax, 128]; pos: device int, cache
- *                          position of query 0.
+ *                          position of query 0.  Prompts whose grid fills the device run 32 queries per CTA, with the same
+ *                          bits; cq_attention_reads_by_32 says which of the two a shape takes.
  *   cq_rms_norm_f32      : out[r] = x[r] * rsqrt(mean(x[r]^2) + eps) * w.
  *   cq_add_rms_norm_f32  : x[r] += residual[r] (stored), then the same normalisation of the new x[r].
  *   cq_add_rms_norm_q8_1, cq_silu_mul_q8_1, cq_attention_q8_1 : the same results stored as the Q8_1 containers the
@@ -289,6 +290,7 @@ int cq_prompt32_timeout_flag(void);
  *   cq_silu_mul_f32      : out[r, i] = silu(gu[r, i]) * gu[r, f + i] for rows gu = [gate | up] of width 2f. */
 void cq_attention_f32(const float *q, const float *k_cache, const float *v_cache, float *out, const int *pos, int batch,
                       int tq, int hq, int hkv, int head_dim, int tmax, float scale, int q_stride, void *stream);
+int cq_attention_reads_by_32(int batch, int tq, int hq, int tmax);
 void cq_rms_norm_f32(const float *x, const float *w, float *out, int rows, int d, float eps, void *stream);
 void cq_add_rms_norm_f32(float *x, const float *residual, const float *w, float *out, int rows, int d, float eps,
                          void *stream);

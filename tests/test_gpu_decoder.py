@@ -421,3 +421,26 @@ def test_prompt_attention_gives_the_bits_of_one_query_at_a_time(lib, cuda_dev, T
     for t in range(0, Tq, 1 if Tq < 80 else 7):
         one = run(wide[:, t:t + 1].contiguous(), pos0 + t, torch.empty((B, 1, Hq, D), device=cuda_dev))
         assert torch.equal(out[:, t], one[:, 0]), t
+
+
+@pytest.mark.parametrize("Tq,pos0,Tmax", [(17, 0, 32), (32, 5, 64), (33, 100, 133), (64, 63, 128), (130, 200, 331), (200, 0, 190), (70, 1060, 1152)])
+def test_prompt_attention_of_many_heads_gives_the_bits_of_one_query_at_a_time(lib, cuda_dev, Tq, pos0, Tmax):
+    """The sizes above with a grid that fills the device, so that cq_attention_f32 runs 32 queries per CTA."""
+    torch.manual_seed(Tq)
+    B, Hq, Hkv, D = 2, 36, 12, 128
+    assert lib.cq_attention_reads_by_32(B, Tq, Hq, Tmax) == 1 and lib.cq_attention_reads_by_32(B, 1, Hq, Tmax) == 0
+    q = torch.randn(B, Tq, Hq * D + 64, device=cuda_dev)
+    kc, vc = torch.randn(B, Hkv, Tmax, D, device=cuda_dev), torch.randn(B, Hkv, Tmax, D, device=cuda_dev)
+    st, scale = torch.cuda.current_stream().cuda_stream, 1.0 / math.sqrt(D)
+
+    def run(q, pos):
+        out = torch.full((B, q.shape[1], Hq, D), float("nan"), device=cuda_dev)
+        p = torch.tensor([pos], dtype=torch.int32, device=cuda_dev)
+        lib.cq_attention_f32(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), p.data_ptr(), B, q.shape[1], Hq, Hkv, D, Tmax, scale,
+                             Hq * D + 64, st)
+        capi.check("attention")
+        return out
+
+    out = run(q, pos0)
+    for t in range(0, Tq, 1 if Tq < 80 else 7):
+        assert torch.equal(out[:, t], run(q[:, t:t + 1].contiguous(), pos0 + t)[:, 0]), t

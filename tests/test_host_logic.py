@@ -88,3 +88,19 @@ def test_decoder_refuses_positions_beyond_max_pos():
     stub2 = types.SimpleNamespace(cfg=DecoderConfig.tiny(), _pos_host=0)
     with pytest.raises(ValueError, match="max_pos"):
         LlamaShapedDecoder.generate(stub2, __import__("torch").zeros((1, 120), dtype=__import__("torch").int64), 10)
+
+
+def test_prompt_attention_is_taken_where_it_is_the_faster(lib):
+    """(batch, queries, heads, cache) with the measured times of a CTA per query and of 32 queries per CTA (us, position 0 or the end
+    of the cache): the slower kernel must not be taken.  Without a device the rule counts 148 SMs."""
+    by_query = [((1, 17, 8, 1152), 21.4, 138.6), ((1, 17, 32, 1152), 54.7, 138.9), ((1, 21, 4, 1152), 13.4, 128.9), ((1, 26, 1, 1024), 13.4, 130.5),
+                ((1, 25, 2, 640), 10.5, 85.4), ((2, 44, 8, 640), 40.0, 80.4), ((1, 32, 4, 64), 11.4, 25.1), ((1, 17, 16, 128), 9.3, 17.9),
+                ((1, 95, 8, 896), 60.5, 116.3), ((1, 839, 2, 896), 81.6, 115.8), ((1, 912, 2, 1152), 112.8, 150.7), ((1, 64, 4, 1152), 26.9, 151.2)]
+    by_32 = [((2, 512, 32, 640), 1181.1, 342.8), ((1, 1024, 32, 1152), 1609.2, 591.8), ((1, 256, 32, 256), 248.9, 78.2), ((1, 64, 32, 128), 60.4, 28.5),
+             ((1, 128, 32, 1152), 309.1, 151.8), ((1, 512, 8, 512), 158.6, 76.3), ((4, 40, 16, 128), 71.3, 26.9)]
+    for shape, slow, fast in by_query:
+        assert slow < fast and lib.cq_attention_reads_by_32(*shape) == 0, shape
+    for shape, slow, fast in by_32:
+        assert fast < slow and lib.cq_attention_reads_by_32(*shape) == 1, shape
+    assert lib.cq_attention_reads_by_32(2, 512, 32, 1161) == 0          # its scores do not fit shared memory
+    assert lib.cq_attention_reads_by_32(64, 16, 64, 128) == 0
