@@ -111,7 +111,8 @@ attention_prompt_kernel(const float *__restrict__ q, const float *__restrict__ k
 
     // ---- softmax: lane = query, warp = every eighth block of 32 keys; the key tile holds the partial results ----
     float *redmax = tile, *redsum = tile + 8 * kQ;          // [8][32], [32 blocks][32]
-    const int my_last = last_of(lane), nblk = min((n_keys + 31) / 32, 32);
+    // at least one block: a context without keys (a position before the cache) divides 0 by 0, as in the other kernel
+    const int my_last = last_of(lane), nblk = min(max((n_keys + 31) / 32, 1), 32);
     float mx = -INFINITY;
     for (int j0 = warp * 32; j0 < n_keys; j0 += 256)
         for (int j = j0; j < min(j0 + 32, n_keys); ++j)
@@ -153,7 +154,7 @@ attention_prompt_kernel(const float *__restrict__ q, const float *__restrict__ k
         for (int w = 1; w < nblk; ++w) den[x] = __fadd_rn(den[x], redsum[w * kQ + q0 + x]);
     }
     __syncthreads();                        // the partial results have been read; the tile takes values now
-    const int rpw = (n_keys + 31) / 32, wg = kValRows / rpw;        // keys per w; w's per value tile (at least one: n_keys <= kMaxKeys)
+    const int rpw = max((n_keys + 31) / 32, 1), wg = kValRows / rpw;        // keys per w; w's per value tile (at least one: n_keys <= kMaxKeys)
     const int ngrp = (32 + wg - 1) / wg, all_see = last_of(0);      // keys up to all_see are in every query's context
     auto load_values = [&](int grp) {
         float *dst = tile + (grp & 1) * kValRows * kD;

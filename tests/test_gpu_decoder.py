@@ -444,3 +444,25 @@ def test_prompt_attention_of_many_heads_gives_the_bits_of_one_query_at_a_time(li
     out = run(q, pos0)
     for t in range(0, Tq, 1 if Tq < 80 else 7):
         assert torch.equal(out[:, t], run(q[:, t:t + 1].contiguous(), pos0 + t)[:, 0]), t
+
+
+def test_prompt_attention_without_keys_is_nan(lib, cuda_dev):
+    """Positions before the cache: the queries that see no key divide 0 by 0, the others keep the bits of a call of their own."""
+    B, Tq, Hq, D, Tmax, pos0 = 2, 70, 36, 128, 64, -40
+    assert lib.cq_attention_reads_by_32(B, Tq, Hq, Tmax) == 1
+    torch.manual_seed(1)
+    q = torch.randn(B, Tq, Hq * D, device=cuda_dev)
+    kc, vc = torch.randn(B, Hq, Tmax, D, device=cuda_dev), torch.randn(B, Hq, Tmax, D, device=cuda_dev)
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run(q, pos):
+        out = torch.zeros((B, q.shape[1], Hq, D), device=cuda_dev)
+        p = torch.tensor([pos], dtype=torch.int32, device=cuda_dev)
+        lib.cq_attention_f32(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), p.data_ptr(), B, q.shape[1], Hq, Hq, D, Tmax, 0.1, Hq * D, st)
+        capi.check("attention")
+        return out
+
+    out = run(q, pos0)
+    assert bool(out[:, :40].isnan().all()) and not bool(out[:, 40:].isnan().any())
+    for t in (40, 41, 63, 64, 69):
+        assert torch.equal(out[:, t], run(q[:, t:t + 1].contiguous(), pos0 + t)[:, 0]), t
