@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 const int rs = it & 1;
                 if (a.use_map) {
-                    if (it >= 2 && !wait_bar(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (it >= 2 && !wait_warp(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
                         cq_tmap::load_2d(raw0 + rs * R::kBytes, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes<kMins>();
                 for (int half = 0; half < 2; ++half, ++ti) {
                     const int s = ti % kStagesT;
-                    if (ti >= kStagesT && !wait_bar(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (ti >= kStagesT && !wait_warp(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         const unsigned bytes = (unsigned)n * 256;
                         if (half == 0) {

@@ -87,13 +87,10 @@ __device__ __forceinline__ bool wait_slow(uint64_t *bar, unsigned parity, volati
     }
     return true;
 }
-__device__ __forceinline__ bool wait_bar(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    return try_wait_suspended(bar, parity) || wait_slow(bar, parity, abort_flag);
-}
-
-// A warp that goes on to a warp-wide tcgen05 instruction must decide as one whether its wait gave up.
+// There is no per-lane form: every role goes on to warp-wide instructions, so its warp decides as one whether a wait gave up (lanes
+// that left at different places would meet at different warp-wide instructions, which need not end).
 __device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, try_wait_suspended(bar, parity) || wait_slow(bar, parity, abort_flag));
 }
 // One arrival per warp: barriers count warps, not threads.
 __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {

@@ -370,7 +370,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                 const int rs = it % F::kRawStages;
                 if (a.use_map) {
-                    if (it >= F::kRawStages && !wait_bar(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (it >= F::kRawStages && !wait_warp(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
                         cq_tmap::load_2d(raw0 + rs * R::kBytes, second ? &wmap2 : &wmap, (int)(((uint32_t)sb * kCB & ~15u) / 2), (int)cx.wrow0, &bar_raw[rs]);
