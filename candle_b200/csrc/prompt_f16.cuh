@@ -3,8 +3,8 @@
 //
 // Both run the quantized product on `tcgen05.mma kind::f16` with INTEGERS in f16: int8 activations, and weight codes times
 // their integer sub-scales, are whole numbers of at most 11 significant bits, so every product is exact and the f32
-// accumulator holds the exact integer sum as long as it stays below 2^24.  Against int8 operands that saves the second
-// weight plane and the int -> float conversions of the epilogue.
+// accumulator holds the exact integer sum as long as no partial sum passes 2^24: each kernel says how it sees to that.  Against
+// int8 operands this saves the second weight plane (Q4_K) and the int -> float conversions of the epilogue.
 //
 // Operand A (M = 128 weight rows) lives in TENSOR MEMORY: a producer thread owns one row = one TMEM lane, expands its GGUF
 // bytes in registers and stores them with `tcgen05.st`.  Through shared memory the same operand would cost a write and, per
@@ -67,6 +67,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
           "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
           "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
           "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }

@@ -7,22 +7,31 @@
 //
 // Arithmetic: candle's CPU path.  Activations are BlockQ8K (one f32 scale per 256 values, k_quants.rs:2320-2358, bit-identical
 // int8); a super-block contributes  d_a * (d_w * P - dmin_w * L)  (k_quants.rs:1460-1540, 2035-2092) with the integers
-//      Q4_K:  P = sum (sc_g q) . q8,   |sc_g q| <= 945: one f16 plane;   L = sum_j m_j bsum_j,  |bsum_j| <= 2032, one K = 16 step
-//      Q6_K:  P = sum (sc_j (q - 32)) . q8:  q - 32 = n + 16 (b - 2) with the nibble n and the bit pair b:  |sc_j n| <= 1920 and
-//             |sc_j 16 (b - 2)| <= 4096, a multiple of 16, are exact in f16; the two planes add into the same accumulator
-// P is exact below 2^24; above (only reachable when most of the 256 products are near their largest value with one sign) each
-// accumulation step rounds to 24 bits, as the int -> float conversion of an integer accumulator would.  L is always exact.
+//      Q4_K:  P = sum (sc_g q) . q8,   |sc_g q| <= 945: one f16 plane;   L = sum_j m_j bsum_j,  |bsum_j| <= 2048, one K = 16 step
+//      Q6_K:  P = sum (sc_j (q - 32)) . q8:  a product of up to 4096 = A + B, A the next multiple of 8, |B| <= 4:  two f16 planes
+// The accumulators are f32, so every partial sum has to stay within 2^24 to be exact, whatever the data (|q8| <= 127; 128 where an
+// activation is infinite or NaN).  P itself reaches 3.1e7 (Q4_K) and 1.3e8 (Q6_K).
+//      Q6_K:  an accumulator per plane: multiples of 8 up to 256 * 4096 * 128 = 8 * 2^24, and 256 * 4 * 128; P = Pa + Pb.
+//      Q4_K:  945 * sum |q8| bounds the terms.  The quantizer stores sum |q8| per token and super-block; where all tokens of the tile have
+//             945 * sum |q8| <= 2^24 (a mean |q8| of 69; normal inputs have 36, uniform ones 64) one accumulator holds P, else the
+//             super-block is split into one accumulator per 128 elements, 128 * 945 * 128 = 15.5e6; P = P0 + P1.
+// The epilogue joins two accumulators with one f32 operation: P rounded once, as converting an integer sum would.
+// L <= 256 * 63 * 128 is exact.
 //
 // Mapping.  One CTA per SM walks tiles of 128 weight rows x up to 128 tokens.  Warps 0-7 epilogue, 8-15 producers (two sets of
-// four, a weight row per thread), 16 MMA issuer, 17 loader, 18-19 raw bytes where there is no tensor map.  K advances in stages of 64 TMEM columns of operand A = eight MMAs: 128
-// elements of Q4_K, 64 of Q6_K (two planes); the sets take turns.  One barrier says that a stage's operands are there (its
-// producer set and the copied activations), one commit that its MMAs are complete.  Tensor memory, all 512 columns: P in two
-// buffers of 128 (the epilogue of one super-block runs beside the MMAs of the next), L in one (its single step comes last in a
-// super-block, by which time the epilogue has read the previous one), operand A in two (Q4_K) or four stages.
+// four, a weight row per thread), 16 MMA issuer, 17 loader, 18-19 raw bytes where there is no tensor map.  K advances in stages of 64 TMEM
+// columns of operand A = eight MMAs: 128 elements of Q4_K, 64 of Q6_K (two planes); the sets take turns.  One barrier says that a
+// stage's operands are there (its producer set and the copied activations), one commit that its MMAs are complete.  Tensor memory, all
+// 512 columns: two accumulators of 128 for P.  Q4_K alternates between them, so that the epilogue of one super-block runs beside the MMAs
+// of the next, and takes both for a split one; L in 128 (its single step comes last in a super-block, by which time the epilogue has read
+// the previous one); operand A in two stages.  Q6_K takes both for every super-block; operand A in four stages, so that the producers go
+// on while the epilogue reads.
 //
-// Measured (4096 -> 14336, f32, quantizer included): Q4_K 2048 tokens 476 us (int8 kernel) -> 357, 128 tokens 28; Q6_K 14336 -> 4096, 512
-// tokens 171 -> 144.  Bound by the hand-offs between the roles: a super-block of 128 tokens takes about 2400 clocks, its MMAs 1090; the
-// producers' two stages (700 - 1000 clocks each, side by side) and the issuing warp (~900) are the longest.
+// Measured (B200, quantizer included; int8 kernel -> this one): Q4_K 4096 -> 14336, 2048 tokens bf16 478 us -> 313 (f32 286 back to back; 463
+// when every super-block is split), 128 tokens 28; Q6_K 14336 -> 4096, 512 tokens f32 170 -> 148.  With one accumulator for all of P, which
+// rounds past 2^24, they took 306 and 145.  Reading both halves of all accumulators in two 64-token passes instead costs 342 (Q4_K)
+// and 157 (Q6_K): twice the MMAs to issue.  Bound by the hand-offs between the roles: a super-block of 128 tokens takes 1.4 us (Q4_K) and
+// 2.4 us (Q6_K) where its MMAs take 0.55 and 1.05.
 //
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
@@ -38,11 +47,12 @@ constexpr int kEpiWarps = 8, kProdWarps = 8;     // producers: two sets of four
 constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
 constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two: raw bytes without a tensor map
 constexpr int kSlabs = 34;                       // 32 slabs of 8 f16 activations, 2 of f16 run sums (16 bytes per token each)
-constexpr int kTokBytes = kSlabs * 16 + 4;       // + the f32 scale
+constexpr int kTokBytes = kSlabs * 16 + 8;       // + the f32 scale and sum |q8|
 constexpr int kRingT = 2 * 32 * kTokMax * 16;    // token stages: two super-blocks, 128 KiB
 constexpr int kAuxRing = 4;
-constexpr int kAux = 2 * kTokMax * 16 + kTokMax * 4;      // run sums, then scales of one super-block
+constexpr int kAux = 2 * kTokMax * 16 + 2 * kTokMax * 4;  // run sums, scales, sums of |q8| of one super-block
 constexpr int kColL = 256;
+constexpr float kOneAccumulator = (float)((1 << 24) / (63 * 15));      // sum |q8| up to which Q4_K needs one accumulator
 
 __device__ int g_prompt_kq_timeout_flag = 0;
 
@@ -97,7 +107,7 @@ template <typename L>
 __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__restrict__ y, int nsb, int q6k, Tiling tl, GroupInfo gi) {
     constexpr int kPitch = 8 * 16 + 16;
     __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
-    __shared__ float sd[8];
+    __shared__ float sd[16];
     cq_pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sb = blockIdx.x % nsb, g = blockIdx.x / nsb, per_tile = tl.tt / 8;
@@ -158,12 +168,17 @@ __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__
         const int j = lane >> 1;
         *reinterpret_cast<__half *>(sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7)) = __float2half_rn(bs);
     }
-    if (lane == 0) sd[warp] = d;
+    float mag = 0.0f;                   // at most 1024, a whole number
+#pragma unroll
+    for (int c = 0; c < 8; ++c) mag += fabsf(q[c]);
+    const int sum_mag = __reduce_add_sync(0xffffffffu, (int)mag);
+    if (lane == 0) { sd[warp] = d; sd[8 + warp] = (float)sum_mag; }
     __syncthreads();
     uint8_t *blob = y + ((size_t)blob_row * nsb + (size_t)sb * rows) * kTokBytes;
     for (int i = threadIdx.x; i < kSlabs * 8; i += 256)
         *reinterpret_cast<uint4 *>(blob + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 16) = *reinterpret_cast<const uint4 *>(sm + (i >> 3) * kPitch + (i & 7) * 16);
-    if (threadIdx.x < 8) *reinterpret_cast<float *>(blob + (size_t)rows * (kSlabs * 16) + (row0 + threadIdx.x) * 4) = sd[threadIdx.x];
+    if (threadIdx.x < 16)
+        *reinterpret_cast<float *>(blob + (size_t)rows * (kSlabs * 16 + (threadIdx.x >> 3) * 4) + (row0 + (threadIdx.x & 7)) * 4) = sd[threadIdx.x];
 }
 
 // One CTA: the tile table of a grouped launch.  expert_ids ascending (ids outside [0, num_experts) may sit at either end);
@@ -263,8 +278,8 @@ template <> struct Expand<CQ_Q4_K> {
 };
 
 // Q6_K stage 2 h + p: the two 32-element groups pos = p (low nibbles) and p + 2 (high ones) of ql[64 h + 32 p ..], bit pairs pos of
-// qh[32 h ..]; 16 cells of sc * nibble, then 16 of sc * 16 (bits - 2), per group.  Codes sit in the mantissa of 64.0 (unit 1/16),
-// nibble at bits 4-7, bit pair at 8-9, so one fma with -64 sc or -96 sc gives each part exactly.
+// qh[32 h ..]; 16 cells of A, then 16 of B per group.  The 6-bit code q sits in the mantissa of 1024.0; sc * (q - 32) + 12288, where f16 counts
+// in eights, rounds to the next multiple of 8 in one fma, and a second one gives the exact rest.
 template <> struct Expand<CQ_Q6_K> {
     const uint8_t *p;
     uint32_t sc[4];
@@ -285,17 +300,16 @@ template <> struct Expand<CQ_Q6_K> {
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 const __half2 s2 = __half2half2(__short2half_rn((short)(int8_t)(scw >> (8 * hf))));
-                const __half2 cl = __hmul2(s2, __float2half2_rn(-64.0f)), ch = __hmul2(s2, __float2half2_rn(-96.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i] >> (2 * pp);
+                    const uint32_t c = ((nib ? l >> 4 : l) & 0x0F0F0F0Fu) | ((nib ? b : b << 4) & 0x30303030u);
 #pragma unroll
                     for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
-                        const int dn = 8 * od + (nib ? 0 : -4), up = 8 - 4 * nib - 8 * od;
-                        const uint32_t lv = dn >= 0 ? l >> (dn >= 0 ? dn : 0) : l << (dn < 0 ? -dn : 0);
-                        const uint32_t hv = up >= 0 ? b << (up >= 0 ? up : 0) : b >> (up < 0 ? -up : 0);
-                        o[nib][8 * hf + 2 * i + od] = hfma2_bits((lv & 0x00F000F0u) | 0x54005400u, s2, cl);
-                        o[nib][16 + 8 * hf + 2 * i + od] = hfma2_bits((hv & 0x03000300u) | 0x54005400u, s2, ch);
+                        const __half2 y = __hsub2(bits_h2(((od ? c >> 8 : c) & 0x00FF00FFu) | 0x64006400u), __float2half2_rn(1056.0f));
+                        const __half2 a = __hsub2(__hfma2(s2, y, __float2half2_rn(12288.0f)), __float2half2_rn(12288.0f));
+                        o[nib][8 * hf + 2 * i + od] = h2_bits(a);
+                        o[nib][16 + 8 * hf + 2 * i + od] = h2_bits(__hfma2(s2, y, __hneg2(a)));
                     }
                 }
             }
@@ -321,10 +335,11 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     uint64_t *bar_rawfree = bar_raw + 3;                            // [3] read by both producer sets
     uint64_t *bar_full = bar_raw + 6;                               // [kNT] stage: operand A stored (four warps), activations landed
     uint64_t *bar_done = bar_raw + 14;                              // [kNT] its MMAs are complete
-    uint64_t *bar_free = bar_raw + 22;                              // [2] accumulators drained (all epilogue warps)
+    uint64_t *bar_free = bar_raw + 22;                              // [2] accumulators of an even / odd super-block drained (all epilogue warps)
     uint64_t *bar_vis = bar_raw + 24;                               // [2] relay: the scale rings of this super-block are visible
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 256);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 264);
+    int *split_of = reinterpret_cast<int *>(smem + 272);           // [2] the super-block takes both accumulators (Q4_K)
     uint8_t *stT0 = smem + 1024;
     uint8_t *aux0 = stT0 + kRingT;
     uint8_t *ringW = aux0 + kAuxRing * kAux;            // (d, dmin) of the rows: [4][128] float2
@@ -385,7 +400,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                         if (st == 0) {
                             // done with the first stage of it - 2: its MMAs started after the epilogue of it - 4
                             uint8_t *ax = aux0 + (it & 3) * kAux;
-                            const unsigned aux_bytes = (unsigned)n * (F::kMins ? 36 : 4);
+                            const unsigned aux_bytes = (unsigned)n * (F::kMins ? 40 : 4);
                             cq_mbar_expect_tx(&bar_full[s], bytes + aux_bytes);
                             cq_bulk_g2s(ax + (F::kMins ? 0 : n * 32), blob + (size_t)n * (F::kMins ? 512 : 544), aux_bytes, &bar_full[s]);
                         } else {
@@ -433,6 +448,81 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         const uint32_t tm = uniform(tmem_base);
         int it = 0;
         bool alive = true;
+        // ---- Q4_K: the super-blocks alternate between the accumulators of P, a split one takes both ----
+        bool split = false;                         // the last super-block whose first stage has been issued
+        auto epilogue_done = [&](int j) { return j < 0 || wait_warp(&bar_free[j & 1], (j >> 1) & 1, abort_flag); };
+        auto super_block4 = [&](uint32_t n, uint32_t idesc, uint32_t bT) {
+            const int c = it & 1;
+            const uint32_t tp = tm + (uint32_t)(c * kTokMax), tp2 = tm + (uint32_t)((c ^ 1) * kTokMax);
+            // The epilogue has read P of it - 2: known from the wait for L of it - 1, unless that took this accumulator too.
+            if (split && !epilogue_done(it - 1)) return false;
+#pragma unroll
+            for (int st = 0; st < 2; ++st) {
+                const int h = it * 2 + st, s = h % F::kNT;
+                if (st == 1) {
+                    // Where this super-block's second stage goes.  Looked up behind the first stage's MMAs: in front of them it cost 170 clocks.
+                    const float4 m = *reinterpret_cast<const float4 *>(aux0 + (it & 3) * kAux + n * 36 + min(16u * lane, 4u * n - 16u));
+                    split = __any_sync(0xffffffffu, fmaxf(fmaxf(m.x, m.y), fmaxf(m.z, m.w)) > kOneAccumulator);
+                    if (split && !epilogue_done(it - 1)) return false;
+                }
+                if (!wait_warp(&bar_full[s], (h / F::kNT) & 1, abort_flag)) return false;
+                tc_fence_after();
+                const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = tm + (uint32_t)(F::kColA + (h % F::kNA) * 64);
+                if (elect_one()) {
+                    if (st == 1) {
+                        split_of[c] = split;
+                        mbar_arrive(&bar_vis[c]);       // relay: what this warp has acquired is visible to the epilogue
+                    }
+                    if (st == 1 && split) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (j == 0) mma_f16_ts<false>(tp2, a0, b0, idesc);
+                            else mma_f16_ts<true>(tp2, a0 + 8 * j, b0 + 2 * j * n, idesc);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (st == 0 && j == 0) mma_f16_ts<false>(tp, a0, b0, idesc);
+                            else mma_f16_ts<true>(tp, a0 + 8 * j, b0 + 2 * j * n, idesc);
+                        }
+                    }
+                }
+                if (st == 1) {
+                    // L has one buffer: the epilogue of the previous super-block must have read it
+                    if (!epilogue_done(it - 1)) return false;
+                    tc_fence_after();
+                    if (elect_one())
+                        mma_f16_ss(tm + (uint32_t)kColL, (mins + (uint32_t)c * (kRows * 32 >> 4)) | ((uint32_t)kRows << 16),
+                                   (aux + (uint32_t)(it & 3) * (kAux >> 4)) | (n << 16), idesc);
+                }
+                __syncwarp();
+                if (elect_one()) tc_commit(&bar_done[s]);
+            }
+            return true;
+        };
+        // ---- Q6_K: an accumulator per plane ----
+        auto super_block6 = [&](uint32_t n, uint32_t idesc, uint32_t bT) {
+            if (!epilogue_done(it - 1)) return false;
+#pragma unroll
+            for (int st = 0; st < F::kSps; ++st) {
+                const int h = it * F::kSps + st, s = h % F::kNT;
+                if (!wait_warp(&bar_full[s], (h / F::kNT) & 1, abort_flag)) return false;
+                tc_fence_after();
+                const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = tm + (uint32_t)(F::kColA + (h % F::kNA) * 64);
+                if (elect_one()) {
+                    if (st == 0) mbar_arrive(&bar_vis[it & 1]);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {           // a group's two planes (two steps each) meet the same 32 activations
+                        const uint32_t dst = tm + (uint32_t)((j >> 1 & 1) * kTokMax), b1 = b0 + (uint32_t)(4 * (j >> 2) + 2 * (j & 1)) * n;
+                        if (st == 0 && (j & ~2) == 0) mma_f16_ts<false>(dst, a0 + 8 * j, b1, idesc);
+                        else mma_f16_ts<true>(dst, a0 + 8 * j, b1, idesc);
+                    }
+                    tc_commit(&bar_done[s]);
+                }
+                __syncwarp();
+            }
+            return true;
+        };
         for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
             TileCtx cx;
             const bool second = tile >= per_matrix;
@@ -440,37 +530,8 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             const uint32_t n = uniform((uint32_t)cx.n), idesc = idesc_f16((int)n), bT = stT | (n << 16);
 #pragma unroll 1
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
-                const int c = it & 1;
-                const uint32_t tp = tm + (uint32_t)(c * kTokMax);
-                // the epilogue has read P of it - 2 (Q4_K: known from the wait for L below)
-                if (!F::kMins && it >= 2 && !wait_warp(&bar_free[c], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
-#pragma unroll
-                for (int st = 0; st < F::kSps; ++st) {
-                    const int h = it * F::kSps + st, s = h % F::kNT;
-                    if (!wait_warp(&bar_full[s], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
-                    tc_fence_after();
-                    const uint32_t b0 = bT + (uint32_t)s * (kStageT >> 4), a0 = tm + (uint32_t)(F::kColA + (h % F::kNA) * 64);
-                    if (elect_one()) {
-                        if (st == 0) mbar_arrive(&bar_vis[c]);      // relay: what this warp has acquired is visible to the epilogue
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            // Q6_K: a group's two planes (two steps each) meet the same 32 activations
-                            const uint32_t b1 = b0 + (uint32_t)(F::kMins ? 2 * j : 4 * (j >> 2) + 2 * (j & 1)) * n;
-                            if (st == 0 && j == 0) mma_f16_ts<false>(tp, a0, b1, idesc);
-                            else mma_f16_ts<true>(tp, a0 + 8 * j, b1, idesc);
-                        }
-                    }
-                    if (F::kMins && st == F::kSps - 1) {
-                        // L has one buffer: the epilogue of the previous super-block must have read it
-                        if (it >= 1 && !wait_warp(&bar_free[c ^ 1], ((it - 1) >> 1) & 1, abort_flag)) { alive = false; break; }
-                        tc_fence_after();
-                        if (elect_one())
-                            mma_f16_ss(tm + (uint32_t)kColL, (mins + (uint32_t)c * (kRows * 32 >> 4)) | ((uint32_t)kRows << 16),
-                                       (aux + (uint32_t)(it & 3) * (kAux >> 4)) | (n << 16), idesc);
-                    }
-                    __syncwarp();
-                    if (elect_one()) tc_commit(&bar_done[s]);
-                }
+                if constexpr (F::kMins) alive = super_block4(n, idesc, bT);
+                else alive = super_block6(n, idesc, bT);
             }
         }
     }
@@ -524,6 +585,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         const int quad = warp & 3, ch0 = warp >> 2;
         const int r = quad * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        [[maybe_unused]] const uint64_t one = pack2f(1.0f, 1.0f);
         int it = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
@@ -545,13 +607,27 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                 const float2 ws = *reinterpret_cast<const float2 *>(ringW + (it & 3) * kRows * 8 + r * 8);
                 const uint64_t dw = pack2f(ws.x, ws.x), ndm = pack2f(-ws.y, -ws.y);
                 const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * kAux + cx.n * 32);
+                const uint32_t tp = tlane + (uint32_t)(F::kMins ? c * kTokMax : 0);
+                if (F::kMins && split_of[c]) {      // rare: P0 + P1 into the place of P
+#pragma unroll 1
+                    for (int col = ch0 * 16; col < cx.n; col += 32) {
+                        uint32_t p[16], p1[16];
+                        tmem_ld16(tp + (uint32_t)col, p);
+                        tmem_ld16(tlane + (uint32_t)((c ^ 1) * kTokMax + col), p1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) p[i] = __float_as_uint(__fadd_rn(__uint_as_float(p[i]), __uint_as_float(p1[i])));
+                        tmem_st16(tp + (uint32_t)col, p);
+                    }
+                    tmem_st_wait();
+                }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
                     const int col = (2 * g + ch0) * 16;
                     if (col < cx.n) {           // warp-uniform
-                        uint32_t p[16], l[16];
-                        tmem_ld16(tlane + (uint32_t)(c * kTokMax + col), p);
-                        if constexpr (F::kMins) tmem_ld16(tlane + (uint32_t)(kColL + col), l);
+                        uint32_t p[16], l[16];      // l: L, or the sum of the second plane
+                        tmem_ld16(tp + (uint32_t)col, p);
+                        tmem_ld16(tlane + (uint32_t)((F::kMins ? kColL : kTokMax) + col), l);
                         tmem_ld_wait();
 #pragma unroll
                         for (int i = 0; i < 8; i += 2) {
@@ -559,10 +635,10 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 #pragma unroll
                             for (int e = 0; e < 2; ++e) {
                                 const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
-                                const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
+                                const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]), lv = pack2(l[2 * (i + e)], l[2 * (i + e) + 1]);
                                 uint64_t tv;
-                                if constexpr (F::kMins) tv = fma2(dw, pv, mul2(ndm, pack2(l[2 * (i + e)], l[2 * (i + e) + 1])));
-                                else tv = mul2(dw, pv);
+                                if constexpr (F::kMins) tv = fma2(dw, pv, mul2(ndm, lv));
+                                else tv = mul2(dw, fma2(one, pv, lv));
                                 acc[g][i + e] = fma2(dd, tv, acc[g][i + e]);
                             }
                         }

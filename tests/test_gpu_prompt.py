@@ -10,7 +10,7 @@ import torch
 
 from candle_b200 import capi
 from candle_b200.quantized import GgmlDType, QMatMul, QTensor
-from helpers import make_case, rel_err
+from helpers import TSIZE, make_case, rel_err
 
 pytestmark = pytest.mark.gpu
 ELEM = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
@@ -58,6 +58,63 @@ def test_prompt_matmul(lib, oracle, cuda_dev, tokens, k, n, wtype, dtype):
     if dtype == torch.float32 and tokens <= 333:
         assert rel_err(out.cpu().numpy(), oracle.matmul(wtype, x, wq, n)) <= 1e-5
     assert torch.equal(out, _int8(lib, wtype, w_dev, x_dev, k, n))
+
+
+def _large_sums(wtype, n, k, kind, rng):
+    """Blocks whose integer sums leave 24 bits: scales and codes near their largest, odd ones among them.  "two signs": the second
+    half of a super-block takes back what the first has added."""
+    nsb = k // 256
+    b = rng.integers(0, 256, (n * nsb, TSIZE[wtype]), dtype=np.uint8)
+    d = (rng.random((n * nsb, 2)) * 1e-4 + 1e-4).astype(np.float16)
+    if wtype == 12:
+        b[:, :4] = d.view(np.uint8)
+        b[:, 4:16] = 0xFF                                        # scales and minima 63
+        b[:, 16:] |= 0 if kind == "two signs" else 0xCC          # codes any, or 12 .. 15
+    else:
+        b[:, :192] |= 0xFC                                       # codes 60 .. 63
+        sc = rng.integers(117, 128, (n * nsb, 16)).astype(np.int8)
+        if kind == "two signs":
+            sc[:, 8:] *= -1
+        b[:, 192:208] = sc.view(np.uint8)
+        b[:, 208:] = d[:, :1].view(np.uint8)
+    return b.reshape(n, -1)
+
+
+# every accumulator of a tile: two halves of the tokens, ragged ones, a tile of 16
+@pytest.mark.parametrize("tokens", [16, 40, 128, 150])
+@pytest.mark.parametrize("wtype", [12, 14])
+@pytest.mark.parametrize("kind", ["one sign", "two signs", "some super-blocks"])
+def test_prompt_matmul_of_sums_past_24_bits(lib, oracle, cuda_dev, tokens, wtype, kind):
+    """The integers are exact for any data (activations of one sign reach +-127 throughout): the bits of the int32 accumulators."""
+    rng = np.random.default_rng(tokens + wtype)
+    k, n = (1024, 200) if kind != "some super-blocks" else (2304, 20000)        # the second: several tiles per CTA
+    wq = _large_sums(wtype, n, k, kind, rng)
+    x = (1.0 - 0.06 * rng.random((tokens, k))).astype(np.float32)
+    x[1::3] *= -1
+    if kind == "some super-blocks":         # 1, 4, 5, 6 of one sign (6 for one token only), the others normal
+        other = ~np.isin(np.arange(k) // 256, (1, 4, 5, 6))
+        x[:, other] = rng.standard_normal((tokens, int(other.sum())))
+        x[:tokens - 1, 6 * 256:7 * 256] = rng.standard_normal((tokens - 1, 256))
+    if kind == "two signs" and wtype == 12:
+        x[:, np.arange(k) % 256 >= 128] *= -1
+    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
+    out = _prompt(lib, wtype, w_dev, x_dev, k, n)
+    assert torch.equal(out, _int8(lib, wtype, w_dev, x_dev, k, n))
+    if kind == "one sign":
+        assert rel_err(out.cpu().numpy(), oracle.matmul(wtype, x, wq, n)) <= 1e-5
+
+
+@pytest.mark.parametrize("wtype", [12, 14])
+def test_prompt_matmul_of_non_finite_activations(lib, oracle, cuda_dev, wtype):
+    """NaN and infinite activations (int8 -128): the same bits, NaNs in the same places, the other tokens untouched."""
+    _, x, wq = make_case(oracle, wtype, 512, 65, 40, seed=9)
+    x[3, 5], x[7, ::2], x[11, 300], x[13, 256:] = np.nan, np.nan, np.inf, -np.inf
+    x[17] = 1e-41
+    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
+    scratch, out = torch.zeros(lib.cq_prompt_scratch_bytes(40, 512), dtype=torch.uint8, device=cuda_dev), torch.empty((40, 65), device=cuda_dev)
+    lib.cq_prompt_matmul(wtype, w_dev.data_ptr(), x_dev.data_ptr(), capi.F32, out.data_ptr(), scratch.data_ptr(), 512, 65, 40, 65, torch.cuda.current_stream().cuda_stream)
+    capi.check("prompt")
+    assert torch.equal(out.nan_to_num(1e30, 2e30, 3e30), _int8(lib, wtype, w_dev, x_dev, 512, 65).nan_to_num(1e30, 2e30, 3e30))
 
 
 def test_prompt_matmul_unaligned_activations(lib, oracle, cuda_dev):

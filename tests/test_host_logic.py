@@ -104,3 +104,16 @@ def test_prompt_attention_is_taken_where_it_is_the_faster(lib):
         assert fast < slow and lib.cq_attention_reads_by_32(*shape) == 1, shape
     assert lib.cq_attention_reads_by_32(2, 512, 32, 1161) == 0          # its scores do not fit shared memory
     assert lib.cq_attention_reads_by_32(64, 16, 64, 128) == 0
+
+
+def test_operands_of_the_super_block_prompt_kernel_are_exact():
+    """csrc/prompt_kq.cu: the f16 operands and the largest partial sum of every accumulator, for all scales and codes."""
+    q, sc = np.meshgrid(np.arange(64), np.arange(-128, 128))
+    y, prod = q - 32, (q - 32) * sc
+    a = (prod + 12288).astype(np.float16).astype(np.int64) - 12288       # f32 -> f16 rounds as the fma does: the product is exact before it
+    assert np.array_equal((1024 + q).astype(np.float16).astype(np.int64) - 1056, y)
+    for part in (a, prod - a):
+        assert np.array_equal(part.astype(np.float16).astype(np.int64), part)
+    assert np.all(a % 8 == 0) and 256 * 128 * np.abs(a).max() <= 8 * 2 ** 24 and 256 * 128 * np.abs(prod - a).max() <= 2 ** 24
+    # Q4_K: one accumulator per 128 elements, or per super-block up to the stored limit of sum |q8|
+    assert 128 * 128 * 63 * 15 <= 2 ** 24 < 256 * 127 * 63 * 15 and (2 ** 24 // 945) * 945 <= 2 ** 24 and 16 * 63 * 2048 <= 2 ** 24
