@@ -110,6 +110,7 @@ def lib() -> C.CDLL:
         L.cq_moe_block_decode_scratch_bytes.argtypes = [i32, i32, i32, i32]
         L.cq_moe_block_decode_scratch_bytes.restype = C.c_size_t
         L.cq_moe_block_decode.argtypes = [i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
+        L.cq_moe_block_decode_pairs.argtypes = [i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
         L.cq_moe_route_f32.argtypes = [vp, vp, vp, i32, i32, i32, i32, vp]
         L.cq_moe_router_f32.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
         L.cq_moe_router_f32.restype = None

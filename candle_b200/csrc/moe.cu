@@ -293,46 +293,73 @@ extern "C" void cq_moe_sort_pairs(const int32_t *ids, int pairs, int num_experts
 
 // The expert products of a block for few tokens: x f32 [tokens, hidden] is quantized once, gate and up run as one launch (the
 // tasks of cq_indexed_moe_forward), up * silu(gate) is stored as Q8_1 containers, down, then the weighted sum over a token's
-// experts: five launches.  The arithmetic of moe_gemm_gguf; wtype / wtype_down: formats of gate and up / of down.
+// experts: five launches.  The arithmetic of moe_gemm_gguf; wtype / wtype_down: formats of gate and up / of down.  The form that ends
+// with the pairs' products is what a rank with a part of the experts runs: ids outside [0, num_experts) take no part.
 extern "C" size_t cq_moe_block_decode_scratch_bytes(int tokens, int topk, int hidden, int ffn) {
     if (tokens <= 0 || topk <= 0 || hidden <= 0 || ffn <= 0) return 0;
     const size_t pairs = (size_t)tokens * topk, kh = (hidden + 511) / 512 * 16 * CQ_Q8_BYTES, kf = (ffn + 511) / 512 * 16 * CQ_Q8_BYTES;
     return (tokens * kh + pairs * kf + 255) / 256 * 256 + pairs * ((size_t)ffn * 8 + (size_t)hidden * 4);
 }
 
+namespace {
+struct BlockScratch {
+    int kh, kf;         // padded row lengths of x and of the activations between the products
+    uint8_t *qx, *qa;
+    float *gate, *up, *y;
+    BlockScratch(void *scratch, int tokens, int topk, int hidden, int ffn) {
+        const size_t pairs = (size_t)tokens * topk;
+        kh = (hidden + 511) / 512 * 512, kf = (ffn + 511) / 512 * 512;
+        const size_t x_bytes = (size_t)tokens * (kh / 32) * CQ_Q8_BYTES, q_bytes = x_bytes + pairs * (kf / 32) * CQ_Q8_BYTES;
+        qx = (uint8_t *)scratch, qa = qx + x_bytes;
+        gate = (float *)(qx + (q_bytes + 255) / 256 * 256), up = gate + pairs * ffn, y = up + pairs * ffn;
+    }
+};
+bool block_pairs(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down, const int32_t *ids, float *y,
+                 const BlockScratch &s, int num_experts, int topk, int tokens, int hidden, int ffn, cudaStream_t st) {
+    const int pairs = tokens * topk;
+    if (!check_common(gate, s.qx, s.gate, wtype, ffn, hidden, pairs, "block") || !check_common(up, s.qx, s.up, wtype, ffn, hidden, pairs, "block") ||
+        !check_common(down, s.qa, y, wtype_down, hidden, ffn, pairs, "block"))
+        return false;
+    cq_quantize_act(x, CQ_ELEM_F32, s.qx, hidden, s.kh, tokens, CQ_ACT_Q8_1_ENC, st);
+    MoeArgs a{};
+    a.w = (const uint8_t *)gate; a.w2 = (const uint8_t *)up; a.y = s.qx; a.out = s.gate; a.out2 = s.up; a.expert_ids = ids;
+    a.stride_col_y = s.kh / 32; a.num_experts = num_experts; a.topk = topk; a.indexed = 1; a.input_dim1 = 1;
+    bool ok = dispatch(wtype, CQ_ACT_Q8_1, a, hidden, ffn, pairs, st);
+    if (ok) {
+        gate_up_q8_1_kernel<<<dim3((ffn + 1023) / 1024, pairs), 256, 0, st>>>(s.gate, s.up, s.qa, ffn, s.kf / 32);
+        a.w = (const uint8_t *)down; a.w2 = nullptr; a.y = s.qa; a.out = y; a.out2 = nullptr;
+        a.stride_col_y = s.kf / 32; a.input_dim1 = topk;
+        ok = dispatch(wtype_down, CQ_ACT_Q8_1, a, ffn, hidden, pairs, st);
+    }
+    if (!ok && cq_last_status() == CQ_OK) cq_set_status(CQ_ERR_UNSUPPORTED, "moe block: shape outside what the kernel covers");
+    return ok;
+}
+bool block_args_ok(const void *x, const void *gate, const void *up, const void *down, const void *ids, const void *out, const void *scratch,
+                   int num_experts, int topk, int tokens) {
+    if (!x || !gate || !up || !down || !ids || !out || !scratch || tokens <= 0 || topk <= 0 || num_experts <= 0 || (int64_t)tokens * topk > 65535 ||
+        (uintptr_t)scratch % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe block: null pointer, empty shape, more than 65535 pairs or misaligned scratch");
+        return false;
+    }
+    return true;
+}
+}  // namespace
+
 extern "C" void cq_moe_block_decode(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down,
                                     const int32_t *ids, const float *topk_weights, float *out, void *scratch, int num_experts, int topk,
                                     int tokens, int hidden, int ffn, void *stream) {
-    if (!x || !gate || !up || !down || !ids || !topk_weights || !out || !scratch || tokens <= 0 || topk <= 0 || num_experts <= 0 ||
-        (int64_t)tokens * topk > 65535 || (uintptr_t)scratch % 256 != 0) {
-        cq_set_status(CQ_ERR_BAD_ARG, "moe block: null pointer, empty shape, more than 65535 pairs or misaligned scratch");
-        return;
-    }
-    cudaStream_t st = (cudaStream_t)stream;
-    const int pairs = tokens * topk, kh = (hidden + 511) / 512 * 512, kf = (ffn + 511) / 512 * 512;
-    const size_t q_bytes = ((size_t)tokens * (kh / 32) + (size_t)pairs * (kf / 32)) * CQ_Q8_BYTES;
-    uint8_t *qx = (uint8_t *)scratch, *qa = qx + (size_t)tokens * (kh / 32) * CQ_Q8_BYTES;
-    float *g = (float *)(qx + (q_bytes + 255) / 256 * 256);
-    float *u = g + (size_t)pairs * ffn, *y = u + (size_t)pairs * ffn;
-    if (!check_common(gate, qx, g, wtype, ffn, hidden, pairs, "block") || !check_common(up, qx, u, wtype, ffn, hidden, pairs, "block") ||
-        !check_common(down, qa, y, wtype_down, hidden, ffn, pairs, "block"))
-        return;
-    cq_quantize_act(x, CQ_ELEM_F32, qx, hidden, kh, tokens, CQ_ACT_Q8_1_ENC, st);
-    MoeArgs a{};
-    a.w = (const uint8_t *)gate; a.w2 = (const uint8_t *)up; a.y = qx; a.out = g; a.out2 = u; a.expert_ids = ids;
-    a.stride_col_y = kh / 32; a.num_experts = num_experts; a.topk = topk; a.indexed = 1; a.input_dim1 = 1;
-    bool ok = dispatch(wtype, CQ_ACT_Q8_1, a, hidden, ffn, pairs, st);
-    if (ok) {
-        gate_up_q8_1_kernel<<<dim3((ffn + 1023) / 1024, pairs), 256, 0, st>>>(g, u, qa, ffn, kf / 32);
-        a.w = (const uint8_t *)down; a.w2 = nullptr; a.y = qa; a.out = y; a.out2 = nullptr;
-        a.stride_col_y = kf / 32; a.input_dim1 = topk;
-        ok = dispatch(wtype_down, CQ_ACT_Q8_1, a, ffn, hidden, pairs, st);
-    }
-    if (!ok) {
-        if (cq_last_status() == CQ_OK) cq_set_status(CQ_ERR_UNSUPPORTED, "moe block: shape outside what the kernel covers");
-        return;
-    }
-    cq_moe_weighted_sum_f32(y, topk_weights, out, tokens, topk, hidden, st);
+    if (!block_args_ok(x, gate, up, down, ids, topk_weights ? out : nullptr, scratch, num_experts, topk, tokens)) return;
+    const BlockScratch s(scratch, tokens, topk, hidden, ffn);
+    if (block_pairs(wtype, wtype_down, x, gate, up, down, ids, s.y, s, num_experts, topk, tokens, hidden, ffn, (cudaStream_t)stream))
+        cq_moe_weighted_sum_f32(s.y, topk_weights, out, tokens, topk, hidden, stream);
+}
+
+extern "C" void cq_moe_block_decode_pairs(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down,
+                                          const int32_t *ids, float *out, void *scratch, int num_experts, int topk, int tokens, int hidden,
+                                          int ffn, void *stream) {
+    if (!block_args_ok(x, gate, up, down, ids, out, scratch, num_experts, topk, tokens)) return;
+    block_pairs(wtype, wtype_down, x, gate, up, down, ids, out, BlockScratch(scratch, tokens, topk, hidden, ffn), num_experts, topk, tokens, hidden,
+                ffn, (cudaStream_t)stream);
 }
 
 extern "C" int cq_moe_timeout_flag(void) {

@@ -3,12 +3,13 @@
 Mirrors candle-transformers/src/fused_moe.rs:222-301 (``FusedMoeGGUF::forward``): router logits -> softmax -> the
 ``num_experts_per_tok`` largest weights per token (optionally renormalised) -> (token, expert) pairs sorted by expert ->
 ``moe_gemm_gguf`` for gate and up, ``up * act(gate)``, ``moe_gemm_gguf`` for down with the routing weights applied ->
-sum over the token's experts.  The router is a dense f32 linear layer (candle de-quantizes it at load); routing itself is
-a handful of small tensor operations; everything heavy goes through the expert-indexed GEMV of libcandle_q_b200.
+sum over the token's experts.  The router is a dense f32 linear layer (candle de-quantizes it at load).  The block runs as a few
+launches of libcandle_q_b200 (`_block`); shapes and formats outside of those take the single calls with tensor operations between them.
 
 Expert parallelism: a rank may own a contiguous range of experts.  Pairs routed elsewhere write nothing (the kernels
 skip expert ids outside their range), every pair is produced by exactly one rank, so summing the pair outputs across
-ranks adds one value and zeros - exact in any order - and the result has the same bits for any number of ranks.
+ranks adds one value and zeros - exact in any order.  Which of the two forms runs, and which kernels inside, depends on the layer and
+on the number of pairs only, so the result has the same bits for any number of ranks.
 """
 from __future__ import annotations
 
@@ -57,45 +58,64 @@ class FusedMoeGGUF:
         self.expert_offset, self.group, self.world = expert_offset, group, world
 
     def _block(self, x: torch.Tensor, is_prefill: bool) -> torch.Tensor | None:
-        """The block as a few launches of libcandle_q_b200 (all experts local); None: the general path has to run.  The
-        expert products are those of `moe_gemm_gguf` - same kernels, same rule for which of them a prompt takes."""
-        e, ffn, hidden = self.gate_experts.shape
-        tokens, k = x.shape[0], self.num_experts_per_tok
+        """The block as a few launches of libcandle_q_b200; None: the general path has to run.  The expert products are those of
+        `moe_gemm_gguf` - same kernels, same rule for which of them a prompt takes, on the layer's experts, not this rank's."""
+        local, ffn, hidden = self.gate_experts.shape
+        experts, tokens, k = self.gate.shape[0], x.shape[0], self.num_experts_per_tok
         gu, down = self.gate_experts.dtype, self.down_experts.dtype
-        if self.world > 1 or self.expert_offset != 0 or e != self.gate.shape[0] or e > 1024 or not 0 < k <= min(32, e) or tokens == 0 or \
-                not x.is_cuda or self.up_experts.dtype != gu or gu not in _CODE or down not in _CODE or x.shape[1] != hidden or \
+        if experts > 1024 or not 0 < k <= min(32, experts) or tokens == 0 or not x.is_cuda or self.up_experts.dtype != gu or \
+                gu not in _CODE or down not in _CODE or x.shape[1] != hidden or \
                 any(w.device != x.device for w in (self.gate_experts, self.up_experts, self.down_experts)):
             return None
         pairs, dev, lib = tokens * k, x.device, capi.lib()
         kind = {torch.float16: capi.F16, torch.bfloat16: capi.BF16}.get(self.prefill_dtype)
         if is_prefill:
-            need = lib.cq_moe_block_prompt_scratch_bytes(pairs, e, hidden, ffn)
-            if kind is None or need == 0 or pairs < max(64, 4 * e) or {gu, down} - {GgmlDType.Q4K, GgmlDType.Q6K}:
+            need = lib.cq_moe_block_prompt_scratch_bytes(pairs, local, hidden, ffn)
+            if kind is None or need == 0 or self._few_pairs(pairs) or {gu, down} - {GgmlDType.Q4K, GgmlDType.Q6K}:
                 return None
         else:
             need = lib.cq_moe_block_decode_scratch_bytes(tokens, k, hidden, ffn)
             if pairs > 65535:
                 return None
+        part = self.world > 1 or self.expert_offset != 0 or local != experts       # pairs of other ranks must read as zero
         with torch.cuda.device(dev):
             st = torch.cuda.current_stream(dev).cuda_stream
             logits = torch.nn.functional.linear(x, self.gate).to(torch.float32).contiguous()      # autocast gives 16 bits
             ids = torch.empty((3, pairs), dtype=torch.int32, device=dev)        # by token; then experts and pairs, sorted
             weights = torch.empty((tokens, k), dtype=torch.float32, device=dev)
             scratch = torch.empty(need, dtype=torch.uint8, device=dev)
-            lib.cq_moe_route_f32(logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, e, k, 1 if self.norm_topk_prob else 0, st)
+            lib.cq_moe_route_f32(logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, experts, k, 1 if self.norm_topk_prob else 0, st)
+            if self.expert_offset:
+                ids[0] -= self.expert_offset        # ids outside [0, local) are skipped by the kernels
             g, u, d = (w.device_ptr() for w in (self.gate_experts, self.up_experts, self.down_experts))
+            if is_prefill or part:
+                y = (torch.zeros if part else torch.empty)((pairs, hidden), dtype=torch.float32, device=dev)
             if is_prefill:
-                out = torch.empty((pairs, hidden), dtype=torch.float32, device=dev)
-                lib.cq_moe_sort_pairs(ids.data_ptr(), pairs, e, ids[1].data_ptr(), ids[2].data_ptr(), st)
+                lib.cq_moe_sort_pairs(ids.data_ptr(), pairs, local, ids[1].data_ptr(), ids[2].data_ptr(), st)
                 lib.cq_moe_block_prompt(int(gu), int(down), x.data_ptr(), kind, g, u, d, ids[2].data_ptr(), ids[1].data_ptr(),
-                                        weights.data_ptr(), out.data_ptr(), scratch.data_ptr(), e, k, pairs, hidden, ffn, st)
-                out = out.view(tokens, k, hidden).sum(dim=1)
+                                        weights.data_ptr(), y.data_ptr(), scratch.data_ptr(), local, k, pairs, hidden, ffn, st)
+            elif part:
+                lib.cq_moe_block_decode_pairs(int(gu), int(down), x.data_ptr(), g, u, d, ids.data_ptr(), y.data_ptr(), scratch.data_ptr(),
+                                              local, k, tokens, hidden, ffn, st)
             else:
                 out = torch.empty((tokens, hidden), dtype=torch.float32, device=dev)
                 lib.cq_moe_block_decode(int(gu), int(down), x.data_ptr(), g, u, d, ids.data_ptr(), weights.data_ptr(), out.data_ptr(),
-                                        scratch.data_ptr(), e, k, tokens, hidden, ffn, st)
+                                        scratch.data_ptr(), local, k, tokens, hidden, ffn, st)
+            if self.world > 1:
+                capi.check("moe block")
+                dist.all_reduce(y, op=dist.ReduceOp.SUM, group=self.group)      # one value plus zeros per element: exact
+            if is_prefill:
+                out = y.view(tokens, k, hidden).sum(dim=1)
+            elif part:
+                out = torch.empty((tokens, hidden), dtype=torch.float32, device=dev)
+                lib.cq_moe_weighted_sum_f32(y.data_ptr(), weights.data_ptr(), out.data_ptr(), tokens, k, hidden, st)
         capi.check("moe block")
         return out
+
+    def _few_pairs(self, pairs: int) -> bool:
+        """The rule of `moe_gemm_gguf_prefill` for prompts that stay on the GEMV, counted on the layer's experts so that it does not
+        depend on how many ranks share them."""
+        return pairs < max(64, 4 * self.gate.shape[0]) or self.gate.shape[0] > 1024
 
     def forward(self, xs: torch.Tensor, is_prefill: bool) -> torch.Tensor:
         batch, seq_len, hidden = xs.shape
@@ -108,13 +128,16 @@ class FusedMoeGGUF:
         topk_weights, topk_ids = route(torch.nn.functional.linear(x, self.gate), k, self.norm_topk_prob)
         expert_ids, sorted_token_ids = sort_pairs(topk_ids)
         local_ids = expert_ids - self.expert_offset          # ids outside [0, local experts) are skipped by the kernels
-        xin = x.to(self.prefill_dtype) if is_prefill else x  # the reference casts for its prefill kernel (moe.rs:310-333)
+        cast = (lambda t: t.to(self.prefill_dtype)) if is_prefill else (lambda t: t)      # the reference casts for its prefill kernel (moe.rs:310-333)
+        if is_prefill and self.world > 1 and self._few_pairs(num_tokens * k):
+            # With this rank's experts alone the prompt entry point could take the tensor cores where one rank takes the GEMV; the
+            # decode entry point on the cast values is that GEMV.
+            cast, is_prefill = (lambda t: t.to(self.prefill_dtype).to(torch.float32)), False
+        xin = cast(x)
         zero = self.world > 1                                 # pairs of other ranks must read as zero
         gate = moe_gemm_gguf(xin, self.gate_experts, None, sorted_token_ids, local_ids, k, is_prefill, zero_init=zero)
         up = moe_gemm_gguf(xin, self.up_experts, None, sorted_token_ids, local_ids, k, is_prefill, zero_init=zero)
-        down_in = up * torch.nn.functional.silu(gate)         # [pairs, intermediate]
-        if is_prefill:
-            down_in = down_in.to(self.prefill_dtype)
+        down_in = cast(up * torch.nn.functional.silu(gate))   # [pairs, intermediate]
         ys = moe_gemm_gguf(down_in, self.down_experts, topk_weights, sorted_token_ids, local_ids, k, is_prefill, zero_init=zero)
         if self.world > 1:
             dist.all_reduce(ys, op=dist.ReduceOp.SUM, group=self.group)      # one value plus zeros per element: exact

@@ -214,7 +214,7 @@ void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *
                          const int32_t *expert_ids, const float *topk_weights, float *out, void *scratch, int num_experts,
                          int topk, int size_m, int size_n, int size_k, void *stream);
 
-/* The expert part of a mixture-of-experts block (gate, up, up * silu(gate), down) with all experts in place.
+/* The expert part of a mixture-of-experts block (gate, up, up * silu(gate), down).
  *   cq_moe_sort_pairs   : i32 ids [pairs] -> expert_ids ascending, and the pair numbers in that order (stable); ids outside
  *                         [0, num_experts) come last, as num_experts: the expert products skip those pairs.
  *   cq_moe_block_prompt : many tokens, Q4_K / Q6_K: x f32 [size_m / topk, hidden] rounded to `kind` (CQ_ELEM_F16 / BF16) -> out f32
@@ -222,6 +222,8 @@ void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *
  *                         arithmetic of three cq_moe_prefill_gemm calls on inputs of that type.  hidden, ffn multiples of 256.
  *   cq_moe_block_decode : few tokens, formats of moe_gemm_gguf: x f32 [tokens, hidden], ids i32 / topk_weights f32 [tokens, topk]
  *                         -> out f32 [tokens, hidden], the weighted sums.
+ *   cq_moe_block_decode_pairs : the same up to the products of the pairs, out f32 [tokens * topk, hidden], unscaled; pairs whose id is
+ *                         outside [0, num_experts) are not written (another rank's experts).
  * scratch: the *_scratch_bytes of the call, 256-byte aligned. */
 void cq_moe_sort_pairs(const int32_t *ids, int pairs, int num_experts, int32_t *expert_ids, int32_t *sorted_token_ids, void *stream);
 size_t cq_moe_block_prompt_scratch_bytes(int size_m, int num_experts, int hidden, int ffn);
@@ -232,6 +234,9 @@ size_t cq_moe_block_decode_scratch_bytes(int tokens, int topk, int hidden, int f
 void cq_moe_block_decode(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down,
                          const int32_t *ids, const float *topk_weights, float *out, void *scratch, int num_experts, int topk,
                          int tokens, int hidden, int ffn, void *stream);
+void cq_moe_block_decode_pairs(int wtype, int wtype_down, const float *x, const void *gate, const void *up, const void *down,
+                               const int32_t *ids, float *out, void *scratch, int num_experts, int topk, int tokens, int hidden, int ffn,
+                               void *stream);
 
 /* Prefill path (many tokens) on the int8 tensor cores, Q4_K weights.  Replaces the pair
  * launch_mmq_quantize_q8_1_* + launch_mmq_gguf_q4_k of candle-kernels/src/ffi.rs:424-630 for callers that go through

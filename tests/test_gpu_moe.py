@@ -500,3 +500,33 @@ def test_fused_moe_few_launches_against_the_general_path(cuda_dev, wt_gu, wt_dow
     moe._block = lambda *a: None
     ref = moe.forward(x, is_prefill)
     assert float((ys - ref).norm() / ref.norm()) <= (2e-3 if is_prefill else 1e-4)
+
+
+@pytest.mark.parametrize("wt_gu,wt_down", [(12, 14), (8, 8)])
+@pytest.mark.parametrize("experts,tokens,is_prefill", [(6, 5, False), (6, 33, True), (6, 300, True), (32, 20, True), (32, 70, True)])
+def test_fused_moe_has_the_same_bits_for_any_number_of_ranks(cuda_dev, monkeypatch, wt_gu, wt_down, experts, tokens, is_prefill):
+    """Two ranks run one after the other, the all-reduce replaced by the sum of what both handed to it, against one rank.  (32, 20): few
+    pairs for 32 experts, enough for the tensor cores if the 16 of one rank were counted."""
+    import candle_b200.fused_moe as fm
+    from candle_b200.synth import random_blocks
+    topk, hidden, ffn, half = 4, 512, 768, experts // 2
+    g = torch.Generator(device=cuda_dev).manual_seed(tokens)
+    router = torch.randn(experts, hidden, device=cuda_dev, generator=g) * 0.1
+    x = torch.randn(1, tokens, hidden, device=cuda_dev, generator=g)
+    dims = [(wt_gu, ffn, hidden), (wt_gu, ffn, hidden), (wt_down, hidden, ffn)]
+    blocks = [random_blocks(GgmlDType(wt), experts * n, k, seed=i, device=cuda_dev).reshape(experts, -1) for i, (wt, n, k) in enumerate(dims)]
+
+    def block(lo, hi, world):
+        w = [QTensor.from_device_blocks(b[lo:hi].reshape(-1).clone(), GgmlDType(wt), (hi - lo, n, k)) for b, (wt, n, k) in zip(blocks, dims)]
+        return fm.FusedMoeGGUF(router, *w, topk, expert_offset=lo, world=world)
+
+    one = block(0, experts, 1).forward(x, is_prefill)
+    ranks = [block(0, half, 2), block(half, experts, 2)]
+    sent = []
+    monkeypatch.setattr(fm.dist, "all_reduce", lambda t, **kw: sent.append(t.clone()))
+    for r in ranks:
+        r.forward(x, is_prefill)
+    assert len(sent) == 2 and not bool(((sent[0] != 0) & (sent[1] != 0)).any())
+    monkeypatch.setattr(fm.dist, "all_reduce", lambda t, **kw: t.copy_(sent[0] + sent[1]))
+    for r in ranks:
+        assert torch.equal(r.forward(x, is_prefill), one)
