@@ -5,7 +5,7 @@
 //
 // Both sides of a product carry a scale per 32 elements, so nothing beyond the integer sub-scales of a K-quant can be folded
 // into the operands: every 32-element block is two K = 16 steps into a FRESH accumulator slot, exact (sums below 2^24: at most
-// 31 * 63 * 127 * 32), and the epilogue adds  d_a * (d_w * I) [+ m_w * s_a]  to f32 running sums, two at a time.
+// 31 * 63 * 127 * 32), and the epilogue adds  d_a d_w I [+ m_w s_a]  to f32 running sums, two at a time.
 // Against int8 operands the epilogue needs no int -> float conversion, which was two of its five operations per value.
 //
 // Summation: Q8_0 / Q4_0 add block after block, as the kernel behind cq_prefill32_gemm does (the same f32 operations, the same
@@ -32,22 +32,27 @@ constexpr int kColA = 384;
 
 __device__ int g_prompt_b32_timeout_flag = 0;
 
-// kMins: terms m_w * s_a per block;  kSum: what s_a is
+// kMins: terms m_w * s_a per block;  kSum: what s_a is;  kTerm: a block's terms are summed apart from the running sum.  The codes are unsigned,
+// so d_a d_w I and m_w s_a are both large and nearly cancel for weights around zero; added to the running sum one after the other they left
+// two to four times the decode kernels' error against 64 bits (2-norm, K = 4096, activations of one sign: Q4_1 2.2e-7 for 7.6e-8, Q5_1 2.6e-7
+// for 7.7e-8; now 6.7e-8 and 6.9e-8), for 2 - 4 % of the time.  Q5_K stays below the decode kernel's own error without (normal activations
+// 1.0e-7 for 1.1e-7, one sign 2.8e-7 for 4.9e-7).
 enum { kNoSum, kFloatSum, kIntSum };
 template <int WTYPE> struct Fmt {       // Q8_0, Q4_0
     static constexpr bool kQ81 = false;
     static constexpr int kMins = 0, kSum = kNoSum, kTok = 64, kStagesT = 4;
+    static constexpr bool kTerm = false;
 };
-template <int MINS, int SUM> struct FmtQ81 {
-    static constexpr bool kQ81 = true;
+template <int MINS, int SUM, bool TERM> struct FmtQ81 {
+    static constexpr bool kQ81 = true, kTerm = TERM;
     static constexpr int kMins = MINS, kSum = SUM, kTok = 64, kStagesT = 4;
 };
-template <> struct Fmt<CQ_Q4_1> : FmtQ81<1, kFloatSum> {};
-template <> struct Fmt<CQ_Q5_0> : FmtQ81<1, kFloatSum> {};
-template <> struct Fmt<CQ_Q5_1> : FmtQ81<1, kFloatSum> {};
-template <> struct Fmt<CQ_Q5_K> : FmtQ81<1, kIntSum> {};
-template <> struct Fmt<CQ_Q2_K> : FmtQ81<2, kIntSum> {};     // one per 16 elements
-template <> struct Fmt<CQ_Q3_K> : FmtQ81<0, kNoSum> {};
+template <> struct Fmt<CQ_Q4_1> : FmtQ81<1, kFloatSum, true> {};
+template <> struct Fmt<CQ_Q5_0> : FmtQ81<1, kFloatSum, true> {};
+template <> struct Fmt<CQ_Q5_1> : FmtQ81<1, kFloatSum, true> {};
+template <> struct Fmt<CQ_Q5_K> : FmtQ81<1, kIntSum, false> {};
+template <> struct Fmt<CQ_Q2_K> : FmtQ81<2, kIntSum, true> {};     // one per 16 elements
+template <> struct Fmt<CQ_Q3_K> : FmtQ81<0, kNoSum, false> {};
 
 template <int WTYPE> constexpr int chunk_bytes() { return 256 / cq_block_elems(WTYPE) * cq_type_size(WTYPE); }
 template <int MINS> constexpr int tok_bytes() { return 512 + 32 + 32 * MINS; }        // f16 values, scales, sums of one chunk
@@ -569,10 +574,16 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                                     for (int e = 0; e < 2; ++e) {
                                         const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
                                         const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
-                                        // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel; else d_a (d_w I)
-                                        uint64_t v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
-                                        if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
-                                        if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
+                                        // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel
+                                        uint64_t v;
+                                        if constexpr (F::kTerm) {       // the block's two large parts meet before they are added to others
+                                            v = mul2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y));
+                                            if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
+                                            v = fma2(one, fma2(mul2(dw, dd), pv, v), acc[g][i + e]);      // d_w d_a: two f16, exact
+                                        } else {
+                                            v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
+                                            if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
+                                        }
                                         acc[g][i + e] = v;
                                     }
                                 }

@@ -172,3 +172,60 @@ def test_qmatmul_routes_rows_past_one_decode_launch(oracle, cuda_dev, wtype):
     y = mm.forward(xd.view(3, 7, 512)).view(21, 96)
     ref = torch.cat([mm.forward(xd[i:i + 7]) for i in (0, 7, 14)])
     assert rel_err(y.cpu().numpy(), ref.cpu().numpy()) <= 2e-6
+
+
+@pytest.mark.parametrize("one_sign", [False, True])
+@pytest.mark.parametrize("wtype,scale,minimum,mid", [(3, 0, 2, -7.5), (6, 0, None, 0.0), (7, 0, 2, -15.5), (10, 80, 82, 1.5), (11, 108, None, 0.0), (13, 0, 2, 15.5)])
+def test_prompt32_is_no_further_from_64_bits_than_the_decode_kernel(lib, cuda_dev, wtype, scale, minimum, mid, one_sign):
+    """Weights around zero, whose codes' part and minimum's part nearly cancel in every block.  `scale`, `minimum`: where a block keeps
+    its f16 fields; the minimum is `mid` scales, the middle of the codes.  10 % for the two kernels' different roundings."""
+    n, m, k = 96, 64, 4096
+    per = 32 if wtype < 10 else 256
+    gen = torch.Generator(device=cuda_dev).manual_seed(wtype)
+    b = torch.randint(0, 256, (n * k // per, TSIZE[wtype]), dtype=torch.uint8, device=cuda_dev, generator=gen)
+
+    def put(b, off, v):
+        b[:, off:off + 2] = v.to(torch.float16).view(torch.uint8).view(-1, 2)
+
+    def values(b, d, mn):           # the integers of all elements (d = 1, minimum 0), or the minima's (d = 0, minimum 1), exact in f32
+        b = b.clone()
+        put(b, scale, torch.full((b.shape[0],), d, device=cuda_dev))
+        if minimum is not None:
+            put(b, minimum, torch.full((b.shape[0],), mn, device=cuda_dev))
+        return QTensor.from_device_blocks(b.reshape(-1), GgmlDType(wtype), (n, k)).dequantize(torch.float32).double()
+
+    d = ((torch.rand(b.shape[0], device=cuda_dev, generator=gen) * 0.5 + 0.75) * 1e-3).half().float()
+    put(b, scale, d)
+    if minimum is not None:
+        put(b, minimum, d * mid)
+    if wtype == 10:                 # minima codes = scale codes
+        b[:, :16] = (b[:, :16] & 15) * 17
+    if wtype == 13:                 # the same in the 6-bit fields
+        b[:, 8:12] = b[:, 4:8]
+        b[:, 12:16] = (b[:, 12:16] & 15) * 17
+    spread = lambda off: b[:, off:off + 2].contiguous().view(torch.float16).double().view(n, -1).repeat_interleave(per, 1)
+    codes, dw = values(b, 1.0, 0.0), spread(scale)
+    mins = values(b, 0.0, 1.0) * spread(minimum) if minimum is not None else torch.zeros_like(dw)
+    if wtype == 6:                  # Q5_0: the kernels take the codes unsigned and -16 d as the minimum
+        codes, mins = codes + 16, -16 * dw
+    x = torch.randn(m, k, device=cuda_dev, generator=gen)
+    x = x.abs() if one_sign else x
+    st = torch.cuda.current_stream().cuda_stream
+    y8 = torch.zeros((m, k // 32, 36), dtype=torch.uint8, device=cuda_dev)
+    lib.cq_quantize_act(x.data_ptr(), capi.F32, y8.data_ptr(), k, k, m, 0, st)
+    a = y8.view(-1, 36)
+    da = a[:, 0:2].contiguous().view(torch.float16).double().view(m, -1).repeat_interleave(32, 1)
+    xq = da * a[:, 4:].contiguous().view(torch.int8).double().view(m, k)
+    ref = xq @ (dw * codes).t()
+    if wtype in (3, 6, 7):          # the stored f16 sum of a block's inputs
+        ref += a[:, 2:4].contiguous().view(torch.float16).double().view(m, -1) @ mins[:, ::32].t()
+    else:
+        ref += xq @ mins.t()
+    wq = b.reshape(n, -1)
+    decode = torch.empty((m, n), device=cuda_dev)
+    for r in range(0, m, 8):
+        lib.cq_mmvq(wtype, 0, capi.F32, wq.data_ptr(), y8[r:].data_ptr(), decode[r:].data_ptr(), k, n, k // 32, n, 8, st)
+    capi.check("decode")
+    err = lambda o: float((o.double() - ref).norm() / ref.norm())
+    assert err(decode) <= 1e-6      # the reference is that arithmetic
+    assert err(_prompt32(lib, wtype, wq, x, k, n)) <= 1.1 * err(decode)
