@@ -1,8 +1,6 @@
 // Host side of the quantized matmul (see qtensor.h) and its flat C interface (cqh_*).
 #include "qtensor.h"
 
-#include <algorithm>
-#include <cmath>
 #include <atomic>
 #include <cstring>
 #include <map>
@@ -213,19 +211,13 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     }
     // Formats with an activation scale per 32 elements: Q4_0 / Q8_0 (Q8_0 activations, the CPU path's arithmetic, in every mode)
     // and the six others (Q8_1, the decode kernels' arithmetic, hence already from the first row that no longer fits one
-    // decode launch, and not in the CPU-exact mode).  K must be a whole number of 256-element stages.
+    // decode launch where that is the faster, and not in the CPU-exact mode).  K must be a whole number of 256-element stages.
     const bool plain32 = dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0;
     const bool q8_1_only = !plain32 && dtype_ != GgmlDType::Q4K && dtype_ != GgmlDType::Q6K;
     const bool any_address = dtype_ == GgmlDType::Q2K || dtype_ == GgmlDType::Q3K;
-    // For the six the GEMV slices give the same values, so the faster is taken: a slice of eight rows streams the matrix at
-    // about 1.15 TB/s and costs 7 us at least; the prompt kernel takes a round of 148 tiles (128 weight rows x 64 tokens) per
-    // launch or more, about 1.3 us per 256 elements of K each, and 8 us.  A narrow matrix with a long K leaves most SMs without
-    // a tile: 512 rows of K = 14336 take 80 us however few the tokens, two slices 14 us.
-    const double slices = (double)((rows + MMVQ_MAX_BATCH - 1) / MMVQ_MAX_BATCH), slice_us = std::max(7.0, (double)len_ / 1.15e6);
-    const double rounds = std::ceil((double)((n + 127) / 128) * (double)((rows + 63) / 64) / 148.0);
-    const bool prompt_pays = 8.0 + rounds * (double)(k / 256) * 1.3 < slices * slice_us;
     if (k % 256 == 0 && ((plain32 && rows > kPrefillMinRows) ||
-                         (q8_1_only && rows > MMVQ_MAX_BATCH && prompt_pays && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0)))) {
+                         (q8_1_only && rows > MMVQ_MAX_BATCH && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0) &&
+                          cq_prompt32_pays((int)dtype_, (int)rows, (int)k, (int)n)))) {
         uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt32_scratch_bytes((int)dtype_, (int)rows, (int)k));
         cq_prompt32_matmul((int)dtype_, ptr_, x, (int)x_dtype, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
         lib_check("qmatmul prefill (scales per 32)");

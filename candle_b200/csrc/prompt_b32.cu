@@ -20,6 +20,8 @@
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
 
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace {
@@ -29,6 +31,7 @@ constexpr int kEpiWarps = 8, kProdWarps = 4;
 constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
 constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two: raw bytes without a tensor map
 constexpr int kColA = 384;
+constexpr int kFixedTokens = 40;                // plan_tiling
 
 __device__ int g_prompt_b32_timeout_flag = 0;
 
@@ -653,7 +656,7 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
         attr_done[dev] = true;
     }
     const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
-    const Tiling tl = plan_tiling(tokens, nrt, sm_count(), 40, F::kTok);
+    const Tiling tl = plan_tiling(tokens, nrt, sm_count(), kFixedTokens, F::kTok);
     const long long blocks = (long long)tl.ntt * (tl.tt / 8) * nch;
     if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32: too many tokens for one launch"); return false; }
     const long long row_bytes = (long long)nch * chunk_bytes<WTYPE>();
@@ -682,6 +685,25 @@ int mins_of(int wtype) {
 extern "C" size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k) {
     if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
     return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)(512 + 32 + 32 * mins_of(wtype)) + 256;
+}
+
+// The six Q8_1 formats against slices of eight rows on the decode kernel, which stream the matrix once each.  Both models are fits to 1500
+// shapes (9 - 220 tokens, 32 - 20000 rows, K to 14336; f32, cold weights; this kernel within 2 %, the slices within 6 - 13 % on average): a round
+// of tiles takes a fixed part and one per token and 256 elements of K; a slice its two launches, and time per weight that grows with
+// its rows.  Of those shapes 21 go to the slower side by more than 5 %, by 20 % at most where that is this kernel: a matrix of few rows and
+// long K leaves most SMs without a tile (5467 rows of K = 10240, 11 tokens: 124 us against 54), 4096 -> 14336 at 512 tokens 490 against 2233.
+extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
+    const double sms = cq_sm_count(), weights = 1e-6 * n * (double)k;
+    const Tiling tl = plan_tiling(tokens, (n + kRows - 1) / kRows, (int)sms, kFixedTokens, 64);
+    const double rounds = std::ceil((double)((n + kRows - 1) / kRows) * tl.ntt / sms);
+    const bool super = cq_block_elems(wtype) == 256;
+    const double fixed = wtype == CQ_Q2_K ? 2.52 : wtype == CQ_Q3_K ? 2.09 : 2.27, per_token = wtype == CQ_Q2_K ? 0.046 : 0.036;
+    const double here = 6.7 + rounds * (k / 256) * (fixed + per_token * tl.tt);
+    auto slice = [&](int rows) {
+        return super ? 5.25 + 0.125e-3 * k + weights * (0.05 + 0.084 * rows) : std::max(5.05, 4.7 + 0.018e-3 * k + weights * (0.21 + 0.02 * rows));
+    };
+    const int whole = tokens / 8, left = tokens % 8;
+    return here < (super ? 1.8 : 2.5) + whole * slice(8) + (left ? slice(left) : 0.0);
 }
 
 extern "C" void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,

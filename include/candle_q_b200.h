@@ -277,6 +277,7 @@ size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k);
 void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
                         int stride_dst, void *stream);
 int cq_prompt32_timeout_flag(void);
+int cq_prompt32_pays(int wtype, int tokens, int k, int n);     /* Q8_1 formats: 0 where slices of eight tokens on the decode kernel are the faster */
 
 /* Glue kernels of the decoder harness (f32, fixed order of additions, one launch each).  They stand where candle's
  * quantized models run chains of tensor ops (candle-transformers/src/models/quantized_llama.rs:56-62, 178-262).

@@ -229,3 +229,22 @@ def test_prompt32_is_no_further_from_64_bits_than_the_decode_kernel(lib, cuda_de
     err = lambda o: float((o.double() - ref).norm() / ref.norm())
     assert err(decode) <= 1e-6      # the reference is that arithmetic
     assert err(_prompt32(lib, wtype, wq, x, k, n)) <= 1.1 * err(decode)
+
+
+@pytest.mark.parametrize("wtype,rows,k,n", [(3, 200, 768, 700), (6, 200, 768, 700), (7, 200, 768, 700), (10, 200, 768, 700), (11, 200, 768, 700), (13, 200, 768, 700),
+                                            (3, 40, 5120, 64), (13, 36, 5120, 64)])
+def test_qmatmul_runs_the_kernel_the_rule_names(lib, oracle, cuda_dev, wtype, rows, k, n):
+    """QMatMul.forward against both kernels called directly: the bits of the one the rule names, which differ from the other's."""
+    _, x, wq = make_case(oracle, wtype, k, n, rows, seed=4)
+    x_dev, w_dev, st = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev), torch.cuda.current_stream().cuda_stream
+    prompt, kp = _prompt32(lib, wtype, w_dev, x_dev, k, n), capi.pad(k, 512)
+    y8 = torch.zeros((rows, kp // 32, 36), dtype=torch.uint8, device=cuda_dev)
+    lib.cq_quantize_act(x_dev.data_ptr(), capi.F32, y8.data_ptr(), k, kp, rows, 0, st)
+    slices = torch.empty_like(prompt)
+    for r in range(0, rows, 8):
+        lib.cq_mmvq(wtype, 0, capi.F32, w_dev.data_ptr(), y8[r:].data_ptr(), slices[r:].data_ptr(), k, n, kp // 32, n, min(8, rows - r), st)
+    capi.check("direct")
+    y = QMatMul.from_qtensor(QTensor.from_data(wq, GgmlDType(wtype), (n, k), cuda_dev)).forward(x_dev)
+    assert not torch.equal(prompt, slices)
+    assert lib.cq_prompt32_pays(wtype, rows, k, n) == (1 if rows == 200 else 0)
+    assert torch.equal(y, prompt if rows == 200 else slices)

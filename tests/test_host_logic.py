@@ -117,3 +117,17 @@ def test_operands_of_the_super_block_prompt_kernel_are_exact():
     assert np.all(a % 8 == 0) and 256 * 128 * np.abs(a).max() <= 8 * 2 ** 24 and 256 * 128 * np.abs(prod - a).max() <= 2 ** 24
     # Q4_K: one accumulator per 128 elements, or per super-block up to the stored limit of sum |q8|
     assert 128 * 128 * 63 * 15 <= 2 ** 24 < 256 * 127 * 63 * 15 and (2 ** 24 // 945) * 945 <= 2 ** 24 and 16 * 63 * 2048 <= 2 ** 24
+
+
+def test_prompt_route_of_the_q8_1_formats_takes_the_faster_side(lib):
+    """(type, tokens, K, rows) with the measured times of slices on the decode kernel and of the prompt kernel (us).  Without a device the
+    rule counts 148 SMs."""
+    slices = [((7, 71, 10240, 53), 47.6, 122.0), ((3, 15, 8192, 7620), 42.1, 97.5), ((7, 34, 5120, 100), 27.7, 63.8), ((7, 11, 10240, 5467), 54.1, 123.7),
+              ((7, 12, 14336, 6442), 76.4, 170.7), ((3, 10, 5120, 7202), 28.7, 63.5), ((10, 41, 5120, 34), 33.0, 71.6), ((6, 9, 768, 360), 13.2, 19.5),
+              ((13, 18, 14336, 3248), 83.2, 166.0), ((13, 11, 8192, 7677), 60.4, 101.4), ((6, 11, 8192, 10496), 55.0, 105.5), ((11, 36, 5120, 128), 39.9, 66.6)]
+    prompt = [((13, 512, 4096, 14336), 2233.0, 490.0), ((6, 91, 10240, 1629), 165.6, 124.9), ((3, 16, 768, 8303), 19.7, 15.0), ((10, 154, 10240, 171), 194.7, 139.3),
+              ((3, 183, 14336, 496), 220.3, 168.6), ((6, 9, 512, 5178), 15.5, 12.4)]
+    for shape, fast, slow in slices:
+        assert fast < slow and lib.cq_prompt32_pays(*shape) == 0, shape
+    for shape, slow, fast in prompt:
+        assert fast < slow and lib.cq_prompt32_pays(*shape) == 1, shape
