@@ -190,14 +190,7 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     // Prompt path: many rows of a Q4_K / Q6_K matrix go to the tensor-core kernel.  It quantizes activations like
     // candle's CPU path (Q8_K) in every mode: that is the arithmetic its integer operands are exact for.
     if (rows > kPrefillMinRows && (dtype_ == GgmlDType::Q4K || dtype_ == GgmlDType::Q6K)) {
-        // Q6_K: expanding 128 rows takes 2.0 us per super-block, the int8 kernel 1.4 us for its tiles of 64 rows x 128 tokens (the same
-        // bits).  So a launch that leaves SMs idle either way (few tiles) is faster with the smaller tiles: 4096 rows of
-        // K = 14336 and 100 tokens, 64 tiles for 148 SMs.  Rows that are not a multiple of 16 bytes apart (K % 2048 != 0) have no tiled
-        // copy and cost this kernel more than the int8 one, whose threads read them directly: K = 2304, 8192 rows, 1000 tokens
-        // 125 against 106 us (K = 4096: 41 against 58).
-        const size_t tiles128 = (n + 127) / 128 * ((rows + 127) / 128), tiles64 = (n + 63) / 64 * ((rows + 127) / 128);
-        if (dtype_ == GgmlDType::Q6K && (uintptr_t)ptr_ % 4 == 0 &&
-            (k % 2048 != 0 || (double)((tiles64 + 147) / 148) * 1.4 < (double)((tiles128 + 147) / 148) * 2.0)) {
+        if ((uintptr_t)ptr_ % 4 == 0 && !cq_prompt_pays((int)dtype_, (int)rows, (int)k, (int)n)) {       // Q6_K on the int8 kernel, the same bits
             uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prefill_scratch_bytes((int)rows, (int)k));
             cq_prefill_quantize(x, (int)x_dtype, scratch, (int)k, (int)rows, stream);
             cq_prefill_gemm((int)dtype_, ptr_, scratch, out, (int)x_dtype, (int)k, (int)n, (int)rows, (int)n, stream);

@@ -260,6 +260,7 @@ size_t cq_prompt_scratch_bytes(int tokens, int k);
 void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
                       int stride_dst, void *stream);
 int cq_prompt_timeout_flag(void);
+int cq_prompt_pays(int wtype, int tokens, int k, int n);       /* 0: the pair above is the faster (some Q6_K shapes); the same bits */
 /* The same for the 32-element block formats Q4_0 (wtype 2) and Q8_0 (8): candle-kernels/src/mmq_gguf/mmq_gguf.cuh:305-364,
  * 927-1062, 1169-1296 behind ffi.rs:471-630.  Activations are quantized like candle's CPU path (BlockQ8_0, k_quants.rs:
  * 658-687); every 32-element block is one tcgen05 MMA step into a fresh TMEM accumulator that the epilogue scales by
