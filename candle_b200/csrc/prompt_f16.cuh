@@ -250,26 +250,34 @@ inline int sm_count() { return cq_sm_count(); }
 
 // ---- raw weight bytes: (128 rows, one 256-element chunk) -> shared memory ---------------------------------------
 // One tiled TMA copy when rows are whole multiples of 16 bytes apart; else (Q6_K rows of K % 2048 != 0 and the like) two warps copy
-// 16-byte pieces with cp.async, consecutive lanes along a row, from the 16-byte boundary below each row's chunk - a bulk copy per
-// row was three times slower than the whole int8 kernel.  In shared memory row r starts at r * kPitch, the chunk a few bytes
-// behind it when it does not start on such a boundary.  CB: bytes of a chunk.
+// 16-byte pieces with cp.async, a lane per piece and two rows per warp step, from the 16-byte boundary below each row's chunk - a bulk copy
+// per row was three times slower than the whole int8 kernel, and splitting a running piece number into row and piece made Q6_K of
+// K = 2304 .. 14080 up to 30 % slower than this (128 experts, K = 1792 -> 768, 512 pairs: 157 us, now 125).  In shared memory row r starts
+// at r * kPitch, the chunk a few bytes behind it when it does not start on such a boundary.  CB: bytes of a chunk.
 constexpr int kRawThreads = 64;
 template <int CB> struct Raw {
     static constexpr bool kAligned = CB % 16 == 0;
     static constexpr int kNeed = kAligned ? CB : (CB + 14 + 15) / 16 * 16;       // 16-byte window that covers the chunk
     // pitch: an odd number of 16-byte units, so that eight lanes' 16-byte reads of one column fall into different banks
     static constexpr int kPitch = (kNeed / 16) % 2 ? kNeed : kNeed + 16;
+    static_assert(kAligned || kNeed <= 256, "one unit per thread");
     static constexpr int kBytes = kRows * kPitch;
     // Pieces reach at most the last 16-byte unit that holds a byte of the chunk, rows past the matrix repeat its last one.
     // `bar` counts kRawThreads; `w` points at the chunk of the tile's first row, `rows_left` rows are in memory from there.
     static __device__ __forceinline__ void load_rows(uint8_t *dst, const uint8_t *w, int rows_left, uint32_t row_bytes, int thread, uint64_t *bar) {
-        constexpr int kUnits = kNeed / 16;
-#pragma unroll 1
-        for (int idx = thread; idx < kRows * kUnits; idx += kRawThreads) {
-            const int row = idx / kUnits, u = idx - row * kUnits;
-            const uint8_t *p = w + (size_t)(uint32_t)min(row, rows_left - 1) * row_bytes;
-            const uintptr_t src = ((uintptr_t)p & ~(uintptr_t)15) + 16 * u;
-            if (src < (uintptr_t)p + CB) cq_cp_async16(dst + row * kPitch + 16 * u, (const void *)src);
+        // 16 threads per row (one 16-byte unit each), four rows at a time
+        const int u = thread & 15;
+        if (16 * u < kNeed) {
+            uint32_t to = cq_smem_u32(dst) + (uint32_t)((thread >> 4) * kPitch + 16 * u);
+            const uint8_t *p = w + (size_t)(uint32_t)min(thread >> 4, rows_left - 1) * row_bytes, *last = w + (size_t)(uint32_t)(rows_left - 1) * row_bytes;
+#pragma unroll 8
+            for (int i = 0; i < kRows / 4; ++i) {
+                const uintptr_t src = ((uintptr_t)p & ~(uintptr_t)15) + 16 * u;
+                if (src < (uintptr_t)p + CB) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
+                to += 4 * kPitch;
+                p += 4 * (size_t)row_bytes;
+                if (p > last) p = last;
+            }
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(cq_smem_u32(bar)) : "memory");
     }

@@ -743,16 +743,15 @@ extern "C" size_t cq_prompt_scratch_bytes(int tokens, int k) {
     return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * kTokBytes + 256;
 }
 
-// Q6_K against the int8 kernel behind cq_prefill_gemm (the same bits): a round of tiles of 128 rows takes 2.3 us per super-block here, 1.6 us for
-// its tiles of 64 rows x 128 tokens.  So a launch that leaves SMs idle either way is faster with the smaller tiles (4096 -> 2368, 64 tokens:
-// 56 against 46 us; 4096 -> 3587 of K = 10240, 393 tokens: 99 against 134).  Rows that are not a multiple of 16 bytes apart (K % 2048 != 0)
-// have no tiled copy and cost this kernel more than that one, whose threads read them directly (1024 -> 5504, 24 tokens: 19.1 against
-// 17.1; K = 2816, 512 rows, 156 tokens: 40 against 26).  Of 90 shapes measured the rule takes the slower one three times, by 7 % at most.
+// Q6_K against the int8 kernel behind cq_prefill_gemm (the same bits): a round of tiles of 128 rows takes 2.3 us per super-block here (2.45 where
+// rows are not a multiple of 16 bytes apart and have no tiled copy), 1.6 us for its tiles of 64 rows x 128 tokens.  So a launch that leaves SMs
+// idle either way is faster with the smaller tiles (8192 -> 2368, 86 tokens: 73 against 63 us; 10240 -> 3587, 393 tokens: 99 against
+// 133; K = 9728, 9856 rows, 51 tokens: 97 against 118).  Of 90 shapes measured the rule takes the slower one five times, by 10 % at most.
 extern "C" int cq_prompt_pays(int wtype, int tokens, int k, int n) {
     if (wtype != CQ_Q6_K) return 1;
     const long long sms = cq_sm_count(), tt = (tokens + kTokMax - 1) / kTokMax;
     const long long rounds64 = ((n + 63) / 64 * tt + sms - 1) / sms, rounds128 = ((n + kRows - 1) / kRows * tt + sms - 1) / sms;
-    return k % 2048 == 0 && rounds64 * 1.6 >= rounds128 * 2.3;
+    return rounds64 * 1.6 >= rounds128 * (k % 2048 == 0 ? 2.3 : 2.45);
 }
 
 extern "C" void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,

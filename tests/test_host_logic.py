@@ -136,9 +136,10 @@ def test_prompt_route_of_the_q8_1_formats_takes_the_faster_side(lib):
 def test_prompt_route_of_q6_k_takes_the_faster_kernel(lib):
     """(tokens, K, rows) with the measured times of the prompt kernel and of the int8 kernel (us)."""
     f16 = [((1154, 4096, 3648), 90.9, 110.2), ((24, 4096, 14208), 41.5, 58.0), ((393, 10240, 3587), 98.5, 133.9), ((512, 14336, 4096), 148.0, 170.0),
-           ((707, 8192, 4800), 158.4, 229.5), ((65, 2048, 12091), 24.3, 37.7)]
+           ((707, 8192, 4800), 158.4, 229.5), ((65, 2048, 12091), 24.3, 37.7), ((25, 8704, 13177), 85.5, 108.5), ((51, 9728, 9856), 97.4, 117.5),
+           ((1487, 4608, 9037), 293.0, 354.5)]
     int8 = [((18, 14336, 4096), 124.3, 90.8), ((61, 8192, 3210), 72.9, 62.3), ((899, 6144, 832), 64.1, 52.5), ((19, 14336, 1216), 120.3, 88.6),
-            ((24, 1024, 5504), 19.1, 17.1), ((156, 2816, 512), 39.8, 25.6), ((196, 11776, 704), 147.0, 77.4)]
+            ((54, 11008, 5278), 106.6, 73.7), ((156, 2816, 512), 31.3, 25.5), ((196, 11776, 704), 113.1, 78.3), ((653, 12800, 4653), 267.9, 239.6)]
     for (tokens, k, n), fast, slow in f16:
         assert fast < slow and lib.cq_prompt_pays(14, tokens, k, n) == 1, (tokens, k, n)
     for (tokens, k, n), slow, fast in int8:
