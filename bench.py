@@ -415,7 +415,7 @@ def measure_prefill(dev, rank, world, peak_tops):
                 del x, y, scratch
         del ws, mms
         torch.cuda.empty_cache()
-    assert L.cq_prefill_timeout_flag() == 0, "a prefill launch gave up a bounded wait"
+    assert L.cq_prefill_timeout_flag() == 0 and L.cq_prompt_timeout_flag() == 0, "a prefill launch gave up a bounded wait"
     return out
 
 
@@ -455,7 +455,7 @@ def measure_prefill_block_formats(dev, peak_tops):
             res.append(row)
             del ws, mms, x, y, mmq_scratch, fixup
             torch.cuda.empty_cache()
-    assert L.cq_prefill32_timeout_flag() == 0, "a block-format prefill launch gave up a bounded wait"
+    assert L.cq_prompt32_timeout_flag() == 0, "a block-format prefill launch gave up a bounded wait"
     return res
 
 

@@ -108,3 +108,17 @@ def test_qmatmul_variants_for_unquantized_tensors_and_dequantize_switches(oracle
     assert y16.dtype == torch.float32
     assert np.abs(y16.cpu().numpy().reshape(-1, n) - ref).max() / np.abs(ref).max() <= 2e-2     # f16 weights, inputs and product
     assert torch.equal(mm.dequantize_f16(), mm.dense)
+
+
+@pytest.mark.parametrize("tname", [t for t in TYPES if t not in ("q4_k", "q5_k")])
+@pytest.mark.parametrize("offset", [2, 6])
+def test_blocks_off_a_word_boundary(oracle, cuda_dev, tname, offset):
+    """Bases that are 2 modulo 4: a lane's eight code bytes then start in the middle of a word."""
+    wt, n, k = TYPES[tname], 5, 768
+    wq = torch.from_numpy(_tensor(oracle, wt, n, k, seed=offset).reshape(-1)).to(cuda_dev)
+    buf = torch.full((wq.numel() + 64,), 0xFF, dtype=torch.uint8, device=cuda_dev)
+    buf[offset:offset + wq.numel()] = wq
+    moved = QTensor.from_device_blocks(buf[offset:offset + wq.numel()], GgmlDType(wt), (n, k))
+    aligned = QTensor.from_device_blocks(wq, GgmlDType(wt), (n, k))
+    for dtype in (torch.float32, torch.float16):
+        assert torch.equal(moved.dequantize(dtype), aligned.dequantize(dtype))

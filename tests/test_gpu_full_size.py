@@ -208,4 +208,4 @@ def test_config3_prefill_full_size(lib, oracle, cuda_dev, k, n):
         # the f32 result is rounded once to bf16 (8-bit mantissa): one unit in the last place of the largest output
         assert rel_err(got_b, ref_b) <= 2 ** -8 * 1.01, (m, "bf16")
         del yb, xb, x_dev
-    assert lib.cq_prefill_timeout_flag() == 0
+    assert lib.cq_prompt_timeout_flag() == 0 and lib.cq_prefill_timeout_flag() == 0       # Q6_K may take either kernel

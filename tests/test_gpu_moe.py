@@ -292,6 +292,7 @@ def test_fused_moe_under_autocast(cuda_dev, tokens, is_prefill):
         ref = moe.forward(x, is_prefill)
     assert ys.dtype == x.dtype
     assert float((ys - ref).norm() / ref.norm()) <= (2e-3 if is_prefill else 1e-4)
+    assert capi.lib().cq_prompt_timeout_flag() == 0 and capi.lib().cq_moe_timeout_flag() == 0
 
 
 def test_one_launch_router_and_slot_sum(cuda_dev):
@@ -437,7 +438,7 @@ def test_grouped_tensor_core_gemm_matches_cpu_arithmetic(oracle, cuda_dev, tname
         x = rng.standard_normal((tokens, k)).astype(np.float32)
         tw = None
         out = moe_prefill_gemm(dev(x), qt, None, dev(order), dev(experts_sorted), topk, zero_init=True).cpu().numpy()
-    assert capi.lib().cq_prefill_timeout_flag() == 0
+    assert capi.lib().cq_prompt_timeout_flag() == 0
     ref = np.zeros_like(out)
     for pair in range(tokens * topk):
         ex = flat[pair]
@@ -500,6 +501,7 @@ def test_fused_moe_few_launches_against_the_general_path(cuda_dev, wt_gu, wt_dow
     moe._block = lambda *a: None
     ref = moe.forward(x, is_prefill)
     assert float((ys - ref).norm() / ref.norm()) <= (2e-3 if is_prefill else 1e-4)
+    assert capi.lib().cq_prompt_timeout_flag() == 0 and capi.lib().cq_moe_timeout_flag() == 0
 
 
 @pytest.mark.parametrize("wt_gu,wt_down", [(12, 14), (8, 8)])

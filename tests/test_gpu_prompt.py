@@ -248,3 +248,32 @@ def test_qmatmul_runs_the_kernel_the_rule_names(lib, oracle, cuda_dev, wtype, ro
     assert not torch.equal(prompt, slices)
     assert lib.cq_prompt32_pays(wtype, rows, k, n) == (1 if rows == 200 else 0)
     assert torch.equal(y, prompt if rows == 200 else slices)
+
+
+def _at_offset(w_dev, offset):
+    """The same bytes `offset` bytes into a larger buffer (whose base is 256-byte aligned)."""
+    buf = torch.full((w_dev.numel() + 256,), 0xFF, dtype=torch.uint8, device=w_dev.device)
+    buf[offset:offset + w_dev.numel()] = w_dev.reshape(-1)
+    assert buf.data_ptr() % 256 == 0
+    return buf[offset:offset + w_dev.numel()]
+
+
+@pytest.mark.parametrize("wtype,offset", [(10, 2), (10, 4), (10, 6), (10, 14), (11, 2), (11, 4), (11, 6), (11, 14), (14, 4), (14, 8), (14, 12)])
+@pytest.mark.parametrize("k,n,tokens", [(2048, 200, 40), (768, 129, 20)])
+def test_weights_at_any_address_give_the_bits_of_an_aligned_copy(lib, oracle, cuda_dev, wtype, offset, k, n, tokens):
+    """Bases off the 16-byte grid have no tensor map, and every row its own distance to the boundary below it."""
+    _, x, wq = make_case(oracle, wtype, k, n, tokens, seed=offset)
+    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
+    run = _prompt if wtype == 14 else _prompt32
+    assert torch.equal(run(lib, wtype, _at_offset(w_dev, offset), x_dev, k, n), run(lib, wtype, w_dev, x_dev, k, n))
+
+
+def test_addresses_the_prompt_kernels_do_not_take_are_refused(lib, oracle, cuda_dev):
+    """Q6_K off a 4-byte boundary, Q4_K and Q8_0 off a 16-byte one: an error before any launch, as before these kernels."""
+    for wtype, offset in ((14, 2), (12, 8), (8, 8)):
+        _, x, wq = make_case(oracle, wtype, 512, 64, 20, seed=1)
+        w = _at_offset(torch.from_numpy(wq).to(cuda_dev), offset)
+        mm = QMatMul.from_qtensor(QTensor.from_device_blocks(w, GgmlDType(wtype), (64, 512)))
+        with pytest.raises(capi.CandleQError, match="aligned"):
+            mm.forward(torch.from_numpy(x).to(cuda_dev))
+        lib.cq_clear_status()
