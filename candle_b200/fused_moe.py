@@ -129,7 +129,7 @@ class FusedMoeGGUF:
         expert_ids, sorted_token_ids = sort_pairs(topk_ids)
         local_ids = expert_ids - self.expert_offset          # ids outside [0, local experts) are skipped by the kernels
         cast = (lambda t: t.to(self.prefill_dtype)) if is_prefill else (lambda t: t)      # the reference casts for its prefill kernel (moe.rs:310-333)
-        if is_prefill and self.world > 1 and self._few_pairs(num_tokens * k):
+        if is_prefill and self.world > 1 and self._few_pairs(num_tokens * k) and self.prefill_dtype in (torch.float16, torch.bfloat16):
             # With this rank's experts alone the prompt entry point could take the tensor cores where one rank takes the GEMV; the
             # decode entry point on the cast values is that GEMV.
             cast, is_prefill = (lambda t: t.to(self.prefill_dtype).to(torch.float32)), False

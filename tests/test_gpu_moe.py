@@ -532,3 +532,16 @@ def test_fused_moe_has_the_same_bits_for_any_number_of_ranks(cuda_dev, monkeypat
     monkeypatch.setattr(fm.dist, "all_reduce", lambda t, **kw: t.copy_(sent[0] + sent[1]))
     for r in ranks:
         assert torch.equal(r.forward(x, is_prefill), one)
+
+
+@pytest.mark.parametrize("tokens", [5, 40])
+def test_fused_moe_prompt_type_stays_16_bit_on_every_rank_count(cuda_dev, tokens):
+    """A prompt type other than f16 / bf16 is refused, with few pairs and many, one rank and two."""
+    from candle_b200.fused_moe import FusedMoeGGUF
+    from candle_b200.synth import random_blocks
+    mk = lambda n, k: QTensor.from_device_blocks(random_blocks(GgmlDType.Q4K, 6 * n, k, seed=1, device=cuda_dev).reshape(-1), GgmlDType.Q4K, (6, n, k))
+    w = [mk(256, 512), mk(256, 512), mk(512, 256)]
+    for world in (1, 2):
+        moe = FusedMoeGGUF(torch.randn(6, 512, device=cuda_dev), *w, 2, prefill_dtype=torch.float32, world=world)
+        with pytest.raises(capi.CandleQError, match="f16 or bf16"):
+            moe.forward(torch.randn(1, tokens, 512, device=cuda_dev), True)
