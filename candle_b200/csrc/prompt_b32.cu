@@ -1,7 +1,7 @@
 // Prompt-phase quantized GEMM for activations with one scale per 32 elements, on tcgen05.mma kind::f16 (prompt_f16.cuh):
 //   Q8_0, Q4_0                            BlockQ8_0 activations, candle's CPU arithmetic (k_quants.rs:294-311, 720-738)
 //   Q4_1, Q5_0, Q5_1, Q2_K, Q3_K, Q5_K     Q8_1 activations, the arithmetic of the decode kernels (mmvq_gguf.cu:208-334, 357-381,
-//                                          492-531; gemv_chunks.cuh), which these formats use at every row count
+//                                          492-531; gemv_chunks.cuh), the same arithmetic at every row count
 //
 // Both sides of a product carry a scale per 32 elements, so nothing beyond the integer sub-scales of a K-quant can be folded
 // into the operands: every 32-element block is two K = 16 steps into a FRESH accumulator slot, exact (sums below 2^24: at most
@@ -9,14 +9,14 @@
 // Against int8 operands the epilogue needs no int -> float conversion, which was two of its five operations per value.
 //
 // Summation: Q8_0 / Q4_0 add block after block, as the kernel behind cq_prefill32_gemm does (the same f32 operations, the same
-// bits).  The Q8_1 formats were summed by the decode kernels' balanced tree until now; a plain chain of K / 32 additions would
+// bits).  The decode kernels, which the Q8_1 formats use otherwise, sum by a balanced tree; a plain chain of K / 32 additions would
 // lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
 //
 // Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
 // warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader, 14-15 raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128
 // columns), 128 columns of operand A.  The roles hand over two blocks at a time.  Every wait is bounded as there.
-// Measured (quantizer included): Q5_K 4096 -> 14336, 512 tokens 2235 us (GEMV slices) -> 471; Q8_0 4096 -> 4096, 333 tokens 98 (int8 kernel,
-// 64 x 128 tiles) -> 89.  Two producer sets as in prompt_kq.cu made it 3 % slower: the epilogue, ~2.5 us per 256 k-elements, bounds it.
+// Measured (quantizer included): Q5_K 4096 -> 14336, 512 tokens 2235 us (GEMV slices) -> 490; Q8_0 4096 -> 4096, 333 tokens 98 (int8 kernel,
+// 64 x 128 tiles) -> 88.  Two producer sets as in prompt_kq.cu made it 3 % slower: the epilogue, ~2.5 us per 256 k-elements, bounds it.
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
 

@@ -204,11 +204,11 @@ void cq_moe_gemv_sorted(int wtype, int act, const void *weights, const void *y, 
 void cq_indexed_moe_forward(int wtype, int act, const void *weights, const void *y, const uint32_t *ids, float *out, int n,
                             int k, int batch, int topk, int k_padded, int input_dim1, int num_experts, void *stream);
 int cq_moe_timeout_flag(void);
-/* Grouped prompt-phase GEMM of a quantized MoE layer on the int8 tensor cores (Q4_K / Q6_K experts, num_experts <= 1024,
+/* Grouped prompt-phase GEMM of a quantized MoE layer on the tensor cores (Q4_K / Q6_K experts, num_experts <= 1024,
  * size_k % 256 == 0): same job rules as moe_gemm_gguf (pairs sorted by expert), input of in_elem (CQ_ELEM_*), f32 output
  * rows indexed by pair.  The pairs of an expert are cut into tiles of 128 on the device; `scratch` holds the tile table
- * and the int8 activation tiles (cq_moe_prefill_scratch_bytes, 256-byte aligned).  Arithmetic: Q8_K activations as the
- * dense prefill kernel.  Pairs whose expert id is outside [0, num_experts) are not written. */
+ * and the activation tiles (cq_moe_prefill_scratch_bytes, 256-byte aligned).  Arithmetic: Q8_K activations, that of
+ * cq_prompt_matmul.  Pairs whose expert id is outside [0, num_experts) are not written. */
 size_t cq_moe_prefill_scratch_bytes(int size_m, int num_experts, int k);
 void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *weights, const int32_t *sorted_token_ids,
                          const int32_t *expert_ids, const float *topk_weights, float *out, void *scratch, int num_experts,
@@ -238,7 +238,7 @@ void cq_moe_block_decode_pairs(int wtype, int wtype_down, const float *x, const 
                                const int32_t *ids, float *out, void *scratch, int num_experts, int topk, int tokens, int hidden, int ffn,
                                void *stream);
 
-/* Prefill path (many tokens) on the int8 tensor cores, Q4_K weights.  Replaces the pair
+/* Prefill path (many tokens) on the int8 tensor cores, Q4_K and Q6_K weights, as two calls.  Replaces the pair
  * launch_mmq_quantize_q8_1_* + launch_mmq_gguf_q4_k of candle-kernels/src/ffi.rs:424-630 for callers that go through
  * this library's host objects; the arithmetic is candle's CPU one (BlockQ8K activations, k_quants.rs:1460-1540,
  * 2320-2358), so results match the CPU vec_dot up to f32 summation order.
