@@ -139,6 +139,39 @@ __global__ void __launch_bounds__(256) quantize_q8k_tiles_kernel(const T *__rest
                              TileBlob::tile_rows(tokens, tt), tl, lane);
 }
 
+// ---- grouped (expert-indexed) mode ------------------------------------------------------------------------
+// The jobs and the tile table of prompt_kq.cu: entry t = (expert, first job, valid rows, -), entry max_tiles = the number of tiles in use.
+// Tiles past it have nothing to do; a tile's blob lies at 128 rows times its number.
+struct GroupInfo {
+    const int *tiles;                  // null: dense mode
+    const int32_t *sorted_token_ids;
+    const float *topk_weights;
+    long long expert_stride;           // bytes between experts
+    int topk;
+};
+
+// One warp per (tile row, super-block): the input row of that job, or zeros for the padding rows of a tile.
+template <typename T>
+__global__ void __launch_bounds__(256) quantize_q8k_tiles_grouped_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k,
+                                                                         int max_tiles, GroupInfo gi) {
+    const int lane = threadIdx.x & 31;
+    const int nsb = k / 256;
+    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= (int64_t)max_tiles * kTokTile * nsb) return;
+    const int sb = (int)(item % nsb);
+    const int64_t slot = item / nsb;
+    const int tt = (int)(slot / kTokTile), tl = (int)(slot % kTokTile);
+    if (tt >= gi.tiles[4 * max_tiles]) return;              // nobody reads its blob
+    const int *ti = gi.tiles + 4 * tt;
+    const T *xr = nullptr;
+    if (tl < ti[2]) {
+        const int pair = gi.sorted_token_ids[ti[1] + tl];
+        const int64_t in_row = gi.topk_weights ? pair : pair / gi.topk;
+        xr = x + in_row * k + sb * 256 + lane * 8;
+    }
+    quantize_q8k_row_part<T>(xr, y + TileBlob::offset(max_tiles * kTokTile, nsb, tt, sb), kTokTile, tl, lane);
+}
+
 // ---- weight planes -----------------------------------------------------------------------------------------
 // RawBlock<T>: the GGUF bytes one producer thread needs for (weight row r, super-block sb, half h, part jh) and their
 // expansion into two int8 planes of 16-byte K slabs:  plane j of row r, slab s  ->  stB + s*kSlabB + (64*j + r)*16,
@@ -276,13 +309,31 @@ template <> struct RawBlock<CQ_Q6_K> {
 //   E(i) after M(i) [bar_acc] and after the relay arrive on bar_vis, which carries the visibility of the scale rings.
 // The scale rings are 8 deep: an entry is rewritten for i+8 only after M(i+5), which itself waited for E(i+3).
 // Warps: 0-7 epilogue (TMEM lane quadrant = warp % 4, weight rows 32 * (warp / 4) ..), 8-15 producers, 16 MMA, 17 loader.
-struct TileCtx { int row0, tt; };
-__device__ __forceinline__ TileCtx tile_ctx(int t, int ntt) { return TileCtx{(t / ntt) * kRowTile, t % ntt}; }
+struct TileCtx {
+    const uint8_t *w;       // weight matrix of this tile (grouped mode: of its expert)
+    int row0, tt, valid, job0;
+};
+// false: nothing to do for tile t (grouped mode, unused tile).  Every role evaluates this for the same t, so all skip alike.
+__device__ __forceinline__ bool tile_ctx(int t, int ntt, const uint8_t *w, const GroupInfo &gi, TileCtx &c) {
+    c.row0 = (t / ntt) * kRowTile;
+    c.tt = t % ntt;
+    c.valid = kTokTile;
+    c.job0 = 0;
+    c.w = w;
+    if (gi.tiles) {
+        if (c.tt >= gi.tiles[4 * ntt]) return false;
+        const int *ti = gi.tiles + 4 * c.tt;
+        c.valid = ti[2];
+        c.w = w + (long long)ti[0] * gi.expert_stride;
+        c.job0 = ti[1];
+    }
+    return true;
+}
 
 template <int WTYPE>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, void *__restrict__ out_v, int out_kind, int k,
-                   int nrows, int tokens, int stride_out, int dbg, int ntt, int ntiles) {
+                   int nrows, int tokens, int stride_out, int dbg, int ntt, int ntiles, const GroupInfo gi) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bar_fullA = reinterpret_cast<uint64_t *>(smem);         // [3] activations landed (TMA bytes)
     uint64_t *bar_fullB = bar_fullA + 3;                               // [3] weight planes written (all producer threads)
@@ -339,21 +390,27 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
             uint8_t *z = stB0 + st * kStageB + (16 + which) * kSlabB + ((which ? 0 : kRowTile) + row) * 16;
             *reinterpret_cast<uint4 *>(z) = make_uint4(0u, 0u, 0u, 0u);
         }
-        auto row_of = [&](int t) -> const uint8_t * {
-            int grow = tile_ctx(t, ntt).row0 + r;
+        auto row_of = [&](const TileCtx &c) -> const uint8_t * {
+            int grow = c.row0 + r;
             if (grow >= nrows) grow = nrows - 1;        // ragged last tile: duplicate a valid row, never stored
-            return w + (size_t)grow * row_bytes;
+            return c.w + (size_t)grow * row_bytes;
+        };
+        auto next_tile = [&](int t, TileCtx &c) -> int {      // first tile >= t of this CTA that has work, or ntiles
+            while (t < ntiles && !tile_ctx(t, ntt, w, gi, c)) t += gridDim.x;
+            return t;
         };
         // the GGUF bytes of the next super-block (of this or of the next tile) are fetched one iteration ahead of their use
-        int t = blockIdx.x;
-        const uint8_t *wrow = t < ntiles ? row_of(t) : nullptr;
+        TileCtx cx;
+        int t = next_tile(blockIdx.x, cx);
+        const uint8_t *wrow = t < ntiles ? row_of(cx) : nullptr;
         RawBlock<WTYPE> nxt_raw;
         if (t < ntiles) nxt_raw.load(wrow, 0, h, jh);
         int it = 0;
         bool alive = true;
         while (t < ntiles && alive) {
-            const int tn = t + gridDim.x;
-            const uint8_t *wnext = tn < ntiles ? row_of(tn) : nullptr;
+            TileCtx nx;
+            const int tn = next_tile(t + gridDim.x, nx);
+            const uint8_t *wnext = tn < ntiles ? row_of(nx) : nullptr;
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int s = it % kStagesB;
                 uint8_t *stB = stB0 + s * kStageB;
@@ -375,7 +432,8 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
             int it = 0;
             bool alive = true;
             for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-                const TileCtx cx = tile_ctx(t, ntt);
+                TileCtx cx;
+                if (!tile_ctx(t, ntt, w, gi, cx)) continue;
                 const int tile_rows = (int)TileBlob::tile_rows(tokens, cx.tt);
                 for (int sb = 0; sb < nsb; ++sb, ++it) {
                     const int a = it % kStagesA;
@@ -399,6 +457,8 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
         int it = 0;
         bool alive = true;
         for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
+            TileCtx cx;
+            if (!tile_ctx(t, ntt, w, gi, cx)) continue;
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int a = it % kStagesA, s = it % kStagesB, c = it & 1;
                 if (!wait_or_abort(&bar_fullA[a], (it / kStagesA) & 1, abort_flag) ||
@@ -432,7 +492,8 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
         int it = 0;
         bool alive = true;
         for (int t = blockIdx.x; t < ntiles && alive; t += gridDim.x) {
-            const TileCtx cx = tile_ctx(t, ntt);
+            TileCtx cx;
+            if (!tile_ctx(t, ntt, w, gi, cx)) continue;
             const int tok = cx.tt * kTokTile + tok_local;
             float acc[kMyRows];
 #pragma unroll
@@ -490,8 +551,20 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
                 mbar_arrive(&bar_free[c]);
             }
             if (!alive) break;
-            const bool store = tok < tokens;
-            const int64_t orow = tok;
+            bool store = tok < tokens;
+            int64_t orow = tok;
+            if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight
+                store = tok_local < cx.valid;
+                if (store) {
+                    const int pair = gi.sorted_token_ids[cx.job0 + tok_local];
+                    orow = pair;
+                    if (gi.topk_weights) {
+                        const float sc = gi.topk_weights[pair];
+#pragma unroll
+                        for (int i = 0; i < kMyRows; ++i) acc[i] = __fmul_rn(acc[i], sc);
+                    }
+                }
+            }
             const int c0 = cx.row0 + rh * kMyRows;
             // The branches below are chosen by warp-uniform values only (`store` differs between the lanes of a ragged token
             // tile and must not decide whether a lane reaches the shuffles of the f32 branch).
@@ -507,7 +580,7 @@ prefill_kernel(const uint8_t *__restrict__ w, const uint8_t *__restrict__ act, v
                         if (c0 + i < nrows) cq_store_out(out_v, out_kind, orow * stride_out + c0 + i, acc[i]);
                 }
               }
-            } else if (c0 + kMyRows <= nrows && (stride_out & 3) == 0 && (c0 & 3) == 0 && (((uintptr_t)out_v) & 15) == 0) {
+            } else if (!gi.tiles && c0 + kMyRows <= nrows && (stride_out & 3) == 0 && (c0 & 3) == 0 && (((uintptr_t)out_v) & 15) == 0) {
                 // f32, whole 32-row slice (warp-uniform test): three exchange steps turn "a lane holds 32 rows of its token" into
                 // "a lane holds 4 rows of 8 tokens", so that eight lanes write one token's 128 contiguous bytes per store
                 // instruction (four full lines per instruction instead of 32 quarter lines).
@@ -576,6 +649,17 @@ static unsigned prefill_grid(int ntiles) {
     return (unsigned)(ntiles < n ? ntiles : n);
 }
 
+void prefill_smem_attr(int ti) {        // 0: Q4_K, 1: Q6_K
+    static bool attr_done[2][64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !attr_done[ti][dev]) {
+        if (ti == 0) cudaFuncSetAttribute(prefill_kernel<CQ_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        else cudaFuncSetAttribute(prefill_kernel<CQ_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        attr_done[ti][dev] = true;
+    }
+}
+
 }  // namespace
 
 extern "C" size_t cq_prefill_scratch_bytes(int tokens, int k) {
@@ -613,24 +697,37 @@ extern "C" void cq_prefill_gemm(int wtype, const void *vx, const void *scratch, 
         cq_set_status(CQ_ERR_BAD_ARG, "prefill gemm: misaligned weights (16 bytes for Q4_K, 4 for Q6_K) or scratch (16)");
         return;
     }
-    static bool attr_done[2][64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
     const int ti = wtype == CQ_Q4_K ? 0 : 1;
-    if (dev >= 0 && dev < 64 && !attr_done[ti][dev]) {
-        if (ti == 0) cudaFuncSetAttribute(prefill_kernel<CQ_Q4_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        else cudaFuncSetAttribute(prefill_kernel<CQ_Q6_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-        attr_done[ti][dev] = true;
-    }
+    prefill_smem_attr(ti);
     const int ntt = (tokens + kTokTile - 1) / kTokTile, ntiles = ((nrows_x + kRowTile - 1) / kRowTile) * ntt;
     const unsigned grid = prefill_grid(ntiles);
     if (ti == 0)
         prefill_kernel<CQ_Q4_K><<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
-            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles);
+            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles, GroupInfo{});
     else
         prefill_kernel<CQ_Q6_K><<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(
-            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles);
+            (const uint8_t *)vx, (const uint8_t *)scratch, dst, out_elem, ncols_x, nrows_x, tokens, stride_dst, g_prefill_dbg, ntt, ntiles, GroupInfo{});
     cq_check_launch("prefill gemm");
+}
+
+// ---- grouped mode, for cq_moe_prefill_gemm (prompt_kq.cu): Q6_K, arguments checked there ----
+size_t cq_prefill_grouped_blob_bytes(int max_tiles, int k) { return (size_t)max_tiles * kTokTile * kTokBytes * (k / 256); }
+
+bool cq_prefill_grouped_q6k(const void *input, int in_elem, const void *weights, const int *tiles, int max_tiles, const int32_t *sorted_token_ids,
+                            const float *topk_weights, float *out, uint8_t *blobs, int topk, int n, int k, cudaStream_t st) {
+    const GroupInfo gi{tiles, sorted_token_ids, topk_weights, (long long)n * (k / 256) * cq_type_size(CQ_Q6_K), topk};
+    const int64_t items = (int64_t)max_tiles * kTokTile * (k / 256);
+    const unsigned qgrid = (unsigned)((items + 7) / 8);
+    if (in_elem == CQ_F32) quantize_q8k_tiles_grouped_kernel<float><<<qgrid, 256, 0, st>>>((const float *)input, blobs, k, max_tiles, gi);
+    else if (in_elem == CQ_F16) quantize_q8k_tiles_grouped_kernel<__half><<<qgrid, 256, 0, st>>>((const __half *)input, blobs, k, max_tiles, gi);
+    else if (in_elem == CQ_BF16)
+        quantize_q8k_tiles_grouped_kernel<__nv_bfloat16><<<qgrid, 256, 0, st>>>((const __nv_bfloat16 *)input, blobs, k, max_tiles, gi);
+    else { cq_set_status(CQ_ERR_BAD_ARG, "moe prefill: unknown input element type"); return false; }
+    prefill_smem_attr(1);
+    const int ntiles = ((n + kRowTile - 1) / kRowTile) * max_tiles;
+    prefill_kernel<CQ_Q6_K><<<prefill_grid(ntiles), kThreads, kSmemBytes, st>>>((const uint8_t *)weights, blobs, out, CQ_F32, k, n,
+                                                                                 max_tiles * kTokTile, n, g_prefill_dbg, max_tiles, ntiles, gi);
+    return cq_check_launch("moe prefill gemm");
 }
 
 #ifdef CQ_EXPERIMENT

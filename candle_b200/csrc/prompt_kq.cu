@@ -38,6 +38,7 @@
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace {
@@ -737,6 +738,11 @@ size_t group_blob_bytes(int size_m, int num_experts, int k) { return ((size_t)si
 
 }  // namespace
 
+// prefill_tcgen05.cu
+size_t cq_prefill_grouped_blob_bytes(int max_tiles, int k);
+bool cq_prefill_grouped_q6k(const void *input, int in_elem, const void *weights, const int *tiles, int max_tiles, const int32_t *sorted_token_ids,
+                            const float *topk_weights, float *out, uint8_t *blobs, int topk, int n, int k, cudaStream_t st);
+
 extern "C" size_t cq_prompt_scratch_bytes(int tokens, int k) {
     if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
     // whatever the tile size, only the last tile is padded, to a multiple of 16 rows
@@ -780,7 +786,20 @@ extern "C" void cq_prompt_matmul(int wtype, const void *vx, const void *x, int e
 // ---- grouped entry point (quantized mixture-of-experts, many tokens) ----
 extern "C" size_t cq_moe_prefill_scratch_bytes(int size_m, int num_experts, int k) {
     if (size_m <= 0 || num_experts <= 0 || num_experts > 1024 || k <= 0 || k % 256 != 0) return 0;
-    return table_bytes(group_max_tiles(size_m, num_experts)) + group_blob_bytes(size_m, num_experts, k) + 256;
+    const int mt = group_max_tiles(size_m, num_experts);
+    return table_bytes(mt) + std::max(group_blob_bytes(size_m, num_experts, k), cq_prefill_grouped_blob_bytes(mt, k)) + 256;
+}
+
+// Q6_K experts against the int8 kernel's grouped form (the same bits), by the rule of cq_prompt_pays on an expected number of token tiles:
+// half way between evenly spread pairs and a tile of each expert besides the full ones.  The int8 kernel is the faster as long as its tiles
+// of 64 rows find an SM each: 8 experts, 320 pairs, K = 2816 -> 768: 46 us against 34; 16 experts, 432 pairs, K = 4096 -> 512, which do
+// not: 52 against 73.  Of 12222 launches measured (1 - 64 experts, 128 - 3584 rows) 712 take the side that is slower by more than 3 %; by
+// this kernel alone 5070 would.
+extern "C" int cq_moe_prompt_pays(int wtype, int size_m, int num_experts, int n) {
+    if (wtype != CQ_Q6_K) return 1;
+    const int experts = size_m < num_experts ? size_m : num_experts;
+    const int even = experts * ((size_m + 128 * num_experts - 1) / (128 * num_experts)), uneven = experts + size_m / 128;
+    return (n + 63) / 64 * (long long)(even + uneven) / 2 > cq_sm_count() * 3 / 4;
 }
 
 // out[pair, :] = W[expert of the pair] . x[input row of the pair] (times topk_weights[pair]) for all size_m sorted pairs
@@ -810,6 +829,10 @@ extern "C" void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, c
     int *tiles = (int *)scratch;
     uint8_t *blobs = (uint8_t *)scratch + table_bytes(mt);
     group_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
+    if (!cq_moe_prompt_pays(wtype, size_m, num_experts, size_n)) {
+        (void)cq_prefill_grouped_q6k(input, in_elem, weights, tiles, mt, sorted_token_ids, topk_weights, out, blobs, topk, size_n, size_k, st);
+        return;
+    }
     const GroupInfo gi{tiles, sorted_token_ids, topk_weights, size_n, topk, topk_weights ? 1 : 0};
     const Tiling tl{mt * kTokMax, kTokMax, mt};
     if (!launch_quantize_rows(wtype, input, in_elem, blobs, size_k, tl, gi, st)) return;

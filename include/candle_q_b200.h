@@ -214,6 +214,8 @@ void cq_moe_prefill_gemm(int wtype, const void *input, int in_elem, const void *
                          const int32_t *expert_ids, const float *topk_weights, float *out, void *scratch, int num_experts,
                          int topk, int size_m, int size_n, int size_k, void *stream);
 
+int cq_moe_prompt_pays(int wtype, int size_m, int num_experts, int n);     /* 0: Q6_K launches of few tiles run the int8 kernel; the same bits */
+
 /* The expert part of a mixture-of-experts block (gate, up, up * silu(gate), down).
  *   cq_moe_sort_pairs   : i32 ids [pairs] -> expert_ids ascending, and the pair numbers in that order (stable); ids outside
  *                         [0, num_experts) come last, as num_experts: the expert products skip those pairs.

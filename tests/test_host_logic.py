@@ -145,3 +145,15 @@ def test_prompt_route_of_q6_k_takes_the_faster_kernel(lib):
     for (tokens, k, n), slow, fast in int8:
         assert fast < slow and lib.cq_prompt_pays(14, tokens, k, n) == 0, (tokens, k, n)
     assert lib.cq_prompt_pays(12, 18, 14336, 4096) == 1
+
+
+def test_grouped_route_of_q6_k_takes_the_faster_kernel(lib):
+    """(pairs, experts, rows) with the measured times of the int8 kernel and of the prompt kernel (us)."""
+    int8 = [((320, 8, 768), 33.7, 45.7), ((396, 2, 1536), 33.6, 45.7), ((150, 2, 256), 25.6, 34.6), ((77 * 2, 8, 512), 33.3, 39.5)]
+    f16 = [((432, 16, 512), 72.6, 52.0), ((832, 32, 256), 84.5, 58.0), ((8192, 128, 768), 220.2, 167.0), ((1024, 64, 1536), 195.6, 142.4),
+           ((180, 16, 768), 42.1, 31.5)]
+    for shape, fast, slow in int8:
+        assert fast < slow and lib.cq_moe_prompt_pays(14, *shape) == 0, shape
+    for shape, slow, fast in f16:
+        assert fast < slow and lib.cq_moe_prompt_pays(14, *shape) == 1, shape
+    assert lib.cq_moe_prompt_pays(12, 64, 2, 256) == 1
