@@ -5,18 +5,37 @@
 //
 // Both sides of a product carry a scale per 32 elements, so nothing beyond the integer sub-scales of a K-quant can be folded
 // into the operands: every 32-element block is two K = 16 steps into a FRESH accumulator slot, exact (sums below 2^24: at most
-// 31 * 63 * 127 * 32), and the epilogue adds  d_a d_w I [+ m_w s_a]  to f32 running sums, two at a time.
-// Against int8 operands the epilogue needs no int -> float conversion, which was two of its five operations per value.
+// 16 * 63 * 127 * 32), and the epilogue adds the scaled slots to f32 running sums, two values per instruction.
+//
+// What moved out of the epilogue, whose instructions per block bound the kernel before:
+//   * The minimum part of the formats that have one.  Codes are CENTRED (signed) in the operand - q - 8, q - 16, sc (q - 16), sc (2 q - 3), sc (q - 4) - and
+//     what the shift and the minimum contribute together is a sum over a chunk of (coefficient of the weights) x (sum of the activations):
+//         Q5_K  sum_g (16 d sc_g - dmin m_g) s_g     Q2_K  sum_j (1.5 d sc_j - dmin m_j) s_j, per 16 elements     Q5_0  sum_g -16 d_g (t_g - s_g)
+//     with s = d_a sum q8 and t the f16 sum of the inputs that Q8_1 stores.  Coefficients and sums are f32; each is split exactly into three
+//     bf16 parts, and the six products of parts down to 2^-16 are K steps of the tensor core into an accumulator of their own, the small
+//     ones first.  The large parts of d q and the minimum cancel in the coefficient and not in sums of thousands, so these formats are
+//     nearer to 64 bits than with f32 additions of both per block (2-norm, K = 4096, normal / one-signed activations: Q5_K 1.0e-7 / 2.9e-7, now
+//     6.5e-8 / 1.2e-7; Q2_K 7.8e-8 / 1.8e-7, now 6.0e-8 / 6.1e-8).  Not for Q4_1 and Q5_1, whose sum can be most of the result: the tensor core
+//     cuts off where an f32 addition rounds (3.7e-7 for 6.6e-8), so their codes stay unsigned and a block's two parts meet in the epilogue.
+//   * A super-block format has one d per 256 elements: a block is then ONE fma per value, sum += d_a I, and d is applied per chunk.
+//   * The accumulators are read with the 16x256b shape of tcgen05.ld: a thread holds four rows x two columns of each eight columns, so one
+//     8-byte shared load of token scales serves eight values (a 16-byte load served four with a row per lane: a broadcast takes as long as the
+//     bytes it delivers, 1.2 loads of 16 bytes a clock and SM).
 //
 // Summation: Q8_0 / Q4_0 add block after block, as the kernel behind cq_prefill32_gemm does (the same f32 operations, the same
 // bits).  The decode kernels, which the Q8_1 formats use otherwise, sum by a balanced tree; a plain chain of K / 32 additions would
 // lose precision against that, so the blocks of a 256-element chunk are added first and the chunks with a compensated sum.
 //
 // Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
-// warps 0-7 epilogue, 8-11 producers, 12 MMA issuer, 13 loader, 14-15 raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128
-// columns), 128 columns of operand A.  The roles hand over two blocks at a time.  Every wait is bounded as there.
-// Measured (quantizer included): Q5_K 4096 -> 14336, 512 tokens 2235 us (GEMV slices) -> 490; Q8_0 4096 -> 4096, 333 tokens 98 (int8 kernel,
-// 64 x 128 tiles) -> 88.  Two producer sets as in prompt_kq.cu made it 3 % slower: the epilogue, ~2.5 us per 256 k-elements, bounds it.
+// warps 0-7 epilogue, 8-15 producers (two sets of four, a weight row per thread, the sets take turns), 16 MMA issuer, 17 loader, 18-19
+// raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128 columns each), 64 columns for the
+// minimum sums where there are any, operand A in two or three buffers of two blocks.  The roles hand over two blocks at a time; where operand
+// A and the accumulators have as many buffers, one commit tells both the producers and the epilogue.  Every wait is bounded as there.
+//
+// Measured (B200, quantizer included; before -> now): Q5_K 4096 -> 14336, 512 tokens 493 us -> 263, Q8_0 4096 -> 4096, 333 tokens 88 -> 76.  A chunk of
+// 256 elements takes 2.1 us and 11 ns per token, 11 - 13 thousand warp instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
+// Tried: tiles of 128 tokens with one producer set (Q5_K 327), the group's first warp polling for the others (534: branches and barrier reads outweigh
+// the polls), a branch on the tile's tokens inside the block loop (312: the compiler then moves every running sum).
 #include "../../include/candle_q_b200.h"
 #include "prompt_f16.cuh"
 
@@ -27,52 +46,72 @@
 namespace {
 using namespace cq_prompt;
 
-constexpr int kEpiWarps = 8, kProdWarps = 4;
+constexpr int kEpiWarps = 8, kProdWarps = 8;     // producers: two sets of four
 constexpr int kMmaWarp = kEpiWarps + kProdWarps, kLoadWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
 constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two: raw bytes without a tensor map
-constexpr int kColA = 384;
-constexpr int kFixedTokens = 40;                // plan_tiling
+constexpr int kTok = 64;                         // tokens per tile, at most
+constexpr int kSlots = 3;                        // accumulator slots of two blocks
+constexpr int kStagesT = 4;                      // token stages of half a chunk
+constexpr int kFixedTokens = 180;                // plan_tiling: 2.1 us + 11 ns per token and chunk
+// registers: 640 threads x 96 at launch = 256 * 144 + 256 * 72 + 128 * 48
+constexpr int kRegsEpi32 = 144, kRegsProd32 = 72, kRegsMisc32 = 48;
 
 __device__ int g_prompt_b32_timeout_flag = 0;
 
-// kMins: terms m_w * s_a per block;  kSum: what s_a is;  kTerm: a block's terms are summed apart from the running sum.  The codes are unsigned,
-// so d_a d_w I and m_w s_a are both large and nearly cancel for weights around zero; added to the running sum one after the other they left
-// two to four times the decode kernels' error against 64 bits (2-norm, K = 4096, activations of one sign: Q4_1 2.2e-7 for 7.6e-8, Q5_1 2.6e-7
-// for 7.7e-8; now 6.7e-8 and 6.9e-8), for 2 - 4 % of the time.  Q5_K stays below the decode kernel's own error without (normal activations
-// 1.0e-7 for 1.1e-7, one sign 2.8e-7 for 4.9e-7).
-enum { kNoSum, kFloatSum, kIntSum };
-template <int WTYPE> struct Fmt {       // Q8_0, Q4_0
-    static constexpr bool kQ81 = false;
-    static constexpr int kMins = 0, kSum = kNoSum, kTok = 64, kStagesT = 4;
+// kSum: the activations' sums of the minimum part: none; s per 32 (Q5_K) or 16 (Q2_K) elements, t - s (Q5_0), which meet their coefficients on the tensor
+// core; t, in the epilogue (Q4_1, Q5_1: kTerm).
+enum { kNoSum, kSum32, kSum16, kDelta, kTermSum };
+template <int WTYPE> struct Fmt {       // Q8_0, Q4_0, Q3_K
+    static constexpr bool kQ81 = WTYPE == CQ_Q3_K, kBlockScale = WTYPE != CQ_Q3_K;
+    static constexpr int kSum = kNoSum;
     static constexpr bool kTerm = false;
 };
-template <int MINS, int SUM, bool TERM> struct FmtQ81 {
-    static constexpr bool kQ81 = true, kTerm = TERM;
-    static constexpr int kMins = MINS, kSum = SUM, kTok = 64, kStagesT = 4;
+template <int SUM, bool BLOCK> struct FmtMin {
+    static constexpr bool kQ81 = true, kBlockScale = BLOCK, kTerm = SUM == kTermSum;
+    static constexpr int kSum = SUM;
 };
-template <> struct Fmt<CQ_Q4_1> : FmtQ81<1, kFloatSum, true> {};
-template <> struct Fmt<CQ_Q5_0> : FmtQ81<1, kFloatSum, true> {};
-template <> struct Fmt<CQ_Q5_1> : FmtQ81<1, kFloatSum, true> {};
-template <> struct Fmt<CQ_Q5_K> : FmtQ81<1, kIntSum, false> {};
-template <> struct Fmt<CQ_Q2_K> : FmtQ81<2, kIntSum, true> {};     // one per 16 elements
-template <> struct Fmt<CQ_Q3_K> : FmtQ81<0, kNoSum, false> {};
+template <> struct Fmt<CQ_Q4_1> : FmtMin<kTermSum, true> {};
+template <> struct Fmt<CQ_Q5_0> : FmtMin<kDelta, true> {};
+template <> struct Fmt<CQ_Q5_1> : FmtMin<kTermSum, true> {};
+template <> struct Fmt<CQ_Q5_K> : FmtMin<kSum32, false> {};
+template <> struct Fmt<CQ_Q2_K> : FmtMin<kSum16, false> {};
 
+constexpr int sums_of(int sum) { return sum == kNoSum || sum == kTermSum ? 0 : sum == kSum16 ? 16 : 8; }   // coefficients per chunk
+constexpr int kColV = 384;                       // tensor memory column of the minimum sums
+// f16 values; scales, and t where the epilogue takes it; four planes of bf16 sums (lo, mid, hi where finite, hi) of one token and chunk
+constexpr int float_bytes(int sum) { return sum == kTermSum ? 64 : 32; }
+constexpr int tok_bytes(int sum) { return 512 + float_bytes(sum) + 8 * sums_of(sum); }
 template <int WTYPE> constexpr int chunk_bytes() { return 256 / cq_block_elems(WTYPE) * cq_type_size(WTYPE); }
-template <int MINS> constexpr int tok_bytes() { return 512 + 32 + 32 * MINS; }        // f16 values, scales, sums of one chunk
-template <int MINS> constexpr int wscale_bytes() { return MINS == 0 ? 4 : MINS == 1 ? 8 : 16; }
 template <int WTYPE> struct Smem {
     using F = Fmt<WTYPE>;
-    static constexpr int kStageT = 16 * F::kTok * 16, kAux = F::kTok * (32 + 32 * F::kMins), kRingW = 8 * kRows * wscale_bytes<F::kMins>();
-    static constexpr int kBytes = 1024 + F::kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
+    static constexpr int kSums = sums_of(F::kSum), kNA = kSums ? 2 : 3;             // buffers of operand A
+    static constexpr int kColA = kSums ? 448 : 384;
+    static constexpr int kStageT = 16 * kTok * 16, kAux = kTok * (float_bytes(F::kSum) + 8 * kSums);
+    static constexpr int kRingW = kRows * 4 * (F::kTerm ? 16 : F::kBlockScale ? 8 : 1);      // d of the rows (and m), one chunk
+    static constexpr int kRawStages = F::kTerm ? 2 : 3;
+    static constexpr int kCoef = 3 * kRows * 2 * kSums;                              // planes lo, hi, mid of the coefficients
+    static constexpr int kBytes = 1024 + kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * kCoef + kRawStages * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
 };
+
+// v = hi + mid + lo, exactly (8 bits each); a value that is not finite has only its first part
+__device__ __forceinline__ void split3(float v, uint16_t &hi, uint16_t &mid, uint16_t &lo) {
+    auto bits = [](__nv_bfloat16 b) { return __bfloat16_as_ushort(b); };
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    const bool finite = fabsf(__bfloat162float(h)) <= 3.4e38f;
+    const float r = finite ? __fsub_rn(v, __bfloat162float(h)) : 0.0f;
+    const __nv_bfloat16 m = __float2bfloat16_rn(r);
+    hi = bits(h);
+    mid = bits(m);
+    lo = bits(__float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m))));
+}
 
 // ---- activations ---------------------------------------------------------------------------------------------------
 // One warp per (token, chunk of 256), 8 tokens of one chunk per block, through shared memory (see prompt_kq.cu).
-template <typename T, bool Q81, int MINS, int SUM>
+template <typename T, bool Q81, int SUM>
 __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k, Tiling tl) {
-    constexpr int kPitch = 8 * 16 + 16, kVals = 8 * (1 + MINS);
-    __shared__ __align__(16) uint8_t sm[32 * kPitch];
-    __shared__ float sv[kVals][8];      // [value][token]: block scales, then sums
+    constexpr int kPitch = 8 * 16 + 16, kPlane = sums_of(SUM) / 8, kSlabs = 32 + 4 * kPlane, kFloats = float_bytes(SUM) / 4;
+    __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
+    __shared__ float sv[kFloats][8];    // [block][token]: scales, then t
     cq_pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nch = k / 256;
@@ -108,32 +147,48 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, 
     *reinterpret_cast<uint4 *>(sm + lane * kPitch + warp * 16) = pack_q8(q);
     const int b = lane >> 2;
     if ((lane & 3) == 0) sv[b][warp] = dh;
-    if constexpr (SUM == kFloatSum) {
-        // the f16-rounded sum of the inputs, added in the order of a 32-lane xor butterfly over the block (16, 8, 4, 2, 1)
-        float s[8];
+    if constexpr (SUM != kNoSum) {
+        int si = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+        si += __shfl_xor_sync(0xffffffffu, si, 1);
+        if constexpr (SUM != kSum16) si += __shfl_xor_sync(0xffffffffu, si, 2);
+        const float s = __fmul_rn(dh, (float)si);
+        [[maybe_unused]] auto put = [&](int j, float v) {        // sum j of the chunk: element j % 8 of slab j / 8 of each plane
+            uint16_t hi, mid, lo;
+            split3(v, hi, mid, lo);
+            uint8_t *p = sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7);
+            const uint16_t plane[4] = {lo, mid, (uint16_t)((hi & 0x7F80u) == 0x7F80u ? 0 : hi), hi};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(e[i], __shfl_xor_sync(0xffffffffu, e[i], 2));
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint16_t *>(p + i * kPlane * kPitch) = plane[i];
+        };
+        if constexpr (SUM == kSum16) { if ((lane & 1) == 0) put(lane >> 1, s); }
+        else if constexpr (SUM == kSum32) { if ((lane & 3) == 0) put(b, s); }
+        else {
+            // t: the f16-rounded sum of the inputs, added in the order of a 32-lane xor butterfly over the block (16, 8, 4, 2, 1)
+            float u[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], 1));
-        const float t0 = __fadd_rn(__fadd_rn(s[0], s[4]), __fadd_rn(s[2], s[6])), t1 = __fadd_rn(__fadd_rn(s[1], s[5]), __fadd_rn(s[3], s[7]));
-        if ((lane & 3) == 0) sv[8 + b][warp] = __half2float(__float2half_rn(__fadd_rn(t0, t1)));
-    } else if constexpr (SUM == kIntSum) {      // scale times the sum of the int8 values, per block or per 16
-        int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if constexpr (MINS == 1) s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if constexpr (MINS == 1) { if ((lane & 3) == 0) sv[8 + b][warp] = __fmul_rn(dh, (float)s); }
-        else { if ((lane & 1) == 0) sv[8 + 8 * ((lane >> 1) & 1) + b][warp] = __fmul_rn(dh, (float)s); }
+            for (int i = 0; i < 8; ++i) u[i] = __fadd_rn(e[i], __shfl_xor_sync(0xffffffffu, e[i], 2));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) u[i] = __fadd_rn(u[i], __shfl_xor_sync(0xffffffffu, u[i], 1));
+            const float t0 = __fadd_rn(__fadd_rn(u[0], u[4]), __fadd_rn(u[2], u[6])), t1 = __fadd_rn(__fadd_rn(u[1], u[5]), __fadd_rn(u[3], u[7]));
+            const float ts = __half2float(__float2half_rn(__fadd_rn(t0, t1)));
+            if ((lane & 3) == 0) {
+                if constexpr (SUM == kDelta) put(b, __fsub_rn(ts, s));
+                else sv[8 + b][warp] = ts;
+            }
+        }
     }
     __syncthreads();
-    uint8_t *blob = y + ((size_t)t * tl.tt * nch + (size_t)c * rows) * tok_bytes<MINS>();
-    for (int i = threadIdx.x; i < 32 * 8; i += 256)
-        *reinterpret_cast<uint4 *>(blob + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 16) = *reinterpret_cast<const uint4 *>(sm + (i >> 3) * kPitch + (i & 7) * 16);
-    for (int i = threadIdx.x; i < kVals * 8; i += 256)
-        *reinterpret_cast<float *>(blob + (size_t)rows * 512 + ((size_t)(i >> 3) * rows + row0 + (i & 7)) * 4) = sv[i >> 3][i & 7];
+    uint8_t *blob = y + ((size_t)t * tl.tt * nch + (size_t)c * rows) * tok_bytes(SUM);
+    for (int i = threadIdx.x; i < kSlabs * 8; i += 256) {
+        const int slab = i >> 3;
+        *reinterpret_cast<uint4 *>(blob + (size_t)rows * (slab < 32 ? slab * 16 : slab * 16 + 4 * kFloats) + (size_t)(row0 + (i & 7)) * 16) =
+            *reinterpret_cast<const uint4 *>(sm + slab * kPitch + (i & 7) * 16);
+    }
+    if (threadIdx.x < kFloats * 8)
+        *reinterpret_cast<float *>(blob + (size_t)rows * 512 + ((size_t)(threadIdx.x >> 3) * rows + row0 + (threadIdx.x & 7)) * 4) = sv[threadIdx.x >> 3][threadIdx.x & 7];
 }
 
-// ---- producers: chunk CH = 0..3 covers blocks 2 CH (cells 0-15) and 2 CH + 1 (cells 16-31) -----------------------------
-struct WScale { float d, m0, m1; };
+// ---- producers: chunk ch = 0..3 covers blocks 2 ch (cells 0-15) and 2 ch + 1 (cells 16-31) -----------------------------
 
 // 32-bit word at byte offset OFF (even) of a row chunk held as 16-byte vectors from vector V0 on
 template <int OFF, int V0, int NV> __device__ __forceinline__ uint32_t word_at(const uint4 (&v)[NV]) {
@@ -149,6 +204,17 @@ __device__ __forceinline__ void codes4(uint32_t w, float off, uint32_t &a, uint3
     a = h2_bits(__hsub2(bits_h2((w & 0x00FF00FFu) | 0x64006400u), o));
     b = h2_bits(__hsub2(bits_h2(((w >> 8) & 0x00FF00FFu) | 0x64006400u), o));
 }
+__device__ __forceinline__ __half2 twice(uint32_t v) { return __hsub2(bits_h2(v * 0x00010001u | 0x64006400u), bits_h2(0x64006400u)); }   // v < 1024
+// Coefficients j, j + 1 (j even) of a row: planes lo, hi, mid of kSums / 8 slabs of 128 rows x 16 bytes
+template <int SUMS> __device__ __forceinline__ void put_coef(uint8_t *row, int j, float a, float b) {
+    uint16_t h0, m0, l0, h1, m1, l1;
+    split3(a, h0, m0, l0);
+    split3(b, h1, m1, l1);
+    uint8_t *p = row + (j >> 3) * kRows * 16 + 2 * (j & 7);
+    *reinterpret_cast<uint32_t *>(p) = l0 | (uint32_t)l1 << 16;
+    *reinterpret_cast<uint32_t *>(p + SUMS / 8 * kRows * 16) = h0 | (uint32_t)h1 << 16;
+    *reinterpret_cast<uint32_t *>(p + 2 * (SUMS / 8) * kRows * 16) = m0 | (uint32_t)m1 << 16;
+}
 
 template <int WTYPE> struct Expand;
 
@@ -158,12 +224,23 @@ template <int WTYPE> struct ExpandBlock {
     static constexpr bool kHasM = WTYPE == CQ_Q4_1 || WTYPE == CQ_Q5_1, kFive = WTYPE == CQ_Q5_0 || WTYPE == CQ_Q5_1;
     const uint8_t *p;
     __device__ __forceinline__ void header(const uint8_t *rr, int) { p = rr; }
-    template <int B, int V0, int NV> __device__ __forceinline__ WScale block(const uint4 (&v)[NV], uint32_t *o) const {
+    __device__ __forceinline__ void scales(float *dst) const {          // [8 blocks][128 rows] d, then the same of m
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const float d = h16(cq_lds_u16(p + b * kBlk));
+            dst[b * kRows] = d;
+            if constexpr (kHasM) dst[(8 + b) * kRows] = h16(cq_lds_u16(p + b * kBlk + 2));
+        }
+    }
+    __device__ __forceinline__ void coef(uint8_t *row) const {
+        if constexpr (WTYPE == CQ_Q5_0) {
+#pragma unroll
+            for (int b = 0; b < 8; b += 2)
+                put_coef<8>(row, b, __fmul_rn(-16.0f, h16(cq_lds_u16(p + b * kBlk))), __fmul_rn(-16.0f, h16(cq_lds_u16(p + (b + 1) * kBlk))));
+        }
+    }
+    template <int B, int V0, int NV> __device__ __forceinline__ void block(const uint4 (&v)[NV], uint32_t *o) const {
         constexpr int off = B * kBlk, qs = off + 2 + (kHasM ? 2 : 0) + (kFive ? 4 : 0);
-        WScale s;
-        s.d = h16(word_at<off, V0>(v));
-        s.m1 = 0.0f;
-        s.m0 = kHasM ? h16(word_at<off + 2, V0>(v)) : __fmul_rn(-16.0f, s.d);      // Q5_0: the codes stay unsigned, -16 d s
         if constexpr (WTYPE == CQ_Q8_0) {
             auto four = [&](auto ic) {
                 constexpr int i = decltype(ic)::value;
@@ -186,23 +263,28 @@ template <int WTYPE> struct ExpandBlock {
                     lo |= ((((qh >> (4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
                     hi |= ((((qh >> (16 + 4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
                 }
-                constexpr float minus = WTYPE == CQ_Q4_0 ? 8.0f : 0.0f;
+                constexpr float minus = WTYPE == CQ_Q4_0 ? 8.0f : WTYPE == CQ_Q5_0 ? 16.0f : 0.0f;
                 codes4(lo, minus, o[2 * i], o[2 * i + 1]);
                 codes4(hi, minus, o[8 + 2 * i], o[8 + 2 * i + 1]);
             };
             four(std::integral_constant<int, 0>{}); four(std::integral_constant<int, 1>{});
             four(std::integral_constant<int, 2>{}); four(std::integral_constant<int, 3>{});
         }
-        return s;
     }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
+    template <int CH> __device__ __forceinline__ void pair(uint32_t (&o)[32]) const {
         constexpr int v0 = 2 * CH * kBlk / 16, nv = (2 * (CH + 1) * kBlk + 15) / 16 - v0;
         uint4 v[nv + 1];
 #pragma unroll
         for (int i = 0; i < nv; ++i) v[i] = *reinterpret_cast<const uint4 *>(p + 16 * (v0 + i));
         v[nv] = make_uint4(0u, 0u, 0u, 0u);       // word_at may name (not use) the word after the last
-        s[0] = block<2 * CH, v0>(v, o);
-        s[1] = block<2 * CH + 1, v0>(v, o + 16);
+        block<2 * CH, v0>(v, o);
+        block<2 * CH + 1, v0>(v, o + 16);
+    }
+    __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
+        if (ch == 0) pair<0>(o);
+        else if (ch == 1) pair<1>(o);
+        else if (ch == 2) pair<2>(o);
+        else pair<3>(o);
     }
 };
 template <> struct Expand<CQ_Q8_0> : ExpandBlock<CQ_Q8_0> {};
@@ -211,7 +293,10 @@ template <> struct Expand<CQ_Q4_1> : ExpandBlock<CQ_Q4_1> {};
 template <> struct Expand<CQ_Q5_0> : ExpandBlock<CQ_Q5_0> {};
 template <> struct Expand<CQ_Q5_1> : ExpandBlock<CQ_Q5_1> {};
 
-// Q5_K: Q4_K with the fifth bits of sub-block g in bit g of 32 bytes; codes times the 6-bit scale, at most 31 * 63 = 1953.
+// Super-block formats.  A code of b bits goes to the top of the mantissa, or near it, so that scale times (code - middle) is one fma whose
+// addend, -(base + middle) * scale, is exact in f16; one copy of the code for all of a chunk's four pairs (see prompt_kq.cu).
+
+// Q5_K: Q4_K with the fifth bits of sub-block g in bit g of 32 bytes.  Code q in bits 4-8: the value 64 + q.
 template <> struct Expand<CQ_Q5_K> {
     const uint8_t *p;
     uint32_t sc[2], mn[2], dm;
@@ -223,103 +308,122 @@ template <> struct Expand<CQ_Q5_K> {
         sc[1] = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
         mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
     }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
-        const uint4 a = *reinterpret_cast<const uint4 *>(p + 48 + 32 * CH), b = *reinterpret_cast<const uint4 *>(p + 64 + 32 * CH);
+    __device__ __forceinline__ void scales(float *dst) const { *dst = __low2float(bits_h2(dm)); }
+    __device__ __forceinline__ void coef(uint8_t *row) const {
+        const float d16 = __fmul_rn(16.0f, __low2float(bits_h2(dm))), dmin = __high2float(bits_h2(dm));
+        auto c = [&](int g) {       // 16 d sc is exact
+            const float s = (float)((sc[g >> 2] >> (8 * (g & 3))) & 0xFFu), m = (float)((mn[g >> 2] >> (8 * (g & 3))) & 0xFFu);
+            return __fmaf_rn(-dmin, m, __fmul_rn(d16, s));
+        };
+#pragma unroll
+        for (int g = 0; g < 8; g += 2) put_coef<8>(row, g, c(g), c(g + 1));
+    }
+    __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
+        const uint4 a = *reinterpret_cast<const uint4 *>(p + 48 + 32 * ch), b = *reinterpret_cast<const uint4 *>(p + 64 + 32 * ch);
         const uint4 ha = *reinterpret_cast<const uint4 *>(p + 16), hb = *reinterpret_cast<const uint4 *>(p + 32);
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
-        auto byte_of = [](const uint32_t (&t)[2], int j) { return (t[j >> 2] >> (8 * (j & 3))) & 0xFFu; };
-        auto twice = [](uint32_t v) { return __hsub2(bits_h2(v * 0x00010001u | 0x64006400u), bits_h2(0x64006400u)); };
-        const __half2 dmh = bits_h2(dm);
-        const float d = __low2float(dmh), dmin = __high2float(dmh);
-        s[0] = WScale{d, -__fmul_rn(dmin, (float)byte_of(mn, 2 * CH)), 0.0f};
-        s[1] = WScale{d, -__fmul_rn(dmin, (float)byte_of(mn, 2 * CH + 1)), 0.0f};
-        const __half2 s0 = twice(byte_of(sc, 2 * CH)), s1 = twice(byte_of(sc, 2 * CH + 1));
-        const __half2 c0 = __hmul2(s0, __float2half2_rn(-1024.0f));
-        const __half2 m1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-64.0f));
+        const uint32_t s16 = (ch & 2 ? sc[1] : sc[0]) >> (16 * (ch & 1));
+        const __half2 s0 = twice(s16 & 0xFFu), s1 = twice((s16 >> 8) & 0xFFu);
+        const __half2 c0 = __hmul2(s0, __float2half2_rn(-80.0f)), c1 = __hmul2(s1, __float2half2_rn(-80.0f));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-#pragma unroll
-            for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
-                const uint32_t u = od ? w[i] >> 8 : w[i], v = od ? h[i] >> 8 : h[i];
-                const uint32_t lo = (u & 0x000F000Fu) | ((2 * CH >= 4 ? v >> (2 * CH - 4) : v << (4 - 2 * CH)) & 0x00100010u);
-                // high nibbles stay in place, so their codes are 16-fold: the fifth bit goes to bit 8
-                const uint32_t hi = (u & 0x00F000F0u) | ((v << (7 - 2 * CH)) & 0x01000100u);
-                o[2 * i + od] = hfma2_bits(lo | 0x64006400u, s0, c0);
-                o[16 + 2 * i + od] = hfma2_bits(hi | 0x64006400u, m1, c1);
-            }
+            const uint32_t he = h[i] << (7 - 2 * ch), ho = h[i] >> (2 * ch);        // fifth bits 2 ch + 1 | 2 ch in bit 8
+            o[2 * i] = hfma2_bits(((w[i] << 4) & 0x00F000F0u) | ((he << 1) & 0x01000100u) | 0x54005400u, s0, c0);
+            o[2 * i + 1] = hfma2_bits(((w[i] >> 4) & 0x00F000F0u) | (ho & 0x01000100u) | 0x54005400u, s0, c0);
+            o[16 + 2 * i] = hfma2_bits((w[i] & 0x00F000F0u) | (he & 0x01000100u) | 0x54005400u, s1, c1);
+            o[16 + 2 * i + 1] = hfma2_bits(((w[i] >> 8) & 0x00F000F0u) | ((ho >> 1) & 0x01000100u) | 0x54005400u, s1, c1);
         }
     }
 };
 
 // Q2_K / Q3_K: block b = 4 n + pos: bit pair pos of bytes 32 n .. of the codes; a scale per 16 elements, number 2 b + half.
+// Q2_K: code q in bits 8-9: the value 4 + q; the operand is sc (2 q - 3), so the row's scale is d / 2.
 template <> struct Expand<CQ_Q2_K> {
     const uint8_t *p;
-    uint32_t q[8], sc[4];
     float d, dmin;
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;         // a multiple of 4 when the base is, else of 2
-        cq_lds_words<4>(p, sc);
         uint32_t dm[1];
         cq_lds_words<1>(p + 80, dm);
         d = h16(dm[0]); dmin = h16(dm[0] >> 16);
     }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
-        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 16 + 16 * CH, q);
+    __device__ __forceinline__ void scales(float *dst) const { *dst = __fmul_rn(0.5f, d); }
+    __device__ __forceinline__ void coef(uint8_t *row) const {
+        const float d15 = __fmul_rn(1.5f, d);
+        uint32_t sc[4];
+        cq_lds_words<4>(p, sc);
+        auto c = [&](int j) {
+            const uint32_t by = (sc[j >> 2] >> (8 * (j & 3))) & 0xFFu;
+            return __fmaf_rn(-dmin, (float)(by >> 4), __fmul_rn(d15, (float)(by & 0xFu)));
+        };
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) put_coef<16>(row, j, c(j), c(j + 1));
+    }
+    __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
+        uint32_t q[8], sc[1];
+        cq_lds_words<8>(p + 16 + 32 * (ch >> 1), q);
+        cq_lds_words<1>(p + 4 * ch, sc);
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
-            const int b = 2 * CH + bb, pos = b & 3;
-            float m[2];
+            const int pos = 2 * (ch & 1) + bb;
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                const uint32_t by = (sc[(2 * b + hf) >> 2] >> (8 * ((2 * b + hf) & 3))) & 0xFFu;
-                m[hf] = -__fmul_rn(dmin, (float)(by >> 4));
-                const __half2 sv = __hsub2(bits_h2((by & 0xFu) * 0x00010001u | 0x64006400u), bits_h2(0x64006400u));
-                const __half2 cv = __hmul2(sv, __float2half2_rn(-1024.0f));
+                const __half2 sv = twice((sc[0] >> (8 * (2 * bb + hf))) & 0xFu), s2 = __hadd2(sv, sv);
+                const __half2 cv = __hmul2(sv, __float2half2_rn(-11.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint32_t u = q[4 * hf + i] >> (2 * pos);
-                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits((u & 0x00030003u) | 0x64006400u, sv, cv);
-                    o[16 * bb + 8 * hf + 2 * i + 1] = hfma2_bits(((u >> 8) & 0x00030003u) | 0x64006400u, sv, cv);
+                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(((q[4 * hf + i] << (8 - 2 * pos)) & 0x03000300u) | 0x44004400u, s2, cv);
+                    o[16 * bb + 8 * hf + 2 * i + 1] = hfma2_bits(((q[4 * hf + i] >> (2 * pos)) & 0x03000300u) | 0x44004400u, s2, cv);
                 }
             }
-            s[bb] = WScale{d, m[0], m[1]};
         }
     }
 };
+// Q3_K: two bits, plus 4 when the mask bit is set, in bits 7-9: the value 8 + u; the operand is scale * (u - 4).
 template <> struct Expand<CQ_Q3_K> {
     const uint8_t *p;
-    uint32_t q[8], hm[8], sc[3];
-    float d;
+    uint32_t sc[3];
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;         // even
         cq_lds_words<3>(p + 96, sc);
-        cq_lds_words<8>(p, hm);
-        d = __half2float(*reinterpret_cast<const __half *>(p + 108));
     }
-    template <int CH> __device__ __forceinline__ void chunk(uint32_t (&o)[32], WScale (&s)[2]) {
-        if constexpr ((CH & 1) == 0) cq_lds_words<8>(p + 32 + 16 * CH, q);
+    __device__ __forceinline__ void scales(float *dst) const { *dst = __half2float(*reinterpret_cast<const __half *>(p + 108)); }
+    __device__ __forceinline__ void coef(uint8_t *) const {}
+    __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
+        uint32_t q[8], hm[8];
+        cq_lds_words<8>(p + 32 + 32 * (ch >> 1), q);
+        cq_lds_words<8>(p, hm);
+        // scale number j = 4 ch + 2 bb + half: 4 low bits from bytes 0-7, 2 high bits from bytes 8-11
+        const uint32_t scl = (ch & 1 ? sc[1] : sc[0]) >> (ch & 2 ? 4 : 0), sch = sc[2] >> (2 * ch);
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
-            const int b = 2 * CH + bb, pos = b & 3;
+            const int b = 2 * ch + bb, pos = b & 3;
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                const int j = 2 * b + hf;       // scale number: 4 low bits from bytes 0-7, 2 high bits from bytes 8-11
-                const uint32_t lo4 = (sc[(j & 7) >> 2] >> (8 * (j & 3) + (j < 8 ? 0 : 4))) & 0xFu, hi2 = (sc[2] >> (8 * (j & 3) + 2 * (j >> 2))) & 3u;
-                const __half2 sv = __hsub2(bits_h2((lo4 | hi2 << 4) * 0x00010001u | 0x64006400u), __float2half2_rn(1056.0f));
-                const __half2 four = __float2half2_rn(1028.0f);
+                const int j = 2 * bb + hf;
+                const uint32_t s6 = ((scl >> (8 * j)) & 0xFu) | ((sch >> (8 * j)) & 3u) << 4;
+                const __half2 sv = __hsub2(bits_h2(s6 * 0x00010001u | 0x64006400u), __float2half2_rn(1056.0f));
+                const __half2 cv = __hmul2(sv, __float2half2_rn(-12.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    // two bits, plus 4 when the mask bit is set, minus 4
-                    const uint32_t u = ((q[4 * hf + i] >> (2 * pos)) & 0x03030303u) | (((hm[4 * hf + i] >> b) & 0x01010101u) << 2);
-                    o[16 * bb + 8 * hf + 2 * i] = h2_bits(__hmul2(__hsub2(bits_h2((u & 0x00FF00FFu) | 0x64006400u), four), sv));
-                    o[16 * bb + 8 * hf + 2 * i + 1] = h2_bits(__hmul2(__hsub2(bits_h2(((u >> 8) & 0x00FF00FFu) | 0x64006400u), four), sv));
+                    const uint32_t u = q[4 * hf + i], h = hm[4 * hf + i];
+                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(((u << (7 - 2 * pos)) & 0x01800180u) | ((h << (9 - b)) & 0x02000200u) | 0x48004800u, sv, cv);
+                    o[16 * bb + 8 * hf + 2 * i + 1] =
+                        hfma2_bits(((u >> (1 + 2 * pos)) & 0x01800180u) | (((h >> 8) << (9 - b)) & 0x02000200u) | 0x48004800u, sv, cv);
                 }
             }
-            s[bb] = WScale{d, 0.0f, 0.0f};
         }
     }
 };
 
+// bf16 x bf16 from shared memory
+template <bool ACC> __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t desc_a, uint32_t desc_b, uint32_t idesc) {
+    if constexpr (ACC)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "l"(desc_of(desc_a)), "l"(desc_of(desc_b)), "r"(idesc) : "memory");
+    else
+        mma_f16_ss(tmem_d, desc_a, desc_b, idesc);
+}
 struct Args {
     const uint8_t *w, *act;
     void *out;
@@ -330,24 +434,27 @@ template <int WTYPE>
 __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
     using F = Fmt<WTYPE>;
     using S = Smem<WTYPE>;
-    constexpr int kCB = chunk_bytes<WTYPE>(), kMins = F::kMins, kTok = F::kTok, kStagesT = F::kStagesT, kSlots = 3;
+    constexpr int kCB = chunk_bytes<WTYPE>(), kSums = S::kSums, kNA = S::kNA;
+    constexpr bool kOneCommit = kNA == kSlots;      // bar_acc serves the producers too
     using R = Raw<kCB>;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [2] raw weight bytes landed
-    uint64_t *bar_rawfree = bar_raw + 2;                            // [2] read by all producers
-    uint64_t *bar_fullT = bar_raw + 4;                              // [4] token stage (first half: + scales) landed
-    uint64_t *bar_doneT = bar_raw + 8;                              // [4] its MMAs are complete
-    uint64_t *bar_fullW = bar_raw + 12;                             // [4] operand A chunk stored (all producers)
-    uint64_t *bar_doneW = bar_raw + 16;                             // [4] its MMAs are complete
-    uint64_t *bar_vis = bar_raw + 20;                               // [4] relay: the scales of this operand chunk are visible
-    uint64_t *bar_acc = bar_raw + 24;                               // [3] the MMAs of two blocks are complete
-    uint64_t *bar_free = bar_raw + 30;                              // [3] accumulator slot read (all epilogue warps)
+    uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [3] raw weight bytes landed
+    uint64_t *bar_rawfree = bar_raw + 3;                            // [3] read by both producer sets
+    uint64_t *bar_fullT = bar_raw + 6;                              // [4] token stage (first half: + scales) landed
+    uint64_t *bar_doneT = bar_raw + 10;                             // [4] its MMAs are complete
+    uint64_t *bar_fullW = bar_raw + 14;                             // [3] operand A pair stored (a producer set)
+    uint64_t *bar_doneW = bar_raw + 17;                             // [3] its MMAs are complete
+    uint64_t *bar_acc = bar_raw + 20;                               // [3] the MMAs of two blocks are complete
+    uint64_t *bar_free = bar_raw + 23;                              // [3] accumulator slot read (all epilogue warps)
+    uint64_t *bar_vis = bar_raw + 26;                               // [2] relay: the scales of this chunk are visible
+    uint64_t *bar_vfree = bar_raw + 28;                             // minimum sums read (all epilogue warps)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 520);
     uint8_t *stT0 = smem + 1024;
-    uint8_t *aux0 = stT0 + kStagesT * S::kStageT;       // [4] scales [8][n], then sums [kMins][8][n]
-    uint8_t *ringW = aux0 + 4 * S::kAux;                // [4][8 blocks][128 rows] weight scales (and minima)
-    uint8_t *raw0 = ringW + 4 * S::kRingW;              // 128-byte aligned
+    uint8_t *aux0 = stT0 + kStagesT * S::kStageT;       // [4] scales [8][n], then planes of sums
+    uint8_t *ringW = aux0 + 4 * S::kAux;                // [4][1 or 8][128 rows] d
+    uint8_t *coef0 = ringW + 4 * S::kRingW;             // [2] planes of coefficients
+    uint8_t *raw0 = coef0 + 2 * S::kCoef;               // 128-byte aligned
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nch = a.nch;
@@ -355,15 +462,16 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     const GroupInfo gi{};
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
-        for (int i = 0; i < 4; ++i) {
-            cq_mbar_init(&bar_fullT[i], 1);
-            cq_mbar_init(&bar_doneT[i], 1);
-            cq_mbar_init(&bar_fullW[i], kProdWarps);
+        for (int i = 0; i < S::kRawStages; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < kStagesT; ++i) { cq_mbar_init(&bar_fullT[i], 1); cq_mbar_init(&bar_doneT[i], 1); }
+        for (int i = 0; i < 3; ++i) {
+            cq_mbar_init(&bar_fullW[i], kProdWarps / 2);
             cq_mbar_init(&bar_doneW[i], 1);
-            cq_mbar_init(&bar_vis[i], 1);
+            cq_mbar_init(&bar_acc[i], 1);
+            cq_mbar_init(&bar_free[i], kEpiWarps);
         }
-        for (int i = 0; i < kSlots; ++i) { cq_mbar_init(&bar_acc[i], 1); cq_mbar_init(&bar_free[i], kEpiWarps); }
+        for (int i = 0; i < 2; ++i) cq_mbar_init(&bar_vis[i], 1);
+        cq_mbar_init(bar_vfree, kEpiWarps);
         *abort_flag = 0;
         cq_fence_mbar_init();
     }
@@ -377,72 +485,27 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     cq_pdl_wait();
 
-    if (warp >= kEpiWarps && warp < kMmaWarp) {
-        // ===== producers: thread = weight row = TMEM lane =====
-        const int r = tid - kEpiWarps * 32;
-        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
-        int it = 0, wi = 0;
-        bool alive = true;
-        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
-            TileCtx cx;
-            tile_ctx(tile, tl.ntt, tl, gi, cx);
-            long long wr = cx.wrow0 + r;
-            if (wr >= a.nrows) wr = a.nrows - 1;
-            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
-            for (int c = 0; c < nch && alive; ++c, ++it) {
-                const int rs = it & 1;
-                if (!wait_warp(&bar_raw[rs], (it >> 1) & 1, abort_flag)) { alive = false; break; }
-                Expand<WTYPE> ex;
-                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
-                uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
-                auto step = [&](auto chc) {
-                    constexpr int CH = decltype(chc)::value;
-                    if (!alive) return;
-                    uint32_t o[32];
-                    WScale s[2];
-                    ex.template chunk<CH>(o, s);
-                    if constexpr (CH == 3) arrive_warp(&bar_rawfree[rs], lane);
-                    const int buf = wi & 3;
-                    if (wi >= 4 && !wait_warp(&bar_doneW[buf], ((wi >> 2) - 1) & 1, abort_flag)) { alive = false; return; }
-                    tc_fence_after();
-                    // the first operand chunk of it - 1 is done, so its MMAs had started and the epilogue, at most three
-                    // operand chunks behind them, has finished it - 3: entry it - 4 of the ring is free
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        uint8_t *dst = rw + (2 * CH + b) * kRows * wscale_bytes<kMins>();
-                        if constexpr (kMins == 0) *reinterpret_cast<float *>(dst) = s[b].d;
-                        else if constexpr (kMins == 1) *reinterpret_cast<float2 *>(dst) = make_float2(s[b].d, s[b].m0);
-                        else *reinterpret_cast<float4 *>(dst) = make_float4(s[b].d, s[b].m0, s[b].m1, 0.0f);
-                    }
-                    tmem_st32(ta + buf * 32, o);
-                    tmem_st_wait();
-                    tc_fence_before();
-                    arrive_warp(&bar_fullW[buf], lane);
-                    ++wi;
-                };
-                step(std::integral_constant<int, 0>{}); step(std::integral_constant<int, 1>{});
-                step(std::integral_constant<int, 2>{}); step(std::integral_constant<int, 3>{});
-            }
-        }
-    } else if (warp == kLoadWarp) {
+    if (warp >= kMmaWarp) {
+    regs_down<kRegsMisc32>();
+    if (warp == kLoadWarp) {
         // ===== loader =====
-        int it = 0, ti = 0;
+        int it = 0, ti = 0, rs = 0, rs_phase = 1;       // rs_phase: parity of the wait for this stage's previous use
         bool alive = true;
         for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
             TileCtx cx;
             tile_ctx(tile, tl.ntt, tl, gi, cx);
             const int n = cx.n;
-            const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes<kMins>();
+            const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes(F::kSum);
             for (int c = 0; c < nch && alive; ++c, ++it) {
-                const int rs = it & 1;
                 if (a.use_map) {
-                    if (it >= 2 && !wait_warp(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                    if (it >= S::kRawStages && !wait_warp(&bar_rawfree[rs], rs_phase, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
                         cq_tmap::load_2d(raw0 + rs * R::kBytes, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
                     }
+                    if (++rs == S::kRawStages) { rs = 0; rs_phase ^= 1; }
                 }
-                const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes<kMins>();
+                const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes(F::kSum);
                 for (int half = 0; half < 2; ++half, ++ti) {
                     const int s = ti % kStagesT;
                     if (ti >= kStagesT && !wait_warp(&bar_doneT[s], (ti / kStagesT - 1) & 1, abort_flag)) { alive = false; break; }
@@ -450,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         const unsigned bytes = (unsigned)n * 256;
                         if (half == 0) {
                             // a stage of chunk it - 2 (or later) is done: its MMAs had started, so the epilogue has finished it - 4
-                            const unsigned aux_bytes = (unsigned)n * (32 + 32 * kMins);
+                            const unsigned aux_bytes = (unsigned)n * (float_bytes(F::kSum) + 8 * kSums);
                             cq_mbar_expect_tx(&bar_fullT[s], bytes + aux_bytes);
                             cq_bulk_g2s(aux0 + (it & 3) * S::kAux, blob + (size_t)n * 512, aux_bytes, &bar_fullT[s]);
                         } else {
@@ -464,7 +527,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         }
         // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
         if (lane == 0 && (!alive || *abort_flag)) {
-            for (int j = it >= 2 ? it - 1 : 0; a.use_map && j <= it; ++j) (void)cq_mbar_wait_bounded(&bar_raw[j & 1], (j >> 1) & 1);
+            for (int j = it >= S::kRawStages ? it - S::kRawStages + 1 : 0; a.use_map && j <= it; ++j)
+                (void)cq_mbar_wait_bounded(&bar_raw[j % S::kRawStages], (j / S::kRawStages) & 1);
             for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j % kStagesT], (j / kStagesT) & 1);
         }
         __syncwarp();
@@ -478,8 +542,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 tile_ctx(tile, tl.ntt, tl, gi, cx);
                 const uint8_t *w0 = a.w + cx.wrow0 * row_bytes;
                 for (int c = 0; c < nch; ++c, ++it) {
-                    const int rs = it & 1;
-                    if (it >= 2 && !wait_warp(&bar_rawfree[rs], ((it >> 1) - 1) & 1, abort_flag)) { alive = false; break; }
+                    const int rs = it % S::kRawStages;
+                    if (it >= S::kRawStages && !wait_warp(&bar_rawfree[rs], (it / S::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                     R::load_rows(raw0 + rs * R::kBytes, w0 + (uint32_t)c * kCB, min(a.nrows - cx.row0, kRows), row_bytes, tid - kRawWarp * 32, &bar_raw[rs]);
                 }
             }
@@ -488,7 +552,9 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     } else if (warp == kMmaWarp) {
         // ===== MMA issuer (the warp runs the loop, one elected lane issues): a block = two K = 16 steps into fresh columns =====
         const uint32_t stT = uniform(cq_smem_u32(stT0) >> 4), tm = uniform(tmem_base);
-        int it = 0, wi = 0, s = 0, s_phase = 0, slot = 0, round = 0;      // token stage; accumulator slot and how often all have been used
+        [[maybe_unused]] const uint32_t coef = uniform(cq_smem_u32(coef0) >> 4), aux = uniform(cq_smem_u32(aux0) >> 4);
+        int it = 0, s = 0, s_phase = 0, slot = 0, round = 0;      // token stage; accumulator slot and how often all have been used
+        int buf = 0, buf_phase = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
             TileCtx cx;
@@ -497,137 +563,211 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
 #pragma unroll 1
             for (int c = 0; c < nch && alive; ++c, ++it) {
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch, ++wi) {
-                    const int buf = wi & 3;
+                for (int ch = 0; ch < 4; ++ch) {
                     if (((ch & 1) == 0 && !wait_warp(&bar_fullT[s], s_phase, abort_flag)) ||
-                        !wait_warp(&bar_fullW[buf], (wi >> 2) & 1, abort_flag) ||
-                        (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag))) { alive = false; break; }
+                        !wait_warp(&bar_fullW[buf], buf_phase, abort_flag) ||
+                        (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag)) ||
+                        (kSums && ch == 3 && it > 0 && !wait_warp(bar_vfree, (it - 1) & 1, abort_flag))) { alive = false; break; }
                     tc_fence_after();
-                    const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = tm + (uint32_t)(kColA + buf * 32);
+                    const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = tm + (uint32_t)(S::kColA + buf * 32);
                     const uint32_t td = tm + (uint32_t)(slot * 2 * kTok);
                     if (elect_one()) {
-                        mbar_arrive(&bar_vis[buf]);     // what this warp has acquired is visible to the epilogue
+                        if (ch == 0) mbar_arrive(&bar_vis[it & 1]);     // what this warp has acquired is visible to the epilogue
                         mma_f16_ts<false>(td, a0, b0, idesc);
                         mma_f16_ts<true>(td, a0 + 8, b0 + 2 * n, idesc);
                         mma_f16_ts<false>(td + kTok, a0 + 16, b0 + 4 * n, idesc);
                         mma_f16_ts<true>(td + kTok, a0 + 24, b0 + 6 * n, idesc);
+                        if constexpr (kSums > 0) {
+                            if (ch == 3) {          // A planes lo, hi, mid; B planes lo, mid, hi where finite, hi
+                                const uint32_t tv = tm + (uint32_t)kColV, idb = idesc | (1u << 7) | (1u << 10);      // bf16 x bf16
+                                const uint32_t ca = (coef + (uint32_t)(it & 1) * (S::kCoef >> 4)) | ((uint32_t)kRows << 16);
+                                const uint32_t cb = (aux + (uint32_t)(it & 3) * (S::kAux >> 4) + (float_bytes(F::kSum) / 16) * n) | (n << 16);
+                                if constexpr (kSums == 8) {         // a step is two planes of eight
+                                    mma_ss<false>(tv, ca + kRows, cb, idb);                 // hi lo + mid mid
+                                    mma_ss<true>(tv, ca + kRows, cb + n, idb);              // hi mid + mid hi
+                                    mma_ss<true>(tv, ca, cb + 2 * n, idb);                  // lo hi + hi hi
+                                } else {
+                                    mma_ss<false>(tv, ca + 2 * kRows, cb, idb);             // hi lo
+                                    mma_ss<true>(tv, ca + 4 * kRows, cb + 2 * n, idb);      // mid mid
+                                    mma_ss<true>(tv, ca, cb + 4 * n, idb);                  // lo hi
+                                    mma_ss<true>(tv, ca + 2 * kRows, cb + 2 * n, idb);      // hi mid
+                                    mma_ss<true>(tv, ca + 4 * kRows, cb + 4 * n, idb);      // mid hi
+                                    mma_ss<true>(tv, ca + 2 * kRows, cb + 6 * n, idb);      // hi hi
+                                }
+                            }
+                        }
                         tc_commit(&bar_acc[slot]);
                         if (ch & 1) tc_commit(&bar_doneT[s]);
-                        tc_commit(&bar_doneW[buf]);
+                        if constexpr (!kOneCommit) tc_commit(&bar_doneW[buf]);
                     }
                     __syncwarp();
                     if (++slot == kSlots) { slot = 0; ++round; }
+                    if (++buf == kNA) { buf = 0; buf_phase ^= 1; }
                     if ((ch & 1) && ++s == kStagesT) { s = 0; s_phase ^= 1; }
                 }
             }
         }
-    } else {
-        // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
-        constexpr int kG = kTok / 32;
-        constexpr bool kComp = F::kQ81;
-        const int quad = warp & 3, ch0 = warp >> 2;
-        const int r = quad * 32 + lane;
-        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
-        const uint64_t minus1 = pack2f(-1.0f, -1.0f), one = pack2f(1.0f, 1.0f);
-        int it = 0, slot = 0, round = 0;
+    }
+    } else if (warp >= kEpiWarps) {
+        regs_down<kRegsProd32>();
+        // ===== producers: thread = weight row = TMEM lane; set 0 takes the even pairs of blocks, set 1 the odd ones =====
+        const int set = (warp - kEpiWarps) >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)S::kColA;
+        int it = 0, rs = 0, rs_phase = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
             TileCtx cx;
             tile_ctx(tile, tl.ntt, tl, gi, cx);
-            uint64_t acc[kG][8];                                              // running sums (or those of this chunk)
-            uint64_t sum[kComp ? kG : 1][8], low[kComp ? kG : 1][8];          // compensated sum of the chunks
-#pragma unroll
-            for (int g = 0; g < kG; ++g)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    acc[g][i] = 0ull;
-                    if constexpr (kComp) { sum[g][i] = 0ull; low[g][i] = 0ull; }
-                }
+            long long wr = cx.wrow0 + r;
+            if (wr >= a.nrows) wr = a.nrows - 1;
+            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
             for (int c = 0; c < nch && alive; ++c, ++it) {
-                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux);
-                const uint8_t *rw = ringW + (it & 3) * S::kRingW + r * wscale_bytes<kMins>();
+                if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
+                Expand<WTYPE> ex;
+                ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
+                // This set has waited for a pair of it - 2 or later (its last pair of it - 1 took over the buffer of one), so the sums step of
+                // it - 2 is complete where there is one, and the epilogue, at most three pairs behind the MMAs, has finished it - 4.
+                if (set == 0) ex.scales(reinterpret_cast<float *>(ringW + (it & 3) * S::kRingW) + r);
+                else if constexpr (kSums > 0) {
+                    ex.coef(coef0 + (it & 1) * S::kCoef + r * 16);
+                    fence_proxy_async_smem();
+                }
+#pragma unroll 1
+                for (int ch = set; ch < 4; ch += 2) {
+                    uint32_t o[32];
+                    ex.chunk(ch, o);
+                    if (ch >= 2) arrive_warp(&bar_rawfree[rs], lane);
+                    const int wi = 4 * it + ch, buf = wi % kNA, turn = wi / kNA;
+                    if (turn > 0 && !wait_warp(kOneCommit ? &bar_acc[buf] : &bar_doneW[buf], (turn - 1) & 1, abort_flag)) { alive = false; break; }
+                    tc_fence_after();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) tmem_st8(ta + buf * 32 + 8 * i, o + 8 * i);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    arrive_warp(&bar_fullW[buf], lane);
+                }
+                if (++rs == S::kRawStages) { rs = 0; rs_phase ^= 1; }
+            }
+        }
+    } else {
+        regs_up<kRegsEpi32>();
+        // ===== epilogue: warp = 32 weight rows 32 (warp % 4) .., half of the tokens =====
+        // A thread holds rows r0 + 8 i, columns 8 j + csub, + 1 of its half: pair 2 N8 (i / 2) + 2 j + i % 2.
+        constexpr bool kComp = F::kQ81;
+        const int half = warp >> 2, r0 = (warp & 3) * 32 + (lane >> 2), csub = 2 * (lane & 3);
+        const uint64_t minus1 = pack2f(-1.0f, -1.0f), one = pack2f(1.0f, 1.0f);
+        int it = 0, slot = 0, round = 0;
+        bool alive = true;
+        // A tile whose warps have up to N8 units of eight columns; those past the tile's tokens are computed and dropped.  (The two sizes are separate
+        // loops: a branch on the size inside, over running sums, made the compiler move every sum, a quarter of the epilogue's instructions.)
+        auto run_tile = [&](const TileCtx &cx, auto units) {
+            constexpr int N8 = decltype(units)::value, kP = 4 * N8;
+            const int n = cx.n, col0 = half * (n >> 1), n8 = n >> 4;
+            const uint32_t tq = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
+            uint64_t acc[kP];                                                 // running sums (or those of this chunk)
+            [[maybe_unused]] uint64_t sum[kComp ? kP : 1], low[kComp ? kP : 1];       // compensated sum of the chunks
+#pragma unroll
+            for (int i = 0; i < kP; ++i) {
+                acc[i] = 0ull;
+                if constexpr (kComp) { sum[i] = 0ull; low[i] = 0ull; }
+            }
+            for (int c = 0; c < nch; ++c, ++it) {
+                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux) + col0 + csub;
+                const float *rw = reinterpret_cast<const float *>(ringW + (it & 3) * S::kRingW) + r0;
+                if (!wait_warp(&bar_vis[it & 1], (it >> 1) & 1, abort_flag)) return false;
 #pragma unroll 1
                 for (int ch = 0; ch < 4; ++ch) {
-                    if (!wait_warp(&bar_vis[ch], it & 1, abort_flag) || !wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
+                    if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) return false;
                     tc_fence_after();
 #pragma unroll
                     for (int bb = 0; bb < 2; ++bb) {
                         const int b = 2 * ch + bb;
-                        const uint8_t *wp = rw + b * kRows * wscale_bytes<kMins>();
-                        float wd, m0 = 0.0f, m1 = 0.0f;
-                        if constexpr (kMins == 0) wd = *reinterpret_cast<const float *>(wp);
-                        else if constexpr (kMins == 1) { const float2 v = *reinterpret_cast<const float2 *>(wp); wd = v.x; m0 = v.y; }
-                        else { const float4 v = *reinterpret_cast<const float4 *>(wp); wd = v.x; m0 = v.y; m1 = v.z; }
-                        const uint64_t dw = pack2f(wd, wd), mm0 = pack2f(m0, m0), mm1 = pack2f(m1, m1);
+                        uint32_t p[8 * N8];
+                        const uint32_t ts = tq + (uint32_t)((2 * slot + bb) * kTok);
+                        tmem_ld_16x256b<N8>(ts, p);
+                        tmem_ld_16x256b<N8>(ts + (16u << 16), p + 4 * N8);
+                        [[maybe_unused]] uint64_t dw[4] = {}, mw[4] = {}, dd[N8], ss[N8];
 #pragma unroll
-                        for (int g = 0; g < kG; ++g) {
-                            const int col = (2 * g + ch0) * 16;
-                            if (col < cx.n) {           // warp-uniform
-                                uint32_t p[16];
-                                tmem_ld16(tlane + (uint32_t)((2 * slot + bb) * kTok + col), p);
-                                tmem_ld_wait();
-                                const float *dp = da + b * cx.n + col;
+                        for (int i = 0; i < 4; ++i) {
+                            if constexpr (F::kBlockScale) { const float d = rw[b * kRows + 8 * i]; dw[i] = pack2f(d, d); }
+                            if constexpr (F::kTerm) { const float m = rw[(8 + b) * kRows + 8 * i]; mw[i] = pack2f(m, m); }
+                        }
 #pragma unroll
-                                for (int i = 0; i < 8; i += 2) {
-                                    const float4 d4 = *reinterpret_cast<const float4 *>(dp + 2 * i);
-                                    float4 s4, t4;
-                                    if constexpr (kMins >= 1) s4 = *reinterpret_cast<const float4 *>(dp + 8 * cx.n + 2 * i);
-                                    if constexpr (kMins >= 2) t4 = *reinterpret_cast<const float4 *>(dp + 16 * cx.n + 2 * i);
+                        for (int j = 0; j < N8; ++j) {
+                            dd[j] = *reinterpret_cast<const uint64_t *>(da + b * n + 8 * j);
+                            if constexpr (F::kTerm) ss[j] = *reinterpret_cast<const uint64_t *>(da + (8 + b) * n + 8 * j);
+                        }
+                        tmem_ld_wait();
+                        if (bb == 1) {
+                            tc_fence_before();
+                            arrive_warp(&bar_free[slot], lane);
+                        }
 #pragma unroll
-                                    for (int e = 0; e < 2; ++e) {
-                                        const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
-                                        const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]);
-                                        // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel
-                                        uint64_t v;
-                                        if constexpr (F::kTerm) {       // the block's two large parts meet before they are added to others
-                                            v = mul2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y));
-                                            if constexpr (kMins >= 2) v = fma2(mm1, e ? pack2f(t4.z, t4.w) : pack2f(t4.x, t4.y), v);
-                                            v = fma2(one, fma2(mul2(dw, dd), pv, v), acc[g][i + e]);      // d_w d_a: two f16, exact
-                                        } else {
-                                            v = kComp ? fma2(dd, mul2(dw, pv), acc[g][i + e]) : fma2(mul2(dw, dd), pv, acc[g][i + e]);
-                                            if constexpr (kMins >= 1) v = fma2(mm0, e ? pack2f(s4.z, s4.w) : pack2f(s4.x, s4.y), v);
-                                        }
-                                        acc[g][i + e] = v;
-                                    }
-                                }
+                        for (int j = 0; j < N8; ++j) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                const int x = 2 * N8 * (i >> 1) + 2 * j + (i & 1);
+                                const uint64_t pv = pack2(p[2 * x], p[2 * x + 1]);
+                                // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel
+                                if constexpr (F::kTerm) acc[x] = fma2(one, fma2(mul2(dw[i], dd[j]), pv, mul2(mw[i], ss[j])), acc[x]);
+                                else acc[x] = fma2(F::kBlockScale ? mul2(dw[i], dd[j]) : dd[j], pv, acc[x]);
                             }
                         }
                     }
-                    tc_fence_before();
-                    arrive_warp(&bar_free[slot], lane);
                     if (++slot == kSlots) { slot = 0; ++round; }
                 }
-                if constexpr (kComp) {      // sum += acc with the rounding error kept in `low` (two-sum)
+                if constexpr (kComp) {
+                    // sum += the chunk, the rounding error of the addition into `low` (fast two-sum: exact unless the chunk is larger than
+                    // the sum before it, and then within one rounding of the chunk's own last bit)
+                    uint64_t dw[4];
 #pragma unroll
-                    for (int g = 0; g < kG; ++g)
+                    for (int i = 0; i < 4; ++i) { const float d = F::kBlockScale ? 1.0f : rw[8 * i]; dw[i] = pack2f(d, d); }
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const uint64_t x = acc[g][i], s0 = sum[g][i], s1 = fma2(one, x, s0), bb = fma2(minus1, s0, s1);
-                            const uint64_t e0 = fma2(minus1, fma2(minus1, bb, s1), s0), e1 = fma2(minus1, bb, x);
-                            low[g][i] = fma2(one, fma2(one, e0, e1), low[g][i]);
-                            sum[g][i] = s1;
-                            acc[g][i] = 0ull;
+                    for (int h = 0; h < 2; ++h) {
+                        [[maybe_unused]] uint32_t v[4 * N8];
+                        if constexpr (kSums > 0) {
+                            tmem_ld_16x256b<N8>(tq + (uint32_t)kColV + ((uint32_t)(16 * h) << 16), v);
+                            tmem_ld_wait();
                         }
-                }
-            }
-            if (!alive) break;
-            if (cx.row0 + r < a.nrows) {
 #pragma unroll
-                for (int g = 0; g < kG; ++g) {
-                    const int col = (2 * g + ch0) * 16, left = cx.valid - col;
-                    if (left <= 0) continue;
-                    if constexpr (kComp) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {       // an infinite (or NaN) sum has no error term
-                            const float s0 = lo2(sum[g][i]), s1 = hi2(sum[g][i]);
-                            acc[g][i] = pack2f(fabsf(s0) <= 3.0e38f ? __fadd_rn(s0, lo2(low[g][i])) : s0,
-                                               fabsf(s1) <= 3.0e38f ? __fadd_rn(s1, hi2(low[g][i])) : s1);
+                        for (int i = 0; i < 2 * N8; ++i) {
+                            const int x = 2 * N8 * h + i;
+                            const uint64_t s0 = sum[x];
+                            uint64_t f = dw[2 * h + (x & 1)], y = acc[x];            // the chunk is f y
+                            if constexpr (kSums > 0) { y = fma2(f, y, pack2(v[2 * i], v[2 * i + 1])); f = one; }
+                            const uint64_t s1 = fma2(f, y, s0);
+                            low[x] = fma2(one, fma2(f, y, fma2(minus1, s1, s0)), low[x]);
+                            sum[x] = s1;
+                            acc[x] = 0ull;
                         }
                     }
-                    const int64_t tok = (int64_t)cx.t * tl.tt + col;
-                    store16(acc[g], a.out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
+                    if constexpr (kSums > 0) {
+                        tc_fence_before();
+                        arrive_warp(bar_vfree, lane);
+                    }
                 }
             }
+#pragma unroll
+            for (int x = 0; x < kP; ++x) {
+                const int row = cx.row0 + r0 + 16 * (x / (2 * N8)) + 8 * (x & 1), j = (x >> 1) % N8, c0 = col0 + csub + 8 * j;
+                float v0 = lo2(acc[x]), v1 = hi2(acc[x]);
+                if constexpr (kComp) {          // an infinite (or NaN) sum has no error term
+                    const float s0 = lo2(sum[x]), s1 = hi2(sum[x]);
+                    v0 = fabsf(s0) <= 3.0e38f ? __fadd_rn(s0, lo2(low[x])) : s0;
+                    v1 = fabsf(s1) <= 3.0e38f ? __fadd_rn(s1, hi2(low[x])) : s1;
+                }
+                if (row < a.nrows && j < n8) {
+                    const int64_t at = ((int64_t)cx.t * tl.tt + c0) * a.stride_out + row;
+                    if (c0 < cx.valid) cq_store_out(a.out, a.out_kind, at, v0);
+                    if (c0 + 1 < cx.valid) cq_store_out(a.out, a.out_kind, at + a.stride_out, v1);
+                }
+            }
+            return true;
+        };
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            alive = cx.n > 32 ? run_tile(cx, std::integral_constant<int, 4>{}) : run_tile(cx, std::integral_constant<int, 2>{});
         }
     }
 
@@ -640,12 +780,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
 template <int WTYPE, typename T>
 void launch_quantize(const void *x, void *scratch, int k, const Tiling &tl, unsigned blocks, cudaStream_t st) {
     using F = Fmt<WTYPE>;
-    cq_launch_k(quantize_kernel<T, F::kQ81, F::kMins, F::kSum>, dim3(blocks), dim3(256), 0, st, (const T *)x, (uint8_t *)scratch, k, tl);
+    cq_launch_k(quantize_kernel<T, F::kQ81, F::kSum>, dim3(blocks), dim3(256), 0, st, (const T *)x, (uint8_t *)scratch, k, tl);
 }
 
 template <int WTYPE>
 bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, int k, int n, int tokens, int stride_dst, cudaStream_t st) {
-    using F = Fmt<WTYPE>;
     using R = Raw<chunk_bytes<WTYPE>()>;
     static_assert(Smem<WTYPE>::kBytes <= 232448, "shared memory of one CTA");
     static bool attr_done[64] = {};
@@ -656,7 +795,7 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
         attr_done[dev] = true;
     }
     const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
-    const Tiling tl = plan_tiling(tokens, nrt, sm_count(), kFixedTokens, F::kTok);
+    const Tiling tl = plan_tiling(tokens, nrt, sm_count(), kFixedTokens, kTok);
     const long long blocks = (long long)tl.ntt * (tl.tt / 8) * nch;
     if (blocks > INT32_MAX) { cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32: too many tokens for one launch"); return false; }
     const long long row_bytes = (long long)nch * chunk_bytes<WTYPE>();
@@ -676,29 +815,36 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
     return true;
 }
 
-int mins_of(int wtype) {
-    return (wtype == CQ_Q4_1 || wtype == CQ_Q5_0 || wtype == CQ_Q5_1 || wtype == CQ_Q5_K) ? 1 : wtype == CQ_Q2_K ? 2 : 0;
+int sum_of(int wtype) {
+    return wtype == CQ_Q4_1 || wtype == CQ_Q5_1 ? kTermSum : wtype == CQ_Q5_0 ? kDelta : wtype == CQ_Q5_K ? kSum32 : wtype == CQ_Q2_K ? kSum16 : kNoSum;
 }
 
 }  // namespace
 
 extern "C" size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k) {
     if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
-    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)(512 + 32 + 32 * mins_of(wtype)) + 256;
+    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)tok_bytes(sum_of(wtype)) + 256;
 }
 
-// The six Q8_1 formats against slices of eight rows on the decode kernel, which stream the matrix once each.  Both models are fits to 1500
-// shapes (9 - 220 tokens, 32 - 20000 rows, K to 14336; f32, cold weights; this kernel within 2 %, the slices within 6 - 13 % on average): a round
-// of tiles takes a fixed part and one per token and 256 elements of K; a slice its two launches, and time per weight that grows with
-// its rows.  Of those shapes 21 go to the slower side by more than 5 %, by 20 % at most where that is this kernel: a matrix of few rows and
-// long K leaves most SMs without a tile (5467 rows of K = 10240, 11 tokens: 124 us against 54), 4096 -> 14336 at 512 tokens 490 against 2233.
+// The six Q8_1 formats against slices of eight rows on the decode kernel, which stream the matrix once each.  Models of both sides (9 - 220 tokens,
+// 32 - 20000 rows, K to 14336; f32, cold weights): a round of tiles takes a fixed part and one per token and 256 elements of K, measured at 148
+// tiles; a slice its two launches, and time per weight that grows with its rows (a fit to 1500 shapes).  Of 245 sampled shapes 11 go to the slower side by
+// more than 5 %, most of them to the slices, for a matrix of few rows and long K (145 rows of K = 8448, 93 tokens: 77 us here, 107 in slices).
 extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     const double sms = cq_sm_count(), weights = 1e-6 * n * (double)k;
     const Tiling tl = plan_tiling(tokens, (n + kRows - 1) / kRows, (int)sms, kFixedTokens, 64);
     const double rounds = std::ceil((double)((n + kRows - 1) / kRows) * tl.ntt / sms);
     const bool super = cq_block_elems(wtype) == 256;
-    const double fixed = wtype == CQ_Q2_K ? 2.52 : wtype == CQ_Q3_K ? 2.09 : 2.27, per_token = wtype == CQ_Q2_K ? 0.046 : 0.036;
-    const double here = 6.7 + rounds * (k / 256) * (fixed + per_token * tl.tt);
+    double fixed = 2.16, per_token = 0.0104;        // Q5_K
+    switch (wtype) {
+    case CQ_Q4_1: fixed = 2.1; per_token = 0.0215; break;
+    case CQ_Q5_0: fixed = 2.58; per_token = 0.0081; break;
+    case CQ_Q5_1: fixed = 2.41; per_token = 0.019; break;
+    case CQ_Q2_K: fixed = 2.46; per_token = 0.008; break;
+    case CQ_Q3_K: fixed = 2.64; per_token = 0.005; break;
+    }
+    const double idle = (double)((n + kRows - 1) / kRows) * tl.ntt < 0.6 * sms ? 0.85 : 1.0;      // fewer tiles share the L2
+    const double here = 8.5 + rounds * (k / 256) * (fixed + per_token * tl.tt) * idle;
     auto slice = [&](int rows) {
         return super ? 5.25 + 0.125e-3 * k + weights * (0.05 + 0.084 * rows) : std::max(5.05, 4.7 + 0.018e-3 * k + weights * (0.21 + 0.02 * rows));
     };

@@ -76,6 +76,21 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
           "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+// 8 N columns of 16 lanes: value 4 j + 2 s + e of a thread is lane 8 s + lane / 4, column 8 j + 2 (lane % 4) + e.
+template <int N> __device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr, uint32_t *v) {
+    static_assert(N == 2 || N == 4, "");
+    if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                       "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]) : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Bounded wait like wait_or_abort, with a hint that lets the hardware suspend the thread until the phase completes (at most about
@@ -97,7 +112,7 @@ __device__ __forceinline__ bool wait_slow(uint64_t *bar, unsigned parity, volati
 // There is no per-lane form: every role goes on to warp-wide instructions, so its warp decides as one whether a wait gave up (lanes
 // that left at different places would meet at different warp-wide instructions, which need not end).
 __device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, try_wait_suspended(bar, parity) || wait_slow(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, cq_mbar_try_wait(bar, parity) || wait_slow(bar, parity, abort_flag));
 }
 // One arrival per warp: barriers count warps, not threads.
 __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {

@@ -154,6 +154,36 @@ def test_prompt32_matmul(lib, oracle, cuda_dev, tokens, k, n, wtype):
         assert rel_err(out.cpu().numpy()[pick], ref) <= 2e-6
 
 
+# tokens per tile at the border of the two sizes of the epilogue (32 | 33), and the multiples of 16 around it
+@pytest.mark.parametrize("tokens", [16, 31, 33, 48])
+@pytest.mark.parametrize("wtype", sorted(NAMES))
+def test_prompt32_tile_sizes_give_the_same_bits(lib, oracle, cuda_dev, tokens, wtype):
+    """A token's result does not depend on the size of the tile it is in."""
+    _, x, wq = make_case(oracle, wtype, 1280, 200, 64, seed=wtype)
+    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
+    assert torch.equal(_prompt32(lib, wtype, w_dev, x_dev[:tokens].contiguous(), 1280, 200), _prompt32(lib, wtype, w_dev, x_dev, 1280, 200)[:tokens])
+
+
+@pytest.mark.parametrize("wtype", [3, 6, 7])
+def test_prompt32_of_block_sums_past_f16(lib, oracle, cuda_dev, wtype):
+    """Q8_1's stored sum is infinite where 32 inputs add up to more than 65504: infinities and NaNs where the decode kernel has them."""
+    k, n, m = 512, 96, 16
+    _, x, wq = make_case(oracle, wtype, k, n, m, seed=1)
+    x[3, 64:96], x[5, 32:64], x[5, 300:330], x[7, 480:] = 3000.0, -2500.0, 4000.0, np.nan
+    x_dev, w_dev, st = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev), torch.cuda.current_stream().cuda_stream
+    y8, decode, out = torch.zeros((m, k // 32, 36), dtype=torch.uint8, device=cuda_dev), torch.empty((m, n), device=cuda_dev), torch.empty((m, n), device=cuda_dev)
+    lib.cq_quantize_act(x_dev.data_ptr(), capi.F32, y8.data_ptr(), k, k, m, 0, st)
+    for r in range(0, m, 8):
+        lib.cq_mmvq(wtype, 0, capi.F32, w_dev.data_ptr(), y8[r:].data_ptr(), decode[r:].data_ptr(), k, n, k // 32, n, 8, st)
+    scratch = torch.zeros(lib.cq_prompt32_scratch_bytes(wtype, m, k), dtype=torch.uint8, device=cuda_dev)
+    lib.cq_prompt32_matmul(wtype, w_dev.data_ptr(), x_dev.data_ptr(), capi.F32, out.data_ptr(), scratch.data_ptr(), k, n, m, n, st)
+    capi.check("prompt32")
+    assert torch.equal(torch.isnan(out), torch.isnan(decode)) and torch.equal(torch.isinf(out), torch.isinf(decode))
+    assert torch.equal(out[torch.isinf(out)], decode[torch.isinf(decode)]) and not bool(torch.isfinite(out[[3, 5, 7]]).all())
+    ok = [i for i in range(m) if i not in (3, 5, 7)]
+    assert rel_err(out[ok].cpu().numpy(), decode[ok].cpu().numpy()) <= 2e-6
+
+
 @pytest.mark.parametrize("wtype", [7, 8, 10, 11, 13])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_prompt32_half_types(lib, oracle, cuda_dev, wtype, dtype):
