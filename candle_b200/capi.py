@@ -118,6 +118,8 @@ def lib() -> C.CDLL:
         L.cq_moe_router_f32.restype = None
         L.cq_moe_weighted_sum_f32.argtypes = [vp, vp, vp, i32, i32, i32, vp]
         L.cq_moe_weighted_sum_f32.restype = None
+        L.cq_argmax_f32.argtypes = [vp, i32, i32, C.c_int64, vp, vp, vp]
+        L.cq_argmax_f32.restype = None
         L.cq_qknorm_rope_store_kv_f32.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32,
                                                   C.c_float, i32, vp]
         L.cq_attention_split_scratch_floats.argtypes = [i32, i32, i32, i32]

@@ -350,6 +350,58 @@ bool norm_args_ok(const void *x, const void *w, const void *out, int rows, int d
     return true;
 }
 
+// First maximum of each row: (value, index + start) as two floats and / or the index + start as a token.  One cluster of kArgmaxCtas CTAs per row:
+// a row of a vocabulary is 0.5 MB, 20 us for a single CTA and 1 us of loads for eight; the CTAs' results meet in the first one's shared memory.
+// As tensor operations (max, compare, index, min, and the same again over the ranks' pairs) a step's choice of one token of 128256 took 75 us.
+// A row with a NaN has no element equal to its maximum: the value is NaN and the index 2^40 / the token the largest int64, as those operations give.
+constexpr int kArgmaxCtas = 8;
+__global__ void __launch_bounds__(1024) argmax_kernel(const float *__restrict__ x, int n, long long start, float *__restrict__ pairs,
+                                                      long long *__restrict__ tokens) {
+    __shared__ float val[32], all_val[kArgmaxCtas];
+    __shared__ int idx[32], all_idx[kArgmaxCtas];
+    const int rank = (int)blockIdx.x % kArgmaxCtas, row = (int)blockIdx.x / kArgmaxCtas, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    cq_pdl_launch_dependents();
+    cq_pdl_wait();
+    const float *xr = x + (size_t)row * n;
+    float v = -INFINITY;
+    int at = INT32_MAX, nan = 0;
+    auto take = [&](float u, int i) {       // ascending i within a thread; a NaN is remembered
+        nan |= u != u;
+        if (u > v || (u == v && i < at)) { v = u; at = i; }
+    };
+#pragma unroll 4
+    for (int i = rank * 1024 + tid; i < n; i += kArgmaxCtas * 1024) take(xr[i], i);
+    auto warp_best = [&] {
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) take(__shfl_xor_sync(0xffffffffu, v, m), __shfl_xor_sync(0xffffffffu, at, m));
+    };
+    warp_best();
+    nan = __syncthreads_or(nan);
+    if (lane == 0) { val[warp] = v; idx[warp] = at; }
+    __syncthreads();
+    if (warp == 0) {
+        v = val[lane]; at = idx[lane];
+        warp_best();
+        if (lane == 0) {                    // the CTA's result to the first CTA of the cluster
+            uint32_t a, b;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(cq_smem_u32(&all_val[rank])));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(b) : "r"(cq_smem_u32(&all_idx[rank])));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(nan ? NAN : v) : "memory");
+            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(b), "r"(at) : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank != 0 || tid != 0) return;
+    v = all_val[0]; at = all_idx[0];
+    nan = v != v;
+    for (int r = 1; r < kArgmaxCtas; ++r) take(all_val[r], all_idx[r]);
+    if (pairs) {
+        pairs[2 * row] = nan ? NAN : v;
+        pairs[2 * row + 1] = nan ? (float)((1LL << 40) + start) : (float)(at + start);
+    }
+    if (tokens) tokens[row] = nan ? INT64_MAX : (long long)(float)(at + start);
+}
+
 }  // namespace
 
 extern "C" void cq_rms_norm_f32(const float *x, const float *w, float *out, int rows, int d, float eps, void *stream) {
@@ -487,4 +539,14 @@ extern "C" void cq_qknorm_rope_store_kv_f32(float *q, float *k, const float *v, 
     cq_launch_k(qknorm_rope_store_kernel, dim3((unsigned)((units + 3) / 4)), dim3(128), 0, (cudaStream_t)stream, q, k, v, q_norm_w,
                 k_norm_w, cosv, sinv, pos, k_cache, v_cache, batch, t, hq, hkv, tmax, q_stride, k_stride, v_stride, eps, neox);
     cq_check_launch("qknorm_rope");
+}
+
+extern "C" void cq_argmax_f32(const float *x, int rows, int n, int64_t start, float *pairs, int64_t *tokens, void *stream) {
+    if (!x || (!pairs && !tokens) || rows <= 0 || rows > 65535 || n <= 0 || start < 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "argmax: null pointer or empty row");
+        return;
+    }
+    cq_launch_cluster_k(argmax_kernel, dim3((unsigned)(rows * kArgmaxCtas)), dim3(1024), 0, (cudaStream_t)stream, kArgmaxCtas, x, n, (long long)start, pairs,
+                        (long long *)tokens);
+    cq_check_launch("argmax");
 }

@@ -18,6 +18,8 @@ import sys
 import torch
 import torch.distributed as dist
 
+from . import capi
+
 
 def shard_rows(n: int, world: int, rank: int, unit: int = 1) -> tuple[int, int]:
     """Contiguous row range [start, start + count) of rank `rank`; `unit` rows stay together (e.g. one head)."""
@@ -294,11 +296,26 @@ def make_gatherer(group=None, world: int | None = None, device=None) -> Gatherer
 def argmax_sharded(local_logits: torch.Tensor, vocab_start: int, gather: Gatherer) -> torch.Tensor:
     """Greedy token over a vocabulary sharded by rows: gather (max, global index) pairs and break ties towards the
     lowest global index, which is what argmax over the whole row returns."""
+    if local_logits.is_cuda and local_logits.dtype == torch.float32 and local_logits.dim() == 2 and local_logits.is_contiguous() and \
+            0 < local_logits.shape[0] <= 65535 and local_logits.shape[1] > 0:
+        rows, n = local_logits.shape
+        st = torch.cuda.current_stream(local_logits.device).cuda_stream
+        one = gather.world == 1         # then the pair is the result
+        out = torch.empty(rows, dtype=torch.int64, device=local_logits.device) if one else \
+            torch.empty((rows, 2), dtype=torch.float32, device=local_logits.device)
+        with torch.cuda.device(local_logits.device):
+            capi.lib().cq_argmax_f32(local_logits.data_ptr(), rows, n, vocab_start, None if one else out.data_ptr(), out.data_ptr() if one else None, st)
+        capi.check("argmax")
+        return out if one else _best_pair(gather(out))
     mx = local_logits.max(dim=-1).values
     ar = torch.arange(local_logits.shape[-1], device=local_logits.device)
     idx = torch.where(local_logits == mx.unsqueeze(-1), ar, ar.new_full((), 1 << 40)).min(dim=-1).values   # first maximum
     pair = torch.stack([mx, (idx + vocab_start).to(mx.dtype)], dim=-1)      # indices < 2^24 are exact in f32
-    allp = gather(pair)                                                      # [rows, 2 * world]
+    return _best_pair(gather(pair))
+
+
+def _best_pair(allp: torch.Tensor) -> torch.Tensor:
+    """Token of the best (value, global index) pair of each row of [rows, 2 * world]."""
     allp = allp.view(allp.shape[0], -1, 2)
     best = allp[..., 0].max(dim=-1, keepdim=True).values
     cand = torch.where(allp[..., 0] == best, allp[..., 1], torch.full_like(allp[..., 1], float("inf")))

@@ -378,6 +378,10 @@ void cq_moe_route_f32(const float *logits, int32_t *ids, float *weights, int tok
 void cq_moe_router_f32(const float *h, const float *router, float *logits, int32_t *ids, float *weights, int *counters, int tokens,
                        int experts, int d, int k, int norm_topk_prob, void *stream);
 void cq_moe_weighted_sum_f32(const float *y, const float *w, float *out, int tokens, int k, int d, void *stream);
+
+/* First maximum of each of `rows` rows of n floats: pairs[r] = (value, index + start) as floats, tokens[r] = index + start (either may be null).  A
+ * row with a NaN gives (NaN, 2^40 + start) and INT64_MAX. */
+void cq_argmax_f32(const float *x, int rows, int n, int64_t start, float *pairs, int64_t *tokens, void *stream);
 void cq_qknorm_rope_store_kv_f32(float *q, float *k, const float *v, const float *q_norm_w, const float *k_norm_w, const float *cosv,
                                  const float *sinv, const int *pos, float *k_cache, float *v_cache, int batch, int t, int hq, int hkv,
                                  int head_dim, int tmax, int q_stride, int k_stride, int v_stride, float eps, int neox, void *stream);

@@ -311,6 +311,23 @@ def test_decode_tokens_do_not_depend_on_fusion_or_dependent_launch(lib, cuda_dev
         lib.cq_set_pdl(1)
 
 
+@pytest.mark.parametrize("rows,n", [(1, 1), (1, 128256), (3, 8193), (2, 50), (65, 1024)])
+def test_argmax_is_the_first_maximum(lib, cuda_dev, rows, n):
+    gen = torch.Generator(device=cuda_dev).manual_seed(n)
+    x = torch.randint(-3, 4, (rows, n), device=cuda_dev, generator=gen).float()       # many equal maxima
+    x[0] = -float("inf")
+    if rows > 2:
+        x[1, n // 2], x[2] = float("nan"), torch.randn(n, device=cuda_dev, generator=gen)
+    pairs, tokens = torch.empty((rows, 2), device=cuda_dev), torch.empty(rows, dtype=torch.int64, device=cuda_dev)
+    lib.cq_argmax_f32(x.data_ptr(), rows, n, 1000, pairs.data_ptr(), tokens.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    capi.check("argmax")
+    mx = x.max(dim=-1).values
+    first = torch.where(x == mx.unsqueeze(-1), torch.arange(n, device=cuda_dev), 1 << 40).min(dim=-1).values + 1000
+    assert torch.equal(pairs.nan_to_num(7e30), torch.stack([mx, first.float()], dim=-1).nan_to_num(7e30))
+    ok = ~torch.isnan(mx)
+    assert torch.equal(tokens[ok], first[ok]) and bool((tokens[~ok] == 2 ** 63 - 1).all())
+
+
 def test_graph_decode_equals_eager_decode(cuda_dev):
     cfg = DecoderConfig.tiny()
     prompt = torch.randint(0, cfg.vocab, (2, 24), device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(2))
