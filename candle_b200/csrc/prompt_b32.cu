@@ -32,7 +32,7 @@
 // minimum sums where there are any, operand A in two or three buffers of two blocks.  The roles hand over two blocks at a time; where operand
 // A and the accumulators have as many buffers, one commit tells both the producers and the epilogue.  Every wait is bounded as there.
 //
-// Measured (B200, quantizer included; before -> now): Q5_K 4096 -> 14336, 512 tokens 493 us -> 263, Q8_0 4096 -> 4096, 333 tokens 88 -> 76.  A chunk of
+// Measured (B200, quantizer included; before -> now): Q5_K 4096 -> 14336, 512 tokens 493 us -> 243, Q8_0 4096 -> 4096, 333 tokens 88 -> 69.  A chunk of
 // 256 elements takes 2.1 us and 11 ns per token, 11 - 13 thousand warp instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
 // Tried: tiles of 128 tokens with one producer set (Q5_K 327), the group's first warp polling for the others (534: branches and barrier reads outweigh
 // the polls), a branch on the tile's tokens inside the block loop (312: the compiler then moves every running sum).
@@ -430,7 +430,8 @@ struct Args {
     int out_kind, nrows, nch, stride_out, use_map, ntiles;
 };
 
-template <int WTYPE>
+// STORE: see prompt_f16.cuh; N8: tiles of up to 16 N8 tokens, 2 or 4
+template <int WTYPE, int STORE, int N8>
 __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
     using F = Fmt<WTYPE>;
     using S = Smem<WTYPE>;
@@ -658,11 +659,13 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         const uint64_t minus1 = pack2f(-1.0f, -1.0f), one = pack2f(1.0f, 1.0f);
         int it = 0, slot = 0, round = 0;
         bool alive = true;
-        // A tile whose warps have up to N8 units of eight columns; those past the tile's tokens are computed and dropped.  (The two sizes are separate
-        // loops: a branch on the size inside, over running sums, made the compiler move every sum, a quarter of the epilogue's instructions.)
-        auto run_tile = [&](const TileCtx &cx, auto units) {
-            constexpr int N8 = decltype(units)::value, kP = 4 * N8;
-            const int n = cx.n, col0 = half * (n >> 1), n8 = n >> 4;
+        // Every warp works on N8 units of eight columns; those past the tile's tokens are computed and dropped.  (A branch on the size inside the loop, over
+        // running sums, made the compiler move every sum, a quarter of the epilogue's instructions.)
+        constexpr int kP = 4 * N8;
+        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            tile_ctx(tile, tl.ntt, tl, gi, cx);
+            const int n = cx.n, col0 = half * (n >> 1);
             const uint32_t tq = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
             uint64_t acc[kP];                                                 // running sums (or those of this chunk)
             [[maybe_unused]] uint64_t sum[kComp ? kP : 1], low[kComp ? kP : 1];       // compensated sum of the chunks
@@ -671,13 +674,13 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 acc[i] = 0ull;
                 if constexpr (kComp) { sum[i] = 0ull; low[i] = 0ull; }
             }
-            for (int c = 0; c < nch; ++c, ++it) {
+            for (int c = 0; c < nch && alive; ++c, ++it) {
                 const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux) + col0 + csub;
                 const float *rw = reinterpret_cast<const float *>(ringW + (it & 3) * S::kRingW) + r0;
-                if (!wait_warp(&bar_vis[it & 1], (it >> 1) & 1, abort_flag)) return false;
+                if (!wait_warp(&bar_vis[it & 1], (it >> 1) & 1, abort_flag)) { alive = false; break; }
 #pragma unroll 1
                 for (int ch = 0; ch < 4; ++ch) {
-                    if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) return false;
+                    if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int bb = 0; bb < 2; ++bb) {
@@ -716,6 +719,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     }
                     if (++slot == kSlots) { slot = 0; ++round; }
                 }
+                if (!alive) break;
                 if constexpr (kComp) {
                     // sum += the chunk, the rounding error of the addition into `low` (fast two-sum: exact unless the chunk is larger than
                     // the sum before it, and then within one rounding of the chunk's own last bit)
@@ -747,27 +751,34 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     }
                 }
             }
+            if (!alive) break;
+            if constexpr (kComp) {
 #pragma unroll
-            for (int x = 0; x < kP; ++x) {
-                const int row = cx.row0 + r0 + 16 * (x / (2 * N8)) + 8 * (x & 1), j = (x >> 1) % N8, c0 = col0 + csub + 8 * j;
-                float v0 = lo2(acc[x]), v1 = hi2(acc[x]);
-                if constexpr (kComp) {          // an infinite (or NaN) sum has no error term
+                for (int x = 0; x < kP; ++x) {          // an infinite (or NaN) sum has no error term
                     const float s0 = lo2(sum[x]), s1 = hi2(sum[x]);
-                    v0 = fabsf(s0) <= 3.0e38f ? __fadd_rn(s0, lo2(low[x])) : s0;
-                    v1 = fabsf(s1) <= 3.0e38f ? __fadd_rn(s1, hi2(low[x])) : s1;
-                }
-                if (row < a.nrows && j < n8) {
-                    const int64_t at = ((int64_t)cx.t * tl.tt + c0) * a.stride_out + row;
-                    if (c0 < cx.valid) cq_store_out(a.out, a.out_kind, at, v0);
-                    if (c0 + 1 < cx.valid) cq_store_out(a.out, a.out_kind, at + a.stride_out, v1);
+                    acc[x] = pack2f(fabsf(s0) <= 3.0e38f ? __fadd_rn(s0, lo2(low[x])) : s0, fabsf(s1) <= 3.0e38f ? __fadd_rn(s1, hi2(low[x])) : s1);
                 }
             }
-            return true;
-        };
-        for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
-            TileCtx cx;
-            tile_ctx(tile, tl.ntt, tl, gi, cx);
-            alive = cx.n > 32 ? run_tile(cx, std::integral_constant<int, 4>{}) : run_tile(cx, std::integral_constant<int, 2>{});
+            const int left = min(n >> 1, cx.valid - col0);          // columns of this warp that hold tokens
+            const int64_t base = ((int64_t)cx.t * tl.tt + col0) * a.stride_out + cx.row0;
+#pragma unroll
+            for (int j = 0; j < N8; ++j) {
+                const uint64_t v[4] = {acc[2 * j], acc[2 * j + 1], acc[2 * N8 + 2 * j], acc[2 * N8 + 2 * j + 1]};       // rows r0 + 8 i
+                if constexpr (STORE == kStore16) {
+                    const int col = 8 * j + (lane >> 2), row = (warp & 3) * 32;
+                    store_rows32_16bit(v, a.out_kind, (uint16_t *)a.out + base + (int64_t)col * a.stride_out + row, col < left ? a.nrows - cx.row0 - row : 0,
+                                       ((a.stride_out & 7) | ((uintptr_t)a.out & 15)) == 0);
+                } else {
+                    const int col = 8 * j + csub;
+                    float *o = (float *)a.out + base + (int64_t)col * a.stride_out + r0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool in = cx.row0 + r0 + 8 * i < a.nrows;
+                        if (in && col < left) o[8 * i] = lo2(v[i]);
+                        if (in && col + 1 < left) o[8 * i + a.stride_out] = hi2(v[i]);
+                    }
+                }
+            }
         }
     }
 
@@ -783,17 +794,21 @@ void launch_quantize(const void *x, void *scratch, int k, const Tiling &tl, unsi
     cq_launch_k(quantize_kernel<T, F::kQ81, F::kSum>, dim3(blocks), dim3(256), 0, st, (const T *)x, (uint8_t *)scratch, k, tl);
 }
 
-template <int WTYPE>
-bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, int k, int n, int tokens, int stride_dst, cudaStream_t st) {
-    using R = Raw<chunk_bytes<WTYPE>()>;
+template <int WTYPE, int STORE, int N8> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const Args &a, const Tiling &tl) {
     static_assert(Smem<WTYPE>::kBytes <= 232448, "shared memory of one CTA");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-        cudaFuncSetAttribute(prompt32_kernel<WTYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<WTYPE>::kBytes);
+        cudaFuncSetAttribute(prompt32_kernel<WTYPE, STORE, N8>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<WTYPE>::kBytes);
         attr_done[dev] = true;
     }
+    cq_launch_k(prompt32_kernel<WTYPE, STORE, N8>, dim3(grid), dim3(kThreads), Smem<WTYPE>::kBytes, st, map, a, tl);
+}
+
+template <int WTYPE>
+bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, int k, int n, int tokens, int stride_dst, cudaStream_t st) {
+    using R = Raw<chunk_bytes<WTYPE>()>;
     const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
     const Tiling tl = plan_tiling(tokens, nrt, sm_count(), kFixedTokens, kTok);
     const long long blocks = (long long)tl.ntt * (tl.tt / 8) * nch;
@@ -811,7 +826,13 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
     else launch_quantize<WTYPE, __nv_bfloat16>(x, scratch, k, tl, (unsigned)blocks, st);
     const Args a{(const uint8_t *)w, (const uint8_t *)scratch, dst, elem, n, nch, stride_dst, use_map ? 1 : 0, nrt * tl.ntt};
     const int grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
-    cq_launch_k(prompt32_kernel<WTYPE>, dim3(grid), dim3(kThreads), Smem<WTYPE>::kBytes, st, map, a, tl);
+    if (elem == CQ_F32) {
+        if (tl.tt <= 32) launch_kernel<WTYPE, kStoreF32, 2>(grid, st, map, a, tl);
+        else launch_kernel<WTYPE, kStoreF32, 4>(grid, st, map, a, tl);
+    } else {
+        if (tl.tt <= 32) launch_kernel<WTYPE, kStore16, 2>(grid, st, map, a, tl);
+        else launch_kernel<WTYPE, kStore16, 4>(grid, st, map, a, tl);
+    }
     return true;
 }
 

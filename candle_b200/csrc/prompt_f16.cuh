@@ -186,17 +186,44 @@ __device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
     return make_uint4(pr(q[0], q[2]), pr(q[1], q[3]), pr(q[4], q[6]), pr(q[5], q[7]));
 }
 
-// 16 consecutive tokens' values of one weight row; `row(i)` gives the output row, values past `valid` are not stored
-template <typename F> __device__ __forceinline__ void store16(const uint64_t (&v)[8], void *out, int kind, int64_t stride, int col, int valid, F &&row) {
-    auto each = [&](auto put) {
+// Eight tokens x 32 weight rows of a warp as a 16-bit kind: v[i] are a thread's values of row 8 i + lane / 4, tokens 2 (lane % 4) and the next (the 16x256b
+// layout).  8 x 8 transposes leave a thread with rows 8 i + 2 (lane % 4), + 1 of token lane / 4, a 4 x 4 transpose over four lanes with eight rows of it, so a
+// token's 32 rows go out as 64 contiguous bytes.  (Stored as they lie, in 16-byte pieces of half a sector, the 2048 x 14336 outputs of a bf16 prompt took
+// 25 us more than twice the bytes as f32.)  `dst`: row 0 of this thread's token; `rows`: how many of the 32 are stored, 0 for a token that is none; `wide`: dst is
+// 16-byte aligned.
+__device__ __forceinline__ void store_rows32_16bit(const uint64_t (&v)[4], int kind, uint16_t *dst, int rows, bool wide) {
+    const int lane = threadIdx.x & 31;
+    uint32_t r[4];
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (i < valid) put(row(i) * stride + col, (i & 1) ? hi2(v[i >> 1]) : lo2(v[i >> 1]));
-    };
-    if (kind == CQ_F32) each([&](int64_t o, float x) { ((float *)out)[o] = x; });
-    else if (kind == CQ_F16) each([&](int64_t o, float x) { ((__half *)out)[o] = __float2half(x); });
-    else each([&](int64_t o, float x) { ((__nv_bfloat16 *)out)[o] = __float2bfloat16(x); });
+    for (int i = 0; i < 4; ++i) {
+        uint32_t w;
+        if (kind == CQ_F16) w = h2_bits(__halves2half2(__float2half(lo2(v[i])), __float2half(hi2(v[i]))));
+        else { const __nv_bfloat162 b = __halves2bfloat162(__float2bfloat16(lo2(v[i])), __float2bfloat16(hi2(v[i]))); w = *reinterpret_cast<const uint32_t *>(&b); }
+        asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r[i]) : "r"(w));
+    }
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {           // swap bit log2 m of the register number with that of the lane
+        const bool up = lane & m;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (!(i & m)) {
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[i] : r[i | m], m);
+                if (up) r[i] = got; else r[i | m] = got;
+            }
+    }
+    dst += 8 * (lane & 3);
+    rows -= 8 * (lane & 3);
+    if (wide && rows >= 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(r[0], r[1], r[2], r[3]);
+    else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < rows) dst[i] = (uint16_t)(r[i >> 1] >> (16 * (i & 1)));
+    }
 }
+
+// What a kernel stores, one instantiation each (the code of the others between the loops of a tile costs them 5 - 10 % in instruction fetches):
+// f32 or 16-bit rows of tokens, or f32 rows of (token, expert) pairs.
+enum { kStoreF32, kStore16, kStorePairs };
 
 // ---- tiles --------------------------------------------------------------------------------------------------
 // The jobs of a grouped (expert-indexed) launch; null `tiles` = dense.

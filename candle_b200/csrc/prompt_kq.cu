@@ -33,6 +33,12 @@
 // and 157 (Q6_K): twice the MMAs to issue.  Bound by the hand-offs between the roles: a super-block of 128 tokens takes 1.4 us (Q4_K) and
 // 2.4 us (Q6_K) where its MMAs take 0.55 and 1.05.
 //
+// The epilogue reads the accumulators in the 16x256b shape (four rows x two columns of each eight per thread), 32 columns at a time: an 8-byte shared load of
+// token scales serves eight values, where a row per thread took a 16-byte load, 4.8 clocks of the SM's shared-memory pipe, for four.  A grouped
+// launch fetches a tile's pair numbers and routing weights, a dependent chain of two L2 round trips, while its super-blocks run.  With one instantiation
+// per kind of output, since the code between the loops costs instruction fetches: expert block of 1024 tokens (below) 457 us -> 340, Q8_0 of prompt_b32.cu
+// 77 -> 69; Q4_K 2048 tokens bf16 313 -> 311 (the clocks fall with the power), 512 tokens f32 99 -> 97.
+//
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
 #include "../../include/candle_q_b200.h"
@@ -325,7 +331,8 @@ struct Args {
     int out_kind, nrows, nsb, stride_out, use_map, nrt;
 };
 
-template <int WTYPE>
+// STORE: see prompt_f16.cuh; Q: tiles of up to 64 Q tokens, 0: of any size (grouped launches, where each tile has its own)
+template <int WTYPE, int STORE, int Q>
 __global__ void __launch_bounds__(kThreads, 1)
 prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2, const Args a, const Tiling tl, const GroupInfo gi) {
     using F = Fmt<WTYPE>;
@@ -571,8 +578,8 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
                     if (before >= 0 && !wait_warp(&bar_done[before % F::kNT], (before / F::kNT) & 1, abort_flag)) { alive = false; break; }
                     tc_fence_after();
                     const uint32_t dst = ta + (uint32_t)((h % F::kNA) * 64);
-                    tmem_st32(dst, o[0]);
-                    tmem_st32(dst + 32, o[1]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) tmem_st8(dst + 8 * i, &o[i >> 2][8 * (i & 3)]);
                     tmem_st_wait();
                     tc_fence_before();
                     arrive_warp(&bar_full[h % F::kNT], lane);
@@ -582,96 +589,130 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         }
     } else {
         regs_up<kRegsEpi>();
-        // ===== epilogue: lane = weight row 32 (warp % 4) + lane; 16-token column groups warp / 4, warp / 4 + 2, ... =====
-        const int quad = warp & 3, ch0 = warp >> 2;
-        const int r = quad * 32 + lane;
-        const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        // ===== epilogue: warp = 32 weight rows 32 (warp % 4) .., half of the tile's tokens =====
+        // A thread holds rows r0 + 8 i, columns 8 j + csub, + 1 of each 32 of its half: pair 8 (i / 2) + 2 j + i % 2 (prompt_f16.cuh, 16x256b).
+        const int half = warp >> 2, r0 = (warp & 3) * 32 + (lane >> 2), csub = 2 * (lane & 3);
+        const uint32_t tlane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         [[maybe_unused]] const uint64_t one = pack2f(1.0f, 1.0f);
         int it = 0;
         bool alive = true;
-        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
-            TileCtx cx;
-            const bool second = tile >= per_matrix;
-            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
-            uint64_t acc[4][8];
+        // A tile whose warps have up to 32 kQ columns; those past its tokens are computed and dropped (a branch on the number of tokens inside, over
+        // running sums, makes the compiler move them).
+        auto run_tile = [&](const TileCtx &cx, bool second, auto quarters) {
+            constexpr int kQ = decltype(quarters)::value;
+            const int n = cx.n, col0 = half * (n >> 1);
+            const uint32_t tcol = tlane + (uint32_t)col0;
+            uint64_t acc[kQ][16];
 #pragma unroll
-            for (int g = 0; g < 4; ++g)
+            for (int q = 0; q < kQ; ++q)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[g][i] = 0ull;
+                for (int i = 0; i < 16; ++i) acc[q][i] = 0ull;
+            // grouped: the pairs of this warp's columns, a lane per column of each 32; their loads have the whole tile to arrive
+            int pair[kQ];
+            float pw[kQ];
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) {
+                pair[q] = 0;
+                pw[q] = 1.0f;
+                if (STORE == kStorePairs && col0 + 32 * q + lane < cx.valid) pair[q] = gi.sorted_token_ids[cx.job0 + col0 + 32 * q + lane];
+            }
             for (int sb = 0; sb < nsb; ++sb, ++it) {
                 const int c = it & 1;
                 // the last stage of the super-block is done; its barrier cannot come round again before this epilogue is through
                 const int h = it * F::kSps + F::kSps - 1;
-                if (!wait_warp(&bar_vis[c], (it >> 1) & 1, abort_flag) ||
-                    !wait_warp(&bar_done[h % F::kNT], (h / F::kNT) & 1, abort_flag)) { alive = false; break; }
+                if (!wait_warp(&bar_vis[c], (it >> 1) & 1, abort_flag) || !wait_warp(&bar_done[h % F::kNT], (h / F::kNT) & 1, abort_flag)) return false;
                 tc_fence_after();
-                const float2 ws = *reinterpret_cast<const float2 *>(ringW + (it & 3) * kRows * 8 + r * 8);
-                const uint64_t dw = pack2f(ws.x, ws.x), ndm = pack2f(-ws.y, -ws.y);
-                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * kAux + cx.n * 32);
-                const uint32_t tp = tlane + (uint32_t)(F::kMins ? c * kTokMax : 0);
+                const float2 *rw = reinterpret_cast<const float2 *>(ringW + (it & 3) * kRows * 8) + r0;
+                const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * kAux + n * 32) + col0 + csub;
+                const uint32_t tp = tcol + (uint32_t)(F::kMins ? c * kTokMax : 0);
                 if (F::kMins && split_of[c]) {      // rare: P0 + P1 into the place of P
 #pragma unroll 1
-                    for (int col = ch0 * 16; col < cx.n; col += 32) {
-                        uint32_t p[16], p1[16];
-                        tmem_ld16(tp + (uint32_t)col, p);
-                        tmem_ld16(tlane + (uint32_t)((c ^ 1) * kTokMax + col), p1);
+                    for (int col = 0; col < n >> 1; col += 8) {
+                        uint32_t p[8], p1[8];
+                        tmem_ld8(tp + (uint32_t)col, p);
+                        tmem_ld8(tcol + (uint32_t)((c ^ 1) * kTokMax + col), p1);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) p[i] = __float_as_uint(__fadd_rn(__uint_as_float(p[i]), __uint_as_float(p1[i])));
-                        tmem_st16(tp + (uint32_t)col, p);
+                        for (int i = 0; i < 8; ++i) p[i] = __float_as_uint(__fadd_rn(__uint_as_float(p[i]), __uint_as_float(p1[i])));
+                        tmem_st8(tp + (uint32_t)col, p);
                     }
                     tmem_st_wait();
                 }
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    const int col = (2 * g + ch0) * 16;
-                    if (col < cx.n) {           // warp-uniform
+                for (int q = 0; q < kQ; ++q) {
+                    uint64_t dd[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) dd[j] = *reinterpret_cast<const uint64_t *>(da + 32 * q + 8 * j);
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
                         uint32_t p[16], l[16];      // l: L, or the sum of the second plane
-                        tmem_ld16(tp + (uint32_t)col, p);
-                        tmem_ld16(tlane + (uint32_t)((F::kMins ? kColL : kTokMax) + col), l);
+                        tmem_ld_16x256b<4>(tp + (uint32_t)(32 * q) + ((uint32_t)(16 * hf) << 16), p);
+                        tmem_ld_16x256b<4>(tcol + (uint32_t)((F::kMins ? kColL : kTokMax) + 32 * q) + ((uint32_t)(16 * hf) << 16), l);
+                        const float2 w0 = rw[16 * hf], w1 = rw[16 * hf + 8];
+                        const uint64_t dw[2] = {pack2f(w0.x, w0.x), pack2f(w1.x, w1.x)}, ndm[2] = {pack2f(-w0.y, -w0.y), pack2f(-w1.y, -w1.y)};
                         tmem_ld_wait();
+                        if (q == kQ - 1 && hf == 1) {
+                            tc_fence_before();
+                            arrive_warp(&bar_free[c], lane);       // (the scales are in registers by now)
+                        }
 #pragma unroll
-                        for (int i = 0; i < 8; i += 2) {
-                            const float4 d4 = *reinterpret_cast<const float4 *>(da + col + 2 * i);
+                        for (int j = 0; j < 4; ++j)
 #pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const uint64_t dd = e ? pack2f(d4.z, d4.w) : pack2f(d4.x, d4.y);
-                                const uint64_t pv = pack2(p[2 * (i + e)], p[2 * (i + e) + 1]), lv = pack2(l[2 * (i + e)], l[2 * (i + e) + 1]);
+                            for (int s = 0; s < 2; ++s) {
+                                const int x = 2 * j + s;
+                                const uint64_t pv = pack2(p[2 * x], p[2 * x + 1]), lv = pack2(l[2 * x], l[2 * x + 1]);
                                 uint64_t tv;
-                                if constexpr (F::kMins) tv = fma2(dw, pv, mul2(ndm, lv));
-                                else tv = mul2(dw, fma2(one, pv, lv));
-                                acc[g][i + e] = fma2(dd, tv, acc[g][i + e]);
+                                if constexpr (F::kMins) tv = fma2(dw[s], pv, mul2(ndm[s], lv));
+                                else tv = mul2(dw[s], fma2(one, pv, lv));
+                                acc[q][8 * hf + x] = fma2(dd[j], tv, acc[q][8 * hf + x]);
                             }
-                        }
                     }
                 }
-                tc_fence_before();
-                arrive_warp(&bar_free[c], lane);
+                if (STORE == kStorePairs && sb == 0 && gi.topk_weights) {
+#pragma unroll
+                    for (int q = 0; q < kQ; ++q)
+                        if (col0 + 32 * q + lane < cx.valid) pw[q] = gi.topk_weights[pair[q]];
+                }
             }
-            if (!alive) break;
-            if (cx.row0 + r < a.nrows) {
-                void *out = second ? a.out2 : a.out;
+            const int left = min(n >> 1, cx.valid - col0);          // columns of this warp that hold tokens
+            void *out = second ? a.out2 : a.out;
+            const int64_t base = ((int64_t)cx.t * tl.tt + col0) * a.stride_out + cx.row0;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    const int col = (2 * g + ch0) * 16, left = cx.valid - col;
-                    if (left <= 0) continue;
-                    if (gi.tiles) {         // output row = the pair of this job, scaled by its routing weight (f32)
-                        const int32_t *pairs = gi.sorted_token_ids + cx.job0 + col;
+            for (int q = 0; q < kQ; ++q)
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            if (i < left) {
-                                const int pair = pairs[i];
-                                float v = (i & 1) ? hi2(acc[g][i >> 1]) : lo2(acc[g][i >> 1]);
-                                if (gi.topk_weights) v = __fmul_rn(v, gi.topk_weights[pair]);
-                                ((float *)out)[(int64_t)pair * a.stride_out + cx.row0 + r] = v;
-                            }
-                        }
+                for (int j = 0; j < 4; ++j) {
+                    const uint64_t v[4] = {acc[q][2 * j], acc[q][2 * j + 1], acc[q][8 + 2 * j], acc[q][9 + 2 * j]};       // rows r0 + 8 i
+                    if constexpr (STORE == kStore16) {
+                        const int col = 32 * q + 8 * j + (lane >> 2), row = (warp & 3) * 32;
+                        store_rows32_16bit(v, a.out_kind, (uint16_t *)out + base + (int64_t)col * a.stride_out + row, col < left ? a.nrows - cx.row0 - row : 0,
+                                           ((a.stride_out & 7) | ((uintptr_t)out & 15)) == 0);
                     } else {
-                        const int64_t tok = (int64_t)cx.t * tl.tt + col;
-                        store16(acc[g], out, a.out_kind, a.stride_out, cx.row0 + r, left, [&](int i) { return tok + i; });
+                        const int col = 32 * q + 8 * j + csub;
+                        float *o0 = (float *)out + base + (int64_t)col * a.stride_out + r0, *o1 = o0 + a.stride_out;
+                        float w0 = 1.0f, w1 = 1.0f;
+                        if constexpr (STORE == kStorePairs) {       // output row = the pair of this job, scaled by its routing weight
+                            const int p0 = __shfl_sync(0xffffffffu, pair[q], col & 31), p1 = __shfl_sync(0xffffffffu, pair[q], (col & 31) + 1);
+                            w0 = __shfl_sync(0xffffffffu, pw[q], col & 31);
+                            w1 = __shfl_sync(0xffffffffu, pw[q], (col & 31) + 1);
+                            o0 = (float *)out + (int64_t)p0 * a.stride_out + cx.row0 + r0;
+                            o1 = (float *)out + (int64_t)p1 * a.stride_out + cx.row0 + r0;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const bool in = cx.row0 + r0 + 8 * i < a.nrows;
+                            if (in && col < left) o0[8 * i] = STORE == kStorePairs ? __fmul_rn(lo2(v[i]), w0) : lo2(v[i]);
+                            if (in && col + 1 < left) o1[8 * i] = STORE == kStorePairs ? __fmul_rn(hi2(v[i]), w1) : hi2(v[i]);
+                        }
                     }
                 }
-            }
+            return true;
+        };
+        for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
+            TileCtx cx;
+            const bool second = tile >= per_matrix;
+            tile_ctx(second ? tile - per_matrix : tile, ntt, tl, gi, cx);
+            if constexpr (Q == 0) alive = cx.n > 64 ? run_tile(cx, second, std::integral_constant<int, 2>{}) : run_tile(cx, second, std::integral_constant<int, 1>{});
+            else alive = run_tile(cx, second, std::integral_constant<int, Q>{});
         }
     }
 
@@ -684,18 +725,22 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 // the fixed part of a tile's time per super-block in tokens (plan_tiling); Q6_K is bound by its producers, 2 us at any token count
 template <int WTYPE> constexpr int fixed_tokens() { return WTYPE == CQ_Q4_K ? 150 : 400; }
 
-template <int WTYPE>
-bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k, int n, long long total_rows, int stride_out, const Tiling &tl,
-                 const GroupInfo &gi, cudaStream_t st, const void *w2 = nullptr, void *out2 = nullptr) {
-    using R = Raw<cq_type_size(WTYPE)>;
+template <int WTYPE, int STORE, int Q> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const CUtensorMap &map2, const Args &a, const Tiling &tl, const GroupInfo &gi) {
     static_assert(smem_bytes<WTYPE>() <= 232448, "shared memory of one CTA");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-        cudaFuncSetAttribute(prompt_kernel<WTYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WTYPE>());
+        cudaFuncSetAttribute(prompt_kernel<WTYPE, STORE, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WTYPE>());
         attr_done[dev] = true;
     }
+    cq_launch_k(prompt_kernel<WTYPE, STORE, Q>, dim3(grid), dim3(kThreads), smem_bytes<WTYPE>(), st, map, map2, a, tl, gi);
+}
+
+template <int WTYPE>
+bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k, int n, long long total_rows, int stride_out, const Tiling &tl,
+                 const GroupInfo &gi, cudaStream_t st, const void *w2 = nullptr, void *out2 = nullptr) {
+    using R = Raw<cq_type_size(WTYPE)>;
     const long long row_bytes = (long long)(k / 256) * cq_type_size(WTYPE);
     CUtensorMap map{}, map2{};
     const uintptr_t both = (uintptr_t)w | (uintptr_t)w2;
@@ -710,7 +755,14 @@ bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k,
                  use_map ? 1 : 0, (n + kRows - 1) / kRows};
     const long long ntiles = (long long)a.nrt * tl.ntt * (w2 ? 2 : 1);
     const int grid = ntiles < sm_count() ? (int)ntiles : sm_count();
-    cq_launch_k(prompt_kernel<WTYPE>, dim3(grid), dim3(kThreads), smem_bytes<WTYPE>(), st, map, map2, a, tl, gi);
+    if (gi.tiles) launch_kernel<WTYPE, kStorePairs, 0>(grid, st, map, map2, a, tl, gi);
+    else if (out_elem == CQ_F32) {
+        if (tl.tt <= 64) launch_kernel<WTYPE, kStoreF32, 1>(grid, st, map, map2, a, tl, gi);
+        else launch_kernel<WTYPE, kStoreF32, 2>(grid, st, map, map2, a, tl, gi);
+    } else {
+        if (tl.tt <= 64) launch_kernel<WTYPE, kStore16, 1>(grid, st, map, map2, a, tl, gi);
+        else launch_kernel<WTYPE, kStore16, 2>(grid, st, map, map2, a, tl, gi);
+    }
     return true;
 }
 
