@@ -240,9 +240,9 @@ __device__ __forceinline__ bool cq_mbar_wait_bounded(uint64_t *bar, unsigned par
 // Read NW consecutive 32-bit words that start at a 2-byte-aligned shared-memory address.
 // Reads one aligned word past the last one (callers keep 4 bytes of slack).
 template <int NW> __device__ __forceinline__ void cq_lds_words(const uint8_t *p, uint32_t (&out)[NW]) {
-    const uintptr_t a = (uintptr_t)p;
-    const uint32_t *w = (const uint32_t *)(a & ~(uintptr_t)3);
-    const unsigned sh = (unsigned)(a & 2) * 8;
+    const unsigned off = (unsigned)(uintptr_t)p & 3u;       // 0 or 2
+    const uint32_t *w = (const uint32_t *)(p - off);        // pointer arithmetic, not a rounded address: the compiler then knows that this is shared memory
+    const unsigned sh = off * 8;
     uint32_t t[NW + 1];
 #pragma unroll
     for (int j = 0; j <= NW; ++j) t[j] = w[j];

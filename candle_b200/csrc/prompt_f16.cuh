@@ -93,21 +93,18 @@ template <int N> __device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr,
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Bounded wait like wait_or_abort, with a hint that lets the hardware suspend the thread until the phase completes (at most about
-// 0.1 ms at a time): fourteen waiting warps that poll took more than half of all issue slots, from the producers above all.
-__device__ __forceinline__ bool try_wait_suspended(uint64_t *bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(cq_smem_u32(bar)), "r"(parity), "r"(100000u) : "memory");
-    return ok != 0;
-}
+// Bounded wait like wait_or_abort; between two tries the warp sleeps, since fourteen waiting warps that poll took more than half of all issue slots, from the
+// producers above all.  The bound counts tries (2^23 sleeps are about a second): every wait is copied into its place - calls do not go with changed register
+// budgets - so its code is kept short.
 __device__ __forceinline__ bool wait_slow(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    const long long t0 = clock64();
-    while (!try_wait_suspended(bar, parity)) {
-        if (*abort_flag) return false;
-        if (clock64() - t0 > 2000000000LL) { *abort_flag = 1; return false; }
+#pragma unroll 1
+    for (unsigned n = 0; n < (1u << 23); ++n) {
+        __nanosleep(64);
+        if (cq_mbar_try_wait(bar, parity)) return true;
+        if ((n & 1023u) == 1023u && *abort_flag) return false;
     }
-    return true;
+    *abort_flag = 1;
+    return false;
 }
 // There is no per-lane form: every role goes on to warp-wide instructions, so its warp decides as one whether a wait gave up (lanes
 // that left at different places would meet at different warp-wide instructions, which need not end).

@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(1024) group_tiles_kernel(const int32_t *__rest
 }
 
 // ---- producers: the GGUF bytes of one row -> stages of 64 TMEM cells ------------------------------------------------
-template <int WTYPE> struct Expand;
+template <int WTYPE, bool MAP> struct Expand;
 
 // Q4_K, a stage is two chunks; chunk ch: elements 64 ch ..: low nibbles of bytes 32 ch .. +31 (sub-block 2 ch), then the high ones (2 ch + 1).
 // A nibble in the low mantissa bits of 1024.0 (or 16 times it, for high nibbles left in place) becomes sc * q in one fma.
-template <> struct Expand<CQ_Q4_K> {
+template <bool MAP> struct Expand<CQ_Q4_K, MAP> {
     const uint8_t *p;
     uint32_t sc[2], mn[2], dm;
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
@@ -287,20 +287,42 @@ template <> struct Expand<CQ_Q4_K> {
 // Q6_K stage 2 h + p: the two 32-element groups pos = p (low nibbles) and p + 2 (high ones) of ql[64 h + 32 p ..], bit pairs pos of
 // qh[32 h ..]; 16 cells of A, then 16 of B per group.  The 6-bit code q sits in the mantissa of 1024.0; sc * (q - 32) + 12288, where f16 counts
 // in eights, rounds to the next multiple of 8 in one fma, and a second one gives the exact rest.
-template <> struct Expand<CQ_Q6_K> {
+template <bool MAP> struct Expand<CQ_Q6_K, MAP> {
     const uint8_t *p;
     uint32_t sc[4];
+    int off;            // distance of p to the 16-byte boundary below it (MAP: the same for all rows)
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;
+        off = shift;
         cq_lds_words<4>(p + 192, sc);
+    }
+    // 32 bytes from an even address.  Eight words read one by one are four-way bank conflicts, whatever the pitch of the rows, a multiple of 16; three
+    // 16-byte reads are none.  Where all rows have the same distance to a 16-byte boundary the words they leave are picked by a uniform branch.
+    __device__ __forceinline__ void words32(const uint8_t *a, uint32_t (&o)[8]) const {
+        if constexpr (!MAP) cq_lds_words<8>(a, o);
+        else {
+            const uint4 *v = reinterpret_cast<const uint4 *>(a - off);
+            const uint4 x = v[0], y = v[1], z = v[2];
+            const uint32_t w[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+            const unsigned sh = (off & 2) * 8;
+            auto pick = [&](auto first) {
+                constexpr int f = decltype(first)::value;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = __funnelshift_r(w[f + i], w[f + i + 1 < 12 ? f + i + 1 : 11], sh);
+            };
+            if (off < 4) pick(std::integral_constant<int, 0>{});
+            else if (off < 8) pick(std::integral_constant<int, 1>{});
+            else if (off < 12) pick(std::integral_constant<int, 2>{});
+            else pick(std::integral_constant<int, 3>{});
+        }
     }
     __device__ __forceinline__ float2 scales() const { return make_float2(__half2float(*reinterpret_cast<const __half *>(p + 208)), 0.0f); }
     __device__ __forceinline__ void mins(uint8_t *) const {}
     __device__ __forceinline__ void stage(int st, uint32_t (&o)[2][32]) const {
         const int h = st >> 1, pp = st & 1;
         uint32_t ql[8], qh[8];
-        cq_lds_words<8>(p + 64 * h + 32 * pp, ql);
-        cq_lds_words<8>(p + 128 + 32 * h, qh);
+        words32(p + 64 * h + 32 * pp, ql);
+        words32(p + 128 + 32 * h, qh);
 #pragma unroll
         for (int nib = 0; nib < 2; ++nib) {         // pos = pp + 2 nib, scales 8 h + 2 pos + {0, 1}
             const uint32_t scw = (h ? sc[2 + nib] : sc[nib]) >> (16 * pp);
@@ -328,11 +350,12 @@ struct Args {
     const uint8_t *w, *w2, *act;        // w2: null, or a second matrix of the same shape for the same activations
     void *out, *out2;
     long long total_rows;               // weight rows in memory (all experts)
-    int out_kind, nrows, nsb, stride_out, use_map, nrt;
+    int out_kind, nrows, nsb, stride_out, nrt;
 };
 
-// STORE: see prompt_f16.cuh; Q: tiles of up to 64 Q tokens, 0: of any size (grouped launches, where each tile has its own)
-template <int WTYPE, int STORE, int Q>
+// STORE: see prompt_f16.cuh; Q: tiles of up to 64 Q tokens, 0: of any size (grouped launches, where each tile has its own); MAP: rows lie a multiple of 16 bytes
+// apart and come by tiled copies, so that a chunk starts at the same distance to a 16-byte boundary in all of them
+template <int WTYPE, int STORE, int Q, bool MAP>
 __global__ void __launch_bounds__(kThreads, 1)
 prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap wmap2, const Args a, const Tiling tl, const GroupInfo gi) {
     using F = Fmt<WTYPE>;
@@ -359,7 +382,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
     const uint32_t row_bytes = (uint32_t)nsb * kCB;
 
     if (tid == 0) {
-        for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < 3; ++i) { cq_mbar_init(&bar_raw[i], MAP ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
         for (int i = 0; i < F::kNT; ++i) { cq_mbar_init(&bar_full[i], 4 + 1); cq_mbar_init(&bar_done[i], 1); }
         for (int i = 0; i < 2; ++i) { cq_mbar_init(&bar_free[i], kEpiWarps); cq_mbar_init(&bar_vis[i], 1); }
         *abort_flag = 0;
@@ -392,7 +415,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nsb * kTokBytes;
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                 const int rs = it % F::kRawStages;
-                if (a.use_map) {
+                if constexpr (MAP) {
                     if (it >= F::kRawStages && !wait_warp(&bar_rawfree[rs], (it / F::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
@@ -423,7 +446,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         // after a give-up the copies of raw bytes must land (or give up themselves) before the shared memory goes away, and those
         // of activations have a second to (their barrier also waits for producers that may have left)
         if (lane == 0 && (!alive || *abort_flag)) {
-            for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; a.use_map && j <= it; ++j)
+            for (int j = it >= F::kRawStages ? it - F::kRawStages + 1 : 0; MAP && j <= it; ++j)
                 (void)cq_mbar_wait_bounded(&bar_raw[j % F::kRawStages], (j / F::kRawStages) & 1);
             for (int j = h > F::kNT ? h - F::kNT : 0; j < h; ++j) {
                 if (cq_mbar_wait_bounded(&bar_full[j % F::kNT], (j / F::kNT) & 1)) continue;
@@ -433,7 +456,7 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
         __syncwarp();
     } else if (warp >= kRawWarp) {
         // ===== raw bytes of rows that are not a multiple of 16 bytes apart =====
-        if (!a.use_map) {
+        if constexpr (!MAP) {
             int it = 0;
             bool alive = true;
             for (int tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x) {
@@ -557,10 +580,10 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
             long long wr = cx.wrow0 + r;
             if (wr >= a.total_rows) wr = a.total_rows - 1;
             // without the tensor map every row has its own distance to the 16-byte boundary below it
-            const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes) & 15);
+            const uint32_t row_off = MAP ? 0u : (uint32_t)((uintptr_t)((second ? a.w2 : a.w) + wr * row_bytes) & 15);
             for (int sb = 0; sb < nsb && alive; ++sb, ++it) {
                 if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
-                Expand<WTYPE> ex;
+                Expand<WTYPE, MAP> ex;
                 ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)sb * kCB) & 15));
                 // This set's wait in super-block it - 1 was for a stage of it - 2: its MMAs had started, so the epilogue had finished it - 4
                 // (the ring entry written here), and set 1's was for the last one, with the sums step that read this copy of the minima.
@@ -725,16 +748,16 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 // the fixed part of a tile's time per super-block in tokens (plan_tiling); Q6_K is bound by its producers, 2 us at any token count
 template <int WTYPE> constexpr int fixed_tokens() { return WTYPE == CQ_Q4_K ? 150 : 400; }
 
-template <int WTYPE, int STORE, int Q> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const CUtensorMap &map2, const Args &a, const Tiling &tl, const GroupInfo &gi) {
+template <int WTYPE, int STORE, int Q, bool MAP> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const CUtensorMap &map2, const Args &a, const Tiling &tl, const GroupInfo &gi) {
     static_assert(smem_bytes<WTYPE>() <= 232448, "shared memory of one CTA");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-        cudaFuncSetAttribute(prompt_kernel<WTYPE, STORE, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WTYPE>());
+        cudaFuncSetAttribute(prompt_kernel<WTYPE, STORE, Q, MAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<WTYPE>());
         attr_done[dev] = true;
     }
-    cq_launch_k(prompt_kernel<WTYPE, STORE, Q>, dim3(grid), dim3(kThreads), smem_bytes<WTYPE>(), st, map, map2, a, tl, gi);
+    cq_launch_k(prompt_kernel<WTYPE, STORE, Q, MAP>, dim3(grid), dim3(kThreads), smem_bytes<WTYPE>(), st, map, map2, a, tl, gi);
 }
 
 template <int WTYPE>
@@ -751,18 +774,19 @@ bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k,
         cq_set_status(CQ_ERR_BAD_ARG, "prompt gemm: Q4_K weights must be 16-byte aligned");
         return false;
     }
-    const Args a{(const uint8_t *)w, (const uint8_t *)w2, (const uint8_t *)act, out, out2, total_rows, out_elem, n, k / 256, stride_out,
-                 use_map ? 1 : 0, (n + kRows - 1) / kRows};
+    const Args a{(const uint8_t *)w, (const uint8_t *)w2, (const uint8_t *)act, out, out2, total_rows, out_elem, n, k / 256, stride_out, (n + kRows - 1) / kRows};
     const long long ntiles = (long long)a.nrt * tl.ntt * (w2 ? 2 : 1);
     const int grid = ntiles < sm_count() ? (int)ntiles : sm_count();
-    if (gi.tiles) launch_kernel<WTYPE, kStorePairs, 0>(grid, st, map, map2, a, tl, gi);
-    else if (out_elem == CQ_F32) {
-        if (tl.tt <= 64) launch_kernel<WTYPE, kStoreF32, 1>(grid, st, map, map2, a, tl, gi);
-        else launch_kernel<WTYPE, kStoreF32, 2>(grid, st, map, map2, a, tl, gi);
-    } else {
-        if (tl.tt <= 64) launch_kernel<WTYPE, kStore16, 1>(grid, st, map, map2, a, tl, gi);
-        else launch_kernel<WTYPE, kStore16, 2>(grid, st, map, map2, a, tl, gi);
-    }
+    auto run = [&](auto map_) {
+        constexpr bool M = decltype(map_)::value;
+        if (gi.tiles) launch_kernel<WTYPE, kStorePairs, 0, M>(grid, st, map, map2, a, tl, gi);
+        else if (out_elem == CQ_F32 && tl.tt <= 64) launch_kernel<WTYPE, kStoreF32, 1, M>(grid, st, map, map2, a, tl, gi);
+        else if (out_elem == CQ_F32) launch_kernel<WTYPE, kStoreF32, 2, M>(grid, st, map, map2, a, tl, gi);
+        else if (tl.tt <= 64) launch_kernel<WTYPE, kStore16, 1, M>(grid, st, map, map2, a, tl, gi);
+        else launch_kernel<WTYPE, kStore16, 2, M>(grid, st, map, map2, a, tl, gi);
+    };
+    if (use_map) run(std::true_type{});
+    else run(std::false_type{});
     return true;
 }
 
