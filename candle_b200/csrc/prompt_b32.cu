@@ -864,7 +864,7 @@ extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     case CQ_Q2_K: fixed = 2.46; per_token = 0.008; break;
     case CQ_Q3_K: fixed = 2.64; per_token = 0.005; break;
     }
-    const double idle = (double)((n + kRows - 1) / kRows) * tl.ntt < 0.6 * sms ? 0.85 : 1.0;      // fewer tiles share the L2
+    const double idle = (double)((n + kRows - 1) / kRows) * tl.ntt < 0.3 * sms ? 0.85 : 1.0;      // few tiles share the L2
     const double here = 8.5 + rounds * (k / 256) * (fixed + per_token * tl.tt) * idle;
     auto slice = [&](int rows) {
         return super ? 5.25 + 0.125e-3 * k + weights * (0.05 + 0.084 * rows) : std::max(5.05, 4.7 + 0.018e-3 * k + weights * (0.21 + 0.02 * rows));
