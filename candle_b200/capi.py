@@ -7,6 +7,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libcandle_q_b200.so")
 
@@ -211,3 +213,28 @@ def check(what: str = "") -> None:
 
 def pad(p: int, q: int) -> int:
     return (p + q - 1) // q * q
+
+
+def stream_of(device: torch.device) -> int:
+    """Handle of the current stream of a CUDA device.  (`torch.cuda.current_stream` builds a stream object: 1.5 us a call.)"""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+class on_device:
+    """Makes a CUDA device current, for library calls that do not do so themselves; nothing to do, in a tenth of the time of
+    `torch.cuda.device`, where it already is."""
+
+    __slots__ = ("_ctx",)
+
+    def __init__(self, device: torch.device):
+        index = device.index
+        self._ctx = None if index is None or torch.cuda.current_device() == index else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self._ctx is not None:
+            self._ctx.__enter__()
+
+    def __exit__(self, *exc):
+        if self._ctx is not None:
+            self._ctx.__exit__(*exc)

@@ -78,8 +78,8 @@ class FusedMoeGGUF:
             if pairs > 65535:
                 return None
         part = self.world > 1 or self.expert_offset != 0 or local != experts       # pairs of other ranks must read as zero
-        with torch.cuda.device(dev):
-            st = torch.cuda.current_stream(dev).cuda_stream
+        with capi.on_device(dev):
+            st = capi.stream_of(dev)
             logits = torch.nn.functional.linear(x, self.gate).to(torch.float32).contiguous()      # autocast gives 16 bits
             ids = torch.empty((3, pairs), dtype=torch.int32, device=dev)        # by token; then experts and pairs, sorted
             weights = torch.empty((tokens, k), dtype=torch.float32, device=dev)

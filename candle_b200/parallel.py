@@ -299,11 +299,11 @@ def argmax_sharded(local_logits: torch.Tensor, vocab_start: int, gather: Gathere
     if local_logits.is_cuda and local_logits.dtype == torch.float32 and local_logits.dim() == 2 and local_logits.is_contiguous() and \
             0 < local_logits.shape[0] <= 65535 and local_logits.shape[1] > 0:
         rows, n = local_logits.shape
-        st = torch.cuda.current_stream(local_logits.device).cuda_stream
+        st = capi.stream_of(local_logits.device)
         one = gather.world == 1         # then the pair is the result
         out = torch.empty(rows, dtype=torch.int64, device=local_logits.device) if one else \
             torch.empty((rows, 2), dtype=torch.float32, device=local_logits.device)
-        with torch.cuda.device(local_logits.device):
+        with capi.on_device(local_logits.device):
             capi.lib().cq_argmax_f32(local_logits.data_ptr(), rows, n, vocab_start, None if one else out.data_ptr(), out.data_ptr() if one else None, st)
         capi.check("argmax")
         return out if one else _best_pair(gather(out))

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import functools
 from typing import Sequence
 
 import numpy as np
@@ -93,6 +94,9 @@ def quantize_blocks(src, dtype: GgmlDType, imatrix=None) -> bytes:
 def _dims(shape: Sequence[int]):
     arr = (C.c_int64 * len(shape))(*[int(d) for d in shape])
     return arr, len(shape)
+
+
+_dims_of = functools.lru_cache(maxsize=512)(_dims)      # of shapes that recur, call after call; the library only reads them
 
 
 class QTensor:
@@ -234,10 +238,8 @@ class QTensor:
         ids32 = ids.to(torch.int32).contiguous()
         topk = ids32.shape[1]
         out = (torch.zeros if zero_init else torch.empty)((batch, topk, self._shape[1]), dtype=torch.float32, device=x.device)
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        with torch.cuda.device(x.device):
-            capi.hcheck(capi.lib().cqh_indexed_moe_forward(self._h, x.data_ptr(), x_dim1, ids32.data_ptr(), batch, topk,
-                                                            out.data_ptr(), stream))
+        capi.hcheck(capi.lib().cqh_indexed_moe_forward(self._h, x.data_ptr(), x_dim1, ids32.data_ptr(), batch, topk,
+                                                        out.data_ptr(), capi.stream_of(x.device)))
         return out
 
     def indexed_moe_forward_q8_1(self, act: torch.Tensor, x_dim1: int, ids: torch.Tensor, zero_init: bool = False) -> torch.Tensor:
@@ -252,10 +254,8 @@ class QTensor:
         if not act.is_cuda or act.dtype != torch.uint8 or not act.is_contiguous() or tuple(act.shape) != (batch * x_dim1, row_bytes):
             raise CandleQError(f"indexed_moe_forward_q8_1 expects a contiguous uint8 CUDA tensor [{batch * x_dim1}, {row_bytes}]")
         out = (torch.zeros if zero_init else torch.empty)((batch, topk, self._shape[1]), dtype=torch.float32, device=act.device)
-        stream = torch.cuda.current_stream(act.device).cuda_stream
-        with torch.cuda.device(act.device):
-            capi.hcheck(capi.lib().cqh_indexed_moe_forward_q8_1(self._h, act.data_ptr(), x_dim1, ids32.data_ptr(), batch, topk,
-                                                                 out.data_ptr(), stream))
+        capi.hcheck(capi.lib().cqh_indexed_moe_forward_q8_1(self._h, act.data_ptr(), x_dim1, ids32.data_ptr(), batch, topk,
+                                                             out.data_ptr(), capi.stream_of(act.device)))
         return out
 
     def dequantize(self, dtype: torch.dtype = torch.float32) -> torch.Tensor:
@@ -263,9 +263,7 @@ class QTensor:
         if dtype not in _ELEM:
             raise CandleQError(f"Expected f32/f16/bf16, got {dtype}")
         out = torch.empty(self._shape, dtype=dtype, device=self._device)
-        stream = torch.cuda.current_stream(self._device).cuda_stream
-        with torch.cuda.device(self._device):
-            capi.hcheck(capi.lib().cqh_qtensor_dequantize(self._h, out.data_ptr(), _ELEM[dtype], stream), "QTensor.dequantize")
+        capi.hcheck(capi.lib().cqh_qtensor_dequantize(self._h, out.data_ptr(), _ELEM[dtype], capi.stream_of(self._device)), "QTensor.dequantize")
         return out
 
     def embedding(self, ids: torch.Tensor, dtype: torch.dtype = torch.float32) -> torch.Tensor:
@@ -353,11 +351,10 @@ class QMatMul:
         n = self.qtensor.shape[0]
         if out is None:
             out = torch.empty((*xs.shape[:-1], n), dtype=xs.dtype, device=xs.device)
-        dims, nd = _dims(xs.shape)
-        stream = torch.cuda.current_stream(xs.device).cuda_stream
-        with torch.cuda.device(xs.device):
-            capi.hcheck(capi.lib().cqh_qmatmul_forward(self.qtensor._h, xs.data_ptr(), _ELEM[xs.dtype], dims, nd,
-                                                        out.data_ptr(), stream))
+        dims, nd = _dims_of(xs.shape)
+        rc = capi.lib().cqh_qmatmul_forward(self.qtensor._h, xs.data_ptr(), _ELEM[xs.dtype], dims, nd, out.data_ptr(), capi.stream_of(xs.device))
+        if rc != 0:     # (the library makes the tensor's device current itself, here and below)
+            capi.hcheck(rc)
         return out
 
     def forward_host(self, xs: torch.Tensor, out: torch.Tensor, stream: int | None = None) -> torch.Tensor:
@@ -396,9 +393,7 @@ class QMatMul:
         rows, n = act.shape[0], self.qtensor.shape[0]
         if out is None:
             out = torch.empty((rows, n), dtype=torch.float32, device=act.device)
-        stream = torch.cuda.current_stream(act.device).cuda_stream
-        with torch.cuda.device(act.device):
-            capi.hcheck(capi.lib().cqh_qmatmul_forward_q8_1(self.qtensor._h, act.data_ptr(), rows, out.data_ptr(), stream))
+        capi.hcheck(capi.lib().cqh_qmatmul_forward_q8_1(self.qtensor._h, act.data_ptr(), rows, out.data_ptr(), capi.stream_of(act.device)))
         return out
 
     def forward_q8_1_pair(self, other: "QMatMul", act: torch.Tensor):
@@ -409,10 +404,8 @@ class QMatMul:
             raise CandleQError("forward_q8_1_pair expects a contiguous uint8 CUDA tensor of Q8_1 containers")
         out_a = torch.empty((rows, self.qtensor.shape[0]), dtype=torch.float32, device=act.device)
         out_b = torch.empty((rows, other.qtensor.shape[0]), dtype=torch.float32, device=act.device)
-        stream = torch.cuda.current_stream(act.device).cuda_stream
-        with torch.cuda.device(act.device):
-            capi.hcheck(capi.lib().cqh_qmatmul_forward_q8_1_pair(self.qtensor._h, other.qtensor._h, act.data_ptr(), rows,
-                                                                 out_a.data_ptr(), out_b.data_ptr(), stream))
+        capi.hcheck(capi.lib().cqh_qmatmul_forward_q8_1_pair(self.qtensor._h, other.qtensor._h, act.data_ptr(), rows,
+                                                             out_a.data_ptr(), out_b.data_ptr(), capi.stream_of(act.device)))
         return out_a, out_b
 
     __call__ = forward
