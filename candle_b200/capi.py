@@ -120,6 +120,10 @@ def lib() -> C.CDLL:
         L.cq_moe_router_f32.restype = None
         L.cq_moe_weighted_sum_f32.argtypes = [vp, vp, vp, i32, i32, i32, vp]
         L.cq_moe_weighted_sum_f32.restype = None
+        L.cq_moe_route_rows_f32.argtypes = [vp] * 5 + [i32] * 5 + [vp]
+        L.cq_moe_route_rows_f32.restype = None
+        L.cq_moe_route_rows_floats.argtypes = [i32] * 3
+        L.cq_moe_route_rows_floats.restype = C.c_size_t
         L.cq_argmax_f32.argtypes = [vp, i32, i32, C.c_int64, vp, vp, vp]
         L.cq_argmax_f32.restype = None
         L.cq_qknorm_rope_store_kv_f32.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32,

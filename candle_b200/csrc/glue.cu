@@ -146,18 +146,23 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const float *__restrict__
 // descending sort of NaNs gives, so that ids stay in range and the NaN stays with its own token.
 // One warp per token; experts <= 1024.  The softmax sum is added lane-strided, then by an xor butterfly.
 // One warp routes one token.  VOLATILE: the logits were written by other CTAs of the running kernel (read around L1).
-template <bool VOLATILE>
+// PER: experts per lane at most; `parts` logits of an expert, `part` floats apart, are added in order first (a router product split over K).
+template <bool VOLATILE, int PER>
 __device__ __forceinline__ void moe_route_row(const float *row, int32_t *__restrict__ ids, float *__restrict__ weights, int tok,
-                                              int experts, int k, int norm, int lane) {
-    constexpr int PER = 32;                    // experts per lane at most (1024 / 32)
+                                              int experts, int k, int norm, int lane, int parts = 1, size_t part = 0) {
     float p[PER];
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int e = lane + 32 * i;
         p[i] = e < experts ? (VOLATILE ? __ldcg(row + e) : row[e]) : -INFINITY;
-        mx = fmaxf(mx, p[i]);
     }
+    for (int s = 1; s < parts; ++s)
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (lane + 32 * i < experts) p[i] = __fadd_rn(p[i], row[s * part + lane + 32 * i]);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) mx = fmaxf(mx, p[i]);
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
     float sum = 0.0f;
@@ -205,15 +210,68 @@ __device__ __forceinline__ void moe_route_row(const float *row, int32_t *__restr
     }
 }
 
+template <int PER>
 __global__ void __launch_bounds__(128) moe_route_kernel(const float *__restrict__ logits, int32_t *__restrict__ ids,
-                                                        float *__restrict__ weights, int tokens, int experts, int k, int norm) {
+                                                        float *__restrict__ weights, int tokens, int experts, int k, int norm, int parts) {
     cq_pdl_launch_dependents();
     cq_pdl_wait();
     const int tok = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (tok >= tokens) return;
-    moe_route_row<false>(logits + (size_t)tok * experts, ids, weights, tok, experts, k, norm, lane);
+    moe_route_row<false, PER>(logits + (size_t)tok * experts, ids, weights, tok, experts, k, norm, lane, parts, (size_t)tokens * experts);
 }
 
+// Router logits of a prompt, f32: logits[s][t, e] = x[t, K part s] . w[e, K part s].  Tiles of 64 tokens x 64 experts, 128 threads with 8 x 4 of them each, the
+// inputs 32 values of K at a time through shared memory; K is split over gridDim.z so that a router of few experts fills the SMs (the library's product
+// of 1024 x 128 x 2048 ran 128 CTAs for 54 us).  Bound by the shared-memory reads, three of 16 bytes per 32 products.
+constexpr int kRtT = 64, kRtE = 64, kRtK = 32, kRtPitch = kRtT + 4;
+__global__ void __launch_bounds__(128) router_logits_kernel(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ logits, int tokens,
+                                                            int experts, int d, int dpart) {
+    __shared__ __align__(16) float xs[kRtK][kRtPitch], ws[kRtK][kRtPitch];
+    const int t0 = blockIdx.x * kRtT, e0 = blockIdx.y * kRtE, k0 = blockIdx.z * dpart, tid = threadIdx.x;
+    const int ty = tid >> 4, tx = tid & 15;
+    const int lr = tid >> 3, lk = (tid & 7) * 4;          // loads: rows lr + 16 i, four values of K
+    float4 xv[4], wv[4];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = t0 + lr + 16 * i, e = e0 + lr + 16 * i;
+            xv[i] = t < tokens ? *reinterpret_cast<const float4 *>(x + (size_t)t * d + k + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+            wv[i] = e < experts ? *reinterpret_cast<const float4 *>(w + (size_t)e * d + k + lk) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    cq_pdl_wait();
+    float acc[8][4] = {};
+    fetch(k0);
+    for (int k = 0; k < dpart; k += kRtK) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = lr + 16 * i;
+            xs[lk][r] = xv[i].x; xs[lk + 1][r] = xv[i].y; xs[lk + 2][r] = xv[i].z; xs[lk + 3][r] = xv[i].w;
+            ws[lk][r] = wv[i].x; ws[lk + 1][r] = wv[i].y; ws[lk + 2][r] = wv[i].z; ws[lk + 3][r] = wv[i].w;
+        }
+        __syncthreads();
+        if (k + kRtK < dpart) fetch(k0 + k + kRtK);
+#pragma unroll 8
+        for (int c = 0; c < kRtK; ++c) {
+            const float4 a0 = *reinterpret_cast<const float4 *>(&xs[c][8 * ty]), a1 = *reinterpret_cast<const float4 *>(&xs[c][8 * ty + 4]);
+            const float4 b = *reinterpret_cast<const float4 *>(&ws[c][4 * tx]);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+    float *out = logits + (size_t)blockIdx.z * tokens * experts;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int t = t0 + 8 * ty + i, e = e0 + 4 * tx + j;
+            if (t < tokens && e < experts) out[(size_t)t * experts + e] = acc[i][j];
+        }
+}
 // Router logits and routing in one launch, for the few rows of a decode step: logits[t, e] = h[t, :] . router[e, :] (f32;
 // one warp per (token, expert): a lane adds its float4 strides in order with FMAs, then an xor butterfly), and the CTA that
 // finishes a token's row last (an arrival counter per token, reset by that CTA) routes it with the warp function above.
@@ -256,7 +314,7 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const float *__restrict
     __syncthreads();
     if (!is_last || warp != 0) return;
     __threadfence();
-    moe_route_row<true>(logits + (size_t)tok * experts, ids, weights, tok, experts, k, norm, lane);
+    moe_route_row<true, 32>(logits + (size_t)tok * experts, ids, weights, tok, experts, k, norm, lane);
     if (lane == 0) counters[tok] = 0;       // ready for the next launch
 }
 
@@ -491,15 +549,52 @@ extern "C" void cq_silu_mul_q8_1(const float *gate_up, void *out_q8, int rows, i
     cq_check_launch("silu_mul_q8_1");
 }
 
+namespace {
+void launch_route(const float *logits, int32_t *ids, float *weights, int tokens, int experts, int k, int norm, int parts, cudaStream_t st) {
+    const dim3 grid((tokens + 3) / 4);
+    if (experts <= 64) cq_launch_k(moe_route_kernel<2>, grid, dim3(128), 0, st, logits, ids, weights, tokens, experts, k, norm, parts);
+    else if (experts <= 128) cq_launch_k(moe_route_kernel<4>, grid, dim3(128), 0, st, logits, ids, weights, tokens, experts, k, norm, parts);
+    else if (experts <= 256) cq_launch_k(moe_route_kernel<8>, grid, dim3(128), 0, st, logits, ids, weights, tokens, experts, k, norm, parts);
+    else cq_launch_k(moe_route_kernel<32>, grid, dim3(128), 0, st, logits, ids, weights, tokens, experts, k, norm, parts);
+}
+// K parts of the router product of a prompt: enough CTAs for two per SM, whole steps of kRtK each
+int router_parts(int tokens, int experts, int d) {
+    const int tiles = ((tokens + kRtT - 1) / kRtT) * ((experts + kRtE - 1) / kRtE);
+    int parts = 1;
+    while (parts < 8 && tiles * parts < 2 * cq_sm_count() && d % (2 * parts * kRtK) == 0) parts *= 2;
+    return parts;
+}
+}  // namespace
+
 extern "C" void cq_moe_route_f32(const float *logits, int32_t *ids, float *weights, int tokens, int experts, int k, int norm_topk_prob,
                                  void *stream) {
     if (!logits || !ids || !weights || tokens <= 0 || experts <= 0 || experts > 1024 || k <= 0 || k > 32 || k > experts) {
         cq_set_status(CQ_ERR_BAD_ARG, "moe_route: bad arguments (experts <= 1024, k <= 32)");
         return;
     }
-    cq_launch_k(moe_route_kernel, dim3((tokens + 3) / 4), dim3(128), 0, (cudaStream_t)stream, logits, ids, weights, tokens, experts, k,
-                norm_topk_prob);
+    launch_route(logits, ids, weights, tokens, experts, k, norm_topk_prob, 1, (cudaStream_t)stream);
     cq_check_launch("moe_route");
+}
+
+// Floats of scratch that cq_moe_route_rows_f32 takes; 0: it does not cover the shape.
+extern "C" size_t cq_moe_route_rows_floats(int tokens, int experts, int d) {
+    if (tokens <= 0 || experts <= 0 || experts > 1024 || d <= 0 || d % kRtK) return 0;
+    return (size_t)tokens * experts * router_parts(tokens, experts, d);
+}
+
+extern "C" void cq_moe_route_rows_f32(const float *x, const float *router, float *scratch, int32_t *ids, float *weights, int tokens, int experts, int d,
+                                      int k, int norm_topk_prob, void *stream) {
+    if (!x || !router || !scratch || !ids || !weights || k <= 0 || k > 32 || k > experts || cq_moe_route_rows_floats(tokens, experts, d) == 0 ||
+        (((uintptr_t)x | (uintptr_t)router) & 15)) {
+        cq_set_status(CQ_ERR_BAD_ARG, "moe_route_rows: bad arguments (experts <= 1024, k <= 32, 16-byte aligned rows)");
+        return;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const int parts = router_parts(tokens, experts, d);
+    cq_launch_k(router_logits_kernel, dim3((tokens + kRtT - 1) / kRtT, (experts + kRtE - 1) / kRtE, parts), dim3(128), 0, st, x, router, scratch, tokens,
+                experts, d, d / parts);
+    launch_route(scratch, ids, weights, tokens, experts, k, norm_topk_prob, parts, st);
+    cq_check_launch("moe_route_rows");
 }
 
 extern "C" void cq_moe_router_f32(const float *h, const float *router, float *logits, int32_t *ids, float *weights, int *counters,

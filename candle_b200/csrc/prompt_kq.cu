@@ -188,6 +188,34 @@ __global__ void __launch_bounds__(256) quantize_kernel(const L load, uint8_t *__
         *reinterpret_cast<float *>(blob + (size_t)rows * (kSlabs * 16 + (threadIdx.x >> 3) * 4) + (row0 + (threadIdx.x & 7)) * 4) = sd[threadIdx.x];
 }
 
+// Grouped launches whose input rows occur topk times: rows quantized once, 16 to a tile (quantize_kernel on a dense tiling), are copied to every pair's place,
+// eight pairs and all their super-blocks per block: a block per super-block held three copies per thread behind two dependent loads (28 us at
+// 8192 pairs of 2048 values, against the 45 that quantizing each pair took).
+__global__ void __launch_bounds__(256) copy_rows_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ y, int nsb, Tiling tl, GroupInfo gi) {
+    cq_pdl_wait();
+    const int per_tile = tl.tt / 8, t = blockIdx.x / per_tile, row0 = (blockIdx.x % per_tile) * 8;
+    if (t >= gi.tiles[4 * tl.ntt]) return;
+    const int4 ti = *reinterpret_cast<const int4 *>(gi.tiles + 4 * t);
+    const int rows = (ti.z + 15) / 16 * 16, rr = threadIdx.x & 7;
+    if (row0 >= rows) return;           // block-uniform
+    const int tok = row0 + rr < ti.z ? gi.sorted_token_ids[ti.y + row0 + rr] / gi.topk : -1;
+    const uint8_t *from = src + (size_t)(max(tok, 0) >> 4) * 16 * nsb * kTokBytes;
+    uint8_t *blob = y + (size_t)ti.w * nsb * kTokBytes;
+#pragma unroll 4
+    for (int i = threadIdx.x >> 3; i < nsb * kSlabs; i += 32) {
+        const int sb = i / kSlabs, slab = i - sb * kSlabs;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (tok >= 0) v = *reinterpret_cast<const uint4 *>(from + (size_t)sb * 16 * kTokBytes + (slab * 16 + (tok & 15)) * 16);
+        *reinterpret_cast<uint4 *>(blob + (size_t)sb * rows * kTokBytes + ((size_t)slab * rows + row0 + rr) * 16) = v;
+    }
+    for (int i = threadIdx.x >> 3; i < nsb * 2; i += 32) {          // scales, sums of |q8|
+        const int sb = i >> 1, w = i & 1;
+        float v = 0.0f;
+        if (tok >= 0) v = *reinterpret_cast<const float *>(from + (size_t)sb * 16 * kTokBytes + 16 * (kSlabs * 16 + w * 4) + (tok & 15) * 4);
+        *reinterpret_cast<float *>(blob + (size_t)sb * rows * kTokBytes + (size_t)rows * (kSlabs * 16 + w * 4) + (row0 + rr) * 4) = v;
+    }
+}
+
 // One CTA: the tile table of a grouped launch.  expert_ids ascending (ids outside [0, num_experts) may sit at either end);
 // the jobs of one expert are cut into tiles of kTokMax.
 __global__ void __launch_bounds__(1024) group_tiles_kernel(const int32_t *__restrict__ expert_ids, int m, int num_experts, int max_tiles,
@@ -953,7 +981,12 @@ extern "C" void cq_moe_block_prompt(int wtype, int wtype_down, const float *x, i
     const Tiling tl{mt * kTokMax, kTokMax, mt};
     group_tiles_kernel<<<1, 1024, 0, st>>>(expert_ids, size_m, num_experts, mt, tiles);
     const GroupInfo gu{tiles, sorted_token_ids, nullptr, ffn, topk, 0};
-    if (!launch_quantize(wtype, LoadRounded{x, hidden, kind}, blobs, hidden, tl, gu, st)) return;
+    const int tokens = (size_m + topk - 1) / topk, nsb = hidden / 256;
+    if (topk > 1 && (size_t)(tokens + 15) / 16 * 16 * nsb * kTokBytes <= (size_t)size_m * ffn * 8) {       // each row once, into the space of gate and up
+        const Tiling rows{tokens, 16, (tokens + 15) / 16};
+        if (!launch_quantize(wtype, LoadRounded{x, hidden, kind}, g, hidden, rows, GroupInfo{}, st)) return;
+        cq_launch_k(copy_rows_kernel, dim3(tl.ntt * (tl.tt / 8)), dim3(256), 0, st, (const uint8_t *)g, blobs, nsb, tl, gu);
+    } else if (!launch_quantize(wtype, LoadRounded{x, hidden, kind}, blobs, hidden, tl, gu, st)) return;
     const long long rows_gu = (long long)ffn * num_experts, rows_d = (long long)hidden * num_experts;
     bool ok = wtype == CQ_Q4_K ? launch_gemm<CQ_Q4_K>(gate, blobs, g, CQ_F32, hidden, ffn, rows_gu, ffn, tl, gu, st, up, u)
                                : launch_gemm<CQ_Q6_K>(gate, blobs, g, CQ_F32, hidden, ffn, rows_gu, ffn, tl, gu, st, up, u);

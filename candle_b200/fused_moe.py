@@ -80,11 +80,18 @@ class FusedMoeGGUF:
         part = self.world > 1 or self.expert_offset != 0 or local != experts       # pairs of other ranks must read as zero
         with capi.on_device(dev):
             st = capi.stream_of(dev)
-            logits = torch.nn.functional.linear(x, self.gate).to(torch.float32).contiguous()      # autocast gives 16 bits
             ids = torch.empty((3, pairs), dtype=torch.int32, device=dev)        # by token; then experts and pairs, sorted
             weights = torch.empty((tokens, k), dtype=torch.float32, device=dev)
             scratch = torch.empty(need, dtype=torch.uint8, device=dev)
-            lib.cq_moe_route_f32(logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, experts, k, 1 if self.norm_topk_prob else 0, st)
+            norm, gate = 1 if self.norm_topk_prob else 0, self.gate
+            floats = lib.cq_moe_route_rows_floats(tokens, experts, hidden) if is_prefill else 0
+            if floats and gate.dtype == torch.float32 and gate.device == dev and gate.is_contiguous() and not (gate.data_ptr() | x.data_ptr()) & 15 and \
+                    not torch.is_autocast_enabled("cuda"):
+                logits = torch.empty(floats, dtype=torch.float32, device=dev)
+                lib.cq_moe_route_rows_f32(x.data_ptr(), gate.data_ptr(), logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, experts, hidden, k, norm, st)
+            else:
+                logits = torch.nn.functional.linear(x, gate).to(torch.float32).contiguous()      # autocast gives 16 bits
+                lib.cq_moe_route_f32(logits.data_ptr(), ids.data_ptr(), weights.data_ptr(), tokens, experts, k, norm, st)
             if self.expert_offset:
                 ids[0] -= self.expert_offset        # ids outside [0, local) are skipped by the kernels
             g, u, d = (w.device_ptr() for w in (self.gate_experts, self.up_experts, self.down_experts))

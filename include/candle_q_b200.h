@@ -379,6 +379,12 @@ void cq_moe_router_f32(const float *h, const float *router, float *logits, int32
                        int experts, int d, int k, int norm_topk_prob, void *stream);
 void cq_moe_weighted_sum_f32(const float *y, const float *w, float *out, int tokens, int k, int d, void *stream);
 
+/* The router product in f32 and cq_moe_route_f32 on it: x [tokens, d], router [experts, d], 16-byte aligned rows; scratch: cq_moe_route_rows_floats
+ * floats (0: the shape is not covered; d a multiple of 32). */
+size_t cq_moe_route_rows_floats(int tokens, int experts, int d);
+void cq_moe_route_rows_f32(const float *x, const float *router, float *scratch, int32_t *ids, float *weights, int tokens, int experts, int d, int k,
+                           int norm_topk_prob, void *stream);
+
 /* First maximum of each of `rows` rows of n floats: pairs[r] = (value, index + start) as floats, tokens[r] = index + start (either may be null).  A
  * row with a NaN gives (NaN, 2^40 + start) and INT64_MAX. */
 void cq_argmax_f32(const float *x, int rows, int n, int64_t start, float *pairs, int64_t *tokens, void *stream);

@@ -545,3 +545,52 @@ def test_fused_moe_prompt_type_stays_16_bit_on_every_rank_count(cuda_dev, tokens
         moe = FusedMoeGGUF(torch.randn(6, 512, device=cuda_dev), *w, 2, prefill_dtype=torch.float32, world=world)
         with pytest.raises(capi.CandleQError, match="f16 or bf16"):
             moe.forward(torch.randn(1, tokens, 512, device=cuda_dev), True)
+
+
+@pytest.mark.parametrize("tokens,experts,d", [(1, 6, 32), (63, 64, 96), (64, 65, 2048), (65, 130, 1280), (200, 300, 512)])
+def test_router_rows_split_over_k(cuda_dev, tokens, experts, d):
+    """cq_moe_route_rows_f32: the sum of its K parts against the f64 product (d + 8 roundings of partial sums at most, each of
+    2^-24 of sum |x w|), ids and weights bit for bit those of cq_moe_route_f32 on that sum."""
+    L, st = capi.lib(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device=cuda_dev).manual_seed(tokens)
+    x, w = torch.randn(tokens, d, device=cuda_dev, generator=g), torch.randn(experts, d, device=cuda_dev, generator=g) * 0.05
+    parts = torch.empty(L.cq_moe_route_rows_floats(tokens, experts, d), device=cuda_dev)
+    k = min(6, experts)
+    ids, ids2 = (torch.empty(tokens, k, dtype=torch.int32, device=cuda_dev) for _ in range(2))
+    wt, wt2 = (torch.empty(tokens, k, device=cuda_dev) for _ in range(2))
+    L.cq_moe_route_rows_f32(x.data_ptr(), w.data_ptr(), parts.data_ptr(), ids.data_ptr(), wt.data_ptr(), tokens, experts, d, k, 1, st)
+    logits = torch.zeros(tokens, experts, device=cuda_dev)
+    for p in parts.view(-1, tokens, experts):
+        logits = logits + p
+    L.cq_moe_route_f32(logits.data_ptr(), ids2.data_ptr(), wt2.data_ptr(), tokens, experts, k, 1, st)
+    bound = (d + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((logits.double() - x.double() @ w.double().T).abs() <= bound).all())
+    assert torch.equal(ids, ids2) and torch.equal(wt, wt2)
+    assert L.cq_moe_route_rows_floats(tokens, experts, 48) == 0 and L.cq_moe_route_rows_floats(tokens, 1025, d) == 0
+
+
+@pytest.mark.parametrize("wt_gu,wt_down", [(12, 14), (14, 12)])
+@pytest.mark.parametrize("tokens,experts,topk,hidden", [(17, 4, 3, 256), (50, 3, 2, 1280), (131, 16, 8, 512)])
+def test_moe_prompt_rows_quantized_once(cuda_dev, wt_gu, wt_down, tokens, experts, topk, hidden):
+    """cq_moe_block_prompt quantizes a row once and copies it to the row's topk pairs: the same bits as with the rows repeated per pair and
+    topk = 1, where every pair is quantized in its place."""
+    from candle_b200.synth import random_blocks
+    L, st, ffn, pairs = capi.lib(), torch.cuda.current_stream().cuda_stream, 256, tokens * topk
+    g = torch.Generator(device=cuda_dev).manual_seed(tokens)
+    x = torch.randn(tokens, hidden, device=cuda_dev, generator=g)
+    ids = torch.stack([torch.randperm(experts, device=cuda_dev, generator=g)[:topk] for _ in range(tokens)]).to(torch.int32)
+    weights = torch.rand(tokens, topk, device=cuda_dev, generator=g)
+    gate, up = (random_blocks(GgmlDType(wt_gu), experts * ffn, hidden, seed=s, device=cuda_dev) for s in (1, 2))
+    down = random_blocks(GgmlDType(wt_down), experts * hidden, ffn, seed=3, device=cuda_dev)
+    by_expert, order = (torch.empty(pairs, dtype=torch.int32, device=cuda_dev) for _ in range(2))
+    L.cq_moe_sort_pairs(ids.data_ptr(), pairs, experts, by_expert.data_ptr(), order.data_ptr(), st)
+    scratch = torch.empty(L.cq_moe_block_prompt_scratch_bytes(pairs, experts, hidden, ffn), dtype=torch.uint8, device=cuda_dev)
+    out = []
+    for rows, k in ((x, topk), (x.repeat_interleave(topk, dim=0), 1)):
+        y = torch.zeros(pairs, hidden, device=cuda_dev)
+        L.cq_moe_block_prompt(wt_gu, wt_down, rows.data_ptr(), capi.BF16, gate.data_ptr(), up.data_ptr(), down.data_ptr(), order.data_ptr(),
+                              by_expert.data_ptr(), weights.data_ptr(), y.data_ptr(), scratch.data_ptr(), experts, k, pairs, hidden, ffn, st)
+        capi.check("moe block")
+        out.append(y)
+    assert torch.equal(out[0], out[1]) and float(out[0].abs().max()) > 0
+    assert L.cq_prompt_timeout_flag() == 0
