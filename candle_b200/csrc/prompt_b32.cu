@@ -201,8 +201,8 @@ __device__ __forceinline__ float h16(uint32_t w) { return __half2float(__ushort_
 // pairs (byte 0, byte 2) and (byte 1, byte 3) of a word of small unsigned codes, minus `off`, as f16
 __device__ __forceinline__ void codes4(uint32_t w, float off, uint32_t &a, uint32_t &b) {
     const __half2 o = __float2half2_rn(1024.0f + off);
-    a = h2_bits(__hsub2(bits_h2((w & 0x00FF00FFu) | 0x64006400u), o));
-    b = h2_bits(__hsub2(bits_h2(((w >> 8) & 0x00FF00FFu) | 0x64006400u), o));
+    a = h2_bits(__hsub2(bits_h2(and_or<0x00FF00FFu, 0x64006400u>(w)), o));
+    b = h2_bits(__hsub2(bits_h2(and_or<0x00FF00FFu, 0x64006400u>(w >> 8)), o));
 }
 __device__ __forceinline__ __half2 twice(uint32_t v) { return __hsub2(bits_h2(v * 0x00010001u | 0x64006400u), bits_h2(0x64006400u)); }   // v < 1024
 // Coefficients j, j + 1 (j even) of a row: planes lo, hi, mid of kSums / 8 slabs of 128 rows x 16 bytes
@@ -246,8 +246,8 @@ template <int WTYPE> struct ExpandBlock {
                 constexpr int i = decltype(ic)::value;
                 const uint32_t w = word_at<qs + 4 * i, V0>(v);
                 const __half2 c = __float2half2_rn(1152.0f);        // int8 + 128 in the mantissa of 1024
-                o[2 * i] = h2_bits(__hsub2(bits_h2((w & 0x00FF00FFu) ^ 0x64806480u), c));
-                o[2 * i + 1] = h2_bits(__hsub2(bits_h2(((w >> 8) & 0x00FF00FFu) ^ 0x64806480u), c));
+                o[2 * i] = h2_bits(__hsub2(bits_h2(and_xor<0x00FF00FFu, 0x64806480u>(w)), c));
+                o[2 * i + 1] = h2_bits(__hsub2(bits_h2(and_xor<0x00FF00FFu, 0x64806480u>(w >> 8)), c));
             };
             four(std::integral_constant<int, 0>{}); four(std::integral_constant<int, 1>{}); four(std::integral_constant<int, 2>{});
             four(std::integral_constant<int, 3>{}); four(std::integral_constant<int, 4>{}); four(std::integral_constant<int, 5>{});
@@ -328,10 +328,10 @@ template <> struct Expand<CQ_Q5_K> {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const uint32_t he = h[i] << (7 - 2 * ch), ho = h[i] >> (2 * ch);        // fifth bits 2 ch + 1 | 2 ch in bit 8
-            o[2 * i] = hfma2_bits(((w[i] << 4) & 0x00F000F0u) | ((he << 1) & 0x01000100u) | 0x54005400u, s0, c0);
-            o[2 * i + 1] = hfma2_bits(((w[i] >> 4) & 0x00F000F0u) | (ho & 0x01000100u) | 0x54005400u, s0, c0);
-            o[16 + 2 * i] = hfma2_bits((w[i] & 0x00F000F0u) | (he & 0x01000100u) | 0x54005400u, s1, c1);
-            o[16 + 2 * i + 1] = hfma2_bits(((w[i] >> 8) & 0x00F000F0u) | ((ho >> 1) & 0x01000100u) | 0x54005400u, s1, c1);
+            o[2 * i] = hfma2_bits(and_or<0x00F000F0u>(w[i] << 4, and_or<0x01000100u, 0x54005400u>(he << 1)), s0, c0);
+            o[2 * i + 1] = hfma2_bits(and_or<0x00F000F0u>(w[i] >> 4, and_or<0x01000100u, 0x54005400u>(ho)), s0, c0);
+            o[16 + 2 * i] = hfma2_bits(and_or<0x00F000F0u>(w[i], and_or<0x01000100u, 0x54005400u>(he)), s1, c1);
+            o[16 + 2 * i + 1] = hfma2_bits(and_or<0x00F000F0u>(w[i] >> 8, and_or<0x01000100u, 0x54005400u>(ho >> 1)), s1, c1);
         }
     }
 };
@@ -372,8 +372,8 @@ template <> struct Expand<CQ_Q2_K> {
                 const __half2 cv = __hmul2(sv, __float2half2_rn(-11.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(((q[4 * hf + i] << (8 - 2 * pos)) & 0x03000300u) | 0x44004400u, s2, cv);
-                    o[16 * bb + 8 * hf + 2 * i + 1] = hfma2_bits(((q[4 * hf + i] >> (2 * pos)) & 0x03000300u) | 0x44004400u, s2, cv);
+                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(and_or<0x03000300u, 0x44004400u>(q[4 * hf + i] << (8 - 2 * pos)), s2, cv);
+                    o[16 * bb + 8 * hf + 2 * i + 1] = hfma2_bits(and_or<0x03000300u, 0x44004400u>(q[4 * hf + i] >> (2 * pos)), s2, cv);
                 }
             }
         }
@@ -407,9 +407,9 @@ template <> struct Expand<CQ_Q3_K> {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t u = q[4 * hf + i], h = hm[4 * hf + i];
-                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(((u << (7 - 2 * pos)) & 0x01800180u) | ((h << (9 - b)) & 0x02000200u) | 0x48004800u, sv, cv);
+                    o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(and_or<0x01800180u>(u << (7 - 2 * pos), and_or<0x02000200u, 0x48004800u>(h << (9 - b))), sv, cv);
                     o[16 * bb + 8 * hf + 2 * i + 1] =
-                        hfma2_bits(((u >> (1 + 2 * pos)) & 0x01800180u) | (((h >> 8) << (9 - b)) & 0x02000200u) | 0x48004800u, sv, cv);
+                        hfma2_bits(and_or<0x01800180u>(u >> (1 + 2 * pos), and_or<0x02000200u, 0x48004800u>((h >> 8) << (9 - b))), sv, cv);
                 }
             }
         }

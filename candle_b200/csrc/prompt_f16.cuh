@@ -94,27 +94,25 @@ template <int N> __device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr,
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Bounded wait like wait_or_abort; between two tries the warp sleeps, since fourteen waiting warps that poll took more than half of all issue slots, from the
-// producers above all.  The bound counts tries (2^23 sleeps are about a second): every wait is copied into its place - calls do not go with changed register
+// producers above all.  The votes keep the loop free of divergence, and the expected case falls through.  The bound counts tries (2^23 sleeps are about a second): every wait is copied into its place - calls do not go with changed register
 // budgets - so its code is kept short.
-__device__ __forceinline__ bool wait_slow(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
+// There is no per-lane form: every role goes on to warp-wide instructions, so its warp decides as one whether a wait gave up (lanes
+// that left at different places would meet at different warp-wide instructions, which need not end).
+__device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
+    if (__builtin_expect(__all_sync(0xffffffffu, cq_mbar_try_wait(bar, parity)), 1)) return true;
 #pragma unroll 1
     for (unsigned n = 0; n < (1u << 23); ++n) {
         __nanosleep(64);
-        if (cq_mbar_try_wait(bar, parity)) return true;
-        if ((n & 1023u) == 1023u && *abort_flag) return false;
+        if (__all_sync(0xffffffffu, cq_mbar_try_wait(bar, parity))) return true;
+        if ((n & 1023u) == 1023u && __any_sync(0xffffffffu, *abort_flag)) return false;
     }
     *abort_flag = 1;
     return false;
 }
-// There is no per-lane form: every role goes on to warp-wide instructions, so its warp decides as one whether a wait gave up (lanes
-// that left at different places would meet at different warp-wide instructions, which need not end).
-__device__ __forceinline__ bool wait_warp(uint64_t *bar, unsigned parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, cq_mbar_try_wait(bar, parity) || wait_slow(bar, parity, abort_flag));
-}
 // One arrival per warp: barriers count warps, not threads.
 __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {
     __syncwarp();
-    if (lane == 0) mbar_arrive(bar);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(cq_smem_u32(bar)), "r"(lane) : "memory");
 }
 
 // Register budgets per warpgroup (kernels of 640 threads = 96 registers each at launch, 61,440 in all): the two epilogue
@@ -123,6 +121,23 @@ __device__ __forceinline__ void arrive_warp(uint64_t *bar, int lane) {
 constexpr int kRegsEpi = 128, kRegsProd = 88, kRegsMisc = 48;
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// (x & M) | C and (x & M) ^ C: written in C with two constants they became two instructions each
+template <uint32_t M, uint32_t C> __device__ __forceinline__ uint32_t and_or(uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "n"(M), "n"(C));
+    return r;
+}
+template <uint32_t M, uint32_t C> __device__ __forceinline__ uint32_t and_xor(uint32_t x) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(r) : "r"(x), "n"(M), "n"(C));
+    return r;
+}
+template <uint32_t M> __device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "n"(M), "r"(c));
+    return r;
+}
 
 // two f32 operations per instruction; each half rounds like the scalar operation
 __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {

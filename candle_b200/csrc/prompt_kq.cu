@@ -39,6 +39,12 @@
 // per kind of output, since the code between the loops costs instruction fetches: expert block of 1024 tokens (below) 457 us -> 340, Q8_0 of prompt_b32.cu
 // 77 -> 69; Q4_K 2048 tokens bf16 313 -> 311 (the clocks fall with the power), 512 tokens f32 99 -> 97.
 //
+// Instructions count wherever a hand-off waits for them: nibbles into mantissas by one LOP3 each (two constants written in C became two), waits without
+// divergence, arrivals by predicate: Q4_K 2048 tokens bf16 281 -> 261, 512 tokens f32 95 -> 89, Q6_K 14336 -> 4096, 512 tokens 151 -> 144.
+// Tried on top: scales and minima written by the idle raw warps (no change, Q6_K 148), half a stage expanded at a time in a loop (Q4_K 273, Q6_K 159),
+// row scales stored in pairs (273: 16-byte broadcast reads).  With all of the expansion left out the 2048 tokens still take 243, without the MMAs 249,
+// without the copies 259: what is left are the chains of barrier round trips, none of which bounds it alone.
+//
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
 #include "../../include/candle_q_b200.h"
@@ -303,10 +309,10 @@ template <bool MAP> struct Expand<CQ_Q4_K, MAP> {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const uint32_t u = w[i], v = w[i] >> 8;
-                o[c][2 * i] = hfma2_bits((u & 0x000F000Fu) | 0x64006400u, s0, c0);
-                o[c][2 * i + 1] = hfma2_bits((v & 0x000F000Fu) | 0x64006400u, s0, c0);
-                o[c][16 + 2 * i] = hfma2_bits((u & 0x00F000F0u) | 0x64006400u, m1, c1);
-                o[c][16 + 2 * i + 1] = hfma2_bits((v & 0x00F000F0u) | 0x64006400u, m1, c1);
+                o[c][2 * i] = hfma2_bits(and_or<0x000F000Fu, 0x64006400u>(u), s0, c0);
+                o[c][2 * i + 1] = hfma2_bits(and_or<0x000F000Fu, 0x64006400u>(v), s0, c0);
+                o[c][16 + 2 * i] = hfma2_bits(and_or<0x00F000F0u, 0x64006400u>(u), m1, c1);
+                o[c][16 + 2 * i + 1] = hfma2_bits(and_or<0x00F000F0u, 0x64006400u>(v), m1, c1);
             }
         }
     }
@@ -360,10 +366,10 @@ template <bool MAP> struct Expand<CQ_Q6_K, MAP> {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t l = ql[4 * hf + i], b = qh[4 * hf + i] >> (2 * pp);
-                    const uint32_t c = ((nib ? l >> 4 : l) & 0x0F0F0F0Fu) | ((nib ? b : b << 4) & 0x30303030u);
+                    const uint32_t c = and_or<0x0F0F0F0Fu>(nib ? l >> 4 : l, (nib ? b : b << 4) & 0x30303030u);
 #pragma unroll
                     for (int od = 0; od < 2; ++od) {        // bytes 0, 2 | 1, 3
-                        const __half2 y = __hsub2(bits_h2(((od ? c >> 8 : c) & 0x00FF00FFu) | 0x64006400u), __float2half2_rn(1056.0f));
+                        const __half2 y = __hsub2(bits_h2(and_or<0x00FF00FFu, 0x64006400u>(od ? c >> 8 : c)), __float2half2_rn(1056.0f));
                         const __half2 a = __hsub2(__hfma2(s2, y, __float2half2_rn(12288.0f)), __float2half2_rn(12288.0f));
                         o[nib][8 * hf + 2 * i + od] = h2_bits(a);
                         o[nib][16 + 8 * hf + 2 * i + od] = h2_bits(__hfma2(s2, y, __hneg2(a)));
