@@ -85,7 +85,8 @@ __device__ __forceinline__ void gemv_body(const uint8_t *__restrict__ w, const M
             for (int r = 0; r < RB; ++r) {
                 if (r < nr) {
                     ChunkW<TYPE> cw;
-                    cw.load(srow + r * row_bytes, tid);
+                    if constexpr (B == 1 && (TYPE == CQ_Q3_K || TYPE == CQ_Q6_K || TYPE == CQ_Q8_0)) cw.template load<true>(srow + r * row_bytes, tid);
+                    else cw.load(srow + r * row_bytes, tid);
 #pragma unroll
                     for (int j = 0; j < B; ++j) v[r * B + j] = cw.template dot<ACT>(act[j]);
                 }

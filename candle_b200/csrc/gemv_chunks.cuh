@@ -221,10 +221,10 @@ template <> struct ChunkW<CQ_Q5_1> : ChunkW32<CQ_Q5_1> {};
 template <> struct ChunkW<CQ_Q8_0> {
     uint32_t q[8];
     float d;
-    __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
+    template <bool SHARED = false> __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
         const uint8_t *b = row + chunk * 34;
         d = __half2float(__ushort_as_half((unsigned short)cq_lds_u16(b)));
-        cq_lds_words<8>(b + 2, q);
+        cq_lds_words<8, SHARED>(b + 2, q);
     }
     __device__ __forceinline__ int idot(const ChunkAct<CQ_Q8_0> &a) const {
         int s = 0;
@@ -445,12 +445,12 @@ template <> struct ChunkW<CQ_Q3_K> {
     uint32_t q[4][4];   // [position][word], signed bytes -4..3
     float d;
     int sc[4];
-    __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
+    template <bool SHARED = false> __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
         const int sb = chunk >> 2, n = (chunk >> 1) & 1, h = chunk & 1;
         const uint8_t *b = row + sb * 110;
         uint32_t ql[4], hm[4];
-        cq_lds_words<4>(b + 32 + 32 * n + 16 * h, ql);
-        cq_lds_words<4>(b + 16 * h, hm);
+        cq_lds_words<4, SHARED>(b + 32 + 32 * n + 16 * h, ql);
+        cq_lds_words<4, SHARED>(b + 16 * h, hm);
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
 #pragma unroll
@@ -490,13 +490,13 @@ template <> struct ChunkW<CQ_Q6_K> {
     uint32_t q[4][4];   // [position][word], unsigned 6-bit values
     float d;
     int sc[4];
-    __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
+    template <bool SHARED = false> __device__ __forceinline__ void load(const uint8_t *row, int chunk) {
         const int sb = chunk >> 2, n = (chunk >> 1) & 1, h = chunk & 1;
         const uint8_t *b = row + sb * 210;
         uint32_t la[4], lb[4], hh[4];
-        cq_lds_words<4>(b + 64 * n + 16 * h, la);
-        cq_lds_words<4>(b + 64 * n + 32 + 16 * h, lb);
-        cq_lds_words<4>(b + 128 + 32 * n + 16 * h, hh);
+        cq_lds_words<4, SHARED>(b + 64 * n + 16 * h, la);
+        cq_lds_words<4, SHARED>(b + 64 * n + 32 + 16 * h, lb);
+        cq_lds_words<4, SHARED>(b + 128 + 32 * n + 16 * h, hh);
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             q[0][w] = (la[w] & 0x0F0F0F0Fu) | ((hh[w] << 4) & 0x30303030u);

@@ -344,14 +344,14 @@ template <> struct Expand<CQ_Q2_K> {
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;         // a multiple of 4 when the base is, else of 2
         uint32_t dm[1];
-        cq_lds_words<1>(p + 80, dm);
+        cq_lds_words<1, true>(p + 80, dm);
         d = h16(dm[0]); dmin = h16(dm[0] >> 16);
     }
     __device__ __forceinline__ void scales(float *dst) const { *dst = __fmul_rn(0.5f, d); }
     __device__ __forceinline__ void coef(uint8_t *row) const {
         const float d15 = __fmul_rn(1.5f, d);
         uint32_t sc[4];
-        cq_lds_words<4>(p, sc);
+        cq_lds_words<4, true>(p, sc);
         auto c = [&](int j) {
             const uint32_t by = (sc[j >> 2] >> (8 * (j & 3))) & 0xFFu;
             return __fmaf_rn(-dmin, (float)(by >> 4), __fmul_rn(d15, (float)(by & 0xFu)));
@@ -361,8 +361,8 @@ template <> struct Expand<CQ_Q2_K> {
     }
     __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
         uint32_t q[8], sc[1];
-        cq_lds_words<8>(p + 16 + 32 * (ch >> 1), q);
-        cq_lds_words<1>(p + 4 * ch, sc);
+        cq_lds_words<8, true>(p + 16 + 32 * (ch >> 1), q);
+        cq_lds_words<1, true>(p + 4 * ch, sc);
 #pragma unroll
         for (int bb = 0; bb < 2; ++bb) {
             const int pos = 2 * (ch & 1) + bb;
@@ -385,14 +385,14 @@ template <> struct Expand<CQ_Q3_K> {
     uint32_t sc[3];
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;         // even
-        cq_lds_words<3>(p + 96, sc);
+        cq_lds_words<3, true>(p + 96, sc);
     }
     __device__ __forceinline__ void scales(float *dst) const { *dst = __half2float(*reinterpret_cast<const __half *>(p + 108)); }
     __device__ __forceinline__ void coef(uint8_t *) const {}
     __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
         uint32_t q[8], hm[8];
-        cq_lds_words<8>(p + 32 + 32 * (ch >> 1), q);
-        cq_lds_words<8>(p, hm);
+        cq_lds_words<8, true>(p + 32 + 32 * (ch >> 1), q);
+        cq_lds_words<8, true>(p, hm);
         // scale number j = 4 ch + 2 bb + half: 4 low bits from bytes 0-7, 2 high bits from bytes 8-11
         const uint32_t scl = (ch & 1 ? sc[1] : sc[0]) >> (ch & 2 ? 4 : 0), sch = sc[2] >> (2 * ch);
 #pragma unroll
@@ -764,10 +764,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
 #pragma unroll
             for (int j = 0; j < N8; ++j) {
                 const uint64_t v[4] = {acc[2 * j], acc[2 * j + 1], acc[2 * N8 + 2 * j], acc[2 * N8 + 2 * j + 1]};       // rows r0 + 8 i
-                if constexpr (STORE == kStore16) {
-                    const int col = 8 * j + (lane >> 2), row = (warp & 3) * 32;
-                    store_rows32_16bit(v, a.out_kind, (uint16_t *)a.out + base + (int64_t)col * a.stride_out + row, col < left ? a.nrows - cx.row0 - row : 0,
-                                       ((a.stride_out & 7) | ((uintptr_t)a.out & 15)) == 0);
+                if constexpr (STORE == kStore16 || STORE == kStore16Any) {
+                    const int row = (warp & 3) * 32;
+                    uint16_t *dst = (uint16_t *)a.out + base + (int64_t)(8 * j) * a.stride_out + row;
+                    if constexpr (STORE == kStore16) store_rows32_wide(v, a.out_kind, dst, a.stride_out, a.nrows - cx.row0 - row, left - 8 * j);
+                    else store_rows32_any(v, a.out_kind, dst, a.stride_out, a.nrows - cx.row0 - row, left - 8 * j);
                 } else {
                     const int col = 8 * j + csub;
                     float *o = (float *)a.out + base + (int64_t)col * a.stride_out + r0;
@@ -829,9 +830,12 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
     if (elem == CQ_F32) {
         if (tl.tt <= 32) launch_kernel<WTYPE, kStoreF32, 2>(grid, st, map, a, tl);
         else launch_kernel<WTYPE, kStoreF32, 4>(grid, st, map, a, tl);
-    } else {
+    } else if (rows_16_bytes_apart(dst, stride_dst) && n % 8 == 0) {
         if (tl.tt <= 32) launch_kernel<WTYPE, kStore16, 2>(grid, st, map, a, tl);
         else launch_kernel<WTYPE, kStore16, 4>(grid, st, map, a, tl);
+    } else {
+        if (tl.tt <= 32) launch_kernel<WTYPE, kStore16Any, 2>(grid, st, map, a, tl);
+        else launch_kernel<WTYPE, kStore16Any, 4>(grid, st, map, a, tl);
     }
     return true;
 }

@@ -199,20 +199,20 @@ __device__ __forceinline__ uint4 pack_q8(const int (&q)[8]) {
 }
 
 // Eight tokens x 32 weight rows of a warp as a 16-bit kind: v[i] are a thread's values of row 8 i + lane / 4, tokens 2 (lane % 4) and the next (the 16x256b
-// layout).  8 x 8 transposes leave a thread with rows 8 i + 2 (lane % 4), + 1 of token lane / 4, a 4 x 4 transpose over four lanes with eight rows of it, so a
-// token's 32 rows go out as 64 contiguous bytes.  (Stored as they lie, in 16-byte pieces of half a sector, the 2048 x 14336 outputs of a bf16 prompt took
-// 25 us more than twice the bytes as f32.)  `dst`: row 0 of this thread's token; `rows`: how many of the 32 are stored, 0 for a token that is none; `wide`: dst is
-// 16-byte aligned.
-__device__ __forceinline__ void store_rows32_16bit(const uint64_t (&v)[4], int kind, uint16_t *dst, int rows, bool wide) {
+// layout).  `dst`: row 0 of the first token; `rows`: how many of the 32 are stored; `tokens`: how many of the eight.
+__device__ __forceinline__ uint32_t pair_16bit(uint64_t v, int kind) {
+    if (kind == CQ_F16) return h2_bits(__halves2half2(__float2half(lo2(v)), __float2half(hi2(v))));
+    const __nv_bfloat162 b = __halves2bfloat162(__float2bfloat16(lo2(v)), __float2bfloat16(hi2(v)));
+    return *reinterpret_cast<const uint32_t *>(&b);
+}
+// Rows a multiple of 16 bytes apart: 8 x 8 transposes leave a thread with rows 8 i + 2 (lane % 4), + 1 of token lane / 4, a 4 x 4 transpose over four lanes with
+// eight rows of it, so a token's 32 rows go out as 64 contiguous bytes.  (Stored as they lie, in 16-byte pieces of half a sector, the 2048 x 14336
+// outputs of a bf16 prompt took 25 us more than twice the bytes as f32.)
+__device__ __forceinline__ void store_rows32_wide(const uint64_t (&v)[4], int kind, uint16_t *dst, int64_t stride, int rows, int tokens) {
     const int lane = threadIdx.x & 31;
     uint32_t r[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t w;
-        if (kind == CQ_F16) w = h2_bits(__halves2half2(__float2half(lo2(v[i])), __float2half(hi2(v[i]))));
-        else { const __nv_bfloat162 b = __halves2bfloat162(__float2bfloat16(lo2(v[i])), __float2bfloat16(hi2(v[i]))); w = *reinterpret_cast<const uint32_t *>(&b); }
-        asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r[i]) : "r"(w));
-    }
+    for (int i = 0; i < 4; ++i) asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r[i]) : "r"(pair_16bit(v[i], kind)));
 #pragma unroll
     for (int m = 1; m < 4; m <<= 1) {           // swap bit log2 m of the register number with that of the lane
         const bool up = lane & m;
@@ -223,19 +223,31 @@ __device__ __forceinline__ void store_rows32_16bit(const uint64_t (&v)[4], int k
                 if (up) r[i] = got; else r[i | m] = got;
             }
     }
-    dst += 8 * (lane & 3);
-    rows -= 8 * (lane & 3);
-    if (wide && rows >= 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(r[0], r[1], r[2], r[3]);
-    else {
+    const int row = 8 * (lane & 3), tok = lane >> 2;
+    if (row < rows && tok < tokens) *reinterpret_cast<uint4 *>(dst + tok * stride + row) = make_uint4(r[0], r[1], r[2], r[3]);     // rows: a multiple of eight
+}
+// Any distance: a lane per row, so that a token's rows go out as one run.  (Pieces of two bytes after the transposes above: 4 x the sectors, Q4_K
+// 6144 -> 12108, 320 tokens f16 83 us; this 70.)
+__device__ __forceinline__ void store_rows32_any(const uint64_t (&v)[4], int kind, uint16_t *dst, int64_t stride, int rows, int tokens) {
+    const int lane = threadIdx.x & 31;
+    uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < rows) dst[i] = (uint16_t)(r[i >> 1] >> (16 * (i & 1)));
+    for (int i = 0; i < 4; ++i) w[i] = pair_16bit(v[i], kind);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {               // tokens 2 c and 2 c + 1 of row `lane`
+        uint32_t got[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) got[i] = __shfl_sync(0xffffffffu, w[i], 4 * (lane & 7) + c);
+        const uint32_t x = lane & 16 ? (lane & 8 ? got[3] : got[2]) : (lane & 8 ? got[1] : got[0]);
+        if (lane < rows && 2 * c < tokens) dst[2 * c * stride + lane] = (uint16_t)x;
+        if (lane < rows && 2 * c + 1 < tokens) dst[(2 * c + 1) * stride + lane] = (uint16_t)(x >> 16);
     }
 }
 
 // What a kernel stores, one instantiation each (the code of the others between the loops of a tile costs them 5 - 10 % in instruction fetches):
-// f32 or 16-bit rows of tokens, or f32 rows of (token, expert) pairs.
-enum { kStoreF32, kStore16, kStorePairs };
+// f32 or 16-bit rows of tokens (a multiple of 16 bytes apart, or not), or f32 rows of (token, expert) pairs.
+enum { kStoreF32, kStore16, kStore16Any, kStorePairs };
+inline bool rows_16_bytes_apart(const void *out, int stride) { return ((uintptr_t)out & 15) == 0 && stride % 8 == 0; }
 
 // ---- tiles --------------------------------------------------------------------------------------------------
 // The jobs of a grouped (expert-indexed) launch; null `tiles` = dense.

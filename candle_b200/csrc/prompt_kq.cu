@@ -328,12 +328,12 @@ template <bool MAP> struct Expand<CQ_Q6_K, MAP> {
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
         p = rr + shift;
         off = shift;
-        cq_lds_words<4>(p + 192, sc);
+        cq_lds_words<4, true>(p + 192, sc);
     }
     // 32 bytes from an even address.  Eight words read one by one are four-way bank conflicts, whatever the pitch of the rows, a multiple of 16; three
     // 16-byte reads are none.  Where all rows have the same distance to a 16-byte boundary the words they leave are picked by a uniform branch.
     __device__ __forceinline__ void words32(const uint8_t *a, uint32_t (&o)[8]) const {
-        if constexpr (!MAP) cq_lds_words<8>(a, o);
+        if constexpr (!MAP) cq_lds_words<8, true>(a, o);
         else {
             const uint4 *v = reinterpret_cast<const uint4 *>(a - off);
             const uint4 x = v[0], y = v[1], z = v[2];
@@ -739,10 +739,11 @@ prompt_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ 
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint64_t v[4] = {acc[q][2 * j], acc[q][2 * j + 1], acc[q][8 + 2 * j], acc[q][9 + 2 * j]};       // rows r0 + 8 i
-                    if constexpr (STORE == kStore16) {
-                        const int col = 32 * q + 8 * j + (lane >> 2), row = (warp & 3) * 32;
-                        store_rows32_16bit(v, a.out_kind, (uint16_t *)out + base + (int64_t)col * a.stride_out + row, col < left ? a.nrows - cx.row0 - row : 0,
-                                           ((a.stride_out & 7) | ((uintptr_t)out & 15)) == 0);
+                    if constexpr (STORE == kStore16 || STORE == kStore16Any) {
+                        const int col = 32 * q + 8 * j, row = (warp & 3) * 32;
+                        uint16_t *dst = (uint16_t *)out + base + (int64_t)col * a.stride_out + row;
+                        if constexpr (STORE == kStore16) store_rows32_wide(v, a.out_kind, dst, a.stride_out, a.nrows - cx.row0 - row, left - col);
+                        else store_rows32_any(v, a.out_kind, dst, a.stride_out, a.nrows - cx.row0 - row, left - col);
                     } else {
                         const int col = 32 * q + 8 * j + csub;
                         float *o0 = (float *)out + base + (int64_t)col * a.stride_out + r0, *o1 = o0 + a.stride_out;
@@ -816,8 +817,11 @@ bool launch_gemm(const void *w, const void *act, void *out, int out_elem, int k,
         if (gi.tiles) launch_kernel<WTYPE, kStorePairs, 0, M>(grid, st, map, map2, a, tl, gi);
         else if (out_elem == CQ_F32 && tl.tt <= 64) launch_kernel<WTYPE, kStoreF32, 1, M>(grid, st, map, map2, a, tl, gi);
         else if (out_elem == CQ_F32) launch_kernel<WTYPE, kStoreF32, 2, M>(grid, st, map, map2, a, tl, gi);
-        else if (tl.tt <= 64) launch_kernel<WTYPE, kStore16, 1, M>(grid, st, map, map2, a, tl, gi);
-        else launch_kernel<WTYPE, kStore16, 2, M>(grid, st, map, map2, a, tl, gi);
+        else if (rows_16_bytes_apart(out, stride_out) && n % 8 == 0) {
+            if (tl.tt <= 64) launch_kernel<WTYPE, kStore16, 1, M>(grid, st, map, map2, a, tl, gi);
+            else launch_kernel<WTYPE, kStore16, 2, M>(grid, st, map, map2, a, tl, gi);
+        } else if (tl.tt <= 64) launch_kernel<WTYPE, kStore16Any, 1, M>(grid, st, map, map2, a, tl, gi);
+        else launch_kernel<WTYPE, kStore16Any, 2, M>(grid, st, map, map2, a, tl, gi);
     };
     if (use_map) run(std::true_type{});
     else run(std::false_type{});

@@ -307,3 +307,27 @@ def test_addresses_the_prompt_kernels_do_not_take_are_refused(lib, oracle, cuda_
         with pytest.raises(capi.CandleQError, match="aligned"):
             mm.forward(torch.from_numpy(x).to(cuda_dev))
         lib.cq_clear_status()
+
+
+@pytest.mark.parametrize("wtype", [GgmlDType.Q4K, GgmlDType.Q6K, GgmlDType.Q8_0])
+@pytest.mark.parametrize("n,pad,offset,tokens", [(136, 0, 0, 75), (136, 8, 0, 130), (136, 4, 0, 33), (136, 0, 1, 20), (129, 0, 0, 70), (135, 1, 0, 17), (8, 0, 0, 9), (260, 0, 0, 131)])
+def test_16_bit_rows_at_any_distance(cuda_dev, wtype, n, pad, offset, tokens):
+    """Rows of 16-bit outputs a multiple of 16 bytes apart (stored by eight) or not (a lane per row), ragged in rows and tokens: the f32 outputs
+    rounded, and nothing between the rows."""
+    from candle_b200.synth import random_blocks
+    L, st, k, big = capi.lib(), torch.cuda.current_stream().cuda_stream, 512, wtype in (GgmlDType.Q4K, GgmlDType.Q6K)
+    w = random_blocks(wtype, n, k, seed=n, device=cuda_dev)
+    need = L.cq_prompt_scratch_bytes(tokens, k) if big else L.cq_prompt32_scratch_bytes(int(wtype), tokens, k)
+    scratch = torch.empty(need, dtype=torch.uint8, device=cuda_dev)
+    matmul = L.cq_prompt_matmul if big else L.cq_prompt32_matmul
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(tokens, k, device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(1)).to(dtype)
+        out = []
+        for xs in (x.float(), x):
+            buf = torch.full((tokens * (n + pad) + 16,), -7.0, dtype=xs.dtype, device=cuda_dev)
+            matmul(int(wtype), w.data_ptr(), xs.data_ptr(), ELEM[xs.dtype], buf[offset:].data_ptr(), scratch.data_ptr(), k, n, tokens, n + pad, st)
+            capi.check("prompt")
+            rows = buf[offset:offset + tokens * (n + pad)].view(tokens, n + pad)
+            assert bool((rows[:, n:] == -7.0).all()) and bool((buf[:offset] == -7.0).all()) and bool((buf[offset + tokens * (n + pad):] == -7.0).all())
+            out.append(rows[:, :n])
+        assert torch.equal(out[0].to(dtype), out[1])
