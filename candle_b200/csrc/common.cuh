@@ -240,7 +240,8 @@ __device__ __forceinline__ bool cq_mbar_wait_bounded(uint64_t *bar, unsigned par
 // Read NW consecutive 32-bit words that start at a 2-byte-aligned shared-memory address.
 // Reads one aligned word past the last one (callers keep 4 bytes of slack).
 // SHARED: the aligned address by pointer arithmetic instead of rounding, so that the compiler knows these for shared-memory loads.  The faster form in the
-// prompt kernels, and for one row of activations with Q3_K, Q6_K and Q8_0 (Q6_K 4096 -> 128256 72.0 us -> 68.8, 14336 -> 4096 14.1 -> 13.0); with more rows, or
+// prompt kernels, in the tensor-core decode kernels (Q6_K, eight rows 4096 -> 18944 26.9 us -> 25.2, 4096 -> 128256 153 -> 144), and for one row of activations
+// with Q3_K, Q6_K and Q8_0 (Q6_K 4096 -> 128256 72.0 us -> 68.8, 14336 -> 4096 14.1 -> 13.0); in the dp4a kernels with more rows, or
 // Q4_0, Q4_1 and Q5_1, some shapes get slower (Q3_K 5632 -> 6016, three rows 16.9 -> 19.4; Q4_0, eight rows 25.6 -> 31.7).
 template <int NW, bool SHARED = false> __device__ __forceinline__ void cq_lds_words(const uint8_t *p, uint32_t (&out)[NW]) {
     const uintptr_t a = (uintptr_t)p;

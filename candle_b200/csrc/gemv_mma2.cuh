@@ -116,8 +116,8 @@ template <> struct Unit<CQ_Q8_0> {
         for (int j = 0; j < 4; ++j) {
             const uint8_t *b0 = r0 + j * 34, *b1 = r1 + j * 34;
             uint32_t q0[2], q1[2];
-            cq_lds_words<2>(b0 + 2 + 8 * t, q0);
-            cq_lds_words<2>(b1 + 2 + 8 * t, q1);
+            cq_lds_words<2, true>(b0 + 2 + 8 * t, q0);
+            cq_lds_words<2, true>(b1 + 2 + 8 * t, q1);
             const uint2 bb = *reinterpret_cast<const uint2 *>(ap + j * 256);
             int c4[4];
             mma_k32(c4, q0[0], q1[0], q0[1], q1[1], bb.x, bb.y);
@@ -144,7 +144,7 @@ template <> struct Unit<CQ_Q6_K> {
         float dW[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            cq_lds_words<4>(bb[r] + 192, scw[r]);
+            cq_lds_words<4, true>(bb[r] + 192, scw[r]);
             dW[r] = __half2float(__ushort_as_half((unsigned short)cq_lds_u16(bb[r] + 208)));
         }
         const uint8_t *ap = aq + g * 32 + 4 * t;        // column g, k = 4t .. 4t+3 of a 16-element half
@@ -155,9 +155,9 @@ template <> struct Unit<CQ_Q6_K> {
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 uint32_t la[1], lb[1], hh[1];
-                cq_lds_words<1>(bb[r] + 64 * n + 16 * h + 4 * t, la);
-                cq_lds_words<1>(bb[r] + 64 * n + 32 + 16 * h + 4 * t, lb);
-                cq_lds_words<1>(bb[r] + 128 + 32 * n + 16 * h + 4 * t, hh);
+                cq_lds_words<1, true>(bb[r] + 64 * n + 16 * h + 4 * t, la);
+                cq_lds_words<1, true>(bb[r] + 64 * n + 32 + 16 * h + 4 * t, lb);
+                cq_lds_words<1, true>(bb[r] + 128 + 32 * n + 16 * h + 4 * t, hh);
                 q[r][0] = center((la[0] & 0x0F0F0F0Fu) | ((hh[0] << 4) & 0x30303030u));
                 q[r][1] = center((lb[0] & 0x0F0F0F0Fu) | ((hh[0] << 2) & 0x30303030u));
                 q[r][2] = center(((la[0] >> 4) & 0x0F0F0F0Fu) | (hh[0] & 0x30303030u));
