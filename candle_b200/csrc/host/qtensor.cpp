@@ -207,10 +207,17 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     // decode launch where that is the faster, and not in the CPU-exact mode).  K must be a whole number of 256-element stages.
     const bool plain32 = dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0;
     const bool q8_1_only = !plain32 && dtype_ != GgmlDType::Q4K && dtype_ != GgmlDType::Q6K;
+    const bool old_sums = q8_1_only && x_dtype == DType::BF16;       // bf16 results keep their bits (prompt_b32_bf16.cu)
     const bool any_address = dtype_ == GgmlDType::Q2K || dtype_ == GgmlDType::Q3K;
     if (k % 256 == 0 && ((plain32 && rows > kPrefillMinRows) ||
                          (q8_1_only && rows > MMVQ_MAX_BATCH && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0) &&
-                          cq_prompt32_pays((int)dtype_, (int)rows, (int)k, (int)n)))) {
+                          (old_sums ? cq_prompt32_bf16_pays : cq_prompt32_pays)((int)dtype_, (int)rows, (int)k, (int)n)))) {
+        if (old_sums) {
+            uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt32_bf16_scratch_bytes((int)dtype_, (int)rows, (int)k));
+            cq_prompt32_bf16_matmul((int)dtype_, ptr_, x, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
+            lib_check("qmatmul prefill (scales per 32, bf16)");
+            return;
+        }
         uint8_t *scratch = (uint8_t *)workspace_ensure(device_, cq_prompt32_scratch_bytes((int)dtype_, (int)rows, (int)k));
         cq_prompt32_matmul((int)dtype_, ptr_, x, (int)x_dtype, out, scratch, (int)k, (int)n, (int)rows, (int)n, stream);
         lib_check("qmatmul prefill (scales per 32)");

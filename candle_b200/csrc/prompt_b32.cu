@@ -907,5 +907,6 @@ extern "C" int cq_prompt32_timeout_flag(void) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_prompt_b32_timeout_flag, sizeof v) != cudaSuccess) { (void)cudaGetLastError(); return -1; }
     if (v) cq_set_status(CQ_ERR_TIMEOUT, "prompt32 matmul: a bounded wait gave up");
-    return v;
+    const int bf16 = cq_prompt32_bf16_timeout_flag();
+    return v ? v : bf16;
 }

@@ -331,3 +331,18 @@ def test_16_bit_rows_at_any_distance(cuda_dev, wtype, n, pad, offset, tokens):
             assert bool((rows[:, n:] == -7.0).all()) and bool((buf[:offset] == -7.0).all()) and bool((buf[offset + tokens * (n + pad):] == -7.0).all())
             out.append(rows[:, :n])
         assert torch.equal(out[0].to(dtype), out[1])
+
+
+@pytest.mark.parametrize("wtype", [3, 6, 7, 10, 11, 13])
+@pytest.mark.parametrize("tokens,k,n", [(16, 256, 128), (17, 768, 129), (75, 1280, 200), (130, 512, 300)])
+def test_prompt32_bf16_results_are_neighbours(lib, oracle, cuda_dev, wtype, tokens, k, n):
+    """The bf16 summation against the f32 sums of cq_prompt32_matmul, both within 1e-6 of the sums' 2-norm: a bf16 result is the rounded f32 one or its
+    neighbour (2^-7 of the value at most), and hardly ever the latter (an interval of 4e-6 around boundaries 2^-8 apart, for small sums more)."""
+    _, x, wq = make_case(oracle, wtype, k, n, tokens, seed=wtype)
+    w_dev, xb = torch.from_numpy(wq).to(cuda_dev), torch.from_numpy(x).to(cuda_dev).to(torch.bfloat16)
+    matmul = lambda t, wp, xp, _elem, out, scratch, kk, nn, m, stride, st: lib.cq_prompt32_bf16_matmul(t, wp, xp, out, scratch, kk, nn, m, stride, st)
+    out = _run(lib.cq_prompt32_bf16_scratch_bytes(wtype, tokens, k), matmul, lib.cq_prompt32_timeout_flag, wtype, w_dev, xb, k, n).float()
+    ref = _prompt32(lib, wtype, w_dev, xb.float(), k, n)
+    slack = 4e-6 * float(ref.norm() / ref.numel() ** 0.5)
+    assert bool(((out - ref.to(torch.bfloat16).float()).abs() <= 2.0 ** -7 * ref.abs() + slack).all())
+    assert float((out != ref.to(torch.bfloat16).float()).float().mean()) <= 0.01
