@@ -418,6 +418,9 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *__restrict__ 
     __shared__ float val[32], all_val[kArgmaxCtas];
     __shared__ int idx[32], all_idx[kArgmaxCtas];
     const int rank = (int)blockIdx.x % kArgmaxCtas, row = (int)blockIdx.x / kArgmaxCtas, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // A CTA's shared memory may be written by another only once it runs: every CTA says so here and waits for the others before it writes, with the
+    // loads of the row in between.
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     cq_pdl_launch_dependents();
     cq_pdl_wait();
     const float *xr = x + (size_t)row * n;
@@ -437,6 +440,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *__restrict__ 
     nan = __syncthreads_or(nan);
     if (lane == 0) { val[warp] = v; idx[warp] = at; }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (warp == 0) {
         v = val[lane]; at = idx[lane];
         warp_best();

@@ -157,3 +157,19 @@ def test_grouped_route_of_q6_k_takes_the_faster_kernel(lib):
     for shape, slow, fast in f16:
         assert fast < slow and lib.cq_moe_prompt_pays(14, *shape) == 1, shape
     assert lib.cq_moe_prompt_pays(12, 64, 2, 256) == 1
+
+
+def test_shared_memory_of_another_cta_is_written_after_a_cluster_barrier():
+    """Distributed shared memory may be written only once the CTA it belongs to runs: in every kernel the first remote address is made after a wait at
+    the cluster's barrier (spelled out, or cluster_sync_all)."""
+    import glob
+    import os
+    import re
+    found = 0
+    for path in glob.glob(os.path.join(os.path.dirname(capi.__file__), "csrc", "*.cu*")):
+        for body in re.sub(r"//[^\n]*", "", open(path).read()).split("\n}\n"):      # one function each
+            remote = re.search(r"cluster_map\(|mapa\.shared::cluster", body)
+            if remote and "cluster_map(uint32_t" not in body:
+                found += 1
+                assert re.search(r"barrier\.cluster\.wait|cluster_sync_all\(\)", body[:remote.start()]), (path, body[:80])
+    assert found >= 2
