@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *__restrict__ 
         pairs[2 * row] = nan ? NAN : v;
         pairs[2 * row + 1] = nan ? (float)((1LL << 40) + start) : (float)(at + start);
     }
-    if (tokens) tokens[row] = nan ? INT64_MAX : (long long)(float)(at + start);
+    if (tokens) tokens[row] = nan ? INT64_MAX : at + start;
 }
 
 }  // namespace

@@ -328,6 +328,16 @@ def test_argmax_is_the_first_maximum(lib, cuda_dev, rows, n):
     assert torch.equal(tokens[ok], first[ok]) and bool((tokens[~ok] == 2 ** 63 - 1).all())
 
 
+def test_argmax_tokens_are_exact_past_the_integers_of_f32(lib, cuda_dev):
+    """Tokens are index + start as integers; only the pairs, which ranks exchange, are floats."""
+    x, start = torch.zeros((2, 9001), device=cuda_dev), 2 ** 24 - 7
+    x[0, 4], x[1, 9000] = 1.0, 1.0            # 2^24 - 3 and, odd and above 2^24, 2^24 + 8993
+    tokens = torch.empty(2, dtype=torch.int64, device=cuda_dev)
+    lib.cq_argmax_f32(x.data_ptr(), 2, 9001, start, None, tokens.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    capi.check("argmax")
+    assert tokens.tolist() == [start + 4, start + 9000]
+
+
 def test_graph_decode_equals_eager_decode(cuda_dev):
     cfg = DecoderConfig.tiny()
     prompt = torch.randint(0, cfg.vocab, (2, 24), device=cuda_dev, generator=torch.Generator(device=cuda_dev).manual_seed(2))
