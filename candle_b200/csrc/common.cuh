@@ -227,6 +227,15 @@ __device__ __forceinline__ bool cq_mbar_try_wait(uint64_t *bar, unsigned parity)
                  : "memory");
     return ok != 0;
 }
+// The same without waiting: a try may suspend the thread for a time of its own, a test returns at once.
+__device__ __forceinline__ bool cq_mbar_test_wait(uint64_t *bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(cq_smem_u32(bar)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
 // Wait for a phase of `bar`, giving up after about a second (2e9 SM cycles).  Returns false on give-up.
 __device__ __forceinline__ bool cq_mbar_wait_bounded(uint64_t *bar, unsigned parity) {
     if (cq_mbar_try_wait(bar, parity)) return true;
