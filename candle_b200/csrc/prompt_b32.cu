@@ -721,8 +721,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 }
                 if (!alive) break;
                 if constexpr (kComp) {
-                    // sum += the chunk, the rounding error of the addition into `low` (fast two-sum: exact unless the chunk is larger than
-                    // the sum before it, and then within one rounding of the chunk's own last bit)
+                    // sum += the chunk, the rounding error of the addition into `low`.  An exact two-sum, but for Q5_K and Q2_K: theirs is the fast one, which
+                    // loses up to a rounding of the chunk where the chunk is larger than the sum before it.  It costs the other formats 1 - 9 % of their
+                    // error (Q5_0, K = 1024, a few large blocks 5.7e-8 -> 6.1e-8); these two stay far below the sums with a minimum added per block (Q5_K
+                    // 6.3e-8 for 8.7e-8, Q2_K 6.0e-8 for 7.2e-8), and three more operations per value are 4 % of the time (Q5_K 254 us -> 267).
+                    constexpr bool kExact = F::kBlockScale || kSums == 0;
                     uint64_t dw[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { const float d = F::kBlockScale ? 1.0f : rw[8 * i]; dw[i] = pack2f(d, d); }
@@ -740,7 +743,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                             uint64_t f = dw[2 * h + (x & 1)], y = acc[x];            // the chunk is f y
                             if constexpr (kSums > 0) { y = fma2(f, y, pack2(v[2 * i], v[2 * i + 1])); f = one; }
                             const uint64_t s1 = fma2(f, y, s0);
-                            low[x] = fma2(one, fma2(f, y, fma2(minus1, s1, s0)), low[x]);
+                            if constexpr (kExact) {
+                                const uint64_t bb = fma2(minus1, s0, s1);
+                                const uint64_t e0 = fma2(minus1, fma2(minus1, bb, s1), s0), e1 = fma2(f, y, bb ^ 0x8000000080000000ull);
+                                low[x] = fma2(one, fma2(one, e0, e1), low[x]);
+                            } else low[x] = fma2(one, fma2(f, y, fma2(minus1, s1, s0)), low[x]);
                             sum[x] = s1;
                             acc[x] = 0ull;
                         }

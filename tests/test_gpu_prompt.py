@@ -261,6 +261,111 @@ def test_prompt32_is_no_further_from_64_bits_than_the_decode_kernel(lib, cuda_de
     assert err(_prompt32(lib, wtype, wq, x, k, n)) <= 1.1 * err(decode)
 
 
+MINIMUM = {3: (0, 2, -7.5), 6: (0, None, 0.0), 7: (0, 2, -15.5), 10: (80, 82, 1.5), 11: (108, None, 0.0), 13: (0, 2, 15.5)}     # where d and the minimum are; the middle of the codes
+
+
+def _weights32(wtype, n, k, minimum, gen, dev):
+    """Random blocks with minima of `minimum` x the middle of the codes (1: weights around zero; -1: all of one sign, 0: none, 8: the minimum is most of a
+    weight), and what they hold, in f64: integers [n, k], scales [n, k / 32] and minima [n, k / 32, 1 or 2]."""
+    per, (at_d, at_m, mid) = 32 if wtype < 10 else 256, MINIMUM[wtype]
+    b = torch.randint(0, 256, (n * k // per, TSIZE[wtype]), dtype=torch.uint8, device=dev, generator=gen)
+
+    def put(b, off, v):
+        b[:, off:off + 2] = v.to(torch.float16).view(torch.uint8).view(-1, 2)
+
+    d = ((torch.rand(b.shape[0], device=dev, generator=gen) * 0.5 + 0.75) * 1e-3).half().float()
+    put(b, at_d, d)
+    if at_m is not None:
+        put(b, at_m, d * mid * minimum)
+
+    def values(d, m):
+        c = b.clone()
+        put(c, at_d, torch.full((b.shape[0],), d, device=dev))
+        if at_m is not None:
+            put(c, at_m, torch.full((b.shape[0],), m, device=dev))
+        return QTensor.from_device_blocks(c.reshape(-1), GgmlDType(wtype), (n, k)).dequantize(torch.float32).double()
+
+    spread = lambda off: b[:, off:off + 2].contiguous().view(torch.float16).double().view(n, -1).repeat_interleave(per // 32, 1)
+    codes, scales = values(1.0, 0.0), spread(at_d)
+    if wtype == 6:          # the codes are unsigned, -16 d is the minimum
+        return b.reshape(n, -1), codes + 16, scales, -16 * scales.unsqueeze(-1)
+    if wtype == 11:
+        return b.reshape(n, -1), codes, scales, torch.zeros((n, k // 32, 1), dtype=torch.float64, device=dev)
+    mins = values(0.0, 1.0)[:, ::16 if wtype == 10 else 32].reshape(n, k // 32, -1)
+    return b.reshape(n, -1), codes, scales, mins * spread(at_m).unsqueeze(-1)
+
+
+def _activations32(lib, wtype, x):
+    """What the quantizer makes of them, in f64: integers [m, k], scales [m, k / 32] and sums [m, k / 32, 1 or 2]."""
+    m, k = x.shape
+    y8 = torch.zeros((m, k // 32, 36), dtype=torch.uint8, device=x.device)
+    lib.cq_quantize_act(x.data_ptr(), capi.F32, y8.data_ptr(), k, k, m, 0, torch.cuda.current_stream().cuda_stream)
+    a = y8.view(-1, 36)
+    d, q = a[:, 0:2].contiguous().view(torch.float16).double().view(m, -1), a[:, 4:].contiguous().view(torch.int8).double().view(m, k)
+    if wtype < 10:
+        return q, d, a[:, 2:4].contiguous().view(torch.float16).double().view(m, -1, 1)
+    return q, d, d.unsqueeze(-1) * q.view(m, k // 32, 2 if wtype == 10 else 1, -1).sum(-1)
+
+
+def _plain_sums(wtype, codes, scales, mins, q, d, sums):
+    """The sums with a minimum added per block, in f32 (operations on f64 values, rounded; products of two f32 are exact in f64): the blocks of 256 elements one
+    after the other, the 256s by a two-sum.  Also the exact result."""
+    r = lambda v: v.float().double()
+    m, n, nb = q.shape[0], codes.shape[0], d.shape[1]
+    total, low, acc, exact = (torch.zeros((m, n), dtype=torch.float64, device=q.device) for _ in range(4))
+    for b in range(nb):
+        i = q[:, 32 * b:32 * b + 32] @ codes[:, 32 * b:32 * b + 32].t()
+        dd, dw, terms = d[:, b:b + 1], scales[None, :, b], [sums[:, b, h:h + 1] * mins[None, :, b, h] for h in range(mins.shape[2])]
+        exact += dd * dw * i + sum(terms)
+        if wtype in (11, 13):
+            acc = r(dd * r(dw * i) + acc)
+            if wtype == 13:
+                acc = r(terms[0] + acc)
+        else:
+            v = r(terms[0])
+            if wtype == 10:
+                v = r(terms[1] + v)
+            acc = r(r(dd * dw * i + v) + acc)
+        if b % 8 == 7:
+            s1 = r(total + acc)
+            bb = r(s1 - total)
+            low = r(low + r(r(total - r(s1 - bb)) + r(acc - bb)))
+            total, acc = s1, torch.zeros_like(acc)
+    return r(total + low).float(), exact
+
+
+def _inputs32(kind, m, k, gen, dev):
+    x = torch.randn(m, k, device=dev, generator=gen)
+    if kind != "normal":
+        x = x.abs()
+    if kind == "one sign, a few large":
+        x.view(m, -1, 32)[:, torch.randperm(k // 32, device=dev, generator=gen)[:k // 1024]] *= 50
+    return x
+
+
+@pytest.mark.parametrize("kind", ["normal", "one sign", "one sign, a few large"])
+@pytest.mark.parametrize("tokens,k,n", [(9, 1024, 65), (33, 1280, 14336)])
+@pytest.mark.parametrize("wtype", [3, 7])
+def test_prompt32_sums_of_the_formats_with_a_minimum_per_block(lib, cuda_dev, wtype, tokens, k, n, kind):
+    """Q4_1 and Q5_1, bit for bit: the chunks meet in an exact two-sum, whichever is the larger."""
+    gen = torch.Generator(device=cuda_dev).manual_seed(k)
+    wq, *parts = _weights32(wtype, n, k, 1.0, gen, cuda_dev)
+    x = _inputs32(kind, tokens, k, gen, cuda_dev)
+    assert torch.equal(_prompt32(lib, wtype, wq, x, k, n), _plain_sums(wtype, *parts, *_activations32(lib, wtype, x))[0])
+
+
+@pytest.mark.parametrize("k", [1024, 4096])
+@pytest.mark.parametrize("wtype", [6, 11])
+def test_prompt32_is_no_further_from_64_bits_than_sums_per_block_where_chunks_differ(lib, cuda_dev, wtype, k):
+    """The other formats with an exact two-sum.  3 % for the noise of 16384 values' errors."""
+    gen = torch.Generator(device=cuda_dev).manual_seed(k)
+    wq, *parts = _weights32(wtype, 256, k, 1.0, gen, cuda_dev)
+    x = _inputs32("one sign, a few large", 64, k, gen, cuda_dev)
+    plain, exact = _plain_sums(wtype, *parts, *_activations32(lib, wtype, x))
+    err = lambda o: float((o.double() - exact).norm() / exact.norm())
+    assert err(_prompt32(lib, wtype, wq, x, k, 256)) <= 1.03 * err(plain) <= 1e-6
+
+
 @pytest.mark.parametrize("wtype,rows,k,n", [(3, 200, 768, 700), (6, 200, 768, 700), (7, 200, 768, 700), (10, 200, 768, 700), (11, 200, 768, 700), (13, 200, 768, 700),
                                             (3, 40, 5120, 64), (13, 36, 5120, 64)])
 def test_qmatmul_runs_the_kernel_the_rule_names(lib, oracle, cuda_dev, wtype, rows, k, n):
