@@ -12,11 +12,15 @@
 //     what the shift and the minimum contribute together is a sum over a chunk of (coefficient of the weights) x (sum of the activations):
 //         Q5_K  sum_g (16 d sc_g - dmin m_g) s_g     Q2_K  sum_j (1.5 d sc_j - dmin m_j) s_j, per 16 elements     Q5_0  sum_g -16 d_g (t_g - s_g)
 //     with s = d_a sum q8 and t the f16 sum of the inputs that Q8_1 stores.  Coefficients and sums are f32; each is split exactly into three
-//     bf16 parts, and the six products of parts down to 2^-16 are K steps of the tensor core into an accumulator of their own, the small
-//     ones first.  The large parts of d q and the minimum cancel in the coefficient and not in sums of thousands, so these formats are
-//     nearer to 64 bits than with f32 additions of both per block (2-norm, K = 4096, normal / one-signed activations: Q5_K 1.0e-7 / 2.9e-7, now
-//     6.5e-8 / 1.2e-7; Q2_K 7.8e-8 / 1.8e-7, now 6.0e-8 / 6.1e-8).  Not for Q4_1 and Q5_1, whose sum can be most of the result: the tensor core
-//     cuts off where an f32 addition rounds (3.7e-7 for 6.6e-8), so their codes stay unsigned and a block's two parts meet in the epilogue.
+//     bf16 parts, hi, mid and lo, and the six products of parts down to 2^-16 are K steps of the tensor core.  It cuts sums off where an f32 addition
+//     rounds, a bias that adds up over the chunks of one-signed data, so hi hi has an accumulator of its own and hi no more than 7 bits: its sums of 8 or 16
+//     products fit 24 bits, up to terms 2^-7 of the largest, and the other five products are small enough for a cut not to matter; the two sums are
+//     added in f32.  The large parts of d q and the minimum cancel in the coefficient and not in sums of thousands.  2-norm error against 64
+//     bits, K = 4096, a minimum added per block in f32 / here:  weights around zero, normal activations Q5_K 8.8e-8 / 5.7e-8, Q2_K 7.2e-8 / 5.5e-8, Q5_0
+//     6.7e-8 / 6.5e-8; no minimum and activations of one sign Q5_K 2.5e-8 / 2.5e-8, Q2_K 3.2e-8 / 3.1e-8 (4.9e-8 and 5.3e-8 with all products in one
+//     accumulator).  Larger only where every code of a block is its lowest, which no quantizer writes (Q5_K 6.0e-8 / 6.7e-8).  It costs 7 % (Q5_K
+//     4096 -> 14336, 512 tokens 237 us -> 255).  Not for Q4_1 and Q5_1, whose stored sum can be most of the result: their codes stay unsigned and a
+//     block's two parts meet in the epilogue.
 //   * A super-block format has one d per 256 elements: a block is then ONE fma per value, sum += d_a I, and d is applied per chunk.
 //   * The accumulators are read with the 16x256b shape of tcgen05.ld: a thread holds four rows x two columns of each eight columns, so one
 //     8-byte shared load of token scales serves eight values (a 16-byte load served four with a row per lane: a broadcast takes as long as the
@@ -28,9 +32,9 @@
 //
 // Mapping as in prompt_kq.cu: tiles of 128 weight rows x up to 64 tokens (the compensated sums take three registers per value),
 // warps 0-7 epilogue, 8-15 producers (two sets of four, a weight row per thread, the sets take turns), 16 MMA issuer, 17 loader, 18-19
-// raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128 columns each), 64 columns for the
-// minimum sums where there are any, operand A in two or three buffers of two blocks.  The roles hand over two blocks at a time; where operand
-// A and the accumulators have as many buffers, one commit tells both the producers and the epilogue.  Every wait is bounded as there.
+// raw bytes where there is no tensor map; tensor memory: three accumulator slots of two blocks (128 columns each), which the minimum sums of a chunk take
+// like a fifth pair, and operand A in three buffers of two blocks.  The roles hand over two blocks at a time; where no minimum sums are between
+// them, slots and buffers go together and one commit tells both the producers and the epilogue.  Every wait is bounded as there.
 //
 // Measured (B200, quantizer included; before -> now): Q5_K 4096 -> 14336, 512 tokens 493 us -> 243, Q8_0 4096 -> 4096, 333 tokens 88 -> 69.  A chunk of
 // 256 elements takes 2.1 us and 11 ns per token, 11 - 13 thousand warp instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
@@ -77,30 +81,32 @@ template <> struct Fmt<CQ_Q5_K> : FmtMin<kSum32, false> {};
 template <> struct Fmt<CQ_Q2_K> : FmtMin<kSum16, false> {};
 
 constexpr int sums_of(int sum) { return sum == kNoSum || sum == kTermSum ? 0 : sum == kSum16 ? 16 : 8; }   // coefficients per chunk
-constexpr int kColV = 384;                       // tensor memory column of the minimum sums
-// f16 values; scales, and t where the epilogue takes it; four planes of bf16 sums (lo, mid, hi where finite, hi) of one token and chunk
+constexpr int kColA = 384;                       // tensor memory column of operand A
+// f16 values; scales, and t where the epilogue takes it; planes of bf16 sums (lo, mid, hi where finite, zeros where two planes make a K step, hi) of one
+// token and chunk
 constexpr int float_bytes(int sum) { return sum == kTermSum ? 64 : 32; }
-constexpr int tok_bytes(int sum) { return 512 + float_bytes(sum) + 8 * sums_of(sum); }
+constexpr int planes_of(int sum) { return sums_of(sum) == 8 ? 5 : sums_of(sum) / 4; }
+constexpr int sum_bytes(int sum) { return planes_of(sum) * 2 * sums_of(sum); }
+constexpr int tok_bytes(int sum) { return 512 + float_bytes(sum) + sum_bytes(sum); }
 template <int WTYPE> constexpr int chunk_bytes() { return 256 / cq_block_elems(WTYPE) * cq_type_size(WTYPE); }
 template <int WTYPE> struct Smem {
     using F = Fmt<WTYPE>;
-    static constexpr int kSums = sums_of(F::kSum), kNA = kSums ? 2 : 3;             // buffers of operand A
-    static constexpr int kColA = kSums ? 448 : 384;
-    static constexpr int kStageT = 16 * kTok * 16, kAux = kTok * (float_bytes(F::kSum) + 8 * kSums);
+    static constexpr int kSums = sums_of(F::kSum);
+    static constexpr int kStageT = 16 * kTok * 16, kAux = kTok * (float_bytes(F::kSum) + sum_bytes(F::kSum));
     static constexpr int kRingW = kRows * 4 * (F::kTerm ? 16 : F::kBlockScale ? 8 : 1);      // d of the rows (and m), one chunk
     static constexpr int kRawStages = F::kTerm ? 2 : 3;
     static constexpr int kCoef = 3 * kRows * 2 * kSums;                              // planes lo, hi, mid of the coefficients
     static constexpr int kBytes = 1024 + kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * kCoef + kRawStages * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
 };
 
-// v = hi + mid + lo, exactly (8 bits each); a value that is not finite has only its first part
+// v = hi + mid + lo, exactly (7, 8 and 8 bits, and the signs of the rests); a value that is not finite has only its first part
 __device__ __forceinline__ void split3(float v, uint16_t &hi, uint16_t &mid, uint16_t &lo) {
     auto bits = [](__nv_bfloat16 b) { return __bfloat16_as_ushort(b); };
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    const bool finite = fabsf(__bfloat162float(h)) <= 3.4e38f;
-    const float r = finite ? __fsub_rn(v, __bfloat162float(h)) : 0.0f;
+    const bool finite = fabsf(v) <= 3.3e38f;
+    const uint32_t h = (__float_as_uint(v) + 0x10000u) & 0xFFFE0000u;
+    const float r = finite ? __fsub_rn(v, __uint_as_float(h)) : 0.0f;
     const __nv_bfloat16 m = __float2bfloat16_rn(r);
-    hi = bits(h);
+    hi = finite ? (uint16_t)(h >> 16) : bits(__float2bfloat16_rn(v));
     mid = bits(m);
     lo = bits(__float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m))));
 }
@@ -109,7 +115,7 @@ __device__ __forceinline__ void split3(float v, uint16_t &hi, uint16_t &mid, uin
 // One warp per (token, chunk of 256), 8 tokens of one chunk per block, through shared memory (see prompt_kq.cu).
 template <typename T, bool Q81, int SUM>
 __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k, Tiling tl) {
-    constexpr int kPitch = 8 * 16 + 16, kPlane = sums_of(SUM) / 8, kSlabs = 32 + 4 * kPlane, kFloats = float_bytes(SUM) / 4;
+    constexpr int kPitch = 8 * 16 + 16, kPlane = sums_of(SUM) / 8, kPlanes = planes_of(SUM), kSlabs = 32 + kPlanes * kPlane, kFloats = float_bytes(SUM) / 4;
     __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
     __shared__ float sv[kFloats][8];    // [block][token]: scales, then t
     cq_pdl_wait();
@@ -156,9 +162,9 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, 
             uint16_t hi, mid, lo;
             split3(v, hi, mid, lo);
             uint8_t *p = sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7);
-            const uint16_t plane[4] = {lo, mid, (uint16_t)((hi & 0x7F80u) == 0x7F80u ? 0 : hi), hi};
+            const uint16_t plane[5] = {lo, mid, (uint16_t)((hi & 0x7F80u) == 0x7F80u ? 0 : hi), kPlanes == 5 ? (uint16_t)0 : hi, hi};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint16_t *>(p + i * kPlane * kPitch) = plane[i];
+            for (int i = 0; i < kPlanes; ++i) *reinterpret_cast<uint16_t *>(p + i * kPlane * kPitch) = plane[i];
         };
         if constexpr (SUM == kSum16) { if ((lane & 1) == 0) put(lane >> 1, s); }
         else if constexpr (SUM == kSum32) { if ((lane & 3) == 0) put(b, s); }
@@ -435,8 +441,8 @@ template <int WTYPE, int STORE, int N8>
 __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
     using F = Fmt<WTYPE>;
     using S = Smem<WTYPE>;
-    constexpr int kCB = chunk_bytes<WTYPE>(), kSums = S::kSums, kNA = S::kNA;
-    constexpr bool kOneCommit = kNA == kSlots;      // bar_acc serves the producers too
+    constexpr int kCB = chunk_bytes<WTYPE>(), kSums = S::kSums, kNA = 3;
+    constexpr bool kOneCommit = kSums == 0;         // accumulator slots and buffers of operand A go together: bar_acc serves the producers too
     using R = Raw<kCB>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bar_raw = reinterpret_cast<uint64_t *>(smem);        // [3] raw weight bytes landed
@@ -448,7 +454,6 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     uint64_t *bar_acc = bar_raw + 20;                               // [3] the MMAs of two blocks are complete
     uint64_t *bar_free = bar_raw + 23;                              // [3] accumulator slot read (all epilogue warps)
     uint64_t *bar_vis = bar_raw + 26;                               // [2] relay: the scales of this chunk are visible
-    uint64_t *bar_vfree = bar_raw + 28;                             // minimum sums read (all epilogue warps)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 520);
     uint8_t *stT0 = smem + 1024;
@@ -472,7 +477,6 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             cq_mbar_init(&bar_free[i], kEpiWarps);
         }
         for (int i = 0; i < 2; ++i) cq_mbar_init(&bar_vis[i], 1);
-        cq_mbar_init(bar_vfree, kEpiWarps);
         *abort_flag = 0;
         cq_fence_mbar_init();
     }
@@ -514,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         const unsigned bytes = (unsigned)n * 256;
                         if (half == 0) {
                             // a stage of chunk it - 2 (or later) is done: its MMAs had started, so the epilogue has finished it - 4
-                            const unsigned aux_bytes = (unsigned)n * (float_bytes(F::kSum) + 8 * kSums);
+                            const unsigned aux_bytes = (unsigned)n * (float_bytes(F::kSum) + sum_bytes(F::kSum));
                             cq_mbar_expect_tx(&bar_fullT[s], bytes + aux_bytes);
                             cq_bulk_g2s(aux0 + (it & 3) * S::kAux, blob + (size_t)n * 512, aux_bytes, &bar_fullT[s]);
                         } else {
@@ -567,10 +571,9 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 for (int ch = 0; ch < 4; ++ch) {
                     if (((ch & 1) == 0 && !wait_warp(&bar_fullT[s], s_phase, abort_flag)) ||
                         !wait_warp(&bar_fullW[buf], buf_phase, abort_flag) ||
-                        (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag)) ||
-                        (kSums && ch == 3 && it > 0 && !wait_warp(bar_vfree, (it - 1) & 1, abort_flag))) { alive = false; break; }
+                        (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag))) { alive = false; break; }
                     tc_fence_after();
-                    const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = tm + (uint32_t)(S::kColA + buf * 32);
+                    const uint32_t b0 = bT + (uint32_t)s * (S::kStageT >> 4) + (uint32_t)(8 * (ch & 1)) * n, a0 = tm + (uint32_t)(kColA + buf * 32);
                     const uint32_t td = tm + (uint32_t)(slot * 2 * kTok);
                     if (elect_one()) {
                         if (ch == 0) mbar_arrive(&bar_vis[it & 1]);     // what this warp has acquired is visible to the epilogue
@@ -578,25 +581,6 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         mma_f16_ts<true>(td, a0 + 8, b0 + 2 * n, idesc);
                         mma_f16_ts<false>(td + kTok, a0 + 16, b0 + 4 * n, idesc);
                         mma_f16_ts<true>(td + kTok, a0 + 24, b0 + 6 * n, idesc);
-                        if constexpr (kSums > 0) {
-                            if (ch == 3) {          // A planes lo, hi, mid; B planes lo, mid, hi where finite, hi
-                                const uint32_t tv = tm + (uint32_t)kColV, idb = idesc | (1u << 7) | (1u << 10);      // bf16 x bf16
-                                const uint32_t ca = (coef + (uint32_t)(it & 1) * (S::kCoef >> 4)) | ((uint32_t)kRows << 16);
-                                const uint32_t cb = (aux + (uint32_t)(it & 3) * (S::kAux >> 4) + (float_bytes(F::kSum) / 16) * n) | (n << 16);
-                                if constexpr (kSums == 8) {         // a step is two planes of eight
-                                    mma_ss<false>(tv, ca + kRows, cb, idb);                 // hi lo + mid mid
-                                    mma_ss<true>(tv, ca + kRows, cb + n, idb);              // hi mid + mid hi
-                                    mma_ss<true>(tv, ca, cb + 2 * n, idb);                  // lo hi + hi hi
-                                } else {
-                                    mma_ss<false>(tv, ca + 2 * kRows, cb, idb);             // hi lo
-                                    mma_ss<true>(tv, ca + 4 * kRows, cb + 2 * n, idb);      // mid mid
-                                    mma_ss<true>(tv, ca, cb + 4 * n, idb);                  // lo hi
-                                    mma_ss<true>(tv, ca + 2 * kRows, cb + 2 * n, idb);      // hi mid
-                                    mma_ss<true>(tv, ca + 4 * kRows, cb + 4 * n, idb);      // mid hi
-                                    mma_ss<true>(tv, ca + 2 * kRows, cb + 6 * n, idb);      // hi hi
-                                }
-                            }
-                        }
                         tc_commit(&bar_acc[slot]);
                         if (ch & 1) tc_commit(&bar_doneT[s]);
                         if constexpr (!kOneCommit) tc_commit(&bar_doneW[buf]);
@@ -606,6 +590,31 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     if (++buf == kNA) { buf = 0; buf_phase ^= 1; }
                     if ((ch & 1) && ++s == kStagesT) { s = 0; s_phase ^= 1; }
                 }
+                if constexpr (kSums > 0) {      // the chunk's sums take a slot like two blocks: the products hi hi, and all others
+                    if (!alive || (round > 0 && !wait_warp(&bar_free[slot], (round - 1) & 1, abort_flag))) { alive = false; break; }
+                    tc_fence_after();
+                    if (elect_one()) {      // A planes lo, hi, mid; B planes: planes_of
+                        const uint32_t t1 = tm + (uint32_t)(slot * 2 * kTok), t2 = t1 + kTok, idb = idesc | (1u << 7) | (1u << 10);      // bf16 x bf16
+                        const uint32_t ca = (coef + (uint32_t)(it & 1) * (S::kCoef >> 4)) | ((uint32_t)kRows << 16);
+                        const uint32_t cb = (aux + (uint32_t)(it & 3) * (S::kAux >> 4) + (float_bytes(F::kSum) / 16) * n) | (n << 16);
+                        if constexpr (kSums == 8) {         // a step is two planes of eight
+                            mma_ss<false>(t2, ca + kRows, cb, idb);                 // hi lo + mid mid
+                            mma_ss<true>(t2, ca, cb + 2 * n, idb);                  // lo hi
+                            mma_ss<true>(t2, ca + kRows, cb + n, idb);              // hi mid + mid hi
+                            mma_ss<false>(t1, ca, cb + 3 * n, idb);                 // hi hi
+                        } else {
+                            mma_ss<false>(t2, ca + 2 * kRows, cb, idb);             // hi lo
+                            mma_ss<true>(t2, ca + 4 * kRows, cb + 2 * n, idb);      // mid mid
+                            mma_ss<true>(t2, ca, cb + 4 * n, idb);                  // lo hi
+                            mma_ss<true>(t2, ca + 2 * kRows, cb + 2 * n, idb);      // hi mid
+                            mma_ss<true>(t2, ca + 4 * kRows, cb + 4 * n, idb);      // mid hi
+                            mma_ss<false>(t1, ca + 2 * kRows, cb + 6 * n, idb);     // hi hi
+                        }
+                        tc_commit(&bar_acc[slot]);
+                    }
+                    __syncwarp();
+                    if (++slot == kSlots) { slot = 0; ++round; }
+                }
             }
         }
     }
@@ -613,7 +622,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         regs_down<kRegsProd32>();
         // ===== producers: thread = weight row = TMEM lane; set 0 takes the even pairs of blocks, set 1 the odd ones =====
         const int set = (warp - kEpiWarps) >> 2, r = (warp & 3) * 32 + lane;
-        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)S::kColA;
+        const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)kColA;
         int it = 0, rs = 0, rs_phase = 0;
         bool alive = true;
         for (int tile = blockIdx.x; tile < a.ntiles && alive; tile += gridDim.x) {
@@ -626,8 +635,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
                 Expand<WTYPE> ex;
                 ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
-                // This set has waited for a pair of it - 2 or later (its last pair of it - 1 took over the buffer of one), so the sums step of
-                // it - 2 is complete where there is one, and the epilogue, at most three pairs behind the MMAs, has finished it - 4.
+                // Set 0 has waited for the last pair of it - 2 or later, and the epilogue, at most three slots behind the MMAs, has finished it - 4; set 1
+                // for the first pair of it - 1, whose completion includes the sums of it - 2.
                 if (set == 0) ex.scales(reinterpret_cast<float *>(ringW + (it & 3) * S::kRingW) + r);
                 else if constexpr (kSums > 0) {
                     ex.coef(coef0 + (it & 1) * S::kCoef + r * 16);
@@ -729,19 +738,31 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     uint64_t dw[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { const float d = F::kBlockScale ? 1.0f : rw[8 * i]; dw[i] = pack2f(d, d); }
+                    if constexpr (kSums > 0) {
+                        if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
+                        tc_fence_after();
+                    }
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        [[maybe_unused]] uint32_t v[4 * N8];
+                        [[maybe_unused]] uint32_t v1[4 * N8], v2[4 * N8];
                         if constexpr (kSums > 0) {
-                            tmem_ld_16x256b<N8>(tq + (uint32_t)kColV + ((uint32_t)(16 * h) << 16), v);
+                            tmem_ld_16x256b<N8>(tq + (uint32_t)(2 * slot * kTok) + ((uint32_t)(16 * h) << 16), v1);
+                            tmem_ld_16x256b<N8>(tq + (uint32_t)((2 * slot + 1) * kTok) + ((uint32_t)(16 * h) << 16), v2);
                             tmem_ld_wait();
+                            if (h == 1) {
+                                tc_fence_before();
+                                arrive_warp(&bar_free[slot], lane);
+                            }
                         }
 #pragma unroll
                         for (int i = 0; i < 2 * N8; ++i) {
                             const int x = 2 * N8 * h + i;
                             const uint64_t s0 = sum[x];
                             uint64_t f = dw[2 * h + (x & 1)], y = acc[x];            // the chunk is f y
-                            if constexpr (kSums > 0) { y = fma2(f, y, pack2(v[2 * i], v[2 * i + 1])); f = one; }
+                            if constexpr (kSums > 0) {
+                                y = fma2(f, y, fma2(one, pack2(v2[2 * i], v2[2 * i + 1]), pack2(v1[2 * i], v1[2 * i + 1])));
+                                f = one;
+                            }
                             const uint64_t s1 = fma2(f, y, s0);
                             if constexpr (kExact) {
                                 const uint64_t bb = fma2(minus1, s0, s1);
@@ -753,8 +774,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         }
                     }
                     if constexpr (kSums > 0) {
-                        tc_fence_before();
-                        arrive_warp(bar_vfree, lane);
+                        if (++slot == kSlots) { slot = 0; ++round; }
                     }
                 }
             }

@@ -366,6 +366,41 @@ def test_prompt32_is_no_further_from_64_bits_than_sums_per_block_where_chunks_di
     assert err(_prompt32(lib, wtype, wq, x, k, 256)) <= 1.03 * err(plain) <= 1e-6
 
 
+@pytest.mark.parametrize("kind", ["normal", "one sign", "one sign, a few large"])
+@pytest.mark.parametrize("minimum", [1.0, 0.0, -1.0, 8.0])
+@pytest.mark.parametrize("k", [1024, 4096, 14336])
+@pytest.mark.parametrize("wtype", [6, 10, 13])
+def test_prompt32_minimum_sums_are_no_further_from_64_bits_than_sums_per_block(lib, cuda_dev, wtype, k, minimum, kind):
+    """Minimum sums on the tensor core, also where they are most of the result and of one sign.  3 % for the noise of 16384 values' errors."""
+    gen = torch.Generator(device=cuda_dev).manual_seed(k)
+    wq, *parts = _weights32(wtype, 256, k, minimum, gen, cuda_dev)
+    x = _inputs32(kind, 64, k, gen, cuda_dev)
+    plain, exact = _plain_sums(wtype, *parts, *_activations32(lib, wtype, x))
+    err = lambda o: float((o.double() - exact).norm() / exact.norm())
+    assert err(_prompt32(lib, wtype, wq, x, k, 256)) <= 1.03 * err(plain) <= 1e-6
+
+
+@pytest.mark.parametrize("wtype", [3, 6, 7, 10, 11, 13])
+def test_prompt32_of_infinite_scales_and_inputs(lib, cuda_dev, wtype):
+    """Results are not finite where the decode kernel's are not, and only there."""
+    k, n, m, gen = 512, 96, 16, torch.Generator(device=cuda_dev).manual_seed(wtype)
+    wq, x, st = _weights32(wtype, n, k, 1.0, gen, cuda_dev)[0].clone(), torch.randn(m, k, device=cuda_dev, generator=gen), torch.cuda.current_stream().cuda_stream
+    x[2, 40], x[4, 300], x[6, 7], x[8, 100:140] = float("inf"), float("nan"), 1e9, -65000.0
+    for row, at in ((5, MINIMUM[wtype][0]), (9, MINIMUM[wtype][1])):
+        if at is not None:
+            wq[row, at:at + 2] = torch.tensor([0, 0x7C], dtype=torch.uint8, device=cuda_dev)
+    y8, decode = torch.zeros((m, k // 32, 36), dtype=torch.uint8, device=cuda_dev), torch.empty((m, n), device=cuda_dev)
+    lib.cq_quantize_act(x.data_ptr(), capi.F32, y8.data_ptr(), k, k, m, 0, st)
+    for r in range(0, m, 8):
+        lib.cq_mmvq(wtype, 0, capi.F32, wq.data_ptr(), y8[r:].data_ptr(), decode[r:].data_ptr(), k, n, k // 32, n, 8, st)
+    scratch, out = torch.zeros(lib.cq_prompt32_scratch_bytes(wtype, m, k), dtype=torch.uint8, device=cuda_dev), torch.empty((m, n), device=cuda_dev)
+    lib.cq_prompt32_matmul(wtype, wq.data_ptr(), x.data_ptr(), capi.F32, out.data_ptr(), scratch.data_ptr(), k, n, m, n, st)
+    capi.check("prompt32")
+    ok = torch.isfinite(decode)
+    assert torch.equal(torch.isfinite(out), ok) and not bool(ok[:, 5].any()) and bool(ok[0, 10:].all())
+    assert float((out - decode)[ok].norm() / decode[ok].norm()) <= 2e-6
+
+
 @pytest.mark.parametrize("wtype,rows,k,n", [(3, 200, 768, 700), (6, 200, 768, 700), (7, 200, 768, 700), (10, 200, 768, 700), (11, 200, 768, 700), (13, 200, 768, 700),
                                             (3, 40, 5120, 64), (13, 36, 5120, 64)])
 def test_qmatmul_runs_the_kernel_the_rule_names(lib, oracle, cuda_dev, wtype, rows, k, n):
