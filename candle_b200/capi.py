@@ -68,7 +68,7 @@ def lib() -> C.CDLL:
         L.cq_prompt32_bf16_scratch_bytes.argtypes, L.cq_prompt32_bf16_scratch_bytes.restype = [i32, i32, i32], C.c_size_t
         L.cq_prompt32_bf16_matmul.argtypes, L.cq_prompt32_bf16_matmul.restype = [i32, vp, vp, vp, vp, i32, i32, i32, i32, vp], None
         L.cq_prompt32_timeout_flag.restype = i32
-        for f in (L.cq_prompt_pays, L.cq_prompt32_pays, L.cq_moe_prompt_pays):
+        for f in (L.cq_prompt_pays, L.cq_prompt32_pays, L.cq_prompt32_bf16_pays, L.cq_moe_prompt_pays):
             f.argtypes, f.restype = [i32] * 4, i32
         L.cq_prefill32_scratch_bytes.argtypes = [i32, i32]
         L.cq_prefill32_scratch_bytes.restype = C.c_size_t

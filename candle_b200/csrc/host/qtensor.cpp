@@ -207,7 +207,7 @@ void QCudaStorage::fwd(size_t n, size_t k, const void *x, DType x_dtype, const i
     // decode launch where that is the faster, and not in the CPU-exact mode).  K must be a whole number of 256-element stages.
     const bool plain32 = dtype_ == GgmlDType::Q4_0 || dtype_ == GgmlDType::Q8_0;
     const bool q8_1_only = !plain32 && dtype_ != GgmlDType::Q4K && dtype_ != GgmlDType::Q6K;
-    const bool old_sums = q8_1_only && x_dtype == DType::BF16;       // bf16 results keep their bits (prompt_b32_bf16.cu)
+    const bool old_sums = q8_1_only && x_dtype == DType::BF16;       // sums of their own (prompt_b32.cu, PLAIN)
     const bool any_address = dtype_ == GgmlDType::Q2K || dtype_ == GgmlDType::Q3K;
     if (k % 256 == 0 && ((plain32 && rows > kPrefillMinRows) ||
                          (q8_1_only && rows > MMVQ_MAX_BATCH && !cpu_exact && (any_address || (uintptr_t)ptr_ % 16 == 0) &&

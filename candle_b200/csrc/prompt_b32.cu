@@ -18,7 +18,8 @@
 //     added in f32.  The large parts of d q and the minimum cancel in the coefficient and not in sums of thousands.  2-norm error against 64
 //     bits, K = 4096, a minimum added per block in f32 / here:  weights around zero, normal activations Q5_K 8.8e-8 / 5.7e-8, Q2_K 7.2e-8 / 5.5e-8, Q5_0
 //     6.7e-8 / 6.5e-8; no minimum and activations of one sign Q5_K 2.5e-8 / 2.5e-8, Q2_K 3.2e-8 / 3.1e-8 (4.9e-8 and 5.3e-8 with all products in one
-//     accumulator).  Larger only where every code of a block is its lowest, which no quantizer writes (Q5_K 6.0e-8 / 6.7e-8).  It costs 7 % (Q5_K
+//     accumulator).  Larger only where every code of a block is its lowest and its
+//     scale is not zero, which no quantizer writes (Q5_K 6.0e-8 / 6.7e-8).  It costs 7 % (Q5_K
 //     4096 -> 14336, 512 tokens 237 us -> 255).  Not for Q4_1 and Q5_1, whose stored sum can be most of the result: their codes stay unsigned and a
 //     block's two parts meet in the epilogue.
 //   * A super-block format has one d per 256 elements: a block is then ONE fma per value, sum += d_a I, and d is applied per chunk.
@@ -36,8 +37,13 @@
 // like a fifth pair, and operand A in three buffers of two blocks.  The roles hand over two blocks at a time; where no minimum sums are between
 // them, slots and buffers go together and one commit tells both the producers and the epilogue.  Every wait is bounded as there.
 //
-// Measured (B200, quantizer included; before -> now): Q5_K 4096 -> 14336, 512 tokens 493 us -> 243, Q8_0 4096 -> 4096, 333 tokens 88 -> 69.  A chunk of
-// 256 elements takes 2.1 us and 11 ns per token, 11 - 13 thousand warp instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
+// bf16 results of Q5_0, Q5_K, Q2_K and Q3_K that QMatMul.forward returns come from PLAIN sums: unsigned codes, d and the minimum in the terms of each block, in f32.
+// Sums in the other order differ by 1e-7 of them, and a few in 100 000 bf16 results then round to the neighbouring value, 2^-8 to 2^-7 of it away; bf16
+// results keep their bits instead, for 12 - 50 % more time (512 tokens below: Q5_K 326 us, Q2_K 418, Q5_0 351, Q3_K 296).  Before this mapping: 468, 579, 482, 475.
+//
+// Measured (B200, quantizer included, f32; before this mapping -> now): 4096 -> 14336, 512 tokens Q5_K 493 us -> 257, Q2_K 282, Q5_0 310, Q3_K 259, Q4_1 339, Q5_1 350,
+// Q4_0 226, Q8_0 212; Q8_0 4096 -> 4096, 333 tokens 88 -> 65.  A chunk of 256 elements takes about 2.2 us and 11 ns per token, 11 - 13 thousand warp
+// instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
 // Tried: tiles of 128 tokens with one producer set (Q5_K 327), the group's first warp polling for the others (534: branches and barrier reads outweigh
 // the polls), a branch on the tile's tokens inside the block loop (312: the compiler then moves every running sum).
 #include "../../include/candle_q_b200.h"
@@ -56,6 +62,7 @@ constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;      // the last two
 constexpr int kTok = 64;                         // tokens per tile, at most
 constexpr int kSlots = 3;                        // accumulator slots of two blocks
 constexpr int kStagesT = 4;                      // token stages of half a chunk
+constexpr int kRawStages = 3;                    // chunks of raw weight bytes
 constexpr int kFixedTokens = 180;                // plan_tiling: 2.1 us + 11 ns per token and chunk
 // registers: 640 threads x 96 at launch = 256 * 144 + 256 * 72 + 128 * 48
 constexpr int kRegsEpi32 = 144, kRegsProd32 = 72, kRegsMisc32 = 48;
@@ -63,38 +70,40 @@ constexpr int kRegsEpi32 = 144, kRegsProd32 = 72, kRegsMisc32 = 48;
 __device__ int g_prompt_b32_timeout_flag = 0;
 
 // kSum: the activations' sums of the minimum part: none; s per 32 (Q5_K) or 16 (Q2_K) elements, t - s (Q5_0), which meet their coefficients on the tensor
-// core; t, in the epilogue (Q4_1, Q5_1: kTerm).
-enum { kNoSum, kSum32, kSum16, kDelta, kTermSum };
-template <int WTYPE> struct Fmt {       // Q8_0, Q4_0, Q3_K
-    static constexpr bool kQ81 = WTYPE == CQ_Q3_K, kBlockScale = WTYPE != CQ_Q3_K;
-    static constexpr int kSum = kNoSum;
-    static constexpr bool kTerm = false;
+// core; t (Q4_1, Q5_1), which meets the minima in the epilogue.  PLAIN: all of them in the epilogue, with unsigned codes and a block's d in its own
+// term; no difference for Q8_0, Q4_0, Q4_1 and Q5_1.  kTerm: the terms of a block are added up apart from the running sum: d_a d_w I and m_w s are both large and nearly
+// cancel for weights around zero; added to the running sum one after the other they left two to four times the decode kernels' error against 64 bits (2-norm, K = 4096,
+// activations of one sign: Q4_1 2.2e-7 for 7.6e-8, Q5_1 2.6e-7 for 7.7e-8; now 6.7e-8 and 6.9e-8).  Q5_K stays below the decode kernel's error without.
+enum { kNoSum, kSum32, kSum16, kDelta, kTermSum, kPlain32, kPlain16 };
+template <int SUM, bool Q81, bool BLOCK, bool TERM = false> struct FmtOf {
+    static constexpr bool kQ81 = Q81, kBlockScale = BLOCK, kTerm = TERM;
+    static constexpr int kSum = SUM, kMins = SUM == kTermSum || SUM == kPlain32 ? 1 : SUM == kPlain16 ? 2 : 0;       // minima of a block in the epilogue
 };
-template <int SUM, bool BLOCK> struct FmtMin {
-    static constexpr bool kQ81 = true, kBlockScale = BLOCK, kTerm = SUM == kTermSum;
-    static constexpr int kSum = SUM;
-};
-template <> struct Fmt<CQ_Q4_1> : FmtMin<kTermSum, true> {};
-template <> struct Fmt<CQ_Q5_0> : FmtMin<kDelta, true> {};
-template <> struct Fmt<CQ_Q5_1> : FmtMin<kTermSum, true> {};
-template <> struct Fmt<CQ_Q5_K> : FmtMin<kSum32, false> {};
-template <> struct Fmt<CQ_Q2_K> : FmtMin<kSum16, false> {};
+template <int WTYPE, bool PLAIN> struct Fmt : FmtOf<kNoSum, false, true> {};       // Q8_0, Q4_0
+template <bool PLAIN> struct Fmt<CQ_Q4_1, PLAIN> : FmtOf<kTermSum, true, true, true> {};
+template <bool PLAIN> struct Fmt<CQ_Q5_1, PLAIN> : FmtOf<kTermSum, true, true, true> {};
+template <> struct Fmt<CQ_Q5_0, false> : FmtOf<kDelta, true, true> {};
+template <> struct Fmt<CQ_Q5_0, true> : FmtOf<kTermSum, true, true, true> {};
+template <> struct Fmt<CQ_Q5_K, false> : FmtOf<kSum32, true, false> {};
+template <> struct Fmt<CQ_Q5_K, true> : FmtOf<kPlain32, true, false> {};
+template <> struct Fmt<CQ_Q2_K, false> : FmtOf<kSum16, true, false> {};
+template <> struct Fmt<CQ_Q2_K, true> : FmtOf<kPlain16, true, false, true> {};
+template <bool PLAIN> struct Fmt<CQ_Q3_K, PLAIN> : FmtOf<kNoSum, true, false> {};
 
-constexpr int sums_of(int sum) { return sum == kNoSum || sum == kTermSum ? 0 : sum == kSum16 ? 16 : 8; }   // coefficients per chunk
+constexpr int sums_of(int sum) { return sum == kSum32 || sum == kDelta ? 8 : sum == kSum16 ? 16 : 0; }   // coefficients per chunk
 constexpr int kColA = 384;                       // tensor memory column of operand A
-// f16 values; scales, and t where the epilogue takes it; planes of bf16 sums (lo, mid, hi where finite, zeros where two planes make a K step, hi) of one
+// f16 values; scales, and sums where the epilogue takes them; planes of bf16 sums (lo, mid, hi where finite, zeros where two planes make a K step, hi) of one
 // token and chunk
-constexpr int float_bytes(int sum) { return sum == kTermSum ? 64 : 32; }
+constexpr int float_bytes(int sum) { return sum == kTermSum || sum == kPlain32 ? 64 : sum == kPlain16 ? 96 : 32; }
 constexpr int planes_of(int sum) { return sums_of(sum) == 8 ? 5 : sums_of(sum) / 4; }
 constexpr int sum_bytes(int sum) { return planes_of(sum) * 2 * sums_of(sum); }
 constexpr int tok_bytes(int sum) { return 512 + float_bytes(sum) + sum_bytes(sum); }
 template <int WTYPE> constexpr int chunk_bytes() { return 256 / cq_block_elems(WTYPE) * cq_type_size(WTYPE); }
-template <int WTYPE> struct Smem {
-    using F = Fmt<WTYPE>;
+template <int WTYPE, bool PLAIN> struct Smem {
+    using F = Fmt<WTYPE, PLAIN>;
     static constexpr int kSums = sums_of(F::kSum);
     static constexpr int kStageT = 16 * kTok * 16, kAux = kTok * (float_bytes(F::kSum) + sum_bytes(F::kSum));
-    static constexpr int kRingW = kRows * 4 * (F::kTerm ? 16 : F::kBlockScale ? 8 : 1);      // d of the rows (and m), one chunk
-    static constexpr int kRawStages = F::kTerm ? 2 : 3;
+    static constexpr int kScales = F::kBlockScale ? 8 : 1, kRingW = kRows * 4 * (kScales + 8 * F::kMins);      // d of the rows, then minima, of one chunk
     static constexpr int kCoef = 3 * kRows * 2 * kSums;                              // planes lo, hi, mid of the coefficients
     static constexpr int kBytes = 1024 + kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * kCoef + kRawStages * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
 };
@@ -117,7 +126,7 @@ template <typename T, bool Q81, int SUM>
 __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, uint8_t *__restrict__ y, int k, Tiling tl) {
     constexpr int kPitch = 8 * 16 + 16, kPlane = sums_of(SUM) / 8, kPlanes = planes_of(SUM), kSlabs = 32 + kPlanes * kPlane, kFloats = float_bytes(SUM) / 4;
     __shared__ __align__(16) uint8_t sm[kSlabs * kPitch];
-    __shared__ float sv[kFloats][8];    // [block][token]: scales, then t
+    __shared__ float sv[kFloats][8];    // [value][token]: scales of the blocks, then sums
     cq_pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nch = k / 256;
@@ -156,7 +165,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, 
     if constexpr (SUM != kNoSum) {
         int si = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
         si += __shfl_xor_sync(0xffffffffu, si, 1);
-        if constexpr (SUM != kSum16) si += __shfl_xor_sync(0xffffffffu, si, 2);
+        if constexpr (SUM != kSum16 && SUM != kPlain16) si += __shfl_xor_sync(0xffffffffu, si, 2);
         const float s = __fmul_rn(dh, (float)si);
         [[maybe_unused]] auto put = [&](int j, float v) {        // sum j of the chunk: element j % 8 of slab j / 8 of each plane
             uint16_t hi, mid, lo;
@@ -168,6 +177,8 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, 
         };
         if constexpr (SUM == kSum16) { if ((lane & 1) == 0) put(lane >> 1, s); }
         else if constexpr (SUM == kSum32) { if ((lane & 3) == 0) put(b, s); }
+        else if constexpr (SUM == kPlain16) { if ((lane & 1) == 0) sv[8 + 8 * ((lane >> 1) & 1) + b][warp] = s; }
+        else if constexpr (SUM == kPlain32) { if ((lane & 3) == 0) sv[8 + b][warp] = s; }
         else {
             // t: the f16-rounded sum of the inputs, added in the order of a 32-lane xor butterfly over the block (16, 8, 4, 2, 1)
             float u[8];
@@ -222,20 +233,21 @@ template <int SUMS> __device__ __forceinline__ void put_coef(uint8_t *row, int j
     *reinterpret_cast<uint32_t *>(p + 2 * (SUMS / 8) * kRows * 16) = m0 | (uint32_t)m1 << 16;
 }
 
-template <int WTYPE> struct Expand;
+template <int WTYPE, bool PLAIN> struct Expand;
 
 // the 32-element block formats: their chunk is a whole number of 16-byte vectors
-template <int WTYPE> struct ExpandBlock {
+template <int WTYPE, bool PLAIN> struct ExpandBlock {
     static constexpr int kBlk = cq_type_size(WTYPE);
     static constexpr bool kHasM = WTYPE == CQ_Q4_1 || WTYPE == CQ_Q5_1, kFive = WTYPE == CQ_Q5_0 || WTYPE == CQ_Q5_1;
     const uint8_t *p;
     __device__ __forceinline__ void header(const uint8_t *rr, int) { p = rr; }
-    __device__ __forceinline__ void scales(float *dst) const {          // [8 blocks][128 rows] d, then the same of m
+    __device__ __forceinline__ void scales(float *dst) const {          // [8 blocks][128 rows] d, then the same of the minima
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
             const float d = h16(cq_lds_u16(p + b * kBlk));
             dst[b * kRows] = d;
             if constexpr (kHasM) dst[(8 + b) * kRows] = h16(cq_lds_u16(p + b * kBlk + 2));
+            else if constexpr (WTYPE == CQ_Q5_0 && PLAIN) dst[(8 + b) * kRows] = __fmul_rn(-16.0f, d);
         }
     }
     __device__ __forceinline__ void coef(uint8_t *row) const {
@@ -269,7 +281,7 @@ template <int WTYPE> struct ExpandBlock {
                     lo |= ((((qh >> (4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
                     hi |= ((((qh >> (16 + 4 * i)) & 0xFu) * 0x00204081u) & 0x01010101u) << 4;
                 }
-                constexpr float minus = WTYPE == CQ_Q4_0 ? 8.0f : WTYPE == CQ_Q5_0 ? 16.0f : 0.0f;
+                constexpr float minus = WTYPE == CQ_Q4_0 ? 8.0f : WTYPE == CQ_Q5_0 && !PLAIN ? 16.0f : 0.0f;
                 codes4(lo, minus, o[2 * i], o[2 * i + 1]);
                 codes4(hi, minus, o[8 + 2 * i], o[8 + 2 * i + 1]);
             };
@@ -293,17 +305,17 @@ template <int WTYPE> struct ExpandBlock {
         else pair<3>(o);
     }
 };
-template <> struct Expand<CQ_Q8_0> : ExpandBlock<CQ_Q8_0> {};
-template <> struct Expand<CQ_Q4_0> : ExpandBlock<CQ_Q4_0> {};
-template <> struct Expand<CQ_Q4_1> : ExpandBlock<CQ_Q4_1> {};
-template <> struct Expand<CQ_Q5_0> : ExpandBlock<CQ_Q5_0> {};
-template <> struct Expand<CQ_Q5_1> : ExpandBlock<CQ_Q5_1> {};
+template <bool PLAIN> struct Expand<CQ_Q8_0, PLAIN> : ExpandBlock<CQ_Q8_0, PLAIN> {};
+template <bool PLAIN> struct Expand<CQ_Q4_0, PLAIN> : ExpandBlock<CQ_Q4_0, PLAIN> {};
+template <bool PLAIN> struct Expand<CQ_Q4_1, PLAIN> : ExpandBlock<CQ_Q4_1, PLAIN> {};
+template <bool PLAIN> struct Expand<CQ_Q5_0, PLAIN> : ExpandBlock<CQ_Q5_0, PLAIN> {};
+template <bool PLAIN> struct Expand<CQ_Q5_1, PLAIN> : ExpandBlock<CQ_Q5_1, PLAIN> {};
 
 // Super-block formats.  A code of b bits goes to the top of the mantissa, or near it, so that scale times (code - middle) is one fma whose
-// addend, -(base + middle) * scale, is exact in f16; one copy of the code for all of a chunk's four pairs (see prompt_kq.cu).
+// addend, -(base + middle) * scale, is exact in f16 (PLAIN: no middle); one copy of the code for all of a chunk's four pairs (see prompt_kq.cu).
 
 // Q5_K: Q4_K with the fifth bits of sub-block g in bit g of 32 bytes.  Code q in bits 4-8: the value 64 + q.
-template <> struct Expand<CQ_Q5_K> {
+template <bool PLAIN> struct Expand<CQ_Q5_K, PLAIN> {
     const uint8_t *p;
     uint32_t sc[2], mn[2], dm;
     __device__ __forceinline__ void header(const uint8_t *rr, int) {
@@ -314,7 +326,14 @@ template <> struct Expand<CQ_Q5_K> {
         sc[1] = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
         mn[1] = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
     }
-    __device__ __forceinline__ void scales(float *dst) const { *dst = __low2float(bits_h2(dm)); }
+    __device__ __forceinline__ void scales(float *dst) const {
+        *dst = __low2float(bits_h2(dm));
+        if constexpr (PLAIN) {
+            const float dmin = __high2float(bits_h2(dm));
+#pragma unroll
+            for (int g = 0; g < 8; ++g) dst[(1 + g) * kRows] = -__fmul_rn(dmin, (float)((mn[g >> 2] >> (8 * (g & 3))) & 0xFFu));
+        }
+    }
     __device__ __forceinline__ void coef(uint8_t *row) const {
         const float d16 = __fmul_rn(16.0f, __low2float(bits_h2(dm))), dmin = __high2float(bits_h2(dm));
         auto c = [&](int g) {       // 16 d sc is exact
@@ -330,7 +349,7 @@ template <> struct Expand<CQ_Q5_K> {
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
         const uint32_t s16 = (ch & 2 ? sc[1] : sc[0]) >> (16 * (ch & 1));
         const __half2 s0 = twice(s16 & 0xFFu), s1 = twice((s16 >> 8) & 0xFFu);
-        const __half2 c0 = __hmul2(s0, __float2half2_rn(-80.0f)), c1 = __hmul2(s1, __float2half2_rn(-80.0f));
+        const __half2 base = __float2half2_rn(PLAIN ? -64.0f : -80.0f), c0 = __hmul2(s0, base), c1 = __hmul2(s1, base);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const uint32_t he = h[i] << (7 - 2 * ch), ho = h[i] >> (2 * ch);        // fifth bits 2 ch + 1 | 2 ch in bit 8
@@ -343,8 +362,8 @@ template <> struct Expand<CQ_Q5_K> {
 };
 
 // Q2_K / Q3_K: block b = 4 n + pos: bit pair pos of bytes 32 n .. of the codes; a scale per 16 elements, number 2 b + half.
-// Q2_K: code q in bits 8-9: the value 4 + q; the operand is sc (2 q - 3), so the row's scale is d / 2.
-template <> struct Expand<CQ_Q2_K> {
+// Q2_K: code q in bits 8-9: the value 4 + q; the operand is sc (2 q - 3), so the row's scale is d / 2 (PLAIN: sc q, d).
+template <bool PLAIN> struct Expand<CQ_Q2_K, PLAIN> {
     const uint8_t *p;
     float d, dmin;
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
@@ -353,7 +372,15 @@ template <> struct Expand<CQ_Q2_K> {
         cq_lds_words<1, true>(p + 80, dm);
         d = h16(dm[0]); dmin = h16(dm[0] >> 16);
     }
-    __device__ __forceinline__ void scales(float *dst) const { *dst = __fmul_rn(0.5f, d); }
+    __device__ __forceinline__ void scales(float *dst) const {
+        if constexpr (PLAIN) {
+            uint32_t sc[4];
+            cq_lds_words<4, true>(p, sc);
+            *dst = d;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[(1 + 8 * (j & 1) + (j >> 1)) * kRows] = -__fmul_rn(dmin, (float)((sc[j >> 2] >> (8 * (j & 3) + 4)) & 0xFu));
+        } else *dst = __fmul_rn(0.5f, d);
+    }
     __device__ __forceinline__ void coef(uint8_t *row) const {
         const float d15 = __fmul_rn(1.5f, d);
         uint32_t sc[4];
@@ -374,8 +401,8 @@ template <> struct Expand<CQ_Q2_K> {
             const int pos = 2 * (ch & 1) + bb;
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                const __half2 sv = twice((sc[0] >> (8 * (2 * bb + hf))) & 0xFu), s2 = __hadd2(sv, sv);
-                const __half2 cv = __hmul2(sv, __float2half2_rn(-11.0f));
+                const __half2 sv = twice((sc[0] >> (8 * (2 * bb + hf))) & 0xFu), s2 = PLAIN ? sv : __hadd2(sv, sv);
+                const __half2 cv = __hmul2(sv, __float2half2_rn(PLAIN ? -4.0f : -11.0f));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     o[16 * bb + 8 * hf + 2 * i] = hfma2_bits(and_or<0x03000300u, 0x44004400u>(q[4 * hf + i] << (8 - 2 * pos)), s2, cv);
@@ -386,7 +413,7 @@ template <> struct Expand<CQ_Q2_K> {
     }
 };
 // Q3_K: two bits, plus 4 when the mask bit is set, in bits 7-9: the value 8 + u; the operand is scale * (u - 4).
-template <> struct Expand<CQ_Q3_K> {
+template <bool PLAIN> struct Expand<CQ_Q3_K, PLAIN> {
     const uint8_t *p;
     uint32_t sc[3];
     __device__ __forceinline__ void header(const uint8_t *rr, int shift) {
@@ -437,11 +464,11 @@ struct Args {
 };
 
 // STORE: see prompt_f16.cuh; N8: tiles of up to 16 N8 tokens, 2 or 4
-template <int WTYPE, int STORE, int N8>
+template <int WTYPE, bool PLAIN, int STORE, int N8>
 __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_constant__ CUtensorMap wmap, const Args a, const Tiling tl) {
-    using F = Fmt<WTYPE>;
-    using S = Smem<WTYPE>;
-    constexpr int kCB = chunk_bytes<WTYPE>(), kSums = S::kSums, kNA = 3;
+    using F = Fmt<WTYPE, PLAIN>;
+    using S = Smem<WTYPE, PLAIN>;
+    constexpr int kCB = chunk_bytes<WTYPE>(), kSums = S::kSums, kMins = F::kMins, kNA = 3;
     constexpr bool kOneCommit = kSums == 0;         // accumulator slots and buffers of operand A go together: bar_acc serves the producers too
     using R = Raw<kCB>;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -457,8 +484,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + 512);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 520);
     uint8_t *stT0 = smem + 1024;
-    uint8_t *aux0 = stT0 + kStagesT * S::kStageT;       // [4] scales [8][n], then planes of sums
-    uint8_t *ringW = aux0 + 4 * S::kAux;                // [4][1 or 8][128 rows] d
+    uint8_t *aux0 = stT0 + kStagesT * S::kStageT;       // [4] scales [8][n], then sums: the same, or planes
+    uint8_t *ringW = aux0 + 4 * S::kAux;                // [4] d [1 or 8][128 rows], then minima [kMins][8][128 rows]
     uint8_t *coef0 = ringW + 4 * S::kRingW;             // [2] planes of coefficients
     uint8_t *raw0 = coef0 + 2 * S::kCoef;               // 128-byte aligned
 
@@ -468,7 +495,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     const GroupInfo gi{};
 
     if (tid == 0) {
-        for (int i = 0; i < S::kRawStages; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
+        for (int i = 0; i < kRawStages; ++i) { cq_mbar_init(&bar_raw[i], a.use_map ? 1 : kRawThreads); cq_mbar_init(&bar_rawfree[i], kProdWarps); }
         for (int i = 0; i < kStagesT; ++i) { cq_mbar_init(&bar_fullT[i], 1); cq_mbar_init(&bar_doneT[i], 1); }
         for (int i = 0; i < 3; ++i) {
             cq_mbar_init(&bar_fullW[i], kProdWarps / 2);
@@ -503,12 +530,12 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             const uint8_t *blob0 = a.act + (size_t)cx.blob_row * nch * tok_bytes(F::kSum);
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 if (a.use_map) {
-                    if (it >= S::kRawStages && !wait_warp(&bar_rawfree[rs], rs_phase, abort_flag)) { alive = false; break; }
+                    if (it >= kRawStages && !wait_warp(&bar_rawfree[rs], rs_phase, abort_flag)) { alive = false; break; }
                     if (lane == 0) {
                         cq_mbar_expect_tx(&bar_raw[rs], R::kBytes);
                         cq_tmap::load_2d(raw0 + rs * R::kBytes, &wmap, (int)(((uint32_t)c * kCB & ~15u) / 2), cx.row0, &bar_raw[rs]);
                     }
-                    if (++rs == S::kRawStages) { rs = 0; rs_phase ^= 1; }
+                    if (++rs == kRawStages) { rs = 0; rs_phase ^= 1; }
                 }
                 const uint8_t *blob = blob0 + (size_t)c * n * tok_bytes(F::kSum);
                 for (int half = 0; half < 2; ++half, ++ti) {
@@ -532,8 +559,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
         }
         // after a give-up the copies already issued must land (or give up themselves) before the shared memory goes away
         if (lane == 0 && (!alive || *abort_flag)) {
-            for (int j = it >= S::kRawStages ? it - S::kRawStages + 1 : 0; a.use_map && j <= it; ++j)
-                (void)cq_mbar_wait_bounded(&bar_raw[j % S::kRawStages], (j / S::kRawStages) & 1);
+            for (int j = it >= kRawStages ? it - kRawStages + 1 : 0; a.use_map && j <= it; ++j)
+                (void)cq_mbar_wait_bounded(&bar_raw[j % kRawStages], (j / kRawStages) & 1);
             for (int j = ti > kStagesT ? ti - kStagesT : 0; j < ti; ++j) (void)cq_mbar_wait_bounded(&bar_fullT[j % kStagesT], (j / kStagesT) & 1);
         }
         __syncwarp();
@@ -547,8 +574,8 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 tile_ctx(tile, tl.ntt, tl, gi, cx);
                 const uint8_t *w0 = a.w + cx.wrow0 * row_bytes;
                 for (int c = 0; c < nch; ++c, ++it) {
-                    const int rs = it % S::kRawStages;
-                    if (it >= S::kRawStages && !wait_warp(&bar_rawfree[rs], (it / S::kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
+                    const int rs = it % kRawStages;
+                    if (it >= kRawStages && !wait_warp(&bar_rawfree[rs], (it / kRawStages - 1) & 1, abort_flag)) { alive = false; break; }
                     R::load_rows(raw0 + rs * R::kBytes, w0 + (uint32_t)c * kCB, min(a.nrows - cx.row0, kRows), row_bytes, tid - kRawWarp * 32, &bar_raw[rs]);
                 }
             }
@@ -633,7 +660,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
             const uint32_t row_off = a.use_map ? 0u : (uint32_t)((uintptr_t)(a.w + wr * row_bytes) & 15);
             for (int c = 0; c < nch && alive; ++c, ++it) {
                 if (!wait_warp(&bar_raw[rs], rs_phase, abort_flag)) { alive = false; break; }
-                Expand<WTYPE> ex;
+                Expand<WTYPE, PLAIN> ex;
                 ex.header(raw0 + rs * R::kBytes + r * R::kPitch, R::kAligned ? 0 : (int)((row_off + (uint32_t)c * kCB) & 15));
                 // Set 0 has waited for the last pair of it - 2 or later, and the epilogue, at most three slots behind the MMAs, has finished it - 4; set 1
                 // for the first pair of it - 1, whose completion includes the sums of it - 2.
@@ -656,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     tc_fence_before();
                     arrive_warp(&bar_fullW[buf], lane);
                 }
-                if (++rs == S::kRawStages) { rs = 0; rs_phase ^= 1; }
+                if (++rs == kRawStages) { rs = 0; rs_phase ^= 1; }
             }
         }
     } else {
@@ -687,6 +714,11 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                 const float *da = reinterpret_cast<const float *>(aux0 + (it & 3) * S::kAux) + col0 + csub;
                 const float *rw = reinterpret_cast<const float *>(ringW + (it & 3) * S::kRingW) + r0;
                 if (!wait_warp(&bar_vis[it & 1], (it >> 1) & 1, abort_flag)) { alive = false; break; }
+                [[maybe_unused]] uint64_t dc[4];
+                if constexpr (!F::kBlockScale && PLAIN) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) dc[i] = pack2f(rw[8 * i], rw[8 * i]);
+                }
 #pragma unroll 1
                 for (int ch = 0; ch < 4; ++ch) {
                     if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
@@ -698,16 +730,20 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         const uint32_t ts = tq + (uint32_t)((2 * slot + bb) * kTok);
                         tmem_ld_16x256b<N8>(ts, p);
                         tmem_ld_16x256b<N8>(ts + (16u << 16), p + 4 * N8);
-                        [[maybe_unused]] uint64_t dw[4] = {}, mw[4] = {}, dd[N8], ss[N8];
+                        [[maybe_unused]] uint64_t dw[4] = {}, mw[kMins ? kMins : 1][4], ss[kMins ? kMins : 1][N8];
+                        uint64_t dd[N8];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             if constexpr (F::kBlockScale) { const float d = rw[b * kRows + 8 * i]; dw[i] = pack2f(d, d); }
-                            if constexpr (F::kTerm) { const float m = rw[(8 + b) * kRows + 8 * i]; mw[i] = pack2f(m, m); }
+                            else if constexpr (PLAIN) dw[i] = dc[i];
+#pragma unroll
+                            for (int h = 0; h < kMins; ++h) { const float m = rw[(S::kScales + 8 * h + b) * kRows + 8 * i]; mw[h][i] = pack2f(m, m); }
                         }
 #pragma unroll
                         for (int j = 0; j < N8; ++j) {
                             dd[j] = *reinterpret_cast<const uint64_t *>(da + b * n + 8 * j);
-                            if constexpr (F::kTerm) ss[j] = *reinterpret_cast<const uint64_t *>(da + (8 + b) * n + 8 * j);
+#pragma unroll
+                            for (int h = 0; h < kMins; ++h) ss[h][j] = *reinterpret_cast<const uint64_t *>(da + (8 + 8 * h + b) * n + 8 * j);
                         }
                         tmem_ld_wait();
                         if (bb == 1) {
@@ -720,9 +756,14 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                             for (int i = 0; i < 4; ++i) {
                                 const int x = 2 * N8 * (i >> 1) + 2 * j + (i & 1);
                                 const uint64_t pv = pack2(p[2 * x], p[2 * x + 1]);
-                                // Q8_0 / Q4_0: (d_w d_a) I, the rounding of the int8 kernel
-                                if constexpr (F::kTerm) acc[x] = fma2(one, fma2(mul2(dw[i], dd[j]), pv, mul2(mw[i], ss[j])), acc[x]);
-                                else acc[x] = fma2(F::kBlockScale ? mul2(dw[i], dd[j]) : dd[j], pv, acc[x]);
+                                if constexpr (F::kTerm) {       // d_w d_a: two f16, exact
+                                    uint64_t v = mul2(mw[0][i], ss[0][j]);
+                                    if constexpr (kMins == 2) v = fma2(mw[1][i], ss[1][j], v);
+                                    acc[x] = fma2(one, fma2(mul2(dw[i], dd[j]), pv, v), acc[x]);
+                                } else if constexpr (PLAIN && !F::kBlockScale) {
+                                    acc[x] = fma2(dd[j], mul2(dw[i], pv), acc[x]);
+                                    if constexpr (kMins == 1) acc[x] = fma2(mw[0][i], ss[0][j], acc[x]);
+                                } else acc[x] = fma2(F::kBlockScale ? mul2(dw[i], dd[j]) : dd[j], pv, acc[x]);       // Q8_0 / Q4_0: the rounding of the int8 kernel
                             }
                         }
                     }
@@ -735,9 +776,12 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                     // error (Q5_0, K = 1024, a few large blocks 5.7e-8 -> 6.1e-8); these two stay far below the sums with a minimum added per block (Q5_K
                     // 6.3e-8 for 8.7e-8, Q2_K 6.0e-8 for 7.2e-8), and three more operations per value are 4 % of the time (Q5_K 254 us -> 267).
                     constexpr bool kExact = F::kBlockScale || kSums == 0;
-                    uint64_t dw[4];
+                    constexpr bool kScaled = !F::kBlockScale && !PLAIN;        // the chunk is d times the blocks' sum
+                    [[maybe_unused]] uint64_t dw[4];
+                    if constexpr (kScaled) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) { const float d = F::kBlockScale ? 1.0f : rw[8 * i]; dw[i] = pack2f(d, d); }
+                        for (int i = 0; i < 4; ++i) dw[i] = pack2f(rw[8 * i], rw[8 * i]);
+                    }
                     if constexpr (kSums > 0) {
                         if (!wait_warp(&bar_acc[slot], round & 1, abort_flag)) { alive = false; break; }
                         tc_fence_after();
@@ -758,15 +802,16 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
                         for (int i = 0; i < 2 * N8; ++i) {
                             const int x = 2 * N8 * h + i;
                             const uint64_t s0 = sum[x];
-                            uint64_t f = dw[2 * h + (x & 1)], y = acc[x];            // the chunk is f y
+                            uint64_t f = one, y = acc[x];            // the chunk is f y
+                            if constexpr (kScaled) f = dw[2 * h + (x & 1)];
                             if constexpr (kSums > 0) {
                                 y = fma2(f, y, fma2(one, pack2(v2[2 * i], v2[2 * i + 1]), pack2(v1[2 * i], v1[2 * i + 1])));
                                 f = one;
                             }
                             const uint64_t s1 = fma2(f, y, s0);
                             if constexpr (kExact) {
-                                const uint64_t bb = fma2(minus1, s0, s1);
-                                const uint64_t e0 = fma2(minus1, fma2(minus1, bb, s1), s0), e1 = fma2(f, y, bb ^ 0x8000000080000000ull);
+                                const uint64_t bb = fma2(minus1, s0, s1), e0 = fma2(minus1, fma2(minus1, bb, s1), s0);
+                                const uint64_t e1 = kScaled ? fma2(f, y, bb ^ 0x8000000080000000ull) : fma2(minus1, bb, y);
                                 low[x] = fma2(one, fma2(one, e0, e1), low[x]);
                             } else low[x] = fma2(one, fma2(f, y, fma2(minus1, s1, s0)), low[x]);
                             sum[x] = s1;
@@ -816,25 +861,25 @@ __global__ void __launch_bounds__(kThreads, 1) prompt32_kernel(const __grid_cons
     if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
-template <int WTYPE, typename T>
+template <int WTYPE, bool PLAIN, typename T>
 void launch_quantize(const void *x, void *scratch, int k, const Tiling &tl, unsigned blocks, cudaStream_t st) {
-    using F = Fmt<WTYPE>;
+    using F = Fmt<WTYPE, PLAIN>;
     cq_launch_k(quantize_kernel<T, F::kQ81, F::kSum>, dim3(blocks), dim3(256), 0, st, (const T *)x, (uint8_t *)scratch, k, tl);
 }
 
-template <int WTYPE, int STORE, int N8> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const Args &a, const Tiling &tl) {
-    static_assert(Smem<WTYPE>::kBytes <= 232448, "shared memory of one CTA");
+template <int WTYPE, bool PLAIN, int STORE, int N8> void launch_kernel(int grid, cudaStream_t st, const CUtensorMap &map, const Args &a, const Tiling &tl) {
+    static_assert(Smem<WTYPE, PLAIN>::kBytes <= 232448, "shared memory of one CTA");
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-        cudaFuncSetAttribute(prompt32_kernel<WTYPE, STORE, N8>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<WTYPE>::kBytes);
+        cudaFuncSetAttribute(prompt32_kernel<WTYPE, PLAIN, STORE, N8>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<WTYPE, PLAIN>::kBytes);
         attr_done[dev] = true;
     }
-    cq_launch_k(prompt32_kernel<WTYPE, STORE, N8>, dim3(grid), dim3(kThreads), Smem<WTYPE>::kBytes, st, map, a, tl);
+    cq_launch_k(prompt32_kernel<WTYPE, PLAIN, STORE, N8>, dim3(grid), dim3(kThreads), Smem<WTYPE, PLAIN>::kBytes, st, map, a, tl);
 }
 
-template <int WTYPE>
+template <int WTYPE, bool PLAIN = false>
 bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, int k, int n, int tokens, int stride_dst, cudaStream_t st) {
     using R = Raw<chunk_bytes<WTYPE>()>;
     const int nch = k / 256, nrt = (n + kRows - 1) / kRows;
@@ -849,33 +894,65 @@ bool launch(const void *w, const void *x, int elem, void *dst, void *scratch, in
         cq_set_status(CQ_ERR_BAD_ARG, "prompt32: weights of this format must be 16-byte aligned");
         return false;
     }
-    if (elem == CQ_F32) launch_quantize<WTYPE, float>(x, scratch, k, tl, (unsigned)blocks, st);
-    else if (elem == CQ_F16) launch_quantize<WTYPE, __half>(x, scratch, k, tl, (unsigned)blocks, st);
-    else launch_quantize<WTYPE, __nv_bfloat16>(x, scratch, k, tl, (unsigned)blocks, st);
+    if constexpr (!PLAIN) {
+        if (elem == CQ_F32) launch_quantize<WTYPE, false, float>(x, scratch, k, tl, (unsigned)blocks, st);
+        if (elem == CQ_F16) launch_quantize<WTYPE, false, __half>(x, scratch, k, tl, (unsigned)blocks, st);
+    }
+    if (elem == CQ_BF16) launch_quantize<WTYPE, PLAIN, __nv_bfloat16>(x, scratch, k, tl, (unsigned)blocks, st);
     const Args a{(const uint8_t *)w, (const uint8_t *)scratch, dst, elem, n, nch, stride_dst, use_map ? 1 : 0, nrt * tl.ntt};
     const int grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
-    if (elem == CQ_F32) {
-        if (tl.tt <= 32) launch_kernel<WTYPE, kStoreF32, 2>(grid, st, map, a, tl);
-        else launch_kernel<WTYPE, kStoreF32, 4>(grid, st, map, a, tl);
-    } else if (rows_16_bytes_apart(dst, stride_dst) && n % 8 == 0) {
-        if (tl.tt <= 32) launch_kernel<WTYPE, kStore16, 2>(grid, st, map, a, tl);
-        else launch_kernel<WTYPE, kStore16, 4>(grid, st, map, a, tl);
+    if constexpr (!PLAIN) {
+        if (elem == CQ_F32) {
+            if (tl.tt <= 32) launch_kernel<WTYPE, false, kStoreF32, 2>(grid, st, map, a, tl);
+            else launch_kernel<WTYPE, false, kStoreF32, 4>(grid, st, map, a, tl);
+            return true;
+        }
+    }
+    if (rows_16_bytes_apart(dst, stride_dst) && n % 8 == 0) {
+        if (tl.tt <= 32) launch_kernel<WTYPE, PLAIN, kStore16, 2>(grid, st, map, a, tl);
+        else launch_kernel<WTYPE, PLAIN, kStore16, 4>(grid, st, map, a, tl);
     } else {
-        if (tl.tt <= 32) launch_kernel<WTYPE, kStore16Any, 2>(grid, st, map, a, tl);
-        else launch_kernel<WTYPE, kStore16Any, 4>(grid, st, map, a, tl);
+        if (tl.tt <= 32) launch_kernel<WTYPE, PLAIN, kStore16Any, 2>(grid, st, map, a, tl);
+        else launch_kernel<WTYPE, PLAIN, kStore16Any, 4>(grid, st, map, a, tl);
     }
     return true;
 }
 
-int sum_of(int wtype) {
-    return wtype == CQ_Q4_1 || wtype == CQ_Q5_1 ? kTermSum : wtype == CQ_Q5_0 ? kDelta : wtype == CQ_Q5_K ? kSum32 : wtype == CQ_Q2_K ? kSum16 : kNoSum;
+int sum_of(int wtype, bool plain) {
+    switch (wtype) {
+    case CQ_Q4_1: case CQ_Q5_1: return kTermSum;
+    case CQ_Q5_0: return plain ? kTermSum : kDelta;
+    case CQ_Q5_K: return plain ? kPlain32 : kSum32;
+    case CQ_Q2_K: return plain ? kPlain16 : kSum16;
+    }
+    return kNoSum;
+}
+
+size_t scratch_bytes(int wtype, int tokens, int k, bool plain) {
+    if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
+    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)tok_bytes(sum_of(wtype, plain)) + 256;
+}
+
+bool args_ok(const void *vx, const void *x, const void *dst, const void *scratch, int elem, int ncols_x, int nrows_x, int tokens) {
+    if (!vx || !x || !scratch || !dst || ncols_x <= 0 || nrows_x <= 0 || tokens <= 0 || ncols_x % 256 != 0) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: null pointer, empty shape or K not a multiple of 256");
+        return false;
+    }
+    if ((uintptr_t)scratch % 16 != 0 || (uintptr_t)vx % 2 != 0 || elem < CQ_F32 || elem > CQ_BF16) {
+        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: misaligned scratch or weights, or unknown element type");
+        return false;
+    }
+    return true;
 }
 
 }  // namespace
 
-extern "C" size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k) {
-    if (tokens <= 0 || k <= 0 || k % 256 != 0) return 0;
-    return (size_t)((tokens + 15) / 16 * 16) * (k / 256) * (size_t)tok_bytes(sum_of(wtype)) + 256;
+extern "C" size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k) { return scratch_bytes(wtype, tokens, k, false); }
+extern "C" size_t cq_prompt32_bf16_scratch_bytes(int wtype, int tokens, int k) { return scratch_bytes(wtype, tokens, k, true); }
+
+// time of a slice of up to eight rows on the decode kernel; weights: millions of them
+static double slice_us(bool super, int rows, int k, double weights) {
+    return super ? 5.25 + 0.125e-3 * k + weights * (0.05 + 0.084 * rows) : std::max(5.05, 4.7 + 0.018e-3 * k + weights * (0.21 + 0.02 * rows));
 }
 
 // The six Q8_1 formats against slices of eight rows on the decode kernel, which stream the matrix once each.  Models of both sides (9 - 220 tokens,
@@ -897,23 +974,26 @@ extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     }
     const double idle = (double)((n + kRows - 1) / kRows) * tl.ntt < 0.3 * sms ? 0.85 : 1.0;      // few tiles share the L2
     const double here = 8.5 + rounds * (k / 256) * (fixed + per_token * tl.tt) * idle;
-    auto slice = [&](int rows) {
-        return super ? 5.25 + 0.125e-3 * k + weights * (0.05 + 0.084 * rows) : std::max(5.05, 4.7 + 0.018e-3 * k + weights * (0.21 + 0.02 * rows));
-    };
     const int whole = tokens / 8, left = tokens % 8;
-    return here < (super ? 1.8 : 2.5) + whole * slice(8) + (left ? slice(left) : 0.0);
+    return here < (super ? 1.8 : 2.5) + whole * slice_us(super, 8, k, weights) + (left ? slice_us(super, left, k, weights) : 0.0);
+}
+
+// The same with bf16, whose line has not followed the kernel (its constants are those of a kernel that took 467 us where this one takes 320, Q5_K 4096 ->
+// 14336, 512 tokens): the two sides add in different orders, so a call that changes sides gets a few in 100 000 of its bf16 results as the neighbouring value.
+extern "C" int cq_prompt32_bf16_pays(int wtype, int tokens, int k, int n) {
+    const double sms = cq_sm_count(), weights = 1e-6 * n * (double)k;
+    const Tiling tl = plan_tiling(tokens, (n + kRows - 1) / kRows, (int)sms, 40, 64);
+    const double rounds = std::ceil((double)((n + kRows - 1) / kRows) * tl.ntt / sms);
+    const bool super = cq_block_elems(wtype) == 256;
+    const double fixed = wtype == CQ_Q2_K ? 2.52 : wtype == CQ_Q3_K ? 2.09 : 2.27, per_token = wtype == CQ_Q2_K ? 0.046 : 0.036;
+    const double here = 6.7 + rounds * (k / 256) * (fixed + per_token * tl.tt);
+    const int whole = tokens / 8, left = tokens % 8;
+    return here < (super ? 1.8 : 2.5) + whole * slice_us(super, 8, k, weights) + (left ? slice_us(super, left, k, weights) : 0.0);
 }
 
 extern "C" void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,
                                    int tokens, int stride_dst, void *stream) {
-    if (!vx || !x || !scratch || !dst || ncols_x <= 0 || nrows_x <= 0 || tokens <= 0 || ncols_x % 256 != 0) {
-        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: null pointer, empty shape or K not a multiple of 256");
-        return;
-    }
-    if ((uintptr_t)scratch % 16 != 0 || (uintptr_t)vx % 2 != 0 || elem < CQ_F32 || elem > CQ_BF16) {
-        cq_set_status(CQ_ERR_BAD_ARG, "prompt32 matmul: misaligned scratch or weights, or unknown element type");
-        return;
-    }
+    if (!args_ok(vx, x, dst, scratch, elem, ncols_x, nrows_x, tokens)) return;
     cudaStream_t st = (cudaStream_t)stream;
     bool ok = false;
     switch (wtype) {
@@ -930,10 +1010,27 @@ extern "C" void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int
     if (ok) cq_check_launch("prompt32 matmul");
 }
 
+extern "C" void cq_prompt32_bf16_matmul(int wtype, const void *vx, const void *x, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
+                                        int stride_dst, void *stream) {
+    if (!args_ok(vx, x, dst, scratch, CQ_BF16, ncols_x, nrows_x, tokens)) return;
+    cudaStream_t st = (cudaStream_t)stream;
+    bool ok = false;
+    switch (wtype) {
+    case CQ_Q4_1: ok = launch<CQ_Q4_1>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_1: ok = launch<CQ_Q5_1>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_0: ok = launch<CQ_Q5_0, true>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q2_K: ok = launch<CQ_Q2_K, true>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q3_K: ok = launch<CQ_Q3_K, true>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    case CQ_Q5_K: ok = launch<CQ_Q5_K, true>(vx, x, CQ_BF16, dst, scratch, ncols_x, nrows_x, tokens, stride_dst, st); break;
+    default: cq_set_status(CQ_ERR_UNSUPPORTED, "prompt32 matmul in bf16: Q4_1, Q5_0, Q5_1, Q2_K, Q3_K, Q5_K"); return;
+    }
+    if (ok) cq_check_launch("prompt32 matmul");
+}
+
 extern "C" int cq_prompt32_timeout_flag(void) {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_prompt_b32_timeout_flag, sizeof v) != cudaSuccess) { (void)cudaGetLastError(); return -1; }
     if (v) cq_set_status(CQ_ERR_TIMEOUT, "prompt32 matmul: a bounded wait gave up");
-    const int bf16 = cq_prompt32_bf16_timeout_flag();
-    return v ? v : bf16;
+    return v;
 }
+extern "C" int cq_prompt32_bf16_timeout_flag(void) { return cq_prompt32_timeout_flag(); }

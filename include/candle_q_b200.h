@@ -281,7 +281,8 @@ void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void
                         int stride_dst, void *stream);
 int cq_prompt32_timeout_flag(void);
 int cq_prompt32_pays(int wtype, int tokens, int k, int n);     /* Q8_1 formats: 0 where slices of eight tokens on the decode kernel are the faster */
-/* The same for Q4_1, Q5_0, Q5_1, Q2_K, Q3_K and Q5_K with bf16 inputs and outputs, in the order of summation whose bf16 results QMatMul.forward gives. */
+/* The same for Q4_1, Q5_0, Q5_1, Q2_K, Q3_K and Q5_K with bf16 inputs and outputs, with the minimum added per block in f32: the bf16 results that
+ * QMatMul.forward gives (Q4_1, Q5_1: also those of cq_prompt32_matmul).  Its _pays is the rule of bf16 calls; its timeout flag is the one above. */
 size_t cq_prompt32_bf16_scratch_bytes(int wtype, int tokens, int k);
 void cq_prompt32_bf16_matmul(int wtype, const void *vx, const void *x, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens, int stride_dst,
                              void *stream);

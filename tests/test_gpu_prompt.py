@@ -486,3 +486,29 @@ def test_prompt32_bf16_results_are_neighbours(lib, oracle, cuda_dev, wtype, toke
     slack = 4e-6 * float(ref.norm() / ref.numel() ** 0.5)
     assert bool(((out - ref.to(torch.bfloat16).float()).abs() <= 2.0 ** -7 * ref.abs() + slack).all())
     assert float((out != ref.to(torch.bfloat16).float()).float().mean()) <= 0.01
+
+
+@pytest.mark.parametrize("tokens,k,n,offset", [(200, 768, 700, 0), (70, 1280, 129, 0), (40, 512, 14341, 0), (2000, 512, 2050, 0), (300, 8192, 1500, 0), (100, 1024, 999, 2)])
+@pytest.mark.parametrize("wtype", [3, 6, 7, 10, 11, 13])
+def test_qmatmul_bf16_prompts_are_the_sums_per_block(lib, cuda_dev, wtype, tokens, k, n, offset):
+    """bf16 calls of the Q8_1 formats: the sums with a minimum added per block, rounded once, bit for bit; ragged rows and tokens, both tile sizes, weights
+    at any even address for Q2_K and Q3_K."""
+    gen = torch.Generator(device=cuda_dev).manual_seed(k + n)
+    wq, *parts = _weights32(wtype, n, k, 1.0, gen, cuda_dev)
+    x = torch.randn(tokens, k, device=cuda_dev, generator=gen).to(torch.bfloat16)
+    w = wq.reshape(-1)
+    if offset:
+        w = _at_offset(w, offset if wtype in (10, 11) else 16)
+    assert lib.cq_prompt32_bf16_pays(wtype, tokens, k, n) == 1
+    y = QMatMul.from_qtensor(QTensor.from_device_blocks(w, GgmlDType(wtype), (n, k))).forward(x)
+    assert torch.equal(y, _plain_sums(wtype, *parts, *_activations32(lib, wtype, x.float()))[0].to(torch.bfloat16))
+    assert lib.cq_prompt32_timeout_flag() == 0 and lib.cq_prompt32_bf16_timeout_flag() == 0
+
+
+@pytest.mark.parametrize("wtype,rows,k,n", [(3, 40, 5120, 64), (13, 36, 5120, 64), (10, 12, 14336, 3248), (6, 11, 8192, 1000)])
+def test_qmatmul_bf16_rows_the_rule_leaves_to_the_decode_kernel(lib, cuda_dev, wtype, rows, k, n):
+    gen = torch.Generator(device=cuda_dev).manual_seed(k)
+    mm = QMatMul.from_qtensor(QTensor.from_device_blocks(_weights32(wtype, n, k, 1.0, gen, cuda_dev)[0].reshape(-1), GgmlDType(wtype), (n, k)))
+    x = torch.randn(rows, k, device=cuda_dev, generator=gen).to(torch.bfloat16)
+    assert lib.cq_prompt32_bf16_pays(wtype, rows, k, n) == 0
+    assert torch.equal(mm.forward(x), torch.cat([mm.forward(x[r:r + 8]) for r in range(0, rows, 8)]))
