@@ -957,8 +957,8 @@ static double slice_us(bool super, int rows, int k, double weights) {
 
 // The six Q8_1 formats against slices of eight rows on the decode kernel, which stream the matrix once each.  Models of both sides (9 - 220 tokens,
 // 32 - 20000 rows, K to 14336; f32, cold weights): a round of tiles takes a fixed part and one per token and 256 elements of K, measured at 148
-// tiles; a slice its two launches, and time per weight that grows with its rows (a fit to 1500 shapes).  Of 245 sampled shapes 11 go to the slower side by
-// more than 5 %, most of them to the slices, for a matrix of few rows and long K (145 rows of K = 8448, 93 tokens: 77 us here, 107 in slices).
+// tiles; a slice its two launches, and time per weight that grows with its rows (a fit to 1500 shapes).  Of 240 sampled shapes 10 go to the slower side by
+// more than 5 %, all of them to the slices, mostly a matrix of few rows and long K (192 rows of K = 9216, 123 tokens: 77 us here, 113 in slices).
 extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     const double sms = cq_sm_count(), weights = 1e-6 * n * (double)k;
     const Tiling tl = plan_tiling(tokens, (n + kRows - 1) / kRows, (int)sms, kFixedTokens, 64);
@@ -978,8 +978,9 @@ extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     return here < (super ? 1.8 : 2.5) + whole * slice_us(super, 8, k, weights) + (left ? slice_us(super, left, k, weights) : 0.0);
 }
 
-// The same with bf16, whose line has not followed the kernel (its constants are those of a kernel that took 467 us where this one takes 320, Q5_K 4096 ->
+// The same with bf16, whose line has not followed the kernel (its constants are those of a kernel that took 468 us where this one takes 326, Q5_K 4096 ->
 // 14336, 512 tokens): the two sides add in different orders, so a call that changes sides gets a few in 100 000 of its bf16 results as the neighbouring value.
+// Of the same shapes 19 go to the slower side by more than 5 %, all of them to the slices (36 rows of K = 11520, 205 tokens: 95 us here, 197 in slices).
 extern "C" int cq_prompt32_bf16_pays(int wtype, int tokens, int k, int n) {
     const double sms = cq_sm_count(), weights = 1e-6 * n * (double)k;
     const Tiling tl = plan_tiling(tokens, (n + kRows - 1) / kRows, (int)sms, 40, 64);
@@ -989,6 +990,10 @@ extern "C" int cq_prompt32_bf16_pays(int wtype, int tokens, int k, int n) {
     const double here = 6.7 + rounds * (k / 256) * (fixed + per_token * tl.tt);
     const int whole = tokens / 8, left = tokens % 8;
     return here < (super ? 1.8 : 2.5) + whole * slice_us(super, 8, k, weights) + (left ? slice_us(super, left, k, weights) : 0.0);
+}
+
+extern "C" int cq_prompt32_tile_tokens(int tokens, int n) {
+    return tokens <= 0 || n <= 0 ? 0 : plan_tiling(tokens, (n + kRows - 1) / kRows, sm_count(), kFixedTokens, kTok).tt;
 }
 
 extern "C" void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,

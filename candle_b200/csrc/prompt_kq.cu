@@ -874,6 +874,8 @@ extern "C" int cq_prompt_pays(int wtype, int tokens, int k, int n) {
     return rounds64 * 1.6 >= rounds128 * (k % 2048 == 0 ? 2.3 : 2.45);
 }
 
+extern "C" int cq_prompt_tile_tokens(int wtype, int tokens, int n) { return tokens <= 0 || n <= 0 ? 0 : dense_tiling(wtype, tokens, n).tt; }
+
 extern "C" void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x,
                                  int tokens, int stride_dst, void *stream) {
     if (!vx || !x || !scratch || !dst || ncols_x <= 0 || nrows_x <= 0 || tokens <= 0 || ncols_x % 256 != 0) {

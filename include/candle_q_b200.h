@@ -262,6 +262,7 @@ size_t cq_prompt_scratch_bytes(int tokens, int k);
 void cq_prompt_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
                       int stride_dst, void *stream);
 int cq_prompt_timeout_flag(void);
+int cq_prompt_tile_tokens(int wtype, int tokens, int n);       /* tokens of a tile, a multiple of 16 up to 128; results do not depend on it */
 int cq_prompt_pays(int wtype, int tokens, int k, int n);       /* 0: the pair above is the faster (some Q6_K shapes); the same bits */
 /* The same for the 32-element block formats Q4_0 (wtype 2) and Q8_0 (8): candle-kernels/src/mmq_gguf/mmq_gguf.cuh:305-364,
  * 927-1062, 1169-1296 behind ffi.rs:471-630.  Activations are quantized like candle's CPU path (BlockQ8_0, k_quants.rs:
@@ -280,6 +281,7 @@ size_t cq_prompt32_scratch_bytes(int wtype, int tokens, int k);
 void cq_prompt32_matmul(int wtype, const void *vx, const void *x, int elem, void *dst, void *scratch, int ncols_x, int nrows_x, int tokens,
                         int stride_dst, void *stream);
 int cq_prompt32_timeout_flag(void);
+int cq_prompt32_tile_tokens(int tokens, int n);                /* tokens of a tile, a multiple of 16 up to 64; results do not depend on it */
 int cq_prompt32_pays(int wtype, int tokens, int k, int n);     /* Q8_1 formats: 0 where slices of eight tokens on the decode kernel are the faster */
 /* The same for Q4_1, Q5_0, Q5_1, Q2_K, Q3_K and Q5_K with bf16 inputs and outputs, with the minimum added per block in f32: the bf16 results that
  * QMatMul.forward gives (Q4_1, Q5_1: also those of cq_prompt32_matmul).  Its _pays is the rule of bf16 calls; its timeout flag is the one above. */

@@ -154,16 +154,6 @@ def test_prompt32_matmul(lib, oracle, cuda_dev, tokens, k, n, wtype):
         assert rel_err(out.cpu().numpy()[pick], ref) <= 2e-6
 
 
-# tokens per tile at the border of the two sizes of the epilogue (32 | 33), and the multiples of 16 around it
-@pytest.mark.parametrize("tokens", [16, 31, 33, 48])
-@pytest.mark.parametrize("wtype", sorted(NAMES))
-def test_prompt32_tile_sizes_give_the_same_bits(lib, oracle, cuda_dev, tokens, wtype):
-    """A token's result does not depend on the size of the tile it is in."""
-    _, x, wq = make_case(oracle, wtype, 1280, 200, 64, seed=wtype)
-    x_dev, w_dev = torch.from_numpy(x).to(cuda_dev), torch.from_numpy(wq).to(cuda_dev)
-    assert torch.equal(_prompt32(lib, wtype, w_dev, x_dev[:tokens].contiguous(), 1280, 200), _prompt32(lib, wtype, w_dev, x_dev, 1280, 200)[:tokens])
-
-
 @pytest.mark.parametrize("wtype", [3, 6, 7])
 def test_prompt32_of_block_sums_past_f16(lib, oracle, cuda_dev, wtype):
     """Q8_1's stored sum is infinite where 32 inputs add up to more than 65504: infinities and NaNs where the decode kernel has them."""
@@ -261,7 +251,7 @@ def test_prompt32_is_no_further_from_64_bits_than_the_decode_kernel(lib, cuda_de
     assert err(_prompt32(lib, wtype, wq, x, k, n)) <= 1.1 * err(decode)
 
 
-MINIMUM = {3: (0, 2, -7.5), 6: (0, None, 0.0), 7: (0, 2, -15.5), 10: (80, 82, 1.5), 11: (108, None, 0.0), 13: (0, 2, 15.5)}     # where d and the minimum are; the middle of the codes
+MINIMUM = {2: (0, None, 0.0), 8: (0, None, 0.0), 3: (0, 2, -7.5), 6: (0, None, 0.0), 7: (0, 2, -15.5), 10: (80, 82, 1.5), 11: (108, None, 0.0), 13: (0, 2, 15.5)}     # where d and the minimum are; the middle of the codes
 
 
 def _weights32(wtype, n, k, minimum, gen, dev):
@@ -289,7 +279,7 @@ def _weights32(wtype, n, k, minimum, gen, dev):
     codes, scales = values(1.0, 0.0), spread(at_d)
     if wtype == 6:          # the codes are unsigned, -16 d is the minimum
         return b.reshape(n, -1), codes + 16, scales, -16 * scales.unsqueeze(-1)
-    if wtype == 11:
+    if at_m is None:
         return b.reshape(n, -1), codes, scales, torch.zeros((n, k // 32, 1), dtype=torch.float64, device=dev)
     mins = values(0.0, 1.0)[:, ::16 if wtype == 10 else 32].reshape(n, k // 32, -1)
     return b.reshape(n, -1), codes, scales, mins * spread(at_m).unsqueeze(-1)
@@ -341,6 +331,22 @@ def _inputs32(kind, m, k, gen, dev):
     if kind == "one sign, a few large":
         x.view(m, -1, 32)[:, torch.randperm(k // 32, device=dev, generator=gen)[:k // 1024]] *= 50
     return x
+
+
+# tiles on both sides of the border of the two sizes of the epilogue (32 | 48), ragged ones, a tile and a part of one, several per CTA; rows of outputs a multiple of
+# 16 bytes apart (19000), of 8 (14340) and of 2 (19001)
+@pytest.mark.parametrize("tokens,n,tile", [(16, 14340, 16), (31, 19000, 32), (33, 19001, 48), (50, 19000, 64), (61, 19001, 64), (100, 14340, 64), (130, 19001, 48)])
+@pytest.mark.parametrize("wtype", sorted(NAMES))
+def test_prompt32_tile_sizes_give_the_same_bits(lib, cuda_dev, tokens, n, tile, wtype):
+    """A token's result does not depend on the size of the tile it is in: against few weight rows, for which tiles of 16 tokens are planned."""
+    k = 512
+    assert lib.cq_prompt32_tile_tokens(tokens, n) == tile and lib.cq_prompt32_tile_tokens(tokens, 200) == 16
+    gen = torch.Generator(device=cuda_dev).manual_seed(n)
+    wq, x = _weights32(wtype, n, k, 1.0, gen, cuda_dev)[0], torch.randn(tokens, k, device=cuda_dev, generator=gen)
+    for dtype in (torch.float32, torch.float16, torch.bfloat16):
+        out = _prompt32(lib, wtype, wq, x.to(dtype), k, n)
+        for rows in (slice(0, 200), slice(n - 200, n)):
+            assert torch.equal(out[:, rows], _prompt32(lib, wtype, wq[rows].contiguous(), x.to(dtype), k, 200))
 
 
 @pytest.mark.parametrize("kind", ["normal", "one sign", "one sign, a few large"])
@@ -454,6 +460,20 @@ def test_addresses_the_prompt_kernels_do_not_take_are_refused(lib, oracle, cuda_
 def test_16_bit_rows_at_any_distance(cuda_dev, wtype, n, pad, offset, tokens):
     """Rows of 16-bit outputs a multiple of 16 bytes apart (stored by eight) or not (a lane per row), ragged in rows and tokens: the f32 outputs
     rounded, and nothing between the rows."""
+    _check_16_bit_rows(cuda_dev, wtype, n, pad, offset, tokens)
+
+
+# tiles of several sizes (Q4_K and Q6_K | Q8_0), past the tile's first 64 (32) tokens and with an epilogue of either size
+@pytest.mark.parametrize("wtype", [GgmlDType.Q4K, GgmlDType.Q6K, GgmlDType.Q8_0])
+@pytest.mark.parametrize("n,pad,offset,tokens,tile,tile32", [(19000, 0, 0, 75, 80, 48), (19001, 0, 0, 75, 80, 48), (14340, 4, 0, 130, 80, 48), (19001, 2, 0, 61, 64, 64), (14340, 0, 0, 100, 112, 64),
+                                                             (19000, 8, 0, 50, 64, 64), (14336, 0, 1, 100, 112, 64)])
+def test_16_bit_rows_of_large_tiles(cuda_dev, wtype, n, pad, offset, tokens, tile, tile32):
+    assert (capi.lib().cq_prompt32_tile_tokens(tokens, n) if wtype == GgmlDType.Q8_0 else capi.lib().cq_prompt_tile_tokens(int(wtype), tokens, n)) == \
+        (tile32 if wtype == GgmlDType.Q8_0 else tile)
+    _check_16_bit_rows(cuda_dev, wtype, n, pad, offset, tokens)
+
+
+def _check_16_bit_rows(cuda_dev, wtype, n, pad, offset, tokens):
     from candle_b200.synth import random_blocks
     L, st, k, big = capi.lib(), torch.cuda.current_stream().cuda_stream, 512, wtype in (GgmlDType.Q4K, GgmlDType.Q6K)
     w = random_blocks(wtype, n, k, seed=n, device=cuda_dev)

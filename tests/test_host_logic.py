@@ -119,18 +119,26 @@ def test_operands_of_the_super_block_prompt_kernel_are_exact():
     assert 128 * 128 * 63 * 15 <= 2 ** 24 < 256 * 127 * 63 * 15 and (2 ** 24 // 945) * 945 <= 2 ** 24 and 16 * 63 * 2048 <= 2 ** 24
 
 
-def test_prompt_route_of_the_q8_1_formats_takes_the_faster_side(lib):
-    """(type, tokens, K, rows) with the measured times of slices on the decode kernel and of the prompt kernel (us).  Without a device the
+@pytest.mark.parametrize("rule,slices,prompt", [
+    ("cq_prompt32_pays",
+     [((7, 71, 10240, 53), 57.1, 83.9), ((3, 15, 8192, 7620), 41.8, 66.9), ((7, 34, 5120, 100), 25.9, 44.2), ((7, 11, 10240, 5467), 53.2, 86.1),
+      ((7, 12, 14336, 6442), 77.0, 119.1), ((3, 10, 5120, 7202), 27.8, 44.0), ((10, 41, 5120, 34), 33.2, 43.6), ((6, 9, 768, 360), 7.6, 11.5),
+      ((13, 18, 14336, 3248), 80.1, 101.7), ((13, 11, 8192, 7677), 55.9, 61.4), ((6, 11, 8192, 10496), 48.9, 71.8), ((11, 36, 5120, 128), 34.9, 48.2)],
+     [((13, 512, 4096, 14336), 2235.0, 261.8), ((6, 91, 10240, 1629), 162.0, 87.3), ((3, 16, 768, 8303), 18.5, 11.8),
+      ((10, 154, 10240, 171), 193.9, 83.4), ((3, 183, 14336, 496), 217.9, 114.2), ((6, 9, 512, 5178), 14.7, 9.8)]),
+    ("cq_prompt32_bf16_pays",
+     [((7, 71, 10240, 53), 56.9, 83.1), ((3, 15, 8192, 7620), 42.5, 67.3), ((7, 34, 5120, 100), 26.9, 44.1), ((7, 11, 10240, 5467), 54.2, 85.5),
+      ((7, 12, 14336, 6442), 78.2, 118.0), ((3, 10, 5120, 7202), 28.6, 44.4), ((10, 41, 5120, 34), 34.6, 47.6), ((6, 9, 768, 360), 8.2, 11.3),
+      ((13, 18, 14336, 3248), 80.9, 110.7), ((13, 11, 8192, 7677), 56.3, 66.6), ((6, 11, 8192, 10496), 49.5, 70.8), ((11, 36, 5120, 128), 37.4, 50.1)],
+     [((13, 512, 4096, 14336), 2255.2, 330.1), ((6, 91, 10240, 1629), 169.7, 86.1), ((3, 16, 768, 8303), 19.2, 12.2),
+      ((10, 154, 10240, 171), 198.2, 92.0), ((3, 183, 14336, 496), 226.9, 114.7), ((6, 9, 512, 5178), 15.0, 9.9)])])
+def test_prompt_route_of_the_q8_1_formats_takes_the_faster_side(lib, rule, slices, prompt):
+    """(type, tokens, K, rows) with the measured times of slices on the decode kernel and of the prompt kernel (us), f32 and bf16.  Without a device the
     rule counts 148 SMs."""
-    slices = [((7, 71, 10240, 53), 47.6, 122.0), ((3, 15, 8192, 7620), 42.1, 97.5), ((7, 34, 5120, 100), 27.7, 63.8), ((7, 11, 10240, 5467), 54.1, 123.7),
-              ((7, 12, 14336, 6442), 76.4, 170.7), ((3, 10, 5120, 7202), 28.7, 63.5), ((10, 41, 5120, 34), 33.0, 71.6), ((6, 9, 768, 360), 13.2, 19.5),
-              ((13, 18, 14336, 3248), 83.2, 166.0), ((13, 11, 8192, 7677), 60.4, 101.4), ((6, 11, 8192, 10496), 55.0, 105.5), ((11, 36, 5120, 128), 39.9, 66.6)]
-    prompt = [((13, 512, 4096, 14336), 2233.0, 490.0), ((6, 91, 10240, 1629), 165.6, 124.9), ((3, 16, 768, 8303), 19.7, 15.0), ((10, 154, 10240, 171), 194.7, 139.3),
-              ((3, 183, 14336, 496), 220.3, 168.6), ((6, 9, 512, 5178), 15.5, 12.4)]
     for shape, fast, slow in slices:
-        assert fast < slow and lib.cq_prompt32_pays(*shape) == 0, shape
+        assert fast < slow and getattr(lib, rule)(*shape) == 0, shape
     for shape, slow, fast in prompt:
-        assert fast < slow and lib.cq_prompt32_pays(*shape) == 1, shape
+        assert fast < slow and getattr(lib, rule)(*shape) == 1, shape
 
 
 def test_prompt_route_of_q6_k_takes_the_faster_kernel(lib):
