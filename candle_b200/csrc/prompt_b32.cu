@@ -20,7 +20,7 @@
 //     6.7e-8 / 6.5e-8; no minimum and activations of one sign Q5_K 2.5e-8 / 2.5e-8, Q2_K 3.2e-8 / 3.1e-8 (4.9e-8 and 5.3e-8 with all products in one
 //     accumulator).  Larger only where every code of a block is its lowest and its
 //     scale is not zero, which no quantizer writes (Q5_K 6.0e-8 / 6.7e-8).  It costs 7 % (Q5_K
-//     4096 -> 14336, 512 tokens 237 us -> 255).  Not for Q4_1 and Q5_1, whose stored sum can be most of the result: their codes stay unsigned and a
+//     4096 -> 14336, 512 tokens 237 us -> 253).  Not for Q4_1 and Q5_1, whose stored sum can be most of the result: their codes stay unsigned and a
 //     block's two parts meet in the epilogue.
 //   * A super-block format has one d per 256 elements: a block is then ONE fma per value, sum += d_a I, and d is applied per chunk.
 //   * The accumulators are read with the 16x256b shape of tcgen05.ld: a thread holds four rows x two columns of each eight columns, so one
@@ -39,9 +39,9 @@
 //
 // bf16 results of Q5_0, Q5_K, Q2_K and Q3_K that QMatMul.forward returns come from PLAIN sums: unsigned codes, d and the minimum in the terms of each block, in f32.
 // Sums in the other order differ by 1e-7 of them, and a few in 100 000 bf16 results then round to the neighbouring value, 2^-8 to 2^-7 of it away; bf16
-// results keep their bits instead, for 12 - 50 % more time (512 tokens below: Q5_K 326 us, Q2_K 418, Q5_0 351, Q3_K 296).  Before this mapping: 468, 579, 482, 475.
+// results keep their bits instead, for 14 - 59 % more time (512 tokens below: Q5_K 325 us, Q2_K 418, Q5_0 351, Q3_K 296).  Before this mapping: 468, 579, 482, 475.
 //
-// Measured (B200, quantizer included, f32; before this mapping -> now): 4096 -> 14336, 512 tokens Q5_K 493 us -> 257, Q2_K 282, Q5_0 310, Q3_K 259, Q4_1 339, Q5_1 350,
+// Measured (B200, quantizer included, f32; before this mapping -> now): 4096 -> 14336, 512 tokens Q5_K 493 us -> 253, Q2_K 263, Q5_0 306, Q3_K 259, Q4_1 337, Q5_1 350,
 // Q4_0 226, Q8_0 212; Q8_0 4096 -> 4096, 333 tokens 88 -> 65.  A chunk of 256 elements takes about 2.2 us and 11 ns per token, 11 - 13 thousand warp
 // instructions at 2.3 a clock; two tensor-core steps of a block are 64 clocks.
 // Tried: tiles of 128 tokens with one producer set (Q5_K 327), the group's first warp polling for the others (534: branches and barrier reads outweigh
@@ -108,16 +108,16 @@ template <int WTYPE, bool PLAIN> struct Smem {
     static constexpr int kBytes = 1024 + kStagesT * kStageT + 4 * kAux + 4 * kRingW + 2 * kCoef + kRawStages * Raw<chunk_bytes<WTYPE>()>::kBytes + 16;
 };
 
-// v = hi + mid + lo, exactly (7, 8 and 8 bits, and the signs of the rests); a value that is not finite has only its first part
-__device__ __forceinline__ void split3(float v, uint16_t &hi, uint16_t &mid, uint16_t &lo) {
-    auto bits = [](__nv_bfloat16 b) { return __bfloat16_as_ushort(b); };
-    const bool finite = fabsf(v) <= 3.3e38f;
-    const uint32_t h = (__float_as_uint(v) + 0x10000u) & 0xFFFE0000u;
-    const float r = finite ? __fsub_rn(v, __uint_as_float(h)) : 0.0f;
-    const __nv_bfloat16 m = __float2bfloat16_rn(r);
-    hi = finite ? (uint16_t)(h >> 16) : bits(__float2bfloat16_rn(v));
-    mid = bits(m);
-    lo = bits(__float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m))));
+// a = hi + mid + lo, exactly (bf16 of 7, 8 and 8 bits, and the signs of the rests), b in the upper halves; a value that is not finite has only its first part.
+// (NaNs are results of f32 operations, with all bits set.)
+__device__ __forceinline__ void split3(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+    auto pair = [](float x, float y) { const __nv_bfloat162 v = __floats2bfloat162_rn(x, y); return *reinterpret_cast<const uint32_t *>(&v); };
+    const bool fa = fabsf(a) <= 3.3e38f, fb = fabsf(b) <= 3.3e38f;
+    const uint32_t ha = (__float_as_uint(a) + (fa ? 0x10000u : 0u)) & 0xFFFE0000u, hb = (__float_as_uint(b) + (fb ? 0x10000u : 0u)) & 0xFFFE0000u;
+    const float ra = fa ? __fsub_rn(a, __uint_as_float(ha)) : 0.0f, rb = fb ? __fsub_rn(b, __uint_as_float(hb)) : 0.0f;
+    hi = __byte_perm(ha, hb, 0x7632);
+    mid = pair(ra, rb);
+    lo = pair(__fsub_rn(ra, __uint_as_float(mid << 16)), __fsub_rn(rb, __uint_as_float(mid & 0xFFFF0000u)));
 }
 
 // ---- activations ---------------------------------------------------------------------------------------------------
@@ -168,10 +168,10 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T *__restrict__ x, 
         if constexpr (SUM != kSum16 && SUM != kPlain16) si += __shfl_xor_sync(0xffffffffu, si, 2);
         const float s = __fmul_rn(dh, (float)si);
         [[maybe_unused]] auto put = [&](int j, float v) {        // sum j of the chunk: element j % 8 of slab j / 8 of each plane
-            uint16_t hi, mid, lo;
-            split3(v, hi, mid, lo);
+            uint32_t hi, mid, lo;
+            split3(v, 0.0f, hi, mid, lo);
             uint8_t *p = sm + (32 + (j >> 3)) * kPitch + warp * 16 + 2 * (j & 7);
-            const uint16_t plane[5] = {lo, mid, (uint16_t)((hi & 0x7F80u) == 0x7F80u ? 0 : hi), kPlanes == 5 ? (uint16_t)0 : hi, hi};
+            const uint16_t plane[5] = {(uint16_t)lo, (uint16_t)mid, (uint16_t)((hi & 0x7F80u) == 0x7F80u ? 0 : hi), (uint16_t)(kPlanes == 5 ? 0 : hi), (uint16_t)hi};
 #pragma unroll
             for (int i = 0; i < kPlanes; ++i) *reinterpret_cast<uint16_t *>(p + i * kPlane * kPitch) = plane[i];
         };
@@ -222,15 +222,18 @@ __device__ __forceinline__ void codes4(uint32_t w, float off, uint32_t &a, uint3
     b = h2_bits(__hsub2(bits_h2(and_or<0x00FF00FFu, 0x64006400u>(w >> 8)), o));
 }
 __device__ __forceinline__ __half2 twice(uint32_t v) { return __hsub2(bits_h2(v * 0x00010001u | 0x64006400u), bits_h2(0x64006400u)); }   // v < 1024
-// Coefficients j, j + 1 (j even) of a row: planes lo, hi, mid of kSums / 8 slabs of 128 rows x 16 bytes
-template <int SUMS> __device__ __forceinline__ void put_coef(uint8_t *row, int j, float a, float b) {
-    uint16_t h0, m0, l0, h1, m1, l1;
-    split3(a, h0, m0, l0);
-    split3(b, h1, m1, l1);
-    uint8_t *p = row + (j >> 3) * kRows * 16 + 2 * (j & 7);
-    *reinterpret_cast<uint32_t *>(p) = l0 | (uint32_t)l1 << 16;
-    *reinterpret_cast<uint32_t *>(p + SUMS / 8 * kRows * 16) = h0 | (uint32_t)h1 << 16;
-    *reinterpret_cast<uint32_t *>(p + 2 * (SUMS / 8) * kRows * 16) = m0 | (uint32_t)m1 << 16;
+// The SUMS coefficients c(j) of a row: planes lo, hi, mid of SUMS / 8 slabs of 128 rows x 16 bytes
+template <int SUMS, typename C> __device__ __forceinline__ void put_coefs(uint8_t *row, C &&c) {
+#pragma unroll
+    for (int slab = 0; slab < SUMS / 8; ++slab) {
+        uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split3(c(8 * slab + 2 * i), c(8 * slab + 2 * i + 1), hi[i], mid[i], lo[i]);
+        uint4 *p = reinterpret_cast<uint4 *>(row + slab * kRows * 16);
+        p[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        p[SUMS / 8 * kRows] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        p[2 * (SUMS / 8) * kRows] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    }
 }
 
 template <int WTYPE, bool PLAIN> struct Expand;
@@ -251,11 +254,7 @@ template <int WTYPE, bool PLAIN> struct ExpandBlock {
         }
     }
     __device__ __forceinline__ void coef(uint8_t *row) const {
-        if constexpr (WTYPE == CQ_Q5_0) {
-#pragma unroll
-            for (int b = 0; b < 8; b += 2)
-                put_coef<8>(row, b, __fmul_rn(-16.0f, h16(cq_lds_u16(p + b * kBlk))), __fmul_rn(-16.0f, h16(cq_lds_u16(p + (b + 1) * kBlk))));
-        }
+        if constexpr (WTYPE == CQ_Q5_0) put_coefs<8>(row, [&](int b) { return __fmul_rn(-16.0f, h16(cq_lds_u16(p + b * kBlk))); });
     }
     template <int B, int V0, int NV> __device__ __forceinline__ void block(const uint4 (&v)[NV], uint32_t *o) const {
         constexpr int off = B * kBlk, qs = off + 2 + (kHasM ? 2 : 0) + (kFive ? 4 : 0);
@@ -340,8 +339,7 @@ template <bool PLAIN> struct Expand<CQ_Q5_K, PLAIN> {
             const float s = (float)((sc[g >> 2] >> (8 * (g & 3))) & 0xFFu), m = (float)((mn[g >> 2] >> (8 * (g & 3))) & 0xFFu);
             return __fmaf_rn(-dmin, m, __fmul_rn(d16, s));
         };
-#pragma unroll
-        for (int g = 0; g < 8; g += 2) put_coef<8>(row, g, c(g), c(g + 1));
+        put_coefs<8>(row, c);
     }
     __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
         const uint4 a = *reinterpret_cast<const uint4 *>(p + 48 + 32 * ch), b = *reinterpret_cast<const uint4 *>(p + 64 + 32 * ch);
@@ -389,8 +387,7 @@ template <bool PLAIN> struct Expand<CQ_Q2_K, PLAIN> {
             const uint32_t by = (sc[j >> 2] >> (8 * (j & 3))) & 0xFFu;
             return __fmaf_rn(-dmin, (float)(by >> 4), __fmul_rn(d15, (float)(by & 0xFu)));
         };
-#pragma unroll
-        for (int j = 0; j < 16; j += 2) put_coef<16>(row, j, c(j), c(j + 1));
+        put_coefs<16>(row, c);
     }
     __device__ __forceinline__ void chunk(int ch, uint32_t (&o)[32]) const {
         uint32_t q[8], sc[1];
@@ -978,7 +975,7 @@ extern "C" int cq_prompt32_pays(int wtype, int tokens, int k, int n) {
     return here < (super ? 1.8 : 2.5) + whole * slice_us(super, 8, k, weights) + (left ? slice_us(super, left, k, weights) : 0.0);
 }
 
-// The same with bf16, whose line has not followed the kernel (its constants are those of a kernel that took 468 us where this one takes 326, Q5_K 4096 ->
+// The same with bf16, whose line has not followed the kernel (its constants are those of a kernel that took 468 us where this one takes 325, Q5_K 4096 ->
 // 14336, 512 tokens): the two sides add in different orders, so a call that changes sides gets a few in 100 000 of its bf16 results as the neighbouring value.
 // Of the same shapes 19 go to the slower side by more than 5 %, all of them to the slices (36 rows of K = 11520, 205 tokens: 95 us here, 197 in slices).
 extern "C" int cq_prompt32_bf16_pays(int wtype, int tokens, int k, int n) {
