@@ -27,23 +27,21 @@
 // the previous one); operand A in two stages.  Q6_K takes both for every super-block; operand A in four stages, so that the producers go
 // on while the epilogue reads.
 //
-// Measured (B200, quantizer included; int8 kernel -> this one): Q4_K 4096 -> 14336, 2048 tokens bf16 478 us -> 313 (f32 286 back to back; 463
-// when every super-block is split), 128 tokens 28; Q6_K 14336 -> 4096, 512 tokens f32 170 -> 148.  With one accumulator for all of P, which
-// rounds past 2^24, they took 306 and 145.  Reading both halves of all accumulators in two 64-token passes instead costs 342 (Q4_K)
-// and 157 (Q6_K): twice the MMAs to issue.  Bound by the hand-offs between the roles: a super-block of 128 tokens takes 1.4 us (Q4_K) and
-// 2.4 us (Q6_K) where its MMAs take 0.55 and 1.05.
-//
-// The epilogue reads the accumulators in the 16x256b shape (four rows x two columns of each eight per thread), 32 columns at a time: an 8-byte shared load of
-// token scales serves eight values, where a row per thread took a 16-byte load, 4.8 clocks of the SM's shared-memory pipe, for four.  A grouped
-// launch fetches a tile's pair numbers and routing weights, a dependent chain of two L2 round trips, while its super-blocks run.  With one instantiation
-// per kind of output, since the code between the loops costs instruction fetches: expert block of 1024 tokens (below) 457 us -> 340, Q8_0 of prompt_b32.cu
-// 77 -> 69; Q4_K 2048 tokens bf16 313 -> 311 (the clocks fall with the power), 512 tokens f32 99 -> 97.
-//
-// Instructions count wherever a hand-off waits for them: nibbles into mantissas by one LOP3 each (two constants written in C became two), waits without
-// divergence, arrivals by predicate: Q4_K 2048 tokens bf16 281 -> 261, 512 tokens f32 95 -> 89, Q6_K 14336 -> 4096, 512 tokens 151 -> 144.
-// Tried on top: scales and minima written by the idle raw warps (no change, Q6_K 148), half a stage expanded at a time in a loop (Q4_K 273, Q6_K 159),
-// row scales stored in pairs (273: 16-byte broadcast reads).  With all of the expansion left out the 2048 tokens still take 243, without the MMAs 249,
-// without the copies 259: what is left are the chains of barrier round trips, none of which bounds it alone.
+// Measured (B200, quantizer included, passes back to back; GPUs differ by up to 5 %): Q4_K 4096 -> 14336, 2048 tokens bf16 287 - 293 us (int8 kernel 478),
+// Q6_K 14336 -> 4096, 512 tokens f32 139 - 141 (170).  Bound by the hand-offs between the roles: a super-block of 128 tokens takes 1.4 us (Q4_K) and 2.5 us (Q6_K)
+// where its MMAs take 0.55 and 1.05.  What follows are shares of the time at that step, both sides on one GPU:
+//   * One accumulator for all of P, which rounds past 2^24: 2 % less.  Both halves of all accumulators in two 64-token passes: 9 % (Q4_K) and 6 % (Q6_K) more,
+//     twice the MMAs to issue.  Every super-block split: 48 % more (Q4_K).
+//   * The epilogue reads the accumulators in the 16x256b shape (four rows x two columns of each eight per thread), 32 columns at a time: an 8-byte shared load
+//     of token scales serves eight values, where a row per thread took a 16-byte load, 4.8 clocks of the SM's shared-memory pipe, for four.  A grouped launch
+//     fetches a tile's pair numbers and routing weights, a dependent chain of two L2 round trips, while its super-blocks run.  One instantiation per kind of
+//     output, since the code between the loops costs instruction fetches.  Expert block of 1024 tokens (below) 26 % less, dense Q4_K 1 - 2 %.
+//   * Instructions count wherever a hand-off waits for them: nibbles into mantissas by one LOP3 each (two constants written in C became two), waits without
+//     divergence, arrivals by predicate: Q4_K 6 - 7 % less, Q6_K 5 %.
+//   * Tried on top: scales and minima written by the idle raw warps (Q4_K the same, Q6_K 3 % more), half a stage expanded at a time in a loop (5 % and 10 %
+//     more), row scales stored in pairs (5 % more: 16-byte broadcast reads).
+//   * Left out to see its share (Q4_K, 2048 tokens): all of the expansion 7 %, the MMAs 5 %, the copies 1 %.  What is left are the chains of barrier round trips,
+//     none of which bounds it alone.
 //
 // Every wait is bounded (about a second); a give-up raises a CTA-wide abort flag, all roles leave, copies in flight are waited
 // for, TMEM is released and a device flag is set for the host.
